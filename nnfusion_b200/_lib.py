@@ -61,6 +61,20 @@ class QWeight(ctypes.Structure):
 
 
 _lib = None
+_host_calls = None
+
+
+def host_calls():
+    """The extension module behind repeated calls of a node (``csrc/host_calls.cpp``); raises if it has not been built."""
+    global _host_calls
+    if _host_calls is None:
+        try:
+            from . import _host_calls as module
+        except ImportError as e:
+            raise RuntimeError("nnfusion_b200/_host_calls.so cannot be loaded: build it with "
+                               f"`python -m nnfusion_b200.build` ({e})") from e
+        _host_calls = module
+    return _host_calls
 
 
 def load() -> ctypes.CDLL:

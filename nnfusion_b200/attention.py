@@ -30,6 +30,23 @@ class DecodeAttention:
         self.k_cache = torch.zeros((kv_heads, capacity, head_dim), dtype=torch.float16, device=dev)
         self.v_cache = torch.zeros((kv_heads, capacity, head_dim), dtype=torch.float16, device=dev)
         self._ws: dict = {}
+        self._native = None
+
+    def __setattr__(self, name, value):
+        """The prepared call (``_native``) holds what the attributes said: a change makes it stale."""
+        object.__setattr__(self, name, value)
+        if name != "_native":
+            object.__setattr__(self, "_native", None)
+
+    def _prepared(self, d: L.AttnDesc) -> None:
+        """Later calls skip ``__call__``'s Python path (``csrc/host_calls.cpp``)."""
+        lib = self.ctx.lib
+        fn, ws_fn = (ctypes.cast(f, ctypes.c_void_p).value
+                     for f in (lib.nnf_b200_decode_attention, lib.nnf_b200_decode_attention_workspace_bytes))
+        ws = self._ws.get("ws")
+        self._native = L.host_calls().AttnCall(fn, ws_fn, self.ctx.handle.value, bytes(d),
+                                               ws.data_ptr() if ws is not None else 0,
+                                               ws.numel() if ws is not None else 0, self.ctx.check)
 
     def desc(self, position: int) -> L.AttnDesc:
         d = L.AttnDesc()
@@ -61,6 +78,10 @@ class DecodeAttention:
 
     def __call__(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, position: int,
                  out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        if self._native is not None:
+            y = self._native.call(q, k_new, v_new, self.k_cache, self.v_cache, position, out)
+            if y is not None:
+                return y
         hd, kd = self.heads * self.head_dim, self.kv_heads * self.head_dim
         for t, n in ((q, hd), (k_new, kd), (v_new, kd)):
             if t.dtype != torch.float16 or t.numel() != n or not t.is_contiguous():
@@ -75,4 +96,5 @@ class DecodeAttention:
             self.k_cache.data_ptr(), self.v_cache.data_ptr(), out.data_ptr(),
             ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0)
         self.ctx.check(rc)
+        self._prepared(d)
         return out

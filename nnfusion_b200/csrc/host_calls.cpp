@@ -1,0 +1,397 @@
+// The host side of a node's repeated call, as a CPython extension: what DequantDot / DecodeAttention do between "the
+// user has a tensor" and "the C ABI is called" once a call of the same shape has been seen.
+//
+// A decode step is a chain of launches of a few microseconds each, so the time the host spends per launch is part of
+// the step: through ctypes and torch's Python wrappers (descriptor fields, workspace lookup, current stream, nine
+// converted arguments) a call took 13 to 19 us of host time for 4 to 8 us of GPU time.  Here a call is: look at the
+// tensor, find the entry for its row count and type, allocate the output, take the current stream, call the C ABI.
+//
+// The objects here never decide anything on their own.  Whatever is not the plain, already prepared case (a new row
+// count, a tensor that is not a contiguous CUDA tensor of the right shape, an addend that is missing) makes the call
+// return None, and the Python method runs its full path, which checks, raises and prepares as it always did.
+//
+// Entries are registered and looked up under the interpreter lock.
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <cstring>
+#include <vector>
+
+#include "nnf_b200.h"
+
+namespace
+{
+using LinearFn = int (*)(nnf_b200_ctx*, void*, const nnf_b200_linear_desc*, const void*, const nnf_b200_qweight*,
+                         const nnf_b200_qweight*, const void*, const void*, void*, void*, size_t);
+using AttnFn = int (*)(nnf_b200_ctx*, void*, const nnf_b200_attn_desc*, const void*, const void*, const void*, void*,
+                       void*, void*, void*, size_t);
+using AttnWsFn = size_t (*)(const nnf_b200_ctx*, const nnf_b200_attn_desc*);
+
+// A tensor the C ABI can take as it is, or null.
+const at::Tensor* plain_cuda(PyObject* o)
+{
+    if (!THPVariable_Check(o))
+        return nullptr;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (!t.defined() || !t.is_cuda() || !t.is_contiguous())
+        return nullptr;
+    return &t;
+}
+
+int dtype_code(c10::ScalarType s)
+{
+    return s == at::kHalf ? NNF_B200_F16 : s == at::kFloat ? NNF_B200_F32 : -1;
+}
+
+PyObject* wrapped_empty(at::IntArrayRef sizes, c10::ScalarType dtype, c10::Device device)
+{
+    return THPVariable_Wrap(at::Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt)));
+}
+
+// ---------------------------------------------------------------------------------------------------- linear
+
+struct LinearEntry
+{
+    nnf_b200_linear_desc desc;
+    void* ws;
+    size_t ws_bytes;
+};
+
+struct LinearCall
+{
+    PyObject_HEAD
+    LinearFn fn;
+    nnf_b200_ctx* ctx;
+    nnf_b200_qweight w, w2;
+    int has_w2, add;
+    PyObject* gain;  // tensors or None: their addresses are read at every call
+    PyObject* bias;
+    PyObject* check; // Context.check: raises for a status that is not OK
+    std::vector<LinearEntry>* entries;
+};
+
+const void* address_of(PyObject* o)
+{
+    return o == Py_None ? nullptr : THPVariable_Unpack(o).const_data_ptr();
+}
+
+// y = node(x) with x [..., K]; lead: the output takes x's leading dimensions instead of [M, N].
+PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* paddend, bool lead)
+{
+    const at::Tensor* x = plain_cuda(px);
+    if (!x)
+        Py_RETURN_NONE;
+    const int xd = dtype_code(x->scalar_type());
+    const int64_t dims = x->dim();
+    if (xd < 0 || (lead ? dims < 1 : dims != 2) || self->entries->empty())
+        Py_RETURN_NONE;
+    const int64_t K = self->entries->front().desc.K, N = self->entries->front().desc.N;
+    if (x->size(dims - 1) != K)
+        Py_RETURN_NONE;
+    const int64_t M = x->numel() / K;
+    LinearEntry e; // a copy: the call below runs without the interpreter lock
+    bool found = false;
+    for (const LinearEntry& c : *self->entries)
+        if (c.desc.M == M && c.desc.x_dtype == xd)
+        {
+            e = c, found = true;
+            break;
+        }
+    if (!found || (self->add != 0) != (paddend != Py_None))
+        Py_RETURN_NONE;
+    const c10::ScalarType yt = e.desc.y_dtype == NNF_B200_F16 ? at::kHalf : at::kFloat;
+    const void* bias = nullptr;
+    if (paddend != Py_None)
+    {
+        const at::Tensor* a = plain_cuda(paddend);
+        if (!a || a->dim() != 2 || a->size(0) != M || a->size(1) != N || a->scalar_type() != yt)
+            Py_RETURN_NONE;
+        bias = a->const_data_ptr();
+    }
+    else
+        bias = address_of(self->bias);
+    PyObject* out;
+    if (pout == Py_None)
+    {
+        if (lead)
+        {
+            c10::SmallVector<int64_t, 6> sizes(x->sizes().begin(), x->sizes().end());
+            sizes.back() = N;
+            out = wrapped_empty(sizes, yt, x->device());
+        }
+        else
+            out = wrapped_empty({M, N}, yt, x->device());
+        if (!out)
+            return nullptr;
+    }
+    else
+    {
+        const at::Tensor* o = plain_cuda(pout);
+        if (!o || o->dim() != 2 || o->size(0) != M || o->size(1) != N || o->scalar_type() != yt)
+            Py_RETURN_NONE;
+        out = pout;
+        Py_INCREF(out);
+    }
+    void* y = THPVariable_Unpack(out).mutable_data_ptr();
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    const void *px_data = x->const_data_ptr(), *gain = address_of(self->gain);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = self->fn(self->ctx, stream, &e.desc, px_data, &self->w, self->has_w2 ? &self->w2 : nullptr, gain, bias, y, e.ws,
+                  e.ws_bytes);
+    Py_END_ALLOW_THREADS
+    if (rc != NNF_B200_OK)
+    {
+        Py_DECREF(out);
+        return PyObject_CallFunction(self->check, "i", rc);
+    }
+    return out;
+}
+
+PyObject* guarded(PyObject* (*body)(PyObject*, PyObject* const*), PyObject* self, PyObject* const* args)
+{
+    try
+    {
+        return body(self, args);
+    }
+    catch (const std::exception& e) // an allocation that failed, a CUDA error
+    {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+// call(x, out, addend) -> tensor or None
+PyObject* linear_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
+{
+    if (n != 3)
+        return PyErr_Format(PyExc_TypeError, "call(x, out, addend)");
+    return guarded([](PyObject* s, PyObject* const* a) {
+        return linear_run(reinterpret_cast<LinearCall*>(s), a[0], a[1], a[2], false);
+    }, self, args);
+}
+
+// call_lead(x, wq) -> tensor or None: any leading dimensions; None too when wq is no longer the tensor the node was
+// built for.
+PyObject* linear_call_lead(PyObject* self, PyObject* const* args, Py_ssize_t n)
+{
+    if (n != 2)
+        return PyErr_Format(PyExc_TypeError, "call_lead(x, wq)");
+    return guarded([](PyObject* s, PyObject* const* a) -> PyObject* {
+        LinearCall* self = reinterpret_cast<LinearCall*>(s);
+        if (!THPVariable_Check(a[1]) || THPVariable_Unpack(a[1]).const_data_ptr() != self->w.wq)
+            Py_RETURN_NONE;
+        return linear_run(self, a[0], Py_None, Py_None, true);
+    }, self, args);
+}
+
+// register(desc bytes, workspace address, workspace bytes)
+PyObject* linear_register(PyObject* self, PyObject* args)
+{
+    Py_buffer desc;
+    unsigned long long ws, bytes;
+    if (!PyArg_ParseTuple(args, "y*KK", &desc, &ws, &bytes))
+        return nullptr;
+    LinearCall* c = reinterpret_cast<LinearCall*>(self);
+    const bool ok = desc.len == (Py_ssize_t)sizeof(nnf_b200_linear_desc);
+    if (ok)
+    {
+        LinearEntry e;
+        memcpy(&e.desc, desc.buf, sizeof e.desc);
+        e.ws = reinterpret_cast<void*>(ws);
+        e.ws_bytes = bytes;
+        bool known = false;
+        for (LinearEntry& q : *c->entries)
+            if (q.desc.M == e.desc.M && q.desc.x_dtype == e.desc.x_dtype)
+                q = e, known = true;
+        if (!known)
+            c->entries->push_back(e);
+    }
+    PyBuffer_Release(&desc);
+    if (!ok)
+        return PyErr_Format(PyExc_ValueError, "descriptor size");
+    Py_RETURN_NONE;
+}
+
+PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
+{
+    unsigned long long fn, ctx;
+    Py_buffer w, w2;
+    int add;
+    PyObject *gain, *bias, *check;
+    w2.buf = nullptr;
+    if (!PyArg_ParseTuple(args, "KKy*z*iOOO", &fn, &ctx, &w, &w2, &add, &gain, &bias, &check))
+        return nullptr;
+    LinearCall* c = reinterpret_cast<LinearCall*>(type->tp_alloc(type, 0));
+    if (c)
+    {
+        c->fn = reinterpret_cast<LinearFn>(fn);
+        c->ctx = reinterpret_cast<nnf_b200_ctx*>(ctx);
+        memcpy(&c->w, w.buf, sizeof c->w);
+        c->has_w2 = w2.buf != nullptr;
+        if (c->has_w2)
+            memcpy(&c->w2, w2.buf, sizeof c->w2);
+        c->add = add;
+        c->gain = Py_NewRef(gain), c->bias = Py_NewRef(bias), c->check = Py_NewRef(check);
+        c->entries = new std::vector<LinearEntry>();
+    }
+    PyBuffer_Release(&w);
+    if (w2.buf)
+        PyBuffer_Release(&w2);
+    return reinterpret_cast<PyObject*>(c);
+}
+
+void linear_dealloc(PyObject* self)
+{
+    LinearCall* c = reinterpret_cast<LinearCall*>(self);
+    Py_XDECREF(c->gain);
+    Py_XDECREF(c->bias);
+    Py_XDECREF(c->check);
+    delete c->entries;
+    Py_TYPE(self)->tp_free(self);
+}
+
+PyMethodDef linear_methods[] = {
+    {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(linear_call)), METH_FASTCALL, nullptr},
+    {"call_lead", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(linear_call_lead)), METH_FASTCALL, nullptr},
+    {"register", linear_register, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+// ---------------------------------------------------------------------------------------------------- attention
+
+struct AttnCall
+{
+    PyObject_HEAD
+    AttnFn fn;
+    AttnWsFn ws_fn;
+    nnf_b200_ctx* ctx;
+    nnf_b200_attn_desc desc;
+    void* ws;
+    size_t ws_bytes;
+    PyObject* check;
+};
+
+const at::Tensor* half_of(PyObject* o, int64_t numel)
+{
+    const at::Tensor* t = plain_cuda(o);
+    return t && t->scalar_type() == at::kHalf && t->numel() == numel ? t : nullptr;
+}
+
+// call(q, k_new, v_new, k_cache, v_cache, position, out) -> tensor or None
+PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
+{
+    if (n != 7)
+        return PyErr_Format(PyExc_TypeError, "call(q, k_new, v_new, k_cache, v_cache, position, out)");
+    return guarded([](PyObject* s, PyObject* const* a) -> PyObject* {
+        AttnCall* c = reinterpret_cast<AttnCall*>(s);
+        const int64_t hd = (int64_t)c->desc.heads * c->desc.head_dim, kd = (int64_t)c->desc.kv_heads * c->desc.head_dim;
+        const at::Tensor *q = half_of(a[0], hd), *k = half_of(a[1], kd), *v = half_of(a[2], kd);
+        const at::Tensor *kc = half_of(a[3], kd * c->desc.capacity), *vc = half_of(a[4], kd * c->desc.capacity);
+        if (!q || !k || !v || !kc || !vc || !PyLong_CheckExact(a[5]))
+            Py_RETURN_NONE;
+        const long position = PyLong_AsLong(a[5]);
+        if (position < 0 || position >= c->desc.capacity)
+        {
+            PyErr_Clear();
+            Py_RETURN_NONE;
+        }
+        nnf_b200_attn_desc d = c->desc;
+        d.position = (int32_t)position;
+        const size_t need = c->ws_fn(c->ctx, &d);
+        if (need > c->ws_bytes)
+            Py_RETURN_NONE;
+        PyObject* out;
+        if (a[6] == Py_None)
+        {
+            out = wrapped_empty({1, hd}, at::kHalf, q->device());
+            if (!out)
+                return nullptr;
+        }
+        else
+        {
+            if (!half_of(a[6], hd))
+                Py_RETURN_NONE;
+            out = Py_NewRef(a[6]);
+        }
+        cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+        const void *qp = q->const_data_ptr(), *kp = k->const_data_ptr(), *vp = v->const_data_ptr();
+        void *kcp = kc->mutable_data_ptr(), *vcp = vc->mutable_data_ptr();
+        void* op = THPVariable_Unpack(out).mutable_data_ptr();
+        int rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = c->fn(c->ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? c->ws : nullptr, need ? c->ws_bytes : 0);
+        Py_END_ALLOW_THREADS
+        if (rc != NNF_B200_OK)
+        {
+            Py_DECREF(out);
+            return PyObject_CallFunction(c->check, "i", rc);
+        }
+        return out;
+    }, self, args);
+}
+
+PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
+{
+    unsigned long long fn, ws_fn, ctx, ws, ws_bytes;
+    Py_buffer desc;
+    PyObject* check;
+    if (!PyArg_ParseTuple(args, "KKKy*KKO", &fn, &ws_fn, &ctx, &desc, &ws, &ws_bytes, &check))
+        return nullptr;
+    AttnCall* c = reinterpret_cast<AttnCall*>(type->tp_alloc(type, 0));
+    if (c)
+    {
+        c->fn = reinterpret_cast<AttnFn>(fn), c->ws_fn = reinterpret_cast<AttnWsFn>(ws_fn);
+        c->ctx = reinterpret_cast<nnf_b200_ctx*>(ctx);
+        memcpy(&c->desc, desc.buf, sizeof c->desc);
+        c->ws = reinterpret_cast<void*>(ws), c->ws_bytes = ws_bytes;
+        c->check = Py_NewRef(check);
+    }
+    PyBuffer_Release(&desc);
+    return reinterpret_cast<PyObject*>(c);
+}
+
+void attn_dealloc(PyObject* self)
+{
+    Py_XDECREF(reinterpret_cast<AttnCall*>(self)->check);
+    Py_TYPE(self)->tp_free(self);
+}
+
+PyMethodDef attn_methods[] = {
+    {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(attn_call)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject linear_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+PyTypeObject attn_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host_calls", "Repeated calls of a node, without Python in between.", -1,
+                          nullptr, nullptr, nullptr, nullptr, nullptr};
+} // namespace
+
+PyMODINIT_FUNC PyInit__host_calls(void)
+{
+    linear_type.tp_name = "nnfusion_b200._host_calls.LinearCall";
+    linear_type.tp_basicsize = sizeof(LinearCall);
+    linear_type.tp_flags = Py_TPFLAGS_DEFAULT;
+    linear_type.tp_new = linear_new;
+    linear_type.tp_dealloc = linear_dealloc;
+    linear_type.tp_methods = linear_methods;
+    attn_type.tp_name = "nnfusion_b200._host_calls.AttnCall";
+    attn_type.tp_basicsize = sizeof(AttnCall);
+    attn_type.tp_flags = Py_TPFLAGS_DEFAULT;
+    attn_type.tp_new = attn_new;
+    attn_type.tp_dealloc = attn_dealloc;
+    attn_type.tp_methods = attn_methods;
+    if (PyType_Ready(&linear_type) < 0 || PyType_Ready(&attn_type) < 0)
+        return nullptr;
+    PyObject* m = PyModule_Create(&module_def);
+    if (!m)
+        return nullptr;
+    if (PyModule_AddObjectRef(m, "LinearCall", reinterpret_cast<PyObject*>(&linear_type)) < 0 ||
+        PyModule_AddObjectRef(m, "AttnCall", reinterpret_cast<PyObject*>(&attn_type)) < 0)
+    {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

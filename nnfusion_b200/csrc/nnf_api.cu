@@ -145,6 +145,35 @@ int pick_kernel(const nnf_b200_linear_desc& d)
         return d.kernel;
     return d.M <= 16 ? NNF_B200_KERNEL_GEMV : NNF_B200_KERNEL_GEMM;
 }
+
+// gemv_plan for the calls of a program's loop: rating the launch shapes costs the host about as long as the launch
+// itself, and a program repeats a handful of descriptors.  A direct-mapped table per thread (nothing to lock, a fixed
+// few KB), keyed by everything the plan depends on.
+int cached_gemv_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, nnf::GemvPlan* plan, std::string* why)
+{
+    struct Known
+    {
+        nnf_b200_linear_desc d;
+        int sm_count, smem_optin; // 0 SMs: empty
+        nnf::GemvPlan plan;
+    };
+    constexpr int kSlots = 64;
+    static thread_local Known known[kSlots];
+    uint64_t h = 1469598103934665603ull; // FNV-1a over the descriptor's words
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(&d);
+    for (size_t i = 0; i < sizeof(d) / sizeof(uint32_t); i++)
+        h = (h ^ words[i]) * 1099511628211ull;
+    Known& k = known[(h >> 32) % kSlots];
+    if (k.sm_count == ctx->sm_count && k.smem_optin == ctx->smem_optin && memcmp(&k.d, &d, sizeof(d)) == 0)
+    {
+        *plan = k.plan;
+        return NNF_B200_OK;
+    }
+    const int rc = nnf::gemv_plan(ctx, d, plan, why);
+    if (rc == NNF_B200_OK)
+        k.d = d, k.sm_count = ctx->sm_count, k.smem_optin = ctx->smem_optin, k.plan = *plan;
+    return rc;
+}
 } // namespace
 
 extern "C" {
@@ -415,7 +444,7 @@ static int linear_impl(nnf_b200_ctx* ctx, void* stream, const nnf_b200_linear_de
     {
         nnf::GemvPlan plan;
         std::string why;
-        rc = nnf::gemv_plan(ctx, d, &plan, &why);
+        rc = cached_gemv_plan(ctx, d, &plan, &why);
         if (rc != NNF_B200_OK)
             return nnf::set_error(ctx, rc, why);
         if (plan.workspace_bytes > 0 && (!workspace || workspace_bytes < plan.workspace_bytes))

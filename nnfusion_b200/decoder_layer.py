@@ -36,6 +36,7 @@ class DecoderLayer:
         self.down = DequantDot(down, add=True, ctx=ctx)
         f16 = dict(dtype=torch.float16, device=dev)
         self._qkv = torch.empty((1, q.N + 2 * k.N), **f16)
+        self._q, self._k, self._v = self._qkv.view(-1).split([q.N, k.N, k.N])  # one view each, not one per token
         self._a = torch.empty((1, q.N), **f16)
         self._x1 = torch.empty((1, self.hidden), **f16)
         self._h = torch.empty((1, gate.N), **f16)
@@ -48,12 +49,8 @@ class DecoderLayer:
 
     def __call__(self, x: torch.Tensor, position: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """x: fp16 [1, hidden], the residual stream; returns the layer's output [1, hidden]."""
-        hd, kd = self.heads * self.head_dim, self.kv_heads * self.head_dim
-        qkv = self.qkv(x, out=self._qkv)
-        flat = qkv.view(-1)
-        a = self.attn(flat[:hd], flat[hd:hd + kd], flat[hd + kd:], position, out=self._a)
+        self.qkv(x, out=self._qkv)
+        a = self.attn(self._q, self._k, self._v, position, out=self._a)
         x1 = self.o(a, out=self._x1, addend=x)
         h = self.gate_up(x1, out=self._h)
-        if out is None:
-            out = torch.empty_like(x)
         return self.down(h, out=out, addend=x1)

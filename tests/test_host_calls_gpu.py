@@ -1,0 +1,44 @@
+"""Repeated calls go through ``csrc/host_calls.cpp``: same bits as the first call's Python path, same errors, and no
+stale descriptor after an attribute of the node has changed."""
+import numpy as np
+import pytest
+
+from nnfusion_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,dt,add", [(1, np.float16, False), (3, np.float16, True), (2, np.float32, False),
+                                      (40, np.float16, False)])
+def test_second_call_equals_first(M, dt, add):
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    x, w = synth.u4g128(11, M, 80, 512, x_dtype=dt)
+    op = DequantDot(DeviceWeight.from_host(w), add=add)
+    tx = torch.from_numpy(x).cuda()
+    kw = dict(addend=torch.ones(M, 80, dtype=tx.dtype, device="cuda")) if add else {}
+    first = op(tx, **kw)
+    assert op._native is not None
+    assert torch.equal(op(tx, **kw), first)
+    out = torch.empty_like(first)
+    assert op(tx, out=out, **kw) is out and torch.equal(out, first)
+    with pytest.raises(ValueError):
+        op(tx[:, :256], **kw)
+    with pytest.raises(ValueError):
+        op(tx, **({} if add else dict(addend=first)))
+    op.y_dtype = torch.float32 if dt == np.float16 else torch.float16
+    kw = dict(addend=kw["addend"].to(op.y_dtype)) if add else {}
+    assert op(tx, **kw).dtype == op.y_dtype and op(tx, **kw).dtype == op.y_dtype
+
+
+def test_module_keeps_leading_dimensions_and_follows_its_buffers():
+    import torch
+    from nnfusion_b200.jit import QuantLinear, jit
+    x, w = synth.u4g128(12, 6, 48, 256)
+    m = jit(QuantLinear.from_host(w).cuda())
+    tx = torch.from_numpy(x).cuda().view(2, 3, 256)
+    first = m(tx)
+    assert first.shape == (2, 3, 48) and torch.equal(m(tx), first)
+    assert torch.equal(m(tx.transpose(0, 1)), first.transpose(0, 1))    # not contiguous: the full path
+    m.wq = torch.zeros_like(m.wq)
+    assert not torch.equal(m(tx), first)
