@@ -1,0 +1,25 @@
+"""Decode attention where its launch shape changes: sequences around the lengths at which warps, ranges and clusters of
+ranges start, groups of more query heads than a CTA takes, and enough ranges for the workspace form."""
+import numpy as np
+import pytest
+
+from tests.test_attention_gpu import _check, _run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("pos", [63, 64, 111, 112, 127, 128, 191, 192, 447, 448])
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (9, 1)])
+def test_lengths_around_the_cuts(H, Hkv, pos):
+    outs, ref, caches, caches_ref = _run(H, Hkv, 512, pos, seed=200 + pos, calls=2)
+    _check(outs[0], ref)
+    np.testing.assert_array_equal(outs[0], outs[1])
+    np.testing.assert_array_equal(caches[1], caches_ref[1])
+
+
+@pytest.mark.parametrize("H,Hkv,pos", [(8, 1, 4862), (8, 1, 4864), (24, 1, 8200), (4, 4, 9000), (20, 20, 700)])
+def test_long_sequences_on_few_heads(H, Hkv, pos):
+    """4864 rows: the last length that one cluster of 8 ranges takes; 20 heads: clusters of 5, the most that fit at once."""
+    outs, ref, _, _ = _run(H, Hkv, pos + 1, pos, seed=300 + H, calls=2)
+    _check(outs[0], ref)
+    np.testing.assert_array_equal(outs[0], outs[1])
