@@ -7,29 +7,40 @@
 // elementwise_fused.cpp:42-189) followed by cublasHgemm / cublasSgemm behind cuda::Dot
 // (src/nnfusion/core/kernels/cuda_gpu/kernels/dot.cpp:103-125,264-363).
 //
-// A tile of the output is computed transposed,  D[128 weight rows, 256 batch rows] = Wdq[128, K] . X[256, K]^T,  so
-// that the dequantised weights are the MMA's A operand and can be handed to the tensor core through TENSOR MEMORY
-// instead of shared memory.  One persistent CTA per SM; the launch's work, tiles x raw chunks of K, is cut into equal
-// shares, so that a tile at a seam is computed by two or more CTAs: each writes its fp32 partial sums to a slot of the
-// workspace, and the one that arrives last at the tile adds the slots in the order of their K ranges (bitwise
-// repeatable) and runs the epilogue.  Roles inside a CTA:
-//   * warps "TMA" : one thread streams x tiles (256 rows x 64 fp16, 128-byte swizzle, the MMA's B operand), another
-//                   raw packed-weight chunks (128 rows x 128 bytes, 128-byte swizzle), into shared-memory rings;
-//   * warps "DQ"  : thread r owns weight row r of the tile = TMEM lane r.  Per 64-element k-block it reads its 32
-//                   (uint4) or 64 (uint8) bytes from the raw ring, turns them into fp16 (q - zp) * scale with the
-//                   exponent trick (PRMT + LOP3 + HSUB2 + HMUL2 per pair, exact integer before the scale), and
-//                   writes the 32 packed registers into the A stage in TMEM with tcgen05.st.  Four groups of four
-//                   warps take the k-blocks in turn, so that the conversion keeps ahead of the tensor core;
-//   * warp "MMA"  : one thread issues tcgen05.mma.kind::f16 (A from TMEM, B from the shared-memory descriptor,
-//                   fp32 accumulator D in TMEM, 128 x 256 x 16 per instruction) and releases stages with
-//                   tcgen05.commit;
-//   * epilogue    : the DQ warps read D with tcgen05.ld, apply bias / addend / SiLU(gate) * up, convert and store y.
-// SiLU(x . Wg^T) * (x . Wu^T) runs as two launches: the first leaves the gate products in y, the second multiplies
-// SiLU of what it finds in y into its own products.  Every mbarrier wait is bounded; on a time-out the CTA raises a
-// status flag, skips its remaining work, and still frees its tensor memory.
+// A tile of the output is computed transposed,  D[256 weight rows, BX batch rows] = Wdq[256, K] . X[BX, K]^T,  by a PAIR
+// of CTAs (tcgen05 cta_group::2): each holds 128 of the weight rows and half of the batch rows.  The dequantised weights
+// are the A operand and go to the tensor core through TENSOR MEMORY; x is the B operand in shared memory.  A pair, because
+// with one CTA per tile the operand that both need from shared memory was what bounded the kernel: a 128 x 256 tile reads
+// 64 bytes of x per clock from shared memory while TMA writes another 64, all there is; the pair halves both.
+// BX is any multiple of 16 up to 256, so that a ragged batch is cut into equal tiles (333 rows: two of 176, not 512).
+// Roles inside a CTA:
+//   * warps "W", "X" : one thread each streams raw packed-weight chunks (128 rows x 128 bytes) and this CTA's half of the
+//                   x tiles (BX/2 rows x 64 fp16), both 128-byte swizzled, into shared-memory rings;
+//   * warps "DQ"  : thread r owns weight row r of the CTA's half = TMEM lane r.  Per 64-element k-block it turns its 32
+//                   (uint4) or 64 (uint8) raw bytes into fp16 (q - zp) * scale with the exponent trick (PRMT + LOP3 +
+//                   HSUB2 + HMUL2 per pair, exact integer before the scale) and writes the 32 packed registers into the
+//                   A stage in TMEM with tcgen05.st.  Groups of four warps share the k-blocks;
+//   * warp "MMA"  : one thread of the even CTA issues tcgen05.mma.kind::f16 (256 x BX x 16, fp32 accumulators in both
+//                   CTAs' TMEM) and releases stages in both CTAs with tcgen05.commit;
+//   * warps "EPI" : eight (four) warps read D with tcgen05.ld, apply bias / addend / SiLU(gate) * up, convert and store y while
+//                   the other roles are at the next tile (two accumulators take turns when BX <= 128).
+// How a launch's tiles meet the pairs, chosen by the host from an estimate:
+//   * whole tiles, dealt out to the pairs;
+//   * few tiles: the pairs that share a tile's K are the CTAs of one cluster (2, 3 or 4 pairs) and exchange their partial
+//     sums through distributed shared memory, each finishing its share of the batch rows;
+//   * otherwise tiles x raw chunks of K in equal shares, so that a tile at a seam is computed by two or more pairs: each
+//     writes its fp32 partial sums to a slot of the workspace, and the one that arrives last adds the slots.
+// Partial sums are always added in the order of their K ranges: bitwise repeatable.
+// SiLU(x . Wg^T) * (x . Wu^T): a tile is the gate's chunks followed by the up projection's; the gate products of a tile
+// wait in y (in y's type) for the same threads that wrote them.
+// Every mbarrier wait is bounded; on a time-out the CTA raises a status flag, skips its remaining work, and still frees
+// its tensor memory.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
 
 #include "nnf_internal.h"
 #include "sm100_ptx.cuh"
@@ -38,85 +49,108 @@ namespace
 {
 using namespace nnf::ptx;
 
-// BXV: batch rows per tile, 256, or 64 for launches of up to 64 batch rows (a quarter of the activation bytes, of the
-// tensor time and of the accumulator to read back and, for shared tiles, to pass through the workspace).
-template <int WBITS, int BXV = 256>
+constexpr int kBN = 128;                      // weight rows per CTA (TMEM lanes); a pair's tile has 256
+constexpr int kBK = 64;                       // k-block: one 128-byte swizzle row of fp16
+constexpr int kWStageBytes = kBN * 128;       // one raw chunk
+constexpr int kTmemCols = 512;                // all of it: it starts at column 0
+constexpr int kASlotCols = 32;                // a converted k-block in tensor memory: 64 fp16 per lane
+constexpr int kASlots = 8;
+constexpr int kMaxPairs = 128;                // pairs of a launch, at most
+constexpr int kEpiBarrier = 1;                // named barrier of the epilogue warps
+
+// SMALL: tiles of up to 128 batch rows, whose multiplication takes no longer than the conversion of the weights: four
+// groups of conversion warps instead of two (about 220 clocks per k-block instead of 380; a k-block of 128 batch rows takes
+// the tensor core 256) and a raw ring of 128 KB (HBM's latency at full rate is about 100 KB per SM), paid for with half of
+// the epilogue warps and a smaller x ring.
+template <bool SMALL>
 struct Cfg
 {
-    static_assert(BXV == 256 || BXV == 64, "batch tile of 256 or 64 rows");
-    static constexpr int BN = 128;              // weight rows per tile  (UMMA M, TMEM lanes)
-    static constexpr int BX = BXV;              // batch rows per tile   (UMMA N, accumulator columns)
-    static constexpr int BK = 64;               // k-block: one 128-byte swizzle row of fp16
-    // One ring index for the x tile in shared memory and the converted weights in tensor memory, and one pair of
-    // barriers for every PAIR of k-blocks: the MMA thread, whose own time per k-block is what bounds the kernel,
-    // then waits once and releases once per eight MMAs.
-    static constexpr int PAIRS = 3;             // ring depth in pairs of k-blocks
-    static constexpr int STAGES = 2 * PAIRS;    // k-block stages
-    static constexpr int WSTAGES = 2;
-    static constexpr int KB_PER_CHUNK = (WBITS == 4) ? 4 : 2; // k-blocks per 128-byte raw chunk
-    static constexpr int RAW_BYTES = (WBITS == 4) ? 32 : 64;  // raw bytes per row and k-block
-    static constexpr int DQ_GROUPS = 4;                       // groups of 4 warps that take the k-blocks in turn
-    static constexpr int DQ_WARPS = 4 * DQ_GROUPS;
-    static constexpr int THREADS = (DQ_WARPS + 3) * 32;
-    static constexpr int X_STAGE_BYTES = BX * 128;
-    static constexpr int W_STAGE_BYTES = BN * 128;
-    static constexpr int A_COL0 = BX;            // first TMEM column of the A stages
-    static constexpr int A_STAGE_COLS = BK / 2;  // 64 fp16 per lane = 32 columns
-    static constexpr int TMEM_COLS = BX == 256 ? 512 : 256;
-    // full / empty per ring stage, full / empty per raw-weight stage, then: accumulator full, accumulator drained,
-    // partial sums written, ticket known
-    static constexpr int NUM_BARRIERS = 2 * PAIRS + 2 * WSTAGES + 4;
+    static constexpr int MAX_BX = SMALL ? 128 : 256;
+    static constexpr int DQ_GROUPS = SMALL ? 4 : 2, DQ_WARPS = 4 * DQ_GROUPS;
+    static constexpr int EPI_WARPS = SMALL ? 4 : 8;
+    static constexpr int X_WARP = DQ_WARPS + EPI_WARPS, MMA_WARP = X_WARP + 1, W_WARP = X_WARP + 2;
+    static constexpr int THREADS = (X_WARP + 4) * 32;    // whole warpgroups: registers are moved between them
+    static constexpr int X_BYTES = (SMALL ? 96 : 128) * 1024; // ring of x tiles: as many stages as fit
+    static constexpr int MAX_X_STAGES = 16;
+    static constexpr int W_STAGES = SMALL ? 8 : 6;       // ring of raw chunks
+    // A stage is what the tensor core is handed at a time: waits, commits and bookkeeping cost its warp about 500 clocks a
+    // stage, whatever the stage holds (with two k-blocks of up to 128 batch rows they set the pace: 445 clocks a k-block).
+    static constexpr int STAGE_KB = SMALL ? 4 : 2;       // k-blocks per stage
+    static constexpr int STAGES = kASlots / STAGE_KB;    // ring of stages of converted weights
+    // Large tiles: a group converts whole stages, in turn.  Small ones: every group converts one k-block of every stage.
+    static constexpr int VISIT_KB = 2, VISIT_STAGES = 2;
+    static constexpr int A_COL0 = 256;                   // first TMEM column of the A stages; the accumulators are below
+    static constexpr int PACKED = MAX_BX / (EPI_WARPS / 4) / 2; // registers for an epilogue thread's fp16 results
+    // full / empty per stage of weights, of x and per raw chunk, full / empty per accumulator, exchange ready / complete
+    static constexpr int BARRIERS = 2 * STAGES + 2 * MAX_X_STAGES + 2 * W_STAGES + 6;
     static constexpr size_t SMEM_BYTES =
-        1024 + (size_t)STAGES * X_STAGE_BYTES + (size_t)WSTAGES * W_STAGE_BYTES + NUM_BARRIERS * 8 + 64;
-    static constexpr int SLOT_FLOATS = BX * BN; // one tile's accumulator as fp32: a partial sum in the workspace
-    static_assert(A_COL0 + STAGES * A_STAGE_COLS <= TMEM_COLS, "tensor memory budget");
+        1024 + (size_t)X_BYTES + (size_t)W_STAGES * kWStageBytes + BARRIERS * 8 + 64 + 2 * kMaxPairs * sizeof(int);
+    // Registers a thread: launched with LAUNCH_REGS each, then the roles take what they need.
+    static constexpr int LAUNCH_REGS = SMALL ? 80 : 96;
+    static constexpr int DQ_REGS = SMALL ? 72 : 80, EPI_REGS = SMALL ? 120 : 128, ISSUE_REGS = SMALL ? 72 : 64;
+    static_assert(DQ_GROUPS * DQ_REGS + EPI_WARPS / 4 * EPI_REGS + ISSUE_REGS <= THREADS / 128 * LAUNCH_REGS, "registers the CTA has");
+    static_assert(LAUNCH_REGS * THREADS <= 65536, "registers the SM has");
+    static_assert(A_COL0 + kASlots * kASlotCols <= kTmemCols, "tensor memory budget");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
 
 struct GemmParams
 {
-    const void* scale;
-    const uint8_t* zp;
+    const void* scale[2];
+    const uint8_t* zp[2];
     const float* bias;
     void* y;
     int* status;
-    uint32_t* counters; // [tiles] arrivals at a tile that several CTAs share; zero before and after a launch
-    float* slots;       // [2 * CTAs][SLOT_FLOATS] partial sums of shared tiles
+    uint32_t* counters; // [2 * tiles] arrivals at the halves of a tile that several pairs share; zero before and after
+    float* slots;       // [CTAs][2 * sets][128 * BX] partial sums of shared tiles
     int M, N, K;
     int group, G, zp_row_bytes;
     int y_f32, scale_f32, has_bias;
-    int has_addend; // bias points at an [M,N] tensor of y's type instead of fp32 [N]
-    int m_tiles;    // batch tiles; tile t covers batch tile t % m_tiles of weight-row tile t / m_tiles
-    int tiles;      // output tiles in all
-    int whole_tiles; // every tile is computed by one CTA (no partial sums)
-    int kbpg_shift; // log2(group_size / 64) if that is a power of two, else -1
-    int cpt;        // raw chunks (the unit of work) per tile: ceil(K / 64 / KB_PER_CHUNK)
+    int has_addend;  // bias points at an [M,N] tensor of y's type instead of fp32 [N]
+    int bx;          // batch rows per tile, a multiple of 16
+    int x_stages;    // stages of the x ring
+    int m_tiles;     // batch tiles; tile t covers batch tile t % m_tiles of weight-row tile t / m_tiles
+    int tiles;       // output tiles in all
+    int sets;        // weight sets: 2 for SiLU(gate) * up
+    int whole_tiles; // every tile is computed by one pair (no partial sums)
+    int ksplit;      // pairs of a cluster that share a tile's K (1: none; then the cluster is the pair)
+    int slice;       // ... and the batch rows of the tile that each of them finishes
+    int kbpg_shift;  // log2(group / 64) if that is a power of two, else -1
+    int cpt;         // raw chunks (the unit of work) per tile and weight set
 };
 
-constexpr uint32_t kGemmSpin = 1u << 22;
+constexpr uint32_t kGemmSpin = 1u << 21;
 
-// Bounded wait that also gives up as soon as another role of the CTA has raised the abort flag.
+// Bounded waits that also give up as soon as another role of the CTA has raised the abort flag.  SLEEP: nanoseconds between
+// polls; a waiting role should not compete with the working ones for issue slots.
+// One thread:
+template <int SLEEP>
 __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
     for (uint32_t i = 0; i < kGemmSpin; i++)
     {
         if (mbar_try_wait(bar, parity))
             return true;
-        __nanosleep(40); // a waiting role should not compete with the working ones for issue slots and power
+        if constexpr (SLEEP > 0)
+            __nanosleep(SLEEP);
         if ((i & 255u) == 255u && *abort_flag)
             return false;
     }
     *abort_flag = 1;
     return false;
 }
-
-// Same for the thread that issues the MMAs: it is the kernel's critical path, so it polls without backing off.
-__device__ __forceinline__ bool wait_hot(uint32_t bar, uint32_t parity, volatile int* abort_flag)
+// A whole warp.  Every decision is a vote, which the compiler knows to be the same for all lanes: the warp stays together
+// for the warp-wide tensor-memory instructions that follow, and what follows may use uniform registers.
+template <int SLEEP>
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
     for (uint32_t i = 0; i < kGemmSpin; i++)
     {
-        if (mbar_try_wait(bar, parity))
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
             return true;
-        if ((i & 1023u) == 1023u && *abort_flag)
+        if constexpr (SLEEP > 0)
+            __nanosleep(SLEEP);
+        if ((i & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0))
             return false;
     }
     *abort_flag = 1;
@@ -130,364 +164,554 @@ __device__ __forceinline__ uint64_t smem_desc_k_sw128(uint32_t smem_addr)
            (2ull << 61);
 }
 
-// The CTA's share of the launch: units [u, u_end) of tiles * cpt raw chunks, walked as segments that each lie
-// inside one tile.  Every role of the CTA walks the same list.
+// A pair's share of the launch: units [u, u_end) of tiles * sets * cpt raw chunks, walked as segments that each lie
+// inside one tile and one weight set.  Every role of both CTAs walks the same list.
 struct Segment
 {
     int tile;     // output tile
+    int set;      // weight set
     int c0, c1;   // raw chunks [c0, c1) of the tile
-    int kb0, kb1; // k-blocks [kb0, kb1)
-    bool whole;   // the CTA computes the tile alone
+    bool whole;   // the pair computes the tile (both weight sets of it) alone
+    bool last;    // the pair's last segment of the tile
 };
 
-template <int KB_PER_CHUNK>
 struct WorkList
 {
-    int u, u_end; // tiles * cpt fits 31 bits (checked on the host)
+    int u, u_begin, u_end; // tiles * sets * cpt fits 31 bits (checked on the host)
     __device__ WorkList(const GemmParams& p)
     {
+        if (p.ksplit > 1)
+        {
+            u = u_begin = 0, u_end = p.sets; // this pair's chunks of either weight set
+            return;
+        }
+        const int per_tile = p.sets * p.cpt;
         // whole tiles only: the shares are cut at tile boundaries
-        const long long U = p.whole_tiles ? (long long)p.tiles : (long long)p.tiles * p.cpt;
-        const int scale = p.whole_tiles ? p.cpt : 1;
-        u = (int)((long long)blockIdx.x * U / gridDim.x) * scale;
-        u_end = (int)((long long)(blockIdx.x + 1) * U / gridDim.x) * scale;
+        const long long U = p.whole_tiles ? (long long)p.tiles : (long long)p.tiles * per_tile;
+        const int scale = p.whole_tiles ? per_tile : 1;
+        const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+        u = u_begin = (int)((long long)pair * U / pairs) * scale;
+        u_end = (int)((long long)(pair + 1) * U / pairs) * scale;
     }
     __device__ bool next(const GemmParams& p, Segment& s)
     {
         if (u >= u_end)
             return false;
-        s.tile = u / p.cpt;
-        s.c0 = u - s.tile * p.cpt;
+        if (p.ksplit > 1)
+        {
+            const int pair = blockIdx.x >> 1, part = pair % p.ksplit;
+            s.tile = pair / p.ksplit, s.set = u;
+            s.c0 = part * p.cpt / p.ksplit, s.c1 = (part + 1) * p.cpt / p.ksplit;
+            s.whole = false, s.last = ++u == u_end;
+            return true;
+        }
+        const int per_tile = p.sets * p.cpt;
+        s.tile = u / per_tile;
+        const int base = s.tile * per_tile, in = u - base;
+        s.set = in >= p.cpt ? 1 : 0;
+        s.c0 = in - s.set * p.cpt;
         s.c1 = min(p.cpt, s.c0 + (u_end - u));
-        s.kb0 = s.c0 * KB_PER_CHUNK;
-        s.kb1 = min(p.K / 64, s.c1 * KB_PER_CHUNK);
-        s.whole = s.c0 == 0 && s.c1 == p.cpt;
+        s.whole = u_begin <= base && base + per_tile <= u_end;
         u += s.c1 - s.c0;
+        s.last = u == u_end || u == base + per_tile;
         return true;
     }
 };
 
-// The CTA whose share holds unit u: the largest c with floor(c * U / G) <= u.
-__device__ __forceinline__ int cta_of_unit(long long u, long long U, int G)
+// The pair whose share holds unit u: the largest c with floor(c * U / G) <= u.
+__device__ __forceinline__ int pair_of_unit(long long u, long long U, int G)
 {
     return (int)(((u + 1) * G + U - 1) / U) - 1;
 }
 
-// Where CTA c keeps its partial sum of tile t: slot 2c if t is the first tile of its share, else 2c + 1 (a share has
-// at most two tiles that it does not compute alone, its first and its last).
-__device__ __forceinline__ int slot_of(int c, int t, long long U, int G, int cpt)
+// Where a CTA of pair c keeps its partial sum of weight set `set` of tile t: a share has at most two tiles that it does
+// not compute alone, its first and its last.
+__device__ __forceinline__ int slot_of(const GemmParams& p, int c, int rank, int t, int set, long long U, int G)
 {
-    const int first_tile = (int)(((long long)c * U / G) / cpt);
-    return 2 * c + (t == first_tile ? 0 : 1);
+    const int first_tile = (int)(((long long)c * U / G) / (p.sets * p.cpt));
+    return ((2 * c + rank) * 2 + (t == first_tile ? 0 : 1)) * p.sets + set;
 }
 
-// One finished value on its way to y: SiLU(gate) * v when a gate value is given, bias of the weight row (0 without),
-// full-size addend, conversion.
-__device__ __forceinline__ void store_value(const GemmParams& p, int m, int n, float v, bool gated, float g, float bias)
+// A value the compiler must keep as it is: without this it works out 128 addresses ahead of their stores.
+__device__ __forceinline__ uint32_t held(uint32_t v)
 {
-    const size_t at = (size_t)m * p.N + n;
-    if (gated)
-        v *= g > -80.f ? __fdividef(g, 1.0f + __expf(-g)) : 0.f; // SiLU(g) = g / (1 + e^-g), ~1e-6 relative; 0 far left
-    v += bias;
-    if (p.has_addend)
-        v += p.y_f32 ? reinterpret_cast<const float*>(p.bias)[at]
-                     : __half2float(reinterpret_cast<const __half*>(p.bias)[at]);
-    if (p.y_f32)
-        static_cast<float*>(p.y)[at] = v;
-    else
-        static_cast<__half*>(p.y)[at] = __float2half_rn(v);
+    uint32_t r;
+    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
 }
 
-// The gate product that an earlier launch left at y[m, n], as raw bits (fp32, or fp16 in the low half).
-__device__ __forceinline__ uint32_t gate_bits(const GemmParams& p, int m, int n)
+// SiLU(g) = g / (1 + e^-g), ~1e-6 relative; 0 far left
+__device__ __forceinline__ float silu(float g)
 {
-    const size_t at = (size_t)m * p.N + n;
-    return p.y_f32 ? static_cast<const uint32_t*>(p.y)[at] : (uint32_t)static_cast<const unsigned short*>(p.y)[at];
+    return g > -80.f ? __fdividef(g, 1.0f + __expf(-g)) : 0.f;
 }
-// (a gate product that left the fp16 range on its way through y comes back as the largest fp16 number, so that SiLU
-// stays finite: SiLU(-inf) would be -inf / inf)
-__device__ __forceinline__ float gate_value(const GemmParams& p, uint32_t bits)
+
+// A gate product that waited in y as fp16.  (One that left the fp16 range on its way comes back as the largest fp16
+// number, so that SiLU stays finite: SiLU(-inf) would be -inf / inf.)
+__device__ __forceinline__ float gate_of_half(uint32_t bits)
 {
-    if (p.y_f32)
-        return __uint_as_float(bits);
     return fminf(fmaxf(__half2float(__ushort_as_half((unsigned short)bits)), -65504.f), 65504.f);
 }
 
-// GATED: y holds the gate products of an earlier launch (the second half of SiLU(gate) * up).
-template <int WBITS, bool GATED, int BXV>
-__global__ void __launch_bounds__(Cfg<WBITS, BXV>::THREADS, 1)
-    dq_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap_x,
-                   const __grid_constant__ CUtensorMap tmap_w)
+__device__ __forceinline__ float4 load_part(const float4* p)
 {
-    using C = Cfg<WBITS, BXV>;
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// Adds up the parts of a tile's half that several pairs computed, in the order of their K ranges, and writes y.  A lane
+// keeps four neighbouring weight rows (16-byte loads), a warp takes every WARPS-th batch row; ROWS rows of two parts are
+// asked for at a time.  load(set, part, row): a lane's four sums; parts0 / parts1: how many parts either weight set has.
+template <int SETS, int ROWS, int WARPS, typename Load>
+__device__ __forceinline__ void add_parts(const GemmParams& p, Load load, int parts0, int parts1, int n4, int m0, int rows,
+                                          int ew)
+{
+    if (n4 >= p.N)
+        return;
+    const bool vec = (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15u) == 0 &&
+                     (!p.has_addend || (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0);
+    float bias[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        bias[e] = p.has_bias && n4 + e < p.N ? __ldg(p.bias + n4 + e) : 0.f;
+    for (int row = ew; row < rows; row += ROWS * WARPS)
+    {
+        float v[SETS][ROWS][4];
+#pragma unroll
+        for (int set = 0; set < SETS; set++)
+        {
+#pragma unroll
+            for (int j = 0; j < ROWS; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    v[set][j][e] = 0.f;
+            // (unconditional loads, past the last part or row of the last one: a choice per load costs a branch per load.  No
+            // more of them at a time than registers hold beside the sums: the compiler would take turns)
+            const int parts = set == 0 ? parts0 : parts1;
+            for (int i = 0; i < parts; i += 2)
+            {
+                float4 a[2][ROWS];
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+#pragma unroll
+                    for (int j = 0; j < ROWS; j++)
+                        a[c][j] = load(set, min(i + c, parts - 1), min(row + j * WARPS, rows - 1));
+                const bool two = i + 1 < parts;
+#pragma unroll
+                for (int j = 0; j < ROWS; j++)
+                {
+                    v[set][j][0] += a[0][j].x, v[set][j][1] += a[0][j].y, v[set][j][2] += a[0][j].z, v[set][j][3] += a[0][j].w;
+                    if (two)
+                        v[set][j][0] += a[1][j].x, v[set][j][1] += a[1][j].y, v[set][j][2] += a[1][j].z, v[set][j][3] += a[1][j].w;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; j++)
+        {
+            if (row + j * WARPS >= rows)
+                break;
+            const size_t at = (size_t)(m0 + row + j * WARPS) * p.N + n4;
+            float o[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+            {
+                if constexpr (SETS == 2) // (the gate products pass through y's type here too)
+                    o[e] = v[1][j][e] * silu(p.y_f32 ? v[0][j][e] : gate_of_half(__half_as_ushort(__float2half_rn(v[0][j][e]))));
+                else
+                    o[e] = v[0][j][e] + bias[e];
+            }
+            if (vec)
+            {
+                if (p.y_f32)
+                {
+                    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (p.has_addend)
+                        c = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.bias) + at);
+                    *reinterpret_cast<float4*>(static_cast<float*>(p.y) + at) = make_float4(o[0] + c.x, o[1] + c.y, o[2] + c.z, o[3] + c.w);
+                }
+                else
+                {
+                    if (p.has_addend)
+                    {
+                        const uint2 c = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(p.bias) + at);
+                        const float2 c0 = __half22float2(*reinterpret_cast<const __half2*>(&c.x));
+                        const float2 c1 = __half22float2(*reinterpret_cast<const __half2*>(&c.y));
+                        o[0] += c0.x, o[1] += c0.y, o[2] += c1.x, o[3] += c1.y;
+                    }
+                    const __half2 h0 = __floats2half2_rn(o[0], o[1]), h1 = __floats2half2_rn(o[2], o[3]);
+                    uint2 pk;
+                    pk.x = *reinterpret_cast<const uint32_t*>(&h0), pk.y = *reinterpret_cast<const uint32_t*>(&h1);
+                    *reinterpret_cast<uint2*>(static_cast<__half*>(p.y) + at) = pk;
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (n4 + e < p.N)
+                    {
+                        if (p.has_addend)
+                            o[e] += p.y_f32 ? reinterpret_cast<const float*>(p.bias)[at + e]
+                                            : __half2float(reinterpret_cast<const __half*>(p.bias)[at + e]);
+                        if (p.y_f32)
+                            static_cast<float*>(p.y)[at + e] = o[e];
+                        else
+                            static_cast<__half*>(p.y)[at + e] = __float2half_rn(o[e]);
+                    }
+            }
+        }
+    }
+}
+
+// ONE_GROUP: two neighbouring k-blocks (of a raw chunk) always lie in one quantisation group.
+template <int WBITS, bool ONE_GROUP, bool SMALL>
+__global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
+    dq_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
+                   const __grid_constant__ CUtensorMap tmap_w1)
+{
+    using C = Cfg<SMALL>;
+    constexpr int KBC = (WBITS == 4) ? 4 : 2;           // k-blocks per raw chunk
+    constexpr int RAW_BYTES = (WBITS == 4) ? 32 : 64;   // raw bytes per row and k-block
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* xs = base;                                             // [STAGES][BX][128 B]
-    uint8_t* wsm = xs + (size_t)C::STAGES * C::X_STAGE_BYTES;       // [WSTAGES][128][128 B]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(wsm + (size_t)C::WSTAGES * C::W_STAGE_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NUM_BARRIERS);
+    uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* xs = base;                                        // [x stages][2][BX / 2 rows][128 B]
+    uint8_t* wsm = xs + (size_t)C::X_BYTES;                    // [raw stages][128][128 B]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(wsm + (size_t)C::W_STAGES * kWStageBytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::BARRIERS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile uint32_t* ticket_slot = reinterpret_cast<volatile uint32_t*>(tmem_slot + 2);
+    int* slot_list = reinterpret_cast<int*>(tmem_slot + 4);    // [2][kMaxPairs]
 
     const uint32_t bar0 = smem_u32(bars);
-    // full(q): the x tiles of pair q have landed (TMA transaction bytes) and every conversion thread has stored its
-    // row of both stages (2 * 128 arrivals; where a segment ends on a single k-block, its threads arrive twice);
-    // empty(q): the MMAs that read the pair have completed (tcgen05.commit).
-    auto full = [&](int q) { return bar0 + 8u * q; };
-    auto empty = [&](int q) { return bar0 + 8u * (C::PAIRS + q); };
-    auto full_w = [&](int s) { return bar0 + 8u * (2 * C::PAIRS + s); };
-    auto empty_w = [&](int s) { return bar0 + 8u * (2 * C::PAIRS + C::WSTAGES + s); };
-    const uint32_t acc_full = bar0 + 8u * (C::NUM_BARRIERS - 4);     // a segment's MMAs have completed
-    const uint32_t acc_empty = bar0 + 8u * (C::NUM_BARRIERS - 3);    // every conversion thread has read its part of D
-    const uint32_t part_done = bar0 + 8u * (C::NUM_BARRIERS - 2);    // every conversion thread has written its partial sums
-    const uint32_t ticket_ready = bar0 + 8u * (C::NUM_BARRIERS - 1); // the tile's arrival count is in ticket_slot
+    // full_a(q), in the even CTA: the conversion warps of both CTAs have stored the stage's weights (4 warps each per k-block or stage);
+    // full_x(q), in the even CTA: both CTAs' x tiles of the stage have landed (TMA transaction bytes);
+    // empty_a(q), empty_x(q), in both: the MMAs that read the stage have completed.
+    auto full_a = [&](int q) { return bar0 + 8u * q; };
+    auto empty_a = [&](int q) { return bar0 + 8u * (C::STAGES + q); };
+    auto full_w = [&](int s) { return bar0 + 8u * (2 * C::STAGES + s); };
+    auto empty_w = [&](int s) { return bar0 + 8u * (2 * C::STAGES + C::W_STAGES + s); };
+    auto acc_full = [&](int b) { return bar0 + 8u * (2 * C::STAGES + 2 * C::W_STAGES + b); };      // in both CTAs
+    auto acc_empty = [&](int b) { return bar0 + 8u * (2 * C::STAGES + 2 * C::W_STAGES + 2 + b); }; // in the even CTA
+    auto full_x = [&](int q) { return bar0 + 8u * (2 * C::STAGES + 2 * C::W_STAGES + 4 + q); };
+    auto empty_x = [&](int q) { return bar0 + 8u * (2 * C::STAGES + 2 * C::W_STAGES + 4 + C::MAX_X_STAGES + q); };
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int KB = p.K / C::BK;
-    constexpr int TMA_WARP = C::DQ_WARPS, MMA_WARP = C::DQ_WARPS + 1, TMAW_WARP = C::DQ_WARPS + 2;
+    const uint32_t peers_ready = bar0 + 8u * (C::BARRIERS - 2); // every pair of the cluster has multiplied: its rings are free
+    const uint32_t parts_here = bar0 + 8u * (C::BARRIERS - 1);  // every pair's sums of this CTA's batch rows have arrived
+
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); // (known to be the same for the whole warp)
+    const uint32_t rank = blockIdx.x & 1u;                                    // CTA of the pair
+    const uint32_t even = 2u * ((blockIdx.x >> 1) % (uint32_t)p.ksplit);      // the pair's even CTA in the cluster
+    const int KB = p.K / kBK;
+    const int acc_bufs = p.bx <= 128 ? 2 : 1;
+    WorkList work(p);
+    Segment sg{};
 
     // ---------------------------------------------------------------- set-up (once per CTA)
-    if (tid == 0)
+    if (warp == C::X_WARP)
     {
-        for (int q = 0; q < C::PAIRS; q++)
+        if (lane == 0)
+            prefetch_tensormap(&tmap_x);
+        if (lane < C::STAGES)
         {
-            mbar_init(full(q), 2 * 128 + 1); // every row of both stages and the x tiles
-            mbar_init(empty(q), 1);
+            mbar_init(full_a(lane), 2 * 4 * (C::STAGE_KB / C::VISIT_KB));
+            mbar_init(empty_a(lane), 1);
         }
-        for (int s = 0; s < C::WSTAGES; s++)
+        if (lane < C::MAX_X_STAGES)
         {
-            mbar_init(full_w(s), 1);
-            mbar_init(empty_w(s), C::KB_PER_CHUNK * 128); // 128 rows read per k-block of the chunk
+            mbar_init(full_x(lane), 1);
+            mbar_init(empty_x(lane), 1);
         }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_empty, C::DQ_WARPS * 32);
-        mbar_init(part_done, C::DQ_WARPS * 32);
-        mbar_init(ticket_ready, 1);
-        *abort_flag = 0;
+        if (lane < 2)
+        {
+            mbar_init(acc_full(lane), 1);
+            mbar_init(acc_empty(lane), 2 * C::EPI_WARPS);
+        }
+        if (lane == 0)
+        {
+            mbar_init(peers_ready, (uint32_t)p.ksplit);
+            mbar_init(parts_here, (uint32_t)(p.ksplit * C::EPI_WARPS));
+            *abort_flag = 0;
+        }
         fence_barrier_init();
     }
-    if (warp == MMA_WARP)
+    // Raw weight chunks: the ring belongs to this CTA alone, so that its first round leaves before anything else is set up
+    // (set-up takes 3000 clocks, as long as HBM takes to answer).
+    uint32_t w_asked = 0; // chunks asked for so far
+    auto ask_chunk = [&](const Segment& s, int c) {
+        const int st = (int)(w_asked % C::W_STAGES);
+        mbar_arrive_expect_tx(full_w(st), kWStageBytes);
+        tma_load_2d(smem_u32(wsm + (size_t)st * kWStageBytes), s.set ? &tmap_w1 : &tmap_w0, full_w(st), c * 128,
+                    (s.tile / p.m_tiles) * (2 * kBN) + (int)rank * kBN);
+        w_asked++;
+    };
+    int w_next = 0; // the chunk of segment sg to ask for next (warp W)
+    bool w_more = false;
+    auto next_chunk = [&] {
+        if (++w_next == sg.c1)
+        {
+            w_more = work.next(p, sg);
+            w_next = sg.c0;
+        }
+    };
+    if (warp == C::W_WARP && lane == 0)
     {
-        tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS); // whole warp; the address lands in shared memory
+        for (int s = 0; s < C::W_STAGES; s++)
+        {
+            mbar_init(full_w(s), 1);
+            mbar_init(empty_w(s), 4 * KBC); // (a warp arrives once per k-block)
+        }
+        fence_barrier_init();
+        w_more = work.next(p, sg);
+        w_next = sg.c0;
+        while (w_more && w_asked < C::W_STAGES)
+        {
+            ask_chunk(sg, w_next);
+            next_chunk();
+        }
+    }
+    if (warp == C::MMA_WARP)
+    {
+        tmem_alloc(smem_u32(tmem_slot), kTmemCols); // whole warp of both CTAs; the address lands in shared memory
         tmem_relinquish();
     }
     tcgen05_fence_before();
     __syncthreads();
+    cluster_arrive(); // the other CTA's barriers are initialised, its tensor memory is allocated
+    cluster_wait();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    WorkList<C::KB_PER_CHUNK> work(p);
-    Segment sg;
+    constexpr uint32_t tmem_base = 0; // (a constant, so that the multiplies' addresses are known to be the same for all lanes)
+    if (tid == 0 && *tmem_slot != tmem_base)
+        *abort_flag = 1;
     // Launched as the programmatic dependent of the kernel before it on the stream, this CTA may have started while
-    // that kernel's last CTAs were still running.  Weights, scales and zero-points are constants: the raw-chunk
-    // producer and the conversion into tensor memory start at once.  The activations, the result, the addend and
-    // the workspace may be the earlier kernel's: the activation producer waits before its first load and the
-    // conversion warps before their first read-back.  The launch behind this one may be scheduled from here on.
+    // that kernel's last CTAs were still running.  Weights, scales and zero-points are constants: the raw chunks and the
+    // conversion into tensor memory start at once.  The activations, the result, the addend and the workspace may be the
+    // earlier kernel's: the thread that loads x waits before its first tile and the epilogue warps before their first
+    // segment.  The launch behind this one may be scheduled from here on.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    if (warp == TMA_WARP)
-    {
-        // ------------------------------------------------------------ TMA producer: activation tiles
-        if (lane == 0)
-        {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            bool ok = true;
-            uint32_t pr = 0; // pairs of k-blocks of this CTA so far: ring position (every segment starts a pair)
-            while (ok && work.next(p, sg))
-            {
-                const int m0 = (sg.tile % p.m_tiles) * C::BX;
-                for (int kb = sg.kb0; kb < sg.kb1; kb += 2, pr++)
-                {
-                    const int q = pr % C::PAIRS;
-                    const uint32_t ph = (pr / C::PAIRS) & 1u;
-                    ok = wait_or_abort(empty(q), ph ^ 1u, abort_flag);
-                    if (!ok)
-                        break;
-                    const int nkb = min(2, sg.kb1 - kb);
-                    mbar_arrive_expect_tx(full(q), (uint32_t)(nkb * C::X_STAGE_BYTES));
-                    for (int h = 0; h < nkb; h++)
-                        tma_load_2d(smem_u32(xs + (size_t)(2 * q + h) * C::X_STAGE_BYTES), &tmap_x, full(q),
-                                    (kb + h) * C::BK, m0);
-                }
-            }
-        }
-    }
-    else if (warp == TMAW_WARP)
+    if (warp >= C::X_WARP)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::ISSUE_REGS));
+    if (warp == C::W_WARP)
     {
         // ------------------------------------------------------------ TMA producer: raw weight chunks
-        // A loop of its own: the chunks run as far ahead as their ring allows (WSTAGES * KB_PER_CHUNK k-blocks),
-        // so that their load latency and the conversion stay off the tensor core's critical path.
+        // A thread of its own, as for x: either runs as far ahead as its own ring allows.
+        if (lane == 0)
+            while (w_more)
+            {
+                if (!wait_or_abort<40>(empty_w(w_asked % C::W_STAGES), ((w_asked / C::W_STAGES) & 1u) ^ 1u, abort_flag))
+                    break;
+                ask_chunk(sg, w_next);
+                next_chunk();
+            }
+    }
+    else if (warp == C::X_WARP)
+    {
+        // ------------------------------------------------------------ TMA producer: x tiles
         if (lane == 0)
         {
             bool ok = true;
-            uint32_t wc = 0; // chunks of this CTA so far
+            const int half = p.bx >> 1;
+            const uint32_t x_bytes = (uint32_t)half * 128u; // one k-block of this CTA's batch rows
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            int q = 0;            // stage ...
+            uint32_t phase = 1;   // ... and the parity of its release
+            uint32_t x_dst = smem_u32(xs), bar = map_to_rank(full_x(0), even);
             while (ok && work.next(p, sg))
             {
-                const int n0 = (sg.tile / p.m_tiles) * C::BN;
-                for (int chunk = sg.c0; chunk < sg.c1; chunk++, wc++)
+                const int m0 = (sg.tile % p.m_tiles) * p.bx + (int)rank * half;
+                const int kb_end = min(KB, sg.c1 * KBC);
+                for (int kb = sg.c0 * KBC; kb < kb_end; kb += C::STAGE_KB)
                 {
-                    const int s = wc % C::WSTAGES;
-                    const uint32_t ph = (wc / C::WSTAGES) & 1u;
-                    ok = wait_or_abort(empty_w(s), ph ^ 1u, abort_flag);
+                    ok = wait_or_abort<20>(empty_x(q), phase, abort_flag);
                     if (!ok)
                         break;
-                    mbar_arrive_expect_tx(full_w(s), C::W_STAGE_BYTES);
-                    tma_load_2d(smem_u32(wsm + (size_t)s * C::W_STAGE_BYTES), &tmap_w, full_w(s), chunk * 128, n0);
+                    const int nkb = min(C::STAGE_KB, kb_end - kb);
+                    if (rank == 0) // (counted at the even CTA, for both)
+                        mbar_arrive_expect_tx(full_x(q), 2u * (uint32_t)nkb * x_bytes);
+                    for (int h = 0; h < nkb; h++)
+                        tma_load_2d_pair(x_dst + (uint32_t)h * x_bytes, &tmap_x, bar, (kb + h) * kBK, m0);
+                    if (++q == p.x_stages)
+                        q = 0, phase ^= 1u, x_dst = smem_u32(xs), bar = map_to_rank(full_x(0), even);
+                    else
+                        x_dst += (uint32_t)C::STAGE_KB * x_bytes, bar += 8u;
                 }
             }
         }
     }
-    else if (warp == MMA_WARP)
+    else if (warp == C::MMA_WARP)
     {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0)
+        // ------------------------------------------------------------ MMA issuer (even CTA)
+        // (the whole warp walks the loop, one elected lane issues)
+        if (rank == 0)
         {
-            // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = BX, M = 128
-            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(C::BX >> 3) << 17) | ((uint32_t)(C::BN >> 4) << 24);
+            // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = BX, M = 256
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(p.bx >> 3) << 17) | ((uint32_t)((2 * kBN) >> 4) << 24);
             bool ok = true;
             uint32_t si = 0;
-            // Ring position kept as (slot, phase) with the slot's addresses carried along: this one thread feeds the
-            // tensor core next to four busy conversion warps on its scheduler, so every instruction it does not
-            // need to issue between two MMAs is tensor time.
-            int q = 0;
-            uint32_t phase = 0;
+            // Ring positions kept as (slot, phase) with the slot's addresses carried along: every instruction not needed
+            // between two MMAs is tensor time.
+            int q = 0, qx = 0;
+            uint32_t phase = 0, phase_x = 0;
+            const uint64_t x_block = (uint64_t)(p.bx * 64 >> 4); // one k-block of this CTA's x rows
             const uint64_t xdesc0 = smem_desc_k_sw128(smem_u32(xs));
             const uint32_t a_tmem0 = tmem_base + (uint32_t)C::A_COL0;
-            uint64_t xdesc = xdesc0;  // of slot q: two stages of x ...
-            uint32_t a_tmem = a_tmem0; // ... and two stages of converted weights
-            uint32_t bar_full = full(0), bar_empty = empty(0);
+            const uint32_t issue = elect_one() ? 1u : 0u;
+            const uint16_t pair_mask = (uint16_t)(3u << even);
+            uint64_t xdesc = xdesc0;
+            uint32_t a_tmem = a_tmem0;
             while (ok && work.next(p, sg))
             {
-                if (si > 0)
-                {
-                    // the accumulator still holds the previous segment until the conversion warps have read it
-                    ok = wait_hot(acc_empty, (si - 1) & 1u, abort_flag);
-                    if (!ok)
-                        break;
-                    tcgen05_fence_after();
-                }
+                const uint32_t b = acc_bufs == 2 ? (si & 1u) : 0u, use = acc_bufs == 2 ? si >> 1 : si;
+                // the accumulator still holds an earlier segment until the epilogue warps of both CTAs have read it
+                ok = wait_warp<0>(acc_empty(b), (use & 1u) ^ 1u, abort_flag);
+                if (!ok)
+                    break;
+                tcgen05_fence_after();
+                const uint32_t d_tmem = tmem_base + b * 128u;
                 uint32_t accumulate = 0u; // the segment's first MMA overwrites D
-                for (int kb = sg.kb0; kb < sg.kb1; kb += 2)
+                const int kb_end = min(KB, sg.c1 * KBC);
+                for (int kb = sg.c0 * KBC; kb < kb_end; kb += C::STAGE_KB)
                 {
-                    ok = wait_hot(bar_full, phase, abort_flag);
+                    ok = wait_warp<0>(full_x(qx), phase_x, abort_flag) && wait_warp<0>(full_a(q), phase, abort_flag);
                     if (!ok)
                         break;
                     tcgen05_fence_after();
-                    // (the descriptor's address field counts 16-byte units: stage and k step are plain additions)
+                    // (the descriptor's address field counts 16-byte units: k-block and k step are plain additions)
+                    auto multiply = [&](int h, uint32_t acc) {
 #pragma unroll
-                    for (int kk = 0; kk < C::BK / 16; kk++)
-                    {
-                        tcgen05_mma_ts(tmem_base, a_tmem + kk * 8, xdesc + (uint64_t)(kk * 2), idesc, accumulate);
-                        accumulate = 1u;
-                    }
-                    if (kb + 1 < sg.kb1)
+                        for (int kk = 0; kk < kBK / 16; kk++)
+                            tcgen05_mma_ts(d_tmem, a_tmem + (uint32_t)(h * kASlotCols + kk * 8), xdesc + (uint64_t)h * x_block + (uint64_t)(kk * 2),
+                                           idesc, kk == 0 ? acc : 1u, issue);
+                    };
+                    multiply(0, accumulate);
+                    accumulate = 1u;
+                    if (kb + C::STAGE_KB <= kb_end)
                     {
 #pragma unroll
-                        for (int kk = 0; kk < C::BK / 16; kk++)
-                            tcgen05_mma_ts(tmem_base, a_tmem + C::A_STAGE_COLS + kk * 8,
-                                           xdesc + (uint64_t)((C::X_STAGE_BYTES >> 4) + kk * 2), idesc, 1u);
-                    }
-                    tcgen05_commit(bar_empty); // arrives when the MMAs above have consumed the pair
-                    if (++q == C::PAIRS)
-                    {
-                        q = 0, phase ^= 1u;
-                        xdesc = xdesc0, a_tmem = a_tmem0, bar_full = full(0), bar_empty = empty(0);
+                        for (int h = 1; h < C::STAGE_KB; h++)
+                            multiply(h, 1u);
                     }
                     else
                     {
-                        xdesc += (uint64_t)(2 * (C::X_STAGE_BYTES >> 4)), a_tmem += 2 * C::A_STAGE_COLS;
-                        bar_full += 8u, bar_empty += 8u;
+#pragma unroll 1
+                        for (int h = 1; h < kb_end - kb; h++)
+                            multiply(h, 1u);
                     }
+                    tcgen05_commit_pair(empty_a(q), pair_mask, issue); // arrives when the MMAs above have consumed the stage
+                    tcgen05_commit_pair(empty_x(qx), pair_mask, issue);
+                    if (++q == C::STAGES)
+                        q = 0, phase ^= 1u, a_tmem = a_tmem0;
+                    else
+                        a_tmem += C::STAGE_KB * kASlotCols;
+                    if (++qx == p.x_stages)
+                        qx = 0, phase_x ^= 1u, xdesc = xdesc0;
+                    else
+                        xdesc += C::STAGE_KB * x_block;
                 }
                 if (ok)
-                    tcgen05_commit(acc_full);
+                    tcgen05_commit_pair(acc_full(b), pair_mask, issue);
                 si++;
             }
         }
     }
-    else
+    else if (warp < C::DQ_WARPS)
     {
         // ------------------------------------------------------------ dequantise into tensor memory
-        const int grp = warp >> 2;                   // 0 .. DQ_GROUPS-1
-        const int quarter = warp & 3;
-        const int r = quarter * 32 + lane;           // row of the tile = TMEM lane
-        const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        const int kb_per_group = p.group / C::BK;
-        const uint32_t wsm_s = smem_u32(wsm);
+        if constexpr (C::DQ_REGS < C::LAUNCH_REGS)
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::DQ_REGS));
+        // group g converts k-blocks [2 * part, 2 * part + 2) of every second stage
+        const int turn = (warp >> 2) / (C::STAGE_KB / C::VISIT_KB), part = (warp >> 2) % (C::STAGE_KB / C::VISIT_KB);
+        const int r = (warp & 3) * 32 + lane;                          // weight row of the CTA's half = TMEM lane
+        const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+        const int kb_per_group = p.group / kBK;
+        const uint32_t row_s = smem_u32(wsm) + (uint32_t)(r * 128);
+        const uint32_t col0 = tmem_base + lane_addr + (uint32_t)C::A_COL0;
+        const uint32_t full0 = map_to_rank(full_a(0), even); // the even CTA's barriers
+        constexpr int VKB = C::VISIT_KB, VST = C::VISIT_STAGES, SKB = C::STAGE_KB;
+        // A parity tells a barrier's phase from the one before, no more: a group's next stage must not be two rounds of the
+        // A ring ahead, and its raw chunk not two rounds of the raw ring ahead of what has landed (everything up to the
+        // stage VISIT_STAGES + STAGES back has been multiplied).
+        static_assert(VST <= C::STAGES && (VST + C::STAGES) * SKB <= C::W_STAGES * KBC, "rounds of the rings");
         bool ok = true;
-        uint32_t pr_base = 0; // pairs of k-blocks of this CTA before the segment in hand: ring position of its first
-        uint32_t wc_base = 0; // raw chunks likewise
-        uint32_t si = 0, npart = 0;
-
-        // Scales and zero-points: the raw words of this group's next two k-blocks wait in registers, in two sets
-        // that take turns.  Nothing touches a loaded word before its k-block is converted (a move, a shift or a
-        // conversion right after the load would make the thread sit out the whole load latency there), and the first
-        // two of a segment are asked for before the previous segment's accumulator is read back.
-        struct RawParams
-        {
-            uint32_t s, z;
-            int g;
-        };
-        RawParams pa{0, 0, 0}, pb{0, 0, 0};
-        // This thread's row of scales and of zero-points (rows past N read the last row's, never stored).
-        struct RowParams
-        {
-            const char* scale;
-            const uint8_t* zp;
-        };
-        auto row_of = [&](int tile) {
-            const size_t n = (size_t)min((tile / p.m_tiles) * C::BN + r, p.N - 1);
-            return RowParams{static_cast<const char*>(p.scale) + n * p.G * (p.scale_f32 ? 4 : 2),
-                             p.zp + n * (WBITS == 4 ? p.zp_row_bytes : p.G)};
-        };
-        auto ask = [&](const RowParams& n, int kb, int kb_last, RawParams& q) {
-            const int kbc = min(kb, kb_last);
-            q.g = p.kbpg_shift >= 0 ? (kbc >> p.kbpg_shift) : kbc / kb_per_group;
-            if (p.scale_f32)
-                q.s = __ldg(reinterpret_cast<const uint32_t*>(n.scale) + q.g);
-            else
-                q.s = __ldg(reinterpret_cast<const unsigned short*>(n.scale) + q.g);
-            q.z = __ldg(n.zp + (WBITS == 4 ? q.g >> 1 : q.g));
-        };
-        bool asked = false;
-        bool dep_waited = false; // has this thread waited for the kernel before this one on the stream?
-
+        uint32_t wc_base = 0, st_base = 0; // chunks and stages of this CTA before the segment in hand
         while (ok && work.next(p, sg))
         {
-            const RowParams n = row_of(sg.tile);
-            if (!asked)
-            {
-                ask(n, sg.kb0 + grp, sg.kb1 - 1, pa);
-                ask(n, sg.kb0 + grp + C::DQ_GROUPS, sg.kb1 - 1, pb);
-            }
-
-            // One k-block: raw bytes -> 64 fp16 (q - zp) * scale in k order (register i holds k = 2i in its low half
-            // and k = 2i + 1 in its high half) -> this thread's row of the A stage in tensor memory -> tell the MMA
-            // thread.  The group's k-block after next gets its parameters asked for on the way.
-            auto one = [&](int kb, RawParams& q) -> bool {
-                const int chunk = kb / C::KB_PER_CHUNK, j = kb % C::KB_PER_CHUNK;
-                const uint32_t wci = wc_base + (uint32_t)(chunk - sg.c0);
-                const int sw = wci % C::WSTAGES;
-                if (!wait_or_abort(full_w(sw), (wci / C::WSTAGES) & 1u, abort_flag))
-                    return false;
-                // this row's raw bytes: 16-byte chunk c of row r is stored at chunk c ^ (r & 7)
-                const uint32_t row = wsm_s + (uint32_t)(sw * C::W_STAGE_BYTES + r * 128);
-                constexpr int NV = C::RAW_BYTES / 16;
-                uint4 raw[NV];
+            // This thread's row of scales and of zero-points (rows past N read the last row's, never stored).
+            const size_t n = (size_t)min((sg.tile / p.m_tiles) * (2 * kBN) + (int)rank * kBN + r, p.N - 1);
+            const char* const sc = static_cast<const char*>(p.scale[sg.set]) + n * p.G * (p.scale_f32 ? 4 : 2);
+            const uint8_t* const zp = p.zp[sg.set] + n * p.zp_row_bytes;
+            const int kb0 = sg.c0 * KBC, kb_end = min(KB, sg.c1 * KBC), n_st = (kb_end - kb0 + SKB - 1) / SKB;
+            // The raw words of the group's next visit are asked for one visit ahead, and nothing touches them before that
+            // visit (a move or a conversion right after the load would make the thread sit out the load's latency).
+            constexpr int NP = ONE_GROUP ? 1 : VKB; // (scale, zero-point) pairs per visit
+            uint32_t s_now[NP], z_now[NP], s_next[NP], z_next[NP];
+            int g_now[NP], g_next[NP];
+            // the group's first k-block of stage i of the segment
+            auto kb_of = [&](int i) { return kb0 + i * SKB + part * VKB; };
+            auto ask = [&](int i) {
 #pragma unroll
-                for (int v = 0; v < NV; v++)
-                    raw[v] = lds128(row + (uint32_t)(((j * NV + v) ^ (r & 7)) * 16));
-                const float sc = p.scale_f32 ? __uint_as_float(q.s) : __half2float(__ushort_as_half((unsigned short)q.s));
-                const uint32_t zq = WBITS == 4 ? (q.z >> (4 * (q.g & 1))) & 0xFu : q.z;
-                ask(n, kb + 2 * C::DQ_GROUPS, sg.kb1 - 1, q);
-                const __half2 s2 = __float2half2_rn(sc);
-                uint32_t a[32];
-                if (WBITS == 4)
+                for (int j = 0; j < NP; j++)
                 {
-                    const uint32_t zc = (0x6400u | zq) | ((0x5400u | (zq << 4)) << 16); // (1024 + zp, 64 + zp)
+                    const int kb = min(kb_of(i) + j, KB - 1);
+                    const int g = p.kbpg_shift >= 0 ? kb >> p.kbpg_shift : kb / kb_per_group;
+                    g_next[j] = g;
+                    s_next[j] = p.scale_f32 ? __ldg(reinterpret_cast<const uint32_t*>(sc) + g)
+                                            : (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(sc) + g);
+                    z_next[j] = (uint32_t)__ldg(zp + (WBITS == 4 ? g >> 1 : g));
+                }
+            };
+            const int i_first = (int)(((uint32_t)turn - st_base) & (VST - 1));
+            if (i_first < n_st)
+                ask(i_first);
+            for (int i = i_first; i < n_st; i += VST)
+            {
+#pragma unroll
+                for (int j = 0; j < NP; j++)
+                    s_now[j] = s_next[j], z_now[j] = z_next[j], g_now[j] = g_next[j];
+                const int kb = kb_of(i), nkb = min(VKB, kb_end - kb); // (nkb <= 0: a short stage has nothing for this group)
+                const int chunk = (kb - kb0) / KBC, in_chunk = (kb - kb0) % KBC;
+                const uint32_t wc = wc_base + (uint32_t)chunk, sti = st_base + (uint32_t)i;
+                const int sw = wc % C::W_STAGES, q = sti % C::STAGES;
+                if (nkb > 0)
+                {
+                    ok = wait_warp<20>(full_w(sw), (wc / C::W_STAGES) & 1u, abort_flag);
+                    if (!ok)
+                        break;
+                }
+                if (i + VST < n_st)
+                    ask(i + VST);
+                // this row's raw bytes: 16-byte piece i of row r is stored at piece i ^ (r & 7)
+                const uint32_t row = row_s + (uint32_t)(sw * kWStageBytes);
+                const uint32_t col = col0 + (uint32_t)((q * SKB + part * VKB) * kASlotCols);
+                ok = wait_warp<20>(empty_a(q), ((sti / C::STAGES) & 1u) ^ 1u, abort_flag);
+                if (!ok)
+                    break;
+                tcgen05_fence_after();
+                // Half a k-block at a time: raw bytes -> 32 fp16 (q - zp) * scale in k order (register i holds k = 2i in its
+                // low half and k = 2i + 1 in its high half).  (A loop: unrolled over the visit, a fifth of the issue slots
+                // went to instruction fetch.)
+#pragma unroll 1
+                for (int hb = 0; hb < 2 * nkb; hb++)
+                {
+                    constexpr int NV = RAW_BYTES / 32;
+                    uint4 raw[NV];
 #pragma unroll
                     for (int v = 0; v < NV; v++)
+                        raw[v] = lds128(row + (uint32_t)((((2 * in_chunk + hb) * NV + v) ^ (r & 7)) * 16));
+                    const bool second = !ONE_GROUP && hb >= 2;
+                    const uint32_t sraw = second ? s_now[NP - 1] : s_now[0], zraw = second ? z_now[NP - 1] : z_now[0];
+                    const uint32_t zq = WBITS == 4 ? (zraw >> (4 * ((second ? g_now[NP - 1] : g_now[0]) & 1))) & 0xFu : zraw;
+                    const __half2 from_f32 = __float2half2_rn(__uint_as_float(sraw));
+                    const uint32_t s2 = p.scale_f32 ? *reinterpret_cast<const uint32_t*>(&from_f32) : __byte_perm(sraw, 0u, 0x1010);
+                    const __half2 scale2 = *reinterpret_cast<const __half2*>(&s2);
+                    uint32_t a[16];
+                    if (WBITS == 4)
                     {
-                        const uint32_t w4[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
+                        const uint32_t zc = (0x6400u | zq) | ((0x5400u | (zq << 4)) << 16); // (1024 + zp, 64 + zp)
+                        const uint32_t w4[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
 #pragma unroll
                         for (int wi = 0; wi < 4; wi++)
 #pragma unroll
@@ -497,331 +721,327 @@ __global__ void __launch_bounds__(Cfg<WBITS, BXV>::THREADS, 1)
                                 uint32_t t = __byte_perm(w4[wi], 0u, 0x1111u * b);
                                 asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(t) : "r"(t), "n"(0x00F0000Fu), "n"(0x54006400u));
                                 __half2 h = __hsub2(*reinterpret_cast<__half2*>(&t), *reinterpret_cast<const __half2*>(&zc));
-                                h = __hmul2(h, s2);
-                                a[(v * 4 + wi) * 4 + b] = *reinterpret_cast<uint32_t*>(&h);
+                                h = __hmul2(h, scale2);
+                                a[wi * 4 + b] = *reinterpret_cast<uint32_t*>(&h);
                             }
-                    }
-                }
-                else
-                {
-                    const uint32_t zc = (0x6400u | zq) * 0x00010001u; // 1024 + zp in both halves
-#pragma unroll
-                    for (int v = 0; v < NV; v++)
-                    {
-                        const uint32_t w4[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
-#pragma unroll
-                        for (int wi = 0; wi < 4; wi++)
-#pragma unroll
-                            for (int b = 0; b < 2; b++)
-                            {
-                                uint32_t t = __byte_perm(w4[wi], 0x64646464u, b ? 0x4342 : 0x4140); // 1024 + (b0, b1)
-                                __half2 h = __hsub2(*reinterpret_cast<__half2*>(&t), *reinterpret_cast<const __half2*>(&zc));
-                                h = __hmul2(h, s2);
-                                a[(v * 4 + wi) * 2 + b] = *reinterpret_cast<uint32_t*>(&h);
-                            }
-                    }
-                }
-                // hand the converted k-block to the tensor core: wait for the A stage, store, publish
-                const int rel = kb - sg.kb0;
-                const uint32_t prv = pr_base + (uint32_t)(rel >> 1);
-                const int pq = prv % C::PAIRS, sa = 2 * pq + (rel & 1);
-                // (the vote brings the warp's lanes back together: each polled on its own and may have left the loop
-                // on a different round, and the tensor-memory store below is a warp-wide instruction that every
-                // lane must execute in the same issue)
-                if (!__all_sync(0xffffffffu, wait_or_abort(empty(pq), ((prv / C::PAIRS) & 1u) ^ 1u, abort_flag)))
-                    return false;
-                tcgen05_fence_after();
-                tmem_st_32x32(tmem_base + lane_addr + (uint32_t)(C::A_COL0 + sa * C::A_STAGE_COLS), a);
-                tcgen05_wait_st();
-                tcgen05_fence_before();
-                // The raw stage goes back to the copy engine only now: one arrival per k-block read (the tile's last
-                // k-block also stands in for the k-blocks that a short last chunk does not have).  The arrival must
-                // not be issued before the shared-memory loads have delivered, and nothing but an instruction that
-                // needs their data makes an instruction wait for them: the tensor-memory store above consumed every
-                // loaded word.  (Issued right behind the loads, the arrival could pass a load that was queued behind
-                // a burst of global stores; the next chunk then landed first and the load read its bytes.)
-                mbar_arrive_n(empty_w(sw), kb == KB - 1 ? (uint32_t)(C::KB_PER_CHUNK - j) : 1u);
-                // a segment that ends on the first k-block of a pair: its threads also stand in for the second
-                mbar_arrive_n(full(pq), ((rel & 1) == 0 && kb == sg.kb1 - 1) ? 2u : 1u);
-                return true;
-            };
-            // The groups take the k-blocks in turn.  A group's warps sit on different schedulers next to the other
-            // groups' warps, which hide one another's waits: no second register buffer.
-            for (int kb = sg.kb0 + grp; ok && kb < sg.kb1; kb += 2 * C::DQ_GROUPS)
-            {
-                ok = one(kb, pa);
-                if (ok && kb + C::DQ_GROUPS < sg.kb1)
-                    ok = one(kb + C::DQ_GROUPS, pb);
-            }
-            pr_base += (uint32_t)((sg.kb1 - sg.kb0 + 1) >> 1);
-            wc_base += (uint32_t)(sg.c1 - sg.c0);
-            {
-                WorkList<C::KB_PER_CHUNK> ahead = work;
-                Segment nx;
-                asked = ahead.next(p, nx);
-                if (asked)
-                {
-                    const RowParams n_next = row_of(nx.tile);
-                    ask(n_next, nx.kb0 + grp, nx.kb1 - 1, pa);
-                    ask(n_next, nx.kb0 + grp + C::DQ_GROUPS, nx.kb1 - 1, pb);
-                }
-            }
-
-            // -------------------------------------------------------- the segment's accumulator
-            // D holds y transposed (lane = weight row n, column = batch row m): for one m the 32 lanes of a warp
-            // hold 32 consecutive n.  A tile computed by this CTA alone goes through the epilogue to y; a shared
-            // tile's accumulator goes to this CTA's slot in the workspace as fp32, and the CTA that arrives last
-            // at the tile adds the slots in the order of their K ranges and writes y.  Each warp reads its two
-            // 32-column pieces of D with both loads in flight, then lets the MMA thread have the accumulator back.
-            const int n_base = (sg.tile / p.m_tiles) * C::BN, m0 = (sg.tile % p.m_tiles) * C::BX;
-            const int nrow = n_base + r;
-            // 256 columns: two 32-column pieces per warp.  64 columns: one piece for the warps of the first two groups,
-            // none for the others (which only say that they are done with D).
-            static_assert(C::BX / 32 == 2 * C::DQ_GROUPS || C::BX / 32 == C::DQ_GROUPS / 2, "pieces per warp");
-            constexpr bool kWide = C::BX / 32 == 2 * C::DQ_GROUPS;
-            const bool has_piece = kWide || grp < C::BX / 32; // the same for every lane of a warp
-            const int col0 = grp * 32, col1 = (grp + C::DQ_GROUPS) * 32;
-            // With the gate products in y, those of the first piece are asked for before the accumulator is ready.
-            const float bias = (p.has_bias && nrow < p.N) ? __ldg(p.bias + nrow) : 0.f;
-            const bool gated = GATED && sg.whole;
-            uint32_t gb[GATED ? 32 : 1] = {};
-            // (rows and columns past the edge read the last valid ones: plain loads whose results nothing touches
-            // until the values are needed)
-            auto ask_gates = [&](int col) {
-                if (GATED && gated)
-                {
-                    const int nn = min(nrow, p.N - 1);
-                    if (p.y_f32)
-                    {
-#pragma unroll
-                        for (int jx = 0; jx < (GATED ? 32 : 1); jx++)
-                            gb[jx] = static_cast<const uint32_t*>(p.y)[(size_t)min(m0 + col + jx, p.M - 1) * p.N + nn];
                     }
                     else
                     {
+                        const uint32_t zc = (0x6400u | zq) * 0x00010001u; // 1024 + zp in both halves
 #pragma unroll
-                        for (int jx = 0; jx < (GATED ? 32 : 1); jx++)
-                            gb[jx] = static_cast<const unsigned short*>(p.y)[(size_t)min(m0 + col + jx, p.M - 1) * p.N + nn];
+                        for (int v = 0; v < NV; v++)
+                        {
+                            const uint32_t w4[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
+#pragma unroll
+                            for (int wi = 0; wi < 4; wi++)
+#pragma unroll
+                                for (int b = 0; b < 2; b++)
+                                {
+                                    uint32_t t = __byte_perm(w4[wi], 0x64646464u, b ? 0x4342 : 0x4140); // 1024 + (b0, b1)
+                                    __half2 h = __hsub2(*reinterpret_cast<__half2*>(&t), *reinterpret_cast<const __half2*>(&zc));
+                                    h = __hmul2(h, scale2);
+                                    a[(v * 4 + wi) * 2 + b] = *reinterpret_cast<uint32_t*>(&h);
+                                }
+                        }
                     }
+                    tmem_st_32x16(col + (uint32_t)(hb * 16), a);
                 }
-            };
-            if (!dep_waited)
-            {
-                asm volatile("griddepcontrol.wait;" ::: "memory"); // y, the addend and the workspace are touched from here on
-                dep_waited = true;
+                tcgen05_wait_st();
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                {
+                    mbar_arrive_cluster(full0 + 8u * q);
+                    // The raw stage goes back to the copy engine only now: the arrival must not be issued before the
+                    // shared-memory loads have delivered, and nothing but an instruction that needs their data makes an
+                    // instruction wait for them: the tensor-memory stores above consumed every loaded word.  (One arrival
+                    // per k-block, also for those that a short last chunk does not have.)
+                    if (chunk < sg.c1 - sg.c0)
+                        mbar_arrive_n_relaxed(empty_w(sw), SKB == 2 && kb + VKB >= KB ? (uint32_t)(KBC - in_chunk) : (uint32_t)VKB);
+                }
             }
-            if (has_piece)
-                ask_gates(col0);
-            // (a vote again: the tensor-memory loads below are warp-wide instructions)
-            ok = __all_sync(0xffffffffu, ok && wait_or_abort(acc_full, si & 1u, abort_flag));
+            wc_base += (uint32_t)(sg.c1 - sg.c0);
+            st_base += (uint32_t)n_st;
+        }
+    }
+    else if (warp < C::X_WARP)
+    {
+        // ------------------------------------------------------------ epilogue
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::EPI_REGS));
+        // D holds y transposed (lane = weight row n, column = batch row m): for one m the 32 lanes of a warp hold 32
+        // consecutive n.  Warps 4h .. 4h + 3 take half h of the columns, 16 at a time.
+        // With more than 128 batch rows a tile there is one accumulator, and the tensor core waits until it has been read:
+        // fp16 results are therefore finished and packed first (up to 64 registers; the gates they are multiplied with have
+        // been waiting in the same registers), D is handed back, and the stores follow beside the next tile.  (Storing piece
+        // by piece held D for 14000 clocks of a tile's 33000; drained like this it is 1700.)
+        const int ew = warp - C::DQ_WARPS, half = ew >> 2;
+        const int r = (ew & 3) * 32 + lane;
+        const uint32_t lane_addr = (uint32_t)((ew & 3) * 32) << 16;
+        const int col_mid = C::EPI_WARPS == 4 ? p.bx : (((p.bx >> 4) + 1) >> 1) << 4;
+        const int col_begin = half == 0 ? 0 : col_mid, col_end = half == 0 ? col_mid : p.bx;
+        const int slot_floats = p.bx * kBN;
+        bool ok = true;
+        uint32_t si = 0;
+        asm volatile("griddepcontrol.wait;" ::: "memory"); // y, the addend and the workspace are touched from here on
+        if (p.ksplit > 1)
+            ok = false; // (below)
+        while (ok && work.next(p, sg))
+        {
+            const uint32_t b = acc_bufs == 2 ? (si & 1u) : 0u, use = acc_bufs == 2 ? si >> 1 : si;
             si++;
+            const int n_base = (sg.tile / p.m_tiles) * (2 * kBN) + (int)rank * kBN, m0 = (sg.tile % p.m_tiles) * p.bx;
+            const int n = n_base + r;
+            const bool row_ok = n < p.N;
+            const int m_end = min(p.bx, p.M - m0); // columns that exist
+            const float bias = p.has_bias && row_ok ? __ldg(p.bias + n) : 0.f;
+            const bool gated = sg.set == 1 && sg.whole;
+            const uint32_t d_addr = tmem_base + lane_addr + b * 128u;
+            const long long U = (long long)p.tiles * p.sets * p.cpt;
+            const int G = (int)(gridDim.x >> 1);
+            auto release = [&] { // this warp's last read of D: a later segment may overwrite it
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive_cluster(map_to_rank(acc_empty(b), even));
+            };
+            const int cols = row_ok ? min(m_end, col_end) - col_begin : 0; // this thread's columns that exist
+            const size_t at0 = (size_t)(m0 + col_begin) * p.N + n;
+            const bool packed = sg.whole && !p.y_f32 && !p.has_addend;
+            uint32_t pk[C::PACKED]; // two columns each
+            if (packed && gated)
+            {
+                const unsigned short* g = static_cast<const unsigned short*>(p.y) + at0;
+                const uint32_t step = held(2u * (uint32_t)p.N);
+#pragma unroll
+                for (int i = 0; i < C::PACKED / 8; i++) // sixteen loads in flight
+                {
+                    uint32_t lo[8], hi[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                    {
+                        lo[j] = 16 * i + 2 * j < cols ? (uint32_t)*g : 0u;
+                        g = reinterpret_cast<const unsigned short*>(reinterpret_cast<const char*>(g) + step);
+                        hi[j] = 16 * i + 2 * j + 1 < cols ? (uint32_t)*g : 0u;
+                        g = reinterpret_cast<const unsigned short*>(reinterpret_cast<const char*>(g) + step);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        pk[8 * i + j] = lo[j] | (hi[j] << 16);
+                }
+            }
+            ok = wait_warp<100>(acc_full(b), use & 1u, abort_flag);
             if (!ok)
                 break;
             tcgen05_fence_after();
-            if (sg.whole)
+            if (col_begin == col_end)
+                release();
+            else if (packed)
             {
-                if constexpr (kWide)
-                {
-                    uint32_t d[32];
-                    tmem_ld_32x32(tmem_base + lane_addr + (uint32_t)col0, d);
-                    tcgen05_wait_ld();
-                    if (nrow < p.N)
-                    {
-    #pragma unroll
-                        for (int jx = 0; jx < 32; jx++)
-                            if (m0 + col0 + jx < p.M)
-                                store_value(p, m0 + col0 + jx, nrow, __uint_as_float(d[jx]), gated, gate_value(p, gb[GATED ? jx : 0]), bias);
-                    }
-                    ask_gates(col1);
-                    tmem_ld_32x32(tmem_base + lane_addr + (uint32_t)col1, d);
-                    tcgen05_wait_ld();
-                    tcgen05_fence_before();
-                    mbar_arrive(acc_empty); // this thread's last read of D: the next segment may overwrite it
-                    if (nrow < p.N)
-                    {
-    #pragma unroll
-                        for (int jx = 0; jx < 32; jx++)
-                            if (m0 + col1 + jx < p.M)
-                                store_value(p, m0 + col1 + jx, nrow, __uint_as_float(d[jx]), gated, gate_value(p, gb[GATED ? jx : 0]), bias);
-                    }
-                }
-                else
-                {
-                    if (has_piece)
-                    {
-                        uint32_t d[32];
-                        tmem_ld_32x32(tmem_base + lane_addr + (uint32_t)col0, d);
-                        tcgen05_wait_ld();
-                        tcgen05_fence_before();
-                        mbar_arrive(acc_empty);
-                        if (nrow < p.N)
-                        {
+                // (whether gates are folded in is decided outside the loop: a choice per value costs a branch per value, and
+                // the two or three warps of a scheduler do not hide it)
+                auto drain = [&](auto with_gates) {
 #pragma unroll
-                            for (int jx = 0; jx < 32; jx++)
-                                if (m0 + col0 + jx < p.M)
-                                    store_value(p, m0 + col0 + jx, nrow, __uint_as_float(d[jx]), gated, gate_value(p, gb[GATED ? jx : 0]), bias);
+                    for (int i = 0; i < C::PACKED / 8; i++)
+                        if (col_begin + 16 * i < col_end)
+                        {
+                            uint32_t d[16];
+                            tmem_ld_32x16(d_addr + (uint32_t)(col_begin + 16 * i), d);
+                            tcgen05_wait_ld();
+                            if (col_begin + 16 * i + 16 == col_end)
+                                release();
+#pragma unroll
+                            for (int j = 0; j < 8; j++)
+                            {
+                                float lo = __uint_as_float(d[2 * j]), hi = __uint_as_float(d[2 * j + 1]);
+                                if constexpr (decltype(with_gates)::value)
+                                    lo *= silu(gate_of_half(pk[8 * i + j] & 0xFFFFu)), hi *= silu(gate_of_half(pk[8 * i + j] >> 16));
+                                const __half2 h = __floats2half2_rn(lo + bias, hi + bias);
+                                pk[8 * i + j] = *reinterpret_cast<const uint32_t*>(&h);
+                            }
                         }
-                    }
-                    else
-                    {
-                        tcgen05_fence_before();
-                        mbar_arrive(acc_empty);
-                    }
+                };
+                if (gated)
+                    drain(std::true_type{});
+                else
+                    drain(std::false_type{});
+                unsigned short* y = static_cast<unsigned short*>(p.y) + at0;
+                const uint32_t step = held(2u * (uint32_t)p.N);
+#pragma unroll
+                for (int j = 0; j < C::PACKED; j++)
+                {
+                    if (2 * j < cols)
+                        *y = (unsigned short)pk[j];
+                    y = reinterpret_cast<unsigned short*>(reinterpret_cast<char*>(y) + step);
+                    if (2 * j + 1 < cols)
+                        *y = (unsigned short)(pk[j] >> 16);
+                    y = reinterpret_cast<unsigned short*>(reinterpret_cast<char*>(y) + step);
                 }
             }
             else
             {
-                const long long U = (long long)p.tiles * p.cpt;
-                const int G = (int)gridDim.x;
-                const int c_first = cta_of_unit((long long)sg.tile * p.cpt, U, G);
-                const int c_last = cta_of_unit((long long)(sg.tile + 1) * p.cpt - 1, U, G);
-                const uint32_t pieces = (uint32_t)(c_last - c_first + 1);
-                float* mine = p.slots + (size_t)slot_of((int)blockIdx.x, sg.tile, U, G, p.cpt) * C::SLOT_FLOATS;
-                if constexpr (kWide)
+                float* const mine = p.slots + (size_t)(sg.whole ? 0 : slot_of(p, (int)(blockIdx.x >> 1), (int)rank, sg.tile, sg.set, U, G)) * slot_floats;
+                for (int col = col_begin; col < col_end; col += 16)
                 {
-                    uint32_t d[32];
-                    tmem_ld_32x32(tmem_base + lane_addr + (uint32_t)col0, d);
+                    uint32_t d[16];
+                    tmem_ld_32x16(d_addr + (uint32_t)col, d);
                     tcgen05_wait_ld();
-#pragma unroll
-                    for (int jx = 0; jx < 32; jx++)
-                        mine[(size_t)(col0 + jx) * C::BN + r] = __uint_as_float(d[jx]);
-                    tmem_ld_32x32(tmem_base + lane_addr + (uint32_t)col1, d);
-                    tcgen05_wait_ld();
-                    tcgen05_fence_before();
-                    mbar_arrive(acc_empty);
-#pragma unroll
-                    for (int jx = 0; jx < 32; jx++)
-                        mine[(size_t)(col1 + jx) * C::BN + r] = __uint_as_float(d[jx]);
-                }
-                else if (has_piece)
-                {
-                    uint32_t d[32];
-                    tmem_ld_32x32(tmem_base + lane_addr + (uint32_t)col0, d);
-                    tcgen05_wait_ld();
-                    tcgen05_fence_before();
-                    mbar_arrive(acc_empty);
-#pragma unroll
-                    for (int jx = 0; jx < 32; jx++)
-                        mine[(size_t)(col0 + jx) * C::BN + r] = __uint_as_float(d[jx]);
-                }
-                else
-                {
-                    tcgen05_fence_before();
-                    mbar_arrive(acc_empty);
-                }
-                __threadfence();
-                mbar_arrive(part_done);
-                if (warp == 0)
-                {
-                    // The whole warp waits (a lane spinning on its own while its warp-mates spin on another barrier
-                    // starves), then one lane takes the ticket.
-                    const bool landed = __all_sync(0xffffffffu, wait_or_abort(part_done, npart & 1u, abort_flag));
-                    if (lane == 0 && landed)
+                    if (col + 16 == col_end)
+                        release();
+                    if (!sg.whole)
                     {
-                        __threadfence(); // the partial sums of all threads before the ticket
-                        const uint32_t before = atomicAdd(p.counters + sg.tile, 1u);
-                        __threadfence();
-                        if (before == pieces - 1)
-                            p.counters[sg.tile] = 0u; // leave the counter zeroed for the next call
-                        *ticket_slot = before;
-                        mbar_arrive(ticket_ready);
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            mine[(size_t)(col + j) * kBN + r] = __uint_as_float(d[j]);
+                        continue;
                     }
-                    __syncwarp();
-                }
-                ok = wait_or_abort(ticket_ready, npart & 1u, abort_flag);
-                npart++;
-                if (!ok)
-                    break;
-                if (*ticket_slot == pieces - 1)
-                {
-                    // Last to arrive: add the tile's slots in the order of their K ranges and write y.  Nothing ties
-                    // a thread to a tensor-memory lane here, so every thread takes four neighbouring weight rows of
-                    // one batch row at a time (16-byte loads), four such positions and two slots per round trip
-                    // to L2.
-                    __threadfence();
-                    constexpr int NT = C::DQ_WARPS * 32;        // threads at work
-                    constexpr int Q = C::SLOT_FLOATS / 4;       // float4 per slot
-                    static_assert(Q % (NT * 4) == 0, "four positions per thread and pass");
-                    const bool vec = (p.N % 4 == 0) && !p.has_addend && !GATED &&
-                                     (reinterpret_cast<uintptr_t>(p.y) & 15u) == 0;
-                    for (int q0 = warp * 32 + lane; q0 < Q; q0 += NT * 4)
+                    // fp32 results, or an addend: in pieces
+                    const int left = row_ok ? m_end - col : 0;
+                    const size_t at = (size_t)(m0 + col) * p.N + n;
+                    float v[16], e[16];
+                    if (p.y_f32)
                     {
-                        float4 v[4];
+                        const float* other = p.has_addend ? reinterpret_cast<const float*>(p.bias) : static_cast<const float*>(p.y);
 #pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        for (int c = c_first; c <= c_last; c += 2) // fixed order: repeatable
-                        {
-                            const bool two = c + 1 <= c_last;
-                            const float4* s0 = reinterpret_cast<const float4*>(
-                                p.slots + (size_t)slot_of(c, sg.tile, U, G, p.cpt) * C::SLOT_FLOATS);
-                            const float4* s1 = reinterpret_cast<const float4*>(
-                                p.slots + (size_t)slot_of(two ? c + 1 : c, sg.tile, U, G, p.cpt) * C::SLOT_FLOATS);
-                            float4 a0[4], a1[4];
+                        for (int j = 0; j < 16; j++)
+                            e[j] = (gated || p.has_addend) && j < left ? other[at + (size_t)j * p.N] : 0.f;
+                    }
+                    else
+                    {
 #pragma unroll
-                            for (int j = 0; j < 4; j++)
-                            {
-                                a0[j] = __ldcg(s0 + q0 + j * NT);
-                                a1[j] = __ldcg(s1 + q0 + j * NT);
-                            }
+                        for (int j = 0; j < 16; j++)
+                            e[j] = p.has_addend && j < left ? __half2float(reinterpret_cast<const __half*>(p.bias)[at + (size_t)j * p.N]) : 0.f;
+                    }
 #pragma unroll
-                            for (int j = 0; j < 4; j++)
-                            {
-                                v[j].x += a0[j].x, v[j].y += a0[j].y, v[j].z += a0[j].z, v[j].w += a0[j].w;
-                                if (two)
-                                    v[j].x += a1[j].x, v[j].y += a1[j].y, v[j].z += a1[j].z, v[j].w += a1[j].w;
-                            }
-                        }
+                    for (int j = 0; j < 16; j++)
+                        v[j] = gated ? __uint_as_float(d[j]) * silu(e[j]) : __uint_as_float(d[j]) + (bias + e[j]);
+                    if (p.y_f32)
+                    {
+                        float* y = static_cast<float*>(p.y) + at;
 #pragma unroll
-                        for (int j = 0; j < 4; j++)
-                        {
-                            const int f = (q0 + j * NT) * 4;    // float index in the slot: [batch row][weight row]
-                            const int m = m0 + f / C::BN, n4 = n_base + f % C::BN;
-                            if (m >= p.M)
-                                continue;
-                            float o[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-                            if (vec && n4 + 3 < p.N)
-                            {
-                                if (p.has_bias)
-                                {
+                        for (int j = 0; j < 16; j++)
+                            if (j < left)
+                                y[(size_t)j * p.N] = v[j];
+                    }
+                    else
+                    {
+                        __half* y = static_cast<__half*>(p.y) + at;
 #pragma unroll
-                                    for (int e = 0; e < 4; e++)
-                                        o[e] += __ldg(p.bias + n4 + e);
-                                }
-                                const size_t at = (size_t)m * p.N + n4;
-                                if (p.y_f32)
-                                    *reinterpret_cast<float4*>(static_cast<float*>(p.y) + at) = make_float4(o[0], o[1], o[2], o[3]);
-                                else
-                                {
-                                    const __half2 h0 = __floats2half2_rn(o[0], o[1]), h1 = __floats2half2_rn(o[2], o[3]);
-                                    uint2 pk;
-                                    pk.x = *reinterpret_cast<const uint32_t*>(&h0), pk.y = *reinterpret_cast<const uint32_t*>(&h1);
-                                    *reinterpret_cast<uint2*>(static_cast<__half*>(p.y) + at) = pk;
-                                }
-                            }
-                            else
-                            {
-#pragma unroll
-                                for (int e = 0; e < 4; e++)
-                                    if (n4 + e < p.N)
-                                        store_value(p, m, n4 + e, o[e], GATED,
-                                                    GATED ? gate_value(p, gate_bits(p, m, n4 + e)) : 0.f,
-                                                    p.has_bias ? __ldg(p.bias + n4 + e) : 0.f);
-                            }
-                        }
+                        for (int j = 0; j < 16; j++)
+                            if (j < left)
+                                y[(size_t)j * p.N] = __float2half_rn(v[j]);
                     }
                 }
             }
+            if (!sg.whole && sg.last)
+            {
+                // All of this pair's sums of the tile are in its slots: take a ticket; the last pair to arrive adds the
+                // slots in the order of their K ranges and writes y.
+                const int per_tile = p.sets * p.cpt;
+                const int c_first = pair_of_unit((long long)sg.tile * per_tile, U, G);
+                const int c_last = pair_of_unit((long long)(sg.tile + 1) * per_tile - 1, U, G);
+                // the pairs with a part of the first and of the last weight set (the same one when there is one)
+                const int set_first[2] = {c_first, p.sets == 1 ? c_first : pair_of_unit((long long)sg.tile * per_tile + p.cpt, U, G)};
+                const int set_last[2] = {p.sets == 1 ? c_last : pair_of_unit((long long)sg.tile * per_tile + p.cpt - 1, U, G), c_last};
+                __threadfence();
+                asm volatile("bar.sync %0, %1;" ::"n"(kEpiBarrier), "n"(C::EPI_WARPS * 32) : "memory");
+                if (ew == 0 && lane == 0)
+                {
+                    const uint32_t before = atomicAdd(p.counters + 2 * sg.tile + rank, 1u);
+                    if (before == (uint32_t)(c_last - c_first))
+                        p.counters[2 * sg.tile + rank] = 0u; // leave the counter zeroed for the next call
+                    *ticket_slot = before;
+                }
+                // every weight set's slots in the order of their K ranges, once, while the ticket is on its way: the 64-bit
+                // divisions behind a slot's place are far dearer than the additions
+                for (int set = 0; set < p.sets; set++)
+                    for (int i = (ew - 1) * 32 + lane; i >= 0 && i <= set_last[set] - set_first[set]; i += (C::EPI_WARPS - 1) * 32)
+                        slot_list[set * kMaxPairs + i] = slot_of(p, set_first[set] + i, (int)rank, sg.tile, set, U, G);
+                asm volatile("bar.sync %0, %1;" ::"n"(kEpiBarrier), "n"(C::EPI_WARPS * 32) : "memory");
+                if (*ticket_slot == (uint32_t)(c_last - c_first))
+                {
+                    __threadfence();
+                    auto load = [&](int set, int part, int row) {
+                        return load_part(reinterpret_cast<const float4*>(p.slots + (size_t)slot_list[set * kMaxPairs + part] * slot_floats) +
+                                         row * (kBN / 4) + lane);
+                    };
+                    const int n0 = set_last[0] - set_first[0] + 1, n1 = set_last[1] - set_first[1] + 1;
+                    if (p.sets == 2)
+                        add_parts<2, 4, C::EPI_WARPS>(p, load, n0, n1, n_base + 4 * lane, m0, m_end, ew);
+                    else
+                        add_parts<1, 4, C::EPI_WARPS>(p, load, n0, 0, n_base + 4 * lane, m0, m_end, ew);
+                }
+                // (nobody touches ticket_slot or slot_list again before everybody has passed the next tile's first barrier,
+                // except this tile's slow readers: meet once more)
+                asm volatile("bar.sync %0, %1;" ::"n"(kEpiBarrier), "n"(C::EPI_WARPS * 32) : "memory");
+            }
+        }
+        if (p.ksplit > 1)
+        {
+            // The cluster's pairs have each multiplied their part of K (with two weight sets: both, one per accumulator).
+            // Every CTA sends its sums of each peer's batch rows to that peer's shared memory - where the rings were, free
+            // once the peer has multiplied - and finishes its own batch rows.
+            bool fine = true;
+            for (int set = 0; set < p.sets; set++)
+                fine = fine && wait_warp<100>(acc_full(set), 0u, abort_flag);
+            tcgen05_fence_after();
+            const int pair = blockIdx.x >> 1, part = pair % p.ksplit, tile = pair / p.ksplit;
+            if (fine && ew == 0 && lane < p.ksplit)
+                mbar_arrive_cluster(map_to_rank(peers_ready, 2u * (uint32_t)lane + rank));
+            fine = fine && wait_warp<0>(peers_ready, 0u, abort_flag);
+            const uint32_t buf = smem_u32(xs); // [set][part][batch row of the slice][128] floats
+            if (fine)
+            {
+                for (int set = 0; set < p.sets; set++)
+                    for (int col = col_begin; col < col_end; col += 16)
+                    {
+                        const int dst = col / p.slice; // (slices are multiples of 16 batch rows)
+                        uint32_t d[16];
+                        tmem_ld_32x16(tmem_base + lane_addr + (uint32_t)(set * 128 + col), d);
+                        const uint32_t to = map_to_rank(buf + (uint32_t)(((set * p.ksplit + part) * p.slice + col - dst * p.slice) * kBN + r) * 4u,
+                                                        2u * (uint32_t)dst + rank);
+                        tcgen05_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to + (uint32_t)(j * kBN * 4)), "r"(d[j]) : "memory");
+                    }
+                __syncwarp();
+                if (lane < p.ksplit)
+                    mbar_arrive_cluster_release(map_to_rank(parts_here, 2u * (uint32_t)lane + rank));
+                bool here = false;
+                for (uint32_t i = 0; i < kGemmSpin && !here && !*abort_flag; i++)
+                    here = mbar_try_wait_cluster(parts_here, 0u);
+                fine = __all_sync(0xffffffffu, here);
+            }
+            if (fine)
+            {
+                const int n_base = (tile / p.m_tiles) * (2 * kBN) + (int)rank * kBN, m0 = (tile % p.m_tiles) * p.bx + part * p.slice;
+                const int rows = min(min(p.slice, p.bx - part * p.slice), p.M - m0);
+                auto load = [&](int set, int pt, int row) {
+                    const uint4 v = lds128(buf + (uint32_t)(((set * p.ksplit + pt) * p.slice + row) * kBN + 4 * lane) * 4u);
+                    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+                };
+                if (rows > 0)
+                {
+                    if (p.sets == 2)
+                        add_parts<2, 4, C::EPI_WARPS>(p, load, p.ksplit, p.ksplit, n_base + 4 * lane, m0, rows, ew);
+                    else
+                        add_parts<1, 4, C::EPI_WARPS>(p, load, p.ksplit, 0, n_base + 4 * lane, m0, rows, ew);
+                }
+            }
+            else
+                *abort_flag = 1;
         }
     }
 
     // ---------------------------------------------------------------- tear-down
     tcgen05_fence_before();
     __syncthreads();
-    if (warp == MMA_WARP)
+    cluster_arrive(); // nobody of the pair reaches into the other's shared or tensor memory any more
+    cluster_wait();
+    if (warp == C::MMA_WARP)
     {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, C::TMEM_COLS);
+        tmem_dealloc(tmem_base, kTmemCols);
     }
     if (tid == 0 && *abort_flag)
         atomicExch(p.status, 1);
@@ -871,10 +1091,11 @@ __global__ void __launch_bounds__(256) prep_activations_kernel(const void* x, co
     }
 }
 
-template <int WBITS, bool GATED, int BXV>
-cudaError_t launch(const GemmParams& p, const CUtensorMap& tx, const CUtensorMap& tw, int grid, cudaStream_t stream)
+template <int WBITS, bool ONE_GROUP, bool SMALL>
+cudaError_t launch(const GemmParams& p, const CUtensorMap& tx, const CUtensorMap& tw0, const CUtensorMap& tw1, int pairs,
+                   cudaStream_t stream)
 {
-    using C = Cfg<WBITS, BXV>;
+    using C = Cfg<SMALL>;
     static bool configured[nnf::kMaxDevices] = {}; // the attribute belongs to the device that is current
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -884,24 +1105,35 @@ cudaError_t launch(const GemmParams& p, const CUtensorMap& tx, const CUtensorMap
         return cudaErrorInvalidDevice;
     if (!configured[dev])
     {
-        e = cudaFuncSetAttribute(dq_gemm_kernel<WBITS, GATED, BXV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)C::SMEM_BYTES);
+        e = cudaFuncSetAttribute(dq_gemm_kernel<WBITS, ONE_GROUP, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
         if (e != cudaSuccess)
             return e;
         configured[dev] = true;
     }
     (void)cudaGetLastError();
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(C::THREADS);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    nnf::overlap_attribute(attr, &cfg.numAttrs);
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 2u * (unsigned)p.ksplit;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs].val.clusterDim.z = 1;
+    cfg.numAttrs++;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<WBITS, GATED, BXV>, p, tx, tw);
+    return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<WBITS, ONE_GROUP, SMALL>, p, tx, tw0, tw1);
+}
+
+template <bool SMALL>
+cudaError_t dispatch(int wbits, bool one_group, const GemmParams& p, const CUtensorMap& tx, const CUtensorMap& tw0,
+                     const CUtensorMap& tw1, int pairs, cudaStream_t stream)
+{
+    if (wbits == 4)
+        return one_group ? launch<4, true, SMALL>(p, tx, tw0, tw1, pairs, stream) : launch<4, false, SMALL>(p, tx, tw0, tw1, pairs, stream);
+    return one_group ? launch<8, true, SMALL>(p, tx, tw0, tw1, pairs, stream) : launch<8, false, SMALL>(p, tx, tw0, tw1, pairs, stream);
 }
 } // namespace
 
@@ -918,11 +1150,11 @@ static bool needs_prepass(const nnf_b200_linear_desc& d)
     return d.x_dtype == NNF_B200_F32 || d.prologue == NNF_B200_PROLOGUE_RMSNORM;
 }
 
-// How a launch is laid out: persistent CTAs share tiles * chunks-per-tile units of work evenly; the workspace holds
-// the arrival counters of the tiles, two partial-sum slots per CTA and, when needed, the fp16 copy of x.
+// How a launch is laid out (see the top of this file); the workspace holds the arrival counters of the tiles' halves,
+// partial-sum slots of every CTA and, when needed, the fp16 copy of x.
 struct GemmLayout
 {
-    int bx, m_tiles, n_tiles, tiles, cpt, grid, whole_tiles;
+    int bx, m_tiles, n_tiles, tiles, sets, cpt, pairs, whole_tiles, ksplit;
     size_t counter_bytes, slot_bytes, prepass_bytes;
     size_t total() const { return counter_bytes + slot_bytes + prepass_bytes; }
 };
@@ -930,29 +1162,52 @@ struct GemmLayout
 static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
 {
     GemmLayout L{};
-    L.bx = d.M <= 64 ? 64 : 256; // a narrow batch tile for small batches
-    L.m_tiles = (d.M + L.bx - 1) / L.bx;
-    L.n_tiles = (d.N + 127) / 128;
-    L.tiles = L.m_tiles * L.n_tiles;
+    const int sms = ctx ? ctx->sm_count : 148;
+    const int max_pairs = std::min(std::max(1, sms / 2), kMaxPairs);
+    // clusters of 1, 2, 3 and 4 pairs that 148 SMs hold at once (the occupancy calculator's answers; a launch of more of
+    // them would only take longer)
+    const int held[5] = {0, max_pairs, max_pairs * 33 / 74, max_pairs * 22 / 74, max_pairs * 15 / 74};
+    L.n_tiles = (d.N + 255) / 256;
+    L.sets = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL ? 2 : 1;
     const int kb_per_chunk = d.w_bits == 4 ? 4 : 2;
     L.cpt = (d.K / 64 + kb_per_chunk - 1) / kb_per_chunk;
-    const long long units = (long long)L.tiles * L.cpt;
-    const int sms = ctx ? ctx->sm_count : 148;
-    // Shares cut anywhere (tiles at the seams cost a partial sum in the workspace, a ticket and a final addition:
-    // about 30 k-blocks' worth of time on top of the 8 of an epilogue) or at tile boundaries only (the CTA with the
-    // most tiles sets the time): whichever the estimate, in k-block times, favours.
-    const double kb = d.K / 64.0;
-    // (the same estimate serves the narrow tile: with a lower price for its smaller shared tiles the up projection
-    // at 17 to 64 batch rows was cut across all SMs and took 24.9 us instead of 23.5)
-    const double t_split = (double)L.tiles * kb / sms + 8.0 + 30.0;
-    const double t_whole = (double)((L.tiles + sms - 1) / sms) * (kb + 8.0);
-    L.whole_tiles = t_whole <= t_split;
-    if (L.whole_tiles)
-        L.grid = L.tiles < sms ? L.tiles : sms;
-    else
-        L.grid = (int)(units < sms ? units : sms);
-    L.counter_bytes = ((size_t)L.tiles * sizeof(uint32_t) + 255) / 256 * 256;
-    L.slot_bytes = (size_t)2 * L.grid * 128 * L.bx * sizeof(float); // two slots of one fp32 tile per CTA
+    // Batch tiles of equal width and how K is shared, by an estimate in microseconds fitted to 20 shapes of 32 to 4096 batch
+    // rows times every choice.  What a k-block takes: up to 128 batch rows the conversion of the weights (and handing it
+    // over), 0.21 to 0.24; above, where two groups of warps convert, 0.31 to 0.345, at 256 rows the tensor core at its
+    // clock under load.  Whole tiles cost whole waves.  Partial sums through the workspace (store, ticket, read back) cost
+    // 9 to 26 us, inside a cluster 1 to 4 us.
+    const double kb = (double)d.K / 64.0 * L.sets;
+    double best = 0;
+    const int m_min = (d.M + 255) / 256;
+    for (int mt = m_min; mt <= m_min * 2 + 2 && mt <= (d.M + 15) / 16; mt++)
+    {
+        const int bx = ((d.M + mt - 1) / mt + 15) / 16 * 16;
+        const int m_tiles = (d.M + bx - 1) / bx, tiles = m_tiles * L.n_tiles;
+        const double t_kb = bx <= 128 ? 0.19 + 0.0004 * bx : 0.25 + 0.00037 * bx, out = (double)bx * L.sets;
+        const double tile = kb * t_kb + 0.5 + 3.0 * (L.sets - 1);
+        auto take = [&](double t, int whole, int ksplit) {
+            if (best == 0 || t < best)
+                best = t, L.bx = bx, L.m_tiles = m_tiles, L.whole_tiles = whole, L.ksplit = ksplit;
+        };
+        take(std::ceil((double)tiles / max_pairs) * tile + 0.004 * out, 1, 1);
+        take(std::max((double)tiles / max_pairs, 1.0 / L.cpt) * tile + 6.0 + (tiles < max_pairs ? 0.08 : 0.05) * out, 0, 1);
+        for (int s = 2; s <= 4 && s <= L.cpt; s++)
+            if (tiles <= held[s] && (L.sets == 1 || bx <= 128))
+                take((double)((L.cpt + s - 1) / s) * kb_per_chunk * L.sets * t_kb + 1.0 + 0.008 * out, 0, s);
+    }
+    L.tiles = L.m_tiles * L.n_tiles;
+    const long long units = (long long)L.tiles * L.sets * L.cpt;
+    L.pairs = L.ksplit > 1 ? L.tiles * L.ksplit : (int)std::min<long long>(L.whole_tiles ? L.tiles : units, max_pairs);
+    // Tiles shared through the workspace: counters for both halves of every tile, and slots of 128 x BX for two tiles per CTA
+    // (and weight set).  The size handed out is at least that of 128-row tiles of 64 or 256 batch rows, one counter each,
+    // with two slots per CTA.
+    const bool shared = !L.whole_tiles && L.ksplit == 1;
+    const int wide = d.M <= 64 ? 64 : 256;
+    const long long tiles128 = (long long)((d.M + wide - 1) / wide) * ((d.N + 127) / 128);
+    const long long ctas128 = std::min<long long>(tiles128 * L.cpt, sms);
+    L.counter_bytes = ((size_t)std::max<long long>(shared ? 2ll * L.tiles : 0, tiles128) * sizeof(uint32_t) + 255) / 256 * 256;
+    L.slot_bytes = std::max<size_t>(shared ? (size_t)2 * L.pairs * 2 * L.sets * 128 * L.bx * sizeof(float) : (size_t)0,
+                                    (size_t)2 * ctas128 * 128 * wide * sizeof(float));
     L.prepass_bytes = needs_prepass(d) ? ((size_t)d.M * d.K * sizeof(__half) + 255) / 256 * 256 : 0;
     return L;
 }
@@ -975,10 +1230,10 @@ int gemm_supported(const nnf_b200_ctx*, const nnf_b200_linear_desc& d, std::stri
         *why = "weight rows must be a multiple of 16 bytes";
         return NNF_B200_ENOTSUP;
     }
-    // the kernel counts its units of work (tiles x raw chunks of K) in 32-bit integers
-    const long long tiles = (long long)((d.M + 255) / 256) * ((d.N + 127) / 128);
-    const long long chunks = (d.K / 64 + (d.w_bits == 4 ? 3 : 1)) / (d.w_bits == 4 ? 4 : 2);
-    if (tiles * chunks >= (1ll << 31) || tiles >= (1ll << 30))
+    // the kernel counts its units of work (tiles x weight sets x raw chunks of K) in 32-bit integers
+    const long long tiles = (long long)((d.M + 255) / 256 + 4) * ((d.N + 127) / 128);
+    const long long chunks = 2 * ((d.K / 64 + (d.w_bits == 4 ? 3 : 1)) / (d.w_bits == 4 ? 4 : 2));
+    if (tiles * chunks >= (1ll << 31) || tiles >= (1ll << 29))
     {
         *why = "M * N * K is beyond what one launch counts";
         return NNF_B200_ENOTSUP;
@@ -1015,6 +1270,7 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     }
     const bool silu_mul = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
     const int row_bytes = d.w_bits == 4 ? d.K / 2 : d.K;
+    const bool small = L.bx <= Cfg<true>::MAX_BX;
     GemmParams p{};
     p.y = y;
     p.status = ctx->dev_status;
@@ -1024,53 +1280,52 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     p.zp_row_bytes = d.w_bits == 4 ? (p.G + 1) / 2 : p.G;
     p.y_f32 = d.y_dtype == NNF_B200_F32;
     p.scale_f32 = d.scale_dtype == NNF_B200_F32;
+    p.bx = L.bx;
+    p.x_stages = std::min(Cfg<true>::MAX_X_STAGES, small ? Cfg<true>::X_BYTES / (L.bx * 64 * Cfg<true>::STAGE_KB)
+                                                         : Cfg<false>::X_BYTES / (L.bx * 64 * Cfg<false>::STAGE_KB));
     p.m_tiles = L.m_tiles;
     p.tiles = L.tiles;
+    p.sets = L.sets;
     p.cpt = L.cpt;
     p.whole_tiles = L.whole_tiles;
+    p.ksplit = L.ksplit;
+    p.slice = ((L.bx >> 4) + L.ksplit - 1) / L.ksplit * 16;
+    p.counters = reinterpret_cast<uint32_t*>(ws);
+    p.slots = reinterpret_cast<float*>(ws + L.counter_bytes);
+    p.has_addend = d.epilogue == NNF_B200_EPILOGUE_ADD;
+    p.has_bias = bias != nullptr && !p.has_addend && !silu_mul;
+    p.bias = static_cast<const float*>(bias);
+    const nnf_b200_qweight* sets[2] = {w, silu_mul ? w2 : w};
+    for (int i = 0; i < 2; i++)
+    {
+        p.scale[i] = sets[i]->scale;
+        p.zp[i] = static_cast<const uint8_t*>(sets[i]->zp);
+    }
     p.kbpg_shift = -1;
     for (int sh = 0; sh < 31; sh++)
         if ((p.group / 64) == (1 << sh))
             p.kbpg_shift = sh;
-    p.counters = reinterpret_cast<uint32_t*>(ws);
-    p.slots = reinterpret_cast<float*>(ws + L.counter_bytes);
+    const bool one_group = p.group % 128 == 0 || p.group == d.K;
 
-    // x: fp16 [M][K], boxes of 256 rows x 64 elements (the tensor map is not cached: x moves between calls)
+    // x: fp16 [M][K], boxes of BX/2 rows x 64 elements (the tensor map is not cached: x moves between calls)
     alignas(64) CUtensorMap tx;
     if (!encode_tensor_map_2d(ctx->encode_tiled, &tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)d.K,
-                              (uint64_t)d.M, (uint64_t)d.K * 2, 64, (uint32_t)L.bx, CU_TENSOR_MAP_SWIZZLE_128B))
+                              (uint64_t)d.M, (uint64_t)d.K * 2, 64, (uint32_t)L.bx / 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the activations");
-
-    // SiLU(x . Wg^T) * (x . Wu^T): the gate products go to y first, the second launch folds them in.
-    const int passes = silu_mul ? 2 : 1;
-    for (int pass = 0; pass < passes; pass++)
+    // (copied by value at once: a later lookup may empty the context's cache)
+    alignas(64) CUtensorMap tw[2];
+    for (int i = 0; i < 2; i++)
     {
-        const nnf_b200_qweight* wp = (silu_mul && pass == 1) ? w2 : w;
-        p.scale = wp->scale;
-        p.zp = static_cast<const uint8_t*>(wp->zp);
-        p.has_addend = d.epilogue == NNF_B200_EPILOGUE_ADD;
-        p.has_bias = bias != nullptr && !p.has_addend && !silu_mul;
-        p.bias = static_cast<const float*>(bias);
-        // copied by value at once: a later lookup may empty the context's cache
-        alignas(64) CUtensorMap twv;
-        const CUtensorMap* tw = weight_tensor_map(ctx, wp->wq, d.N, row_bytes, 128, 128);
-        if (!tw)
+        const CUtensorMap* m = weight_tensor_map(ctx, sets[i]->wq, d.N, row_bytes, 128, 128);
+        if (!m)
             return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the weight tensor");
-        twv = *tw;
-        const bool gated = silu_mul && pass == 1;
-        cudaError_t e;
-        if (L.bx == 256)
-            e = d.w_bits == 4
-                    ? (gated ? launch<4, true, 256>(p, tx, twv, L.grid, stream) : launch<4, false, 256>(p, tx, twv, L.grid, stream))
-                    : (gated ? launch<8, true, 256>(p, tx, twv, L.grid, stream) : launch<8, false, 256>(p, tx, twv, L.grid, stream));
-        else
-            e = d.w_bits == 4
-                    ? (gated ? launch<4, true, 64>(p, tx, twv, L.grid, stream) : launch<4, false, 64>(p, tx, twv, L.grid, stream))
-                    : (gated ? launch<8, true, 64>(p, tx, twv, L.grid, stream) : launch<8, false, 64>(p, tx, twv, L.grid, stream));
-        if (e != cudaSuccess)
-            return set_error(ctx, NNF_B200_ECUDA, std::string("dq_gemm launch: ") + cudaGetErrorString(e));
-        ctx->launches++;
+        tw[i] = *m;
     }
+    const cudaError_t e = small ? dispatch<true>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream)
+                                : dispatch<false>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream);
+    if (e != cudaSuccess)
+        return set_error(ctx, NNF_B200_ECUDA, std::string("dq_gemm launch: ") + cudaGetErrorString(e));
+    ctx->launches++;
     return NNF_B200_OK;
 }
 } // namespace nnf
