@@ -40,7 +40,6 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
-#include <type_traits>
 
 #include "nnf_internal.h"
 #include "sm100_ptx.cuh"
@@ -87,7 +86,7 @@ struct Cfg
         1024 + (size_t)X_BYTES + (size_t)W_STAGES * kWStageBytes + BARRIERS * 8 + 64 + 2 * kMaxPairs * sizeof(int);
     // Registers a thread: launched with LAUNCH_REGS each, then the roles take what they need.
     static constexpr int LAUNCH_REGS = SMALL ? 80 : 96;
-    static constexpr int DQ_REGS = SMALL ? 72 : 80, EPI_REGS = SMALL ? 120 : 128, ISSUE_REGS = SMALL ? 72 : 64;
+    static constexpr int DQ_REGS = 72, EPI_REGS = SMALL ? 136 : 144, ISSUE_REGS = SMALL ? 56 : 48;
     static_assert(DQ_GROUPS * DQ_REGS + EPI_WARPS / 4 * EPI_REGS + ISSUE_REGS <= THREADS / 128 * LAUNCH_REGS, "registers the CTA has");
     static_assert(LAUNCH_REGS * THREADS <= 65536, "registers the SM has");
     static_assert(A_COL0 + kASlots * kASlotCols <= kTmemCols, "tensor memory budget");
@@ -771,8 +770,8 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
         // D holds y transposed (lane = weight row n, column = batch row m): for one m the 32 lanes of a warp hold 32
         // consecutive n.  Warps 4h .. 4h + 3 take half h of the columns, 16 at a time.
         // With more than 128 batch rows a tile there is one accumulator, and the tensor core waits until it has been read:
-        // fp16 results are therefore finished and packed first (up to 64 registers; the gates they are multiplied with have
-        // been waiting in the same registers), D is handed back, and the stores follow beside the next tile.  (Storing piece
+        // fp16 results are therefore finished and packed first (up to 64 registers; the gates or the addend that are folded in
+        // have been waiting in the same registers), D is handed back, and the stores follow beside the next tile.  (Storing piece
         // by piece held D for 14000 clocks of a tile's 33000; drained like this it is 1700.)
         const int ew = warp - C::DQ_WARPS, half = ew >> 2;
         const int r = (ew & 3) * 32 + lane;
@@ -806,11 +805,11 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
             };
             const int cols = row_ok ? min(m_end, col_end) - col_begin : 0; // this thread's columns that exist
             const size_t at0 = (size_t)(m0 + col_begin) * p.N + n;
-            const bool packed = sg.whole && !p.y_f32 && !p.has_addend;
+            const bool packed = sg.whole && !p.y_f32;
             uint32_t pk[C::PACKED]; // two columns each
-            if (packed && gated)
+            if (packed && (gated || p.has_addend))
             {
-                const unsigned short* g = static_cast<const unsigned short*>(p.y) + at0;
+                const unsigned short* g = (p.has_addend ? reinterpret_cast<const unsigned short*>(p.bias) : static_cast<const unsigned short*>(p.y)) + at0;
                 const uint32_t step = held(2u * (uint32_t)p.N);
 #pragma unroll
                 for (int i = 0; i < C::PACKED / 8; i++) // sixteen loads in flight
@@ -837,33 +836,43 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                 release();
             else if (packed)
             {
-                // (whether gates are folded in is decided outside the loop: a choice per value costs a branch per value, and
-                // the two or three warps of a scheduler do not hide it)
-                auto drain = [&](auto with_gates) {
+                // (what is folded in is decided once per piece: a choice per value costs a branch per value, and the two or
+                // three warps of a scheduler do not hide it)
 #pragma unroll
-                    for (int i = 0; i < C::PACKED / 8; i++)
-                        if (col_begin + 16 * i < col_end)
+                for (int i = 0; i < C::PACKED / 8; i++)
+                    if (col_begin + 16 * i < col_end)
+                    {
+                        uint32_t d[16];
+                        tmem_ld_32x16(d_addr + (uint32_t)(col_begin + 16 * i), d);
+                        tcgen05_wait_ld();
+                        if (col_begin + 16 * i + 16 == col_end)
+                            release();
+                        if (gated)
                         {
-                            uint32_t d[16];
-                            tmem_ld_32x16(d_addr + (uint32_t)(col_begin + 16 * i), d);
-                            tcgen05_wait_ld();
-                            if (col_begin + 16 * i + 16 == col_end)
-                                release();
 #pragma unroll
                             for (int j = 0; j < 8; j++)
                             {
-                                float lo = __uint_as_float(d[2 * j]), hi = __uint_as_float(d[2 * j + 1]);
-                                if constexpr (decltype(with_gates)::value)
-                                    lo *= silu(gate_of_half(pk[8 * i + j] & 0xFFFFu)), hi *= silu(gate_of_half(pk[8 * i + j] >> 16));
-                                const __half2 h = __floats2half2_rn(lo + bias, hi + bias);
-                                pk[8 * i + j] = *reinterpret_cast<const uint32_t*>(&h);
+                                d[2 * j] = __float_as_uint(__uint_as_float(d[2 * j]) * silu(gate_of_half(pk[8 * i + j] & 0xFFFFu)));
+                                d[2 * j + 1] = __float_as_uint(__uint_as_float(d[2 * j + 1]) * silu(gate_of_half(pk[8 * i + j] >> 16)));
                             }
                         }
-                };
-                if (gated)
-                    drain(std::true_type{});
-                else
-                    drain(std::false_type{});
+                        else if (p.has_addend)
+                        {
+#pragma unroll
+                            for (int j = 0; j < 8; j++)
+                            {
+                                const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&pk[8 * i + j]));
+                                d[2 * j] = __float_as_uint(__uint_as_float(d[2 * j]) + c.x);
+                                d[2 * j + 1] = __float_as_uint(__uint_as_float(d[2 * j + 1]) + c.y);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; j++)
+                        {
+                            const __half2 h = __floats2half2_rn(__uint_as_float(d[2 * j]) + bias, __uint_as_float(d[2 * j + 1]) + bias);
+                            pk[8 * i + j] = *reinterpret_cast<const uint32_t*>(&h);
+                        }
+                    }
                 unsigned short* y = static_cast<unsigned short*>(p.y) + at0;
                 const uint32_t step = held(2u * (uint32_t)p.N);
 #pragma unroll
@@ -879,9 +888,26 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
             }
             else
             {
-                float* const mine = p.slots + (size_t)(sg.whole ? 0 : slot_of(p, (int)(blockIdx.x >> 1), (int)rank, sg.tile, sg.set, U, G)) * slot_floats;
+                float* mine = p.slots + (size_t)(sg.whole ? 0 : slot_of(p, (int)(blockIdx.x >> 1), (int)rank, sg.tile, sg.set, U, G)) * slot_floats +
+                              (size_t)col_begin * kBN + r;
+                // fp32 results, in pieces of 16 batch rows
+                const uint32_t step = held(4u * (uint32_t)p.N);
+                char* y = reinterpret_cast<char*>(static_cast<float*>(p.y) + at0);
+                // what is combined with the products: the gates, or the addend
+                const char* other = reinterpret_cast<const char*>((p.has_addend ? p.bias : static_cast<const float*>(p.y)) + at0);
                 for (int col = col_begin; col < col_end; col += 16)
                 {
+                    const int left = cols - (col - col_begin);
+                    float e[16];
+                    if (sg.whole && (gated || p.has_addend))
+                    {
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                        {
+                            e[j] = j < left ? *reinterpret_cast<const float*>(other) : 0.f;
+                            other += step;
+                        }
+                    }
                     uint32_t d[16];
                     tmem_ld_32x16(d_addr + (uint32_t)col, d);
                     tcgen05_wait_ld();
@@ -891,44 +917,32 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                     {
 #pragma unroll
                         for (int j = 0; j < 16; j++)
-                            mine[(size_t)(col + j) * kBN + r] = __uint_as_float(d[j]);
+                            mine[j * kBN] = __uint_as_float(d[j]);
+                        mine += 16 * kBN;
                         continue;
                     }
-                    // fp32 results, or an addend: in pieces
-                    const int left = row_ok ? m_end - col : 0;
-                    const size_t at = (size_t)(m0 + col) * p.N + n;
-                    float v[16], e[16];
-                    if (p.y_f32)
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        v[j] = __uint_as_float(d[j]) + bias;
+                    if (gated)
                     {
-                        const float* other = p.has_addend ? reinterpret_cast<const float*>(p.bias) : static_cast<const float*>(p.y);
 #pragma unroll
                         for (int j = 0; j < 16; j++)
-                            e[j] = (gated || p.has_addend) && j < left ? other[at + (size_t)j * p.N] : 0.f;
+                            v[j] *= silu(e[j]);
                     }
-                    else
+                    else if (p.has_addend)
                     {
 #pragma unroll
                         for (int j = 0; j < 16; j++)
-                            e[j] = p.has_addend && j < left ? __half2float(reinterpret_cast<const __half*>(p.bias)[at + (size_t)j * p.N]) : 0.f;
+                            v[j] += e[j];
                     }
 #pragma unroll
                     for (int j = 0; j < 16; j++)
-                        v[j] = gated ? __uint_as_float(d[j]) * silu(e[j]) : __uint_as_float(d[j]) + (bias + e[j]);
-                    if (p.y_f32)
                     {
-                        float* y = static_cast<float*>(p.y) + at;
-#pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            if (j < left)
-                                y[(size_t)j * p.N] = v[j];
-                    }
-                    else
-                    {
-                        __half* y = static_cast<__half*>(p.y) + at;
-#pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            if (j < left)
-                                y[(size_t)j * p.N] = __float2half_rn(v[j]);
+                        if (j < left)
+                            *reinterpret_cast<float*>(y) = v[j];
+                        y += step;
                     }
                 }
             }
@@ -1049,7 +1063,8 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
 
 // Pre-pass for activations the tensor-core kernel does not take as they are: fp32 rows are rounded to fp16, and with
 // the RMSNorm prologue every row is scaled by rsqrt(mean(x^2) + eps) * gain on the way (fp32 arithmetic, one
-// rounding).  One CTA per row; the row is read twice when it has to be normalised (the second time from L2).
+// rounding).  One CTA per row, 16-byte accesses, the whole row (up to 8192 elements; the rest is read again) asked for at
+// once and kept in registers.  Bound by HBM; with scalar loads in two rounds 2000 rows of 6016 fp16 took 50 us, now 13.
 // Replaces the reference's Multiply -> Sum -> Divide -> Add -> Rsqrt -> Multiply chain in front of the Dot
 // (reduce: src/nnfusion/core/kernels/cuda_gpu/kernels/reduce.hpp:18-600) and its Convert.
 template <bool XF32>
@@ -1059,18 +1074,50 @@ __global__ void __launch_bounds__(256) prep_activations_kernel(const void* x, co
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float part[8];
-    const size_t row = blockIdx.x;
-    auto load = [&](int k) -> float {
-        return XF32 ? static_cast<const float*>(x)[row * K + k] : __half2float(static_cast<const __half*>(x)[row * K + k]);
+    constexpr int kStep = 256 * 8, kKept = 4; // elements per step of the CTA, steps kept in registers
+    const size_t row = (size_t)blockIdx.x * K;
+    const int k0 = threadIdx.x * 8;
+    auto load = [&](int k, float (&v)[8]) {
+        if (XF32)
+        {
+            const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(x) + row + k);
+            const float4 a = __ldg(src), b = __ldg(src + 1);
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        }
+        else
+        {
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(x) + row + k));
+            const __half2* h = reinterpret_cast<const __half2*>(&a);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                const float2 f = __half22float2(h[j]);
+                v[2 * j] = f.x, v[2 * j + 1] = f.y;
+            }
+        }
     };
+    float kept[kKept][8];
+#pragma unroll
+    for (int s = 0; s < kKept; s++)
+        if (k0 + s * kStep < K) // (K is a multiple of 64)
+            load(k0 + s * kStep, kept[s]);
     float r = 1.f;
     if (gain != nullptr)
     {
         float ss = 0.f;
-        for (int k = threadIdx.x; k < K; k += blockDim.x)
+#pragma unroll
+        for (int s = 0; s < kKept; s++)
+            if (k0 + s * kStep < K)
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    ss = fmaf(kept[s][j], kept[s][j], ss);
+        for (int k = k0 + kKept * kStep; k < K; k += kStep)
         {
-            const float v = load(k);
-            ss += v * v;
+            float v[8];
+            load(k, v);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                ss = fmaf(v[j], v[j], ss);
         }
         for (int o = 16; o > 0; o >>= 1)
             ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -1078,17 +1125,68 @@ __global__ void __launch_bounds__(256) prep_activations_kernel(const void* x, co
             part[threadIdx.x >> 5] = ss;
         __syncthreads();
         float tot = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) // fixed order: repeatable
+#pragma unroll
+        for (int w = 0; w < 8; w++) // fixed order: repeatable
             tot += part[w];
         r = 1.0f / sqrtf(tot / (float)K + eps);
     }
-    for (int k = threadIdx.x; k < K; k += blockDim.x)
-    {
-        float v = load(k) * r;
+    auto store = [&](int k, const float (&v)[8]) {
+        float g[8];
         if (gain != nullptr)
-            v *= gain[k];
-        out[row * K + k] = __float2half_rn(v);
+        {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(gain + k)), b = __ldg(reinterpret_cast<const float4*>(gain + k) + 1);
+            g[0] = a.x, g[1] = a.y, g[2] = a.z, g[3] = a.w, g[4] = b.x, g[5] = b.y, g[6] = b.z, g[7] = b.w;
+        }
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const float lo = gain != nullptr ? v[2 * j] * r * g[2 * j] : v[2 * j], hi = gain != nullptr ? v[2 * j + 1] * r * g[2 * j + 1] : v[2 * j + 1];
+            const __half2 q = __floats2half2_rn(lo, hi);
+            h[j] = *reinterpret_cast<const uint32_t*>(&q);
+        }
+        *reinterpret_cast<uint4*>(out + row + k) = make_uint4(h[0], h[1], h[2], h[3]);
+    };
+#pragma unroll
+    for (int s = 0; s < kKept; s++)
+        if (k0 + s * kStep < K)
+            store(k0 + s * kStep, kept[s]);
+    for (int k = k0 + kKept * kStep; k < K; k += kStep)
+    {
+        float v[8];
+        load(k, v);
+        store(k, v);
     }
+}
+
+// Launched as a programmatic dependent like the linear behind it, which starts on its weights meanwhile; with the shared
+// memory carve-out that the linear wants, so that an SM need not drain before it can hold one of its CTAs.
+template <bool XF32>
+cudaError_t launch_prep(const void* x, const float* gain, __half* out, int M, int K, float eps, cudaStream_t stream)
+{
+    static bool configured[nnf::kMaxDevices] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess)
+        return e;
+    if (dev < 0 || dev >= nnf::kMaxDevices)
+        return cudaErrorInvalidDevice;
+    if (!configured[dev])
+    {
+        e = cudaFuncSetAttribute(prep_activations_kernel<XF32>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess)
+            return e;
+        configured[dev] = true;
+    }
+    (void)cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(M);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    nnf::overlap_attribute(attr, &cfg.numAttrs);
+    cfg.attrs = attr;
+    return cudaLaunchKernelEx(&cfg, prep_activations_kernel<XF32>, x, gain, out, K, eps);
 }
 
 template <int WBITS, bool ONE_GROUP, bool SMALL>
@@ -1257,12 +1355,8 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     {
         __half* xh = reinterpret_cast<__half*>(ws + L.counter_bytes + L.slot_bytes);
         const float* g = d.prologue == NNF_B200_PROLOGUE_RMSNORM ? static_cast<const float*>(gain) : nullptr;
-        (void)cudaGetLastError();
-        if (d.x_dtype == NNF_B200_F32)
-            prep_activations_kernel<true><<<d.M, 256, 0, stream>>>(x, g, xh, d.K, d.rms_eps);
-        else
-            prep_activations_kernel<false><<<d.M, 256, 0, stream>>>(x, g, xh, d.K, d.rms_eps);
-        cudaError_t pe = cudaGetLastError();
+        const cudaError_t pe = d.x_dtype == NNF_B200_F32 ? launch_prep<true>(x, g, xh, d.M, d.K, d.rms_eps, stream)
+                                                         : launch_prep<false>(x, g, xh, d.M, d.K, d.rms_eps, stream);
         if (pe != cudaSuccess)
             return set_error(ctx, NNF_B200_ECUDA, std::string("prep_activations launch: ") + cudaGetErrorString(pe));
         ctx->launches++;
