@@ -442,17 +442,28 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     copy_params(0, min(p.batch, ntiles), 0);
     copy_params(p.batch, min(p.batch, max(ntiles - p.batch, 0)), 1);
 
+    // The RMSNorm gain is a constant as well: its lines come to L1 meanwhile (as plain loads behind the activations they
+    // stood a second round trip to memory into the launch's way: 7B gate/up pair with the prologue 16.6 -> @@NORM@@ us).
+    if (!XSPLIT && p.rmsnorm && g < p.M)
+    {
+#pragma unroll
+        for (int l = 0; l < 2; l++)
+            if (unit_ok[l])
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(p.gain + (2 * slice + l) * F::UE + t * F::LE) : "memory");
+    }
+
     // Everything above reads only constants (weights, scales, zero-points).  The activations, the output and the workspace may belong
     // to the launch before this one on the stream: when this kernel was launched as its programmatic dependent, it
     // has been running beside that launch's tail until here.
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ---------------------------------------------------------------- activations: ask first, set up meanwhile
-    // fp16 activations that are used as they are: the raw loads leave now and are permuted into fragments below.
+    // fp16 activations: the raw loads leave now and are permuted into fragments, or normalised, below.
     const bool plain = !XSPLIT && !p.x_f32 && !p.rmsnorm;
+    const bool raw = plain || (MB == 1 && !XSPLIT && !p.x_f32); // (16 rows to be normalised: no registers for them)
     uint32_t xf[2][XSM ? 1 : MB][XS][NF];
     uint4 xraw[2][MB][F::LE / 8];
-    if (plain)
+    if (raw)
     {
 #pragma unroll
         for (int l = 0; l < 2; l++)
@@ -560,7 +571,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 #pragma unroll
                         for (int j = 0; j < F::LE / 8; j++)
                         {
-                            uint4 v = __ldg(src + j);
+                            const uint4 v = raw ? xraw[l][mb][j] : __ldg(src + j);
                             const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
                             for (int q = 0; q < 4; q++)
@@ -589,22 +600,19 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
                     for (int j = 0; j < F::LE; j++)
                         xv[j] = 0.f;
                 }
-                __half hi[F::LE], lo[F::LE];
-#pragma unroll
-                for (int j = 0; j < F::LE; j++)
-                {
-                    hi[j] = __float2half_rn(xv[j]);
-                    if (XSPLIT)
-                        lo[j] = __float2half_rn(xv[j] - __half2float(hi[j]));
-                }
 #pragma unroll
                 for (int f = 0; f < NF; f++)
                 {
                     const int e0 = (WBITS == 4) ? 8 * (f >> 2) + (f & 3) : 2 * f;
                     const int e1 = (WBITS == 4) ? e0 + 4 : e0 + 1;
-                    frag[0][f] = pack_h2(hi[e0], hi[e1]);
+                    const __half2 hi = __floats2half2_rn(xv[e0], xv[e1]);
+                    frag[0][f] = *reinterpret_cast<const uint32_t*>(&hi);
                     if (XSPLIT)
-                        frag[XS - 1][f] = pack_h2(lo[e0], lo[e1]);
+                    {
+                        const float2 h = __half22float2(hi);
+                        const __half2 lo = __floats2half2_rn(xv[e0] - h.x, xv[e1] - h.y);
+                        frag[XS - 1][f] = *reinterpret_cast<const uint32_t*>(&lo);
+                    }
                 }
             }
             {
@@ -666,16 +674,17 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     }
     cp_async_wait_but_one(); // this thread's pieces of the first batch's parameters have landed
     __syncthreads();         // ... and everybody's; ss_w visible
-    if (p.rmsnorm)
+    if (p.rmsnorm && tid < MPAD) // (read behind the barrier that ends the first batch)
     {
-        if (tid < MPAD)
-        {
-            float v = 0.f;
-            for (int w = 0; w < nwarps; w++)
-                v += ss_w[w * MPAD + tid];
-            ss_cta[tid] = v;
-        }
-        __syncthreads();
+        float part[kMaxWarps];
+#pragma unroll
+        for (int w = 0; w < kMaxWarps; w++)
+            part[w] = w < nwarps ? ss_w[w * MPAD + tid] : 0.f;
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < kMaxWarps; w++)
+            v += part[w];
+        ss_cta[tid] = v;
     }
 
     // ---------------------------------------------------------------- arithmetic on one stage
@@ -1114,15 +1123,26 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
                 const int n = rt * 16 + row;
                 if (m < p.M && n < p.N)
                 {
+                    // (four splits' sums asked for at a time: one after the other they were a round trip to L2 each)
                     float a0 = 0.f, a1 = 0.f, ssum = 0.f;
-                    for (int s = 0; s < p.splits; s++)
+                    const float* slot0 = p.ws_slots + (size_t)rt * p.slot_floats;
+                    const size_t step = (size_t)p.row_tiles * p.slot_floats;
+                    constexpr int SB = MB == 1 && !DUAL ? 4 : 1; // (16 rows, two sets: no registers for more)
+                    for (int s0 = 0; s0 < p.splits; s0 += SB)
                     {
-                        const float* slot = p.ws_slots + ((size_t)s * p.row_tiles + rt) * p.slot_floats;
-                        a0 += __ldcg(slot + o);
-                        if (DUAL)
-                            a1 += __ldcg(slot + MB * 128 + o);
-                        if (p.rmsnorm)
-                            ssum += __ldcg(slot + SETS * MB * 128 + m);
+                        float b0[SB], b1[SB], bs[SB];
+#pragma unroll
+                        for (int q = 0; q < SB; q++)
+                        {
+                            const float* slot = slot0 + (size_t)min(s0 + q, p.splits - 1) * step;
+                            b0[q] = __ldcg(slot + o);
+                            b1[q] = DUAL ? __ldcg(slot + MB * 128 + o) : 0.f;
+                            bs[q] = p.rmsnorm ? __ldcg(slot + SETS * MB * 128 + m) : 0.f;
+                        }
+#pragma unroll
+                        for (int q = 0; q < SB; q++) // in split order: repeatable
+                            if (s0 + q < p.splits)
+                                a0 += b0[q], a1 += b1[q], ssum += bs[q];
                     }
                     if (ar)
                         ar_put(j, m, n, a0);
