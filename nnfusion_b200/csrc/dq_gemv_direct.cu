@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     copy_params(p.batch, min(p.batch, max(ntiles - p.batch, 0)), 1);
 
     // The RMSNorm gain is a constant as well: its lines come to L1 meanwhile (as plain loads behind the activations they
-    // stood a second round trip to memory into the launch's way: 7B gate/up pair with the prologue 16.6 -> @@NORM@@ us).
+    // stood a second round trip to memory into the launch's way: 7B gate/up pair with the prologue 16.6 -> 15.0 us).
     if (!XSPLIT && p.rmsnorm && g < p.M)
     {
 #pragma unroll
