@@ -138,10 +138,6 @@ __device__ __forceinline__ int held(int v)
     asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(v));
     return r;
 }
-__device__ __forceinline__ uint32_t pack_h2(__half a, __half b)
-{
-    return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
-}
 
 // 16 bytes of weights, read once.  Without a line in L1 the load comes back sooner, which is what a short launch
 // needs; with one, an SM sustains more bytes in flight, which is what a long launch needs (the host chooses).

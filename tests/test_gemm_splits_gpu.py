@@ -1,0 +1,47 @@
+"""How the large-M kernel's tiles meet the pairs of CTAs (``gemm_layout`` in ``nnfusion_b200/csrc/dq_gemm_tcgen05.cu``):
+K shared by the 2, 3 or 4 pairs of a cluster, seam shares through the workspace, several whole tiles a pair, at the edges
+of batch tiles (16, 128, 256), of weight tiles (256) and of K chunks, against the oracle."""
+import numpy as np
+import pytest
+
+from nnfusion_b200 import _lib as L
+from nnfusion_b200 import synth
+from oracle import oracle as orc
+from tests.util import TOL_F16, oracle_linear
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K,bits,dual", [
+    (17, 256, 512, 4, False),       # 2 pairs share K, the second one's slice of 16 batch rows is empty
+    (33, 257, 1088, 4, True),       # 3 pairs, gate and up, 17 k-blocks: the last chunk holds one
+    (48, 513, 2112, 8, False),      # 4 pairs, 33 k-blocks of which two make a chunk
+    (128, 130, 2048, 4, True),      # 4 pairs, gate and up
+    (129, 1000, 11008, 4, False),   # a long K cut into 4 uneven ranges
+    (300, 2500, 1088, 4, True),     # 2 or 3 pairs, up to 128 batch rows a tile, gate and up
+    (1040, 2000, 640, 8, True),     # whole tiles
+    (1040, 5000, 1024, 4, False),   # several whole tiles a pair, above 128 batch rows a tile
+    (300, 9000, 1024, 4, True),     # one whole tile a pair, above 128 batch rows, gate and up
+    (18, 19001, 3136, 4, False),    # 75 tiles on 74 pairs: seam shares, scalar stores
+    (130, 19000, 3136, 4, False),   # the same above 128 batch rows a tile
+])
+def test_splits(M, N, K, bits, dual):
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(M + N))
+    x = synth.make_x(rng, M, K, np.float16)
+    w = [synth.make_weights(rng, N, K, bits, 64) for _ in range(1 + dual)]
+    dev = [DeviceWeight.from_host(v) for v in w]
+    tx = torch.from_numpy(x).cuda()
+    r32 = oracle_linear(x, *w, out_dtype=np.float32)
+    for y_dtype, add in [(torch.float16, False), (torch.float32, False)] + [(torch.float16, True), (torch.float32, True)] * (not dual):
+        op = DequantDot(*dev, kernel=L.KERNEL_GEMM, y_dtype=y_dtype, add=add)
+        c = torch.randn(M, N, device="cuda").to(y_dtype) if add else None
+        kw = dict(addend=c) if add else {}
+        y = op(tx, **kw)
+        assert torch.equal(op(tx, **kw), y)          # bitwise repeatable, counters left zeroed
+        op.ctx.device_status()
+        want = r32 + c.float().cpu().numpy() if add else r32
+        err = orc.max_rel_err(y.float().cpu().numpy(), want)
+        # fp16 scale products and, with SiLU, one rounding of the gate to y's type: the kernel's other tests' bounds
+        assert err <= min(TOL_F16, 3e-3 if dual else 2e-3), (y_dtype, add, err)
