@@ -995,14 +995,16 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 
     // Add up the warps' partial sums of the local tiles [first, first + count) and write the results out.
     // (the caller brackets it with the CTA's barriers)
+    // With one batch row every other value is that of a row that does not exist (odd accumulator columns): the loops step
+    // over those, which halves the passes of a long batch (8192 x 28672 cut 7 ways behind its gate/up pair: 86.8 -> 83.6 us for both).
     auto flush = [&](int first, int count) {
         if (p.splits == 1)
         {
             if (ar)
                 ar_begin(first, count, false);
-            for (int idx = tid; idx < count * per_tile; idx += nthreads)
+            for (int idx = tid; idx < count * (per_tile >> M1); idx += nthreads)
             {
-                const int j = idx >> pt_shift, e = idx & (per_tile - 1);
+                const int j = idx >> (pt_shift - M1), e = (idx << M1) & (per_tile - 1);
                 int row, m, o;
                 decode(e, row, m, o);
                 const int n = (tile0 + first + j) * 16 + row;
@@ -1036,9 +1038,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
             auto put = [&](uint32_t float_index, float v) {
                 asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(my_part + float_index * 4u), "f"(v) : "memory");
             };
-            for (int idx = tid; idx < count * per_tile; idx += nthreads)
+            for (int idx = tid; idx < count * (per_tile >> M1); idx += nthreads)
             {
-                const int j = idx >> pt_shift, e = idx & (per_tile - 1);
+                const int j = idx >> (pt_shift - M1), e = (idx << M1) & (per_tile - 1);
                 int row, m, o;
                 decode(e, row, m, o);
                 if (m >= p.M)
@@ -1060,9 +1062,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
             if (ar)
                 ar_begin(first, count, true);
             if (split == 0)
-                for (int idx = tid; idx < count * per_tile; idx += nthreads)
+                for (int idx = tid; idx < count * (per_tile >> M1); idx += nthreads)
                 {
-                    const int j = idx >> pt_shift, e = idx & (per_tile - 1);
+                    const int j = idx >> (pt_shift - M1), e = (idx << M1) & (per_tile - 1);
                     int row, m, o;
                     decode(e, row, m, o);
                     const int n = (tile0 + first + j) * 16 + row;
@@ -1108,9 +1110,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
             }
             else
             {
-                for (int idx = tid; idx < count * per_tile; idx += nthreads)
+                for (int idx = tid; idx < count * (per_tile >> M1); idx += nthreads)
                 {
-                    const int j = idx >> pt_shift, e = idx & (per_tile - 1);
+                    const int j = idx >> (pt_shift - M1), e = (idx << M1) & (per_tile - 1);
                     int row, m, o;
                     decode(e, row, m, o);
                     if (m >= p.M)
@@ -1196,9 +1198,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
             }
             else
             {
-                for (int idx = tid; idx < count * per_tile; idx += nthreads)
+                for (int idx = tid; idx < count * (per_tile >> M1); idx += nthreads)
                 {
-                    const int j = idx >> pt_shift, e = idx & (per_tile - 1);
+                    const int j = idx >> (pt_shift - M1), e = (idx << M1) & (per_tile - 1);
                     if (!last_flag[j])
                         continue;
                     int row, m, o;

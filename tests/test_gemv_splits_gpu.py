@@ -1,4 +1,5 @@
-"""The small-M kernel's sums of a split K through the workspace, four values a thread: odd and even row counts at the edges
+"""The small-M kernel's sums of a split K through the workspace, four values a thread (one row: every
+other value): odd and even row counts at the edges
 of the accumulator's columns (2, 8, 16), ragged N, split counts around the four read back at a time, with every epilogue."""
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bits", [4, 8])
-@pytest.mark.parametrize("M,N,splits", [(2, 4096, 3), (3, 2063, 4), (7, 2049, 5), (8, 4095, 4), (9, 2063, 3), (15, 2048, 5), (16, 2049, 4)])
+@pytest.mark.parametrize("M,N,splits", [(1, 2063, 3), (1, 4096, 5), (2, 4096, 3), (3, 2063, 4), (7, 2049, 5), (8, 4095, 4), (9, 2063, 3), (15, 2048, 5), (16, 2049, 4)])
 def test_four_values_a_thread(M, N, splits, bits):
     rng = np.random.Generator(np.random.PCG64(M * N))
     K = 10240
