@@ -144,7 +144,7 @@ class DequantDot:
 
     Mirrors the fused graph node that stands in for Convert -> Subtract -> Multiply -> Dot(transB)
     (``src/nnfusion/core/operators/op_define/dot.cpp:43-135``).  The workspace is allocated once
-    per (node, M) and zeroed once, as the generated runtime plans temp tensors into its pool
+    per (node, descriptor) and zeroed once, as the generated runtime plans temp tensors into its pool
     (``src/nnfusion/core/kernels/kernel_emitter.cpp:282-319``).
     """
 
@@ -217,7 +217,7 @@ class DequantDot:
         return d
 
     def workspace(self, d: L.LinearDesc) -> Optional[torch.Tensor]:
-        key = (d.M, d.x_dtype)
+        key = bytes(d)  # a buffer serves one descriptor: the counters of another one may lie where this one's sums are
         if key not in self._ws:
             n = int(self.ctx.lib.nnf_b200_linear_workspace_bytes(self.ctx.handle, ctypes.byref(d)))
             if n == 0:

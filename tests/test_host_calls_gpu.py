@@ -42,3 +42,24 @@ def test_module_keeps_leading_dimensions_and_follows_its_buffers():
     assert torch.equal(m(tx.transpose(0, 1)), first.transpose(0, 1))    # not contiguous: the full path
     m.wq = torch.zeros_like(m.wq)
     assert not torch.equal(m(tx), first)
+
+
+def test_a_node_whose_kernel_and_split_change():
+    """Each descriptor has its own workspace: the large-M kernel's partial sums must not be taken for the small-M
+    kernel's arrival counters, nor one split's for another's."""
+    import torch
+    from nnfusion_b200 import _lib as L
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    from oracle import oracle as orc
+    from tests.util import TOL_F16, oracle_linear
+    x, w = synth.u4g128(13, 8, 512, 10240)
+    want = oracle_linear(x, w)
+    op = DequantDot(DeviceWeight.from_host(w))
+    tx = torch.from_numpy(x).cuda()
+    for kernel, split_k in [(L.KERNEL_GEMM, 0), (L.KERNEL_GEMV, 3), (L.KERNEL_GEMV, 5), (L.KERNEL_GEMM, 0),
+                            (L.KERNEL_AUTO, 0), (L.KERNEL_GEMV, 3)]:
+        op.kernel, op.split_k = kernel, split_k
+        for _ in range(2):
+            y = torch.full((8, 512), float("nan"), dtype=torch.float16, device="cuda")  # rows nobody writes stay NaN
+            op(tx, out=y)
+            assert orc.max_rel_err(y.cpu().numpy(), want) <= min(TOL_F16, 2e-3), (kernel, split_k)
