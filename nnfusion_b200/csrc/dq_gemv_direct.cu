@@ -441,14 +441,15 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     copy_params(0, min(p.batch, ntiles), 0);
     copy_params(p.batch, min(p.batch, max(ntiles - p.batch, 0)), 1);
 
-    // The RMSNorm gain is a constant as well: its lines come to L1 meanwhile (as plain loads behind the activations they
-    // stood a second round trip to memory into the launch's way: 7B gate/up pair with the prologue 16.6 -> 15.0 us).
+    // The RMSNorm gain's lines come to L2 meanwhile.  To L2 and no nearer: the gain may be what the launch ahead writes, and
+    // a line in this SM's L1 would not see that.  (Behind the activations a plain load's round trip to memory stood in the
+    // launch's way: 7B gate/up pair with the prologue 16.6 -> 15.0 us; from L1 or from L2 makes no difference to a layer.)
     if (!XSPLIT && p.rmsnorm && g < p.M)
     {
 #pragma unroll
         for (int l = 0; l < 2; l++)
             if (unit_ok[l])
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(p.gain + (2 * slice + l) * F::UE + t * F::LE) : "memory");
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gain + (2 * slice + l) * F::UE + t * F::LE) : "memory");
     }
 
     // Everything above reads only constants (weights, scales, zero-points).  The activations, the output and the workspace may belong
