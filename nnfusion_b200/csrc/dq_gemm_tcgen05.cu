@@ -273,7 +273,7 @@ __device__ __forceinline__ void add_parts(const GemmParams& p, Load load, int pa
     float bias[4];
 #pragma unroll
     for (int e = 0; e < 4; e++)
-        bias[e] = p.has_bias && n4 + e < p.N ? __ldg(p.bias + n4 + e) : 0.f;
+        bias[e] = p.has_bias && n4 + e < p.N ? p.bias[n4 + e] : 0.f;
     for (int row = ew; row < rows; row += ROWS * WARPS)
     {
         float v[SETS][ROWS][4];
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
             const int n = n_base + r;
             const bool row_ok = n < p.N;
             const int m_end = min(p.bx, p.M - m0); // columns that exist
-            const float bias = p.has_bias && row_ok ? __ldg(p.bias + n) : 0.f;
+            const float bias = p.has_bias && row_ok ? p.bias[n] : 0.f;
             const bool gated = sg.set == 1 && sg.whole;
             const uint32_t d_addr = tmem_base + lane_addr + b * 128u;
             const long long U = (long long)p.tiles * p.sets * p.cpt;
@@ -1081,12 +1081,12 @@ __global__ void __launch_bounds__(256) prep_activations_kernel(const void* x, co
         if (XF32)
         {
             const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(x) + row + k);
-            const float4 a = __ldg(src), b = __ldg(src + 1);
+            const float4 a = src[0], b = src[1];
             v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
         }
         else
         {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(x) + row + k));
+            const uint4 a = *reinterpret_cast<const uint4*>(static_cast<const __half*>(x) + row + k);
             const __half2* h = reinterpret_cast<const __half2*>(&a);
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -1134,7 +1134,7 @@ __global__ void __launch_bounds__(256) prep_activations_kernel(const void* x, co
         float g[8];
         if (gain != nullptr)
         {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(gain + k)), b = __ldg(reinterpret_cast<const float4*>(gain + k) + 1);
+            const float4 a = reinterpret_cast<const float4*>(gain + k)[0], b = reinterpret_cast<const float4*>(gain + k)[1];
             g[0] = a.x, g[1] = a.y, g[2] = a.z, g[3] = a.w, g[4] = b.x, g[5] = b.y, g[6] = b.z, g[7] = b.w;
         }
         uint32_t h[4];

@@ -460,7 +460,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
                                                                  unit_of[l] * F::UE + t * F::LE);
 #pragma unroll
                 for (int j = 0; j < F::LE / 8; j++)
-                    xraw[l][mb][j] = (unit_ok[l] && m < p.M) ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+                    xraw[l][mb][j] = (unit_ok[l] && m < p.M) ? src[j] : make_uint4(0u, 0u, 0u, 0u);
             }
     }
     if (lsu)
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
 #pragma unroll
                         for (int j = 0; j < F::LE / 4; j++)
                         {
-                            float4 v = __ldg(src + j);
+                            float4 v = src[j];
                             xv[4 * j + 0] = v.x, xv[4 * j + 1] = v.y, xv[4 * j + 2] = v.z, xv[4 * j + 3] = v.w;
                         }
                     }
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
 #pragma unroll
                         for (int j = 0; j < F::LE / 8; j++)
                         {
-                            uint4 v = __ldg(src + j);
+                            uint4 v = src[j];
                             const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
                             for (int q = 0; q < 4; q++)
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
 #pragma unroll
                         for (int j = 0; j < F::LE / 4; j++)
                         {
-                            float4 gv = __ldg(gsrc + j);
+                            float4 gv = gsrc[j];
                             float* e = xv + 4 * j;
                             ss_local[mb] += e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + e[3] * e[3];
                             e[0] *= gv.x, e[1] *= gv.y, e[2] *= gv.z, e[3] *= gv.w;
@@ -832,7 +832,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
             v = v * sg * u;
         }
         if (p.has_bias)
-            v += __ldg(p.bias + n);
+            v += p.bias[n];
         if (p.has_addend)
             v += p.y_f32 ? reinterpret_cast<const float*>(p.bias)[(size_t)m * p.N + n]
                          : __half2float(reinterpret_cast<const __half*>(p.bias)[(size_t)m * p.N + n]);

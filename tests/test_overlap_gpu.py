@@ -46,3 +46,42 @@ def test_gain_written_by_the_launch_ahead(M, K, dual):
         node = DequantDot(*ws, gain=gain.view(-1))
         return lambda: node(x)
     _chain(make, K)
+
+
+@pytest.mark.parametrize("M,kernel,norm", [(1, 1, False), (1, 1, True), (8, 1, False), (16, 1, True), (2, 2, False), (2, 2, True)])
+def test_activations_and_bias_written_by_the_launch_ahead(M, kernel, norm):
+    """fp32 activations (all rows of one buffer) and a bias, for the small-M kernel and for the large-M kernel's pre-pass."""
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(8))
+    K, N = 2048, 1536
+    w = DeviceWeight.from_host(synth.make_weights(rng, N, K, 4, 128))
+    gain = torch.from_numpy(rng.uniform(0.9, 1.1, K).astype(np.float32)).cuda() if norm else None
+
+    def activations(t):
+        node = DequantDot(w, gain=gain, kernel=kernel)
+        return lambda: node(t.view(M, K))
+    _chain(activations, M * K)
+
+    x = torch.from_numpy(synth.make_x(rng, M, K, np.float16)).cuda()
+
+    def bias(t):
+        node = DequantDot(w, gain=gain, bias=t.view(-1), kernel=kernel)
+        return lambda: node(x)
+    _chain(bias, N)
+
+
+@pytest.mark.parametrize("norm", [False, True])
+def test_exact_zero_point_kernel_behind_the_launch_ahead(norm):
+    import torch
+    from nnfusion_b200 import _lib as L
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(9))
+    K, N = 2048, 1536
+    w = DeviceWeight.from_host(synth.make_weights(rng, N, K, 4, 128))
+    gain = torch.from_numpy(rng.uniform(0.9, 1.1, K).astype(np.float32)).cuda() if norm else None
+
+    def activations(t):
+        node = DequantDot(w, gain=gain, flags=L.FLAG_EXACT_ZP)
+        return lambda: node(t.view(2, K))
+    _chain(activations, 2 * K)
