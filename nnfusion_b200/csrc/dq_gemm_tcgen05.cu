@@ -139,13 +139,14 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
     return false;
 }
 // A whole warp.  Every decision is a vote, which the compiler knows to be the same for all lanes: the warp stays together
-// for the warp-wide tensor-memory instructions that follow, and what follows may use uniform registers.
-template <int SLEEP>
+// for the warp-wide tensor-memory instructions that follow, and what follows may use uniform registers.  CLUSTER: what was
+// announced happened in another CTA of the cluster.
+template <int SLEEP, bool CLUSTER = false>
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
     for (uint32_t i = 0; i < kGemmSpin; i++)
     {
-        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
+        if (__all_sync(0xffffffffu, CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)))
             return true;
         if constexpr (SLEEP > 0)
             __nanosleep(SLEEP);
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
     auto full_x = [&](int q) { return bar0 + 8u * (2 * C::STAGES + 2 * C::W_STAGES + 4 + q); };
     auto empty_x = [&](int q) { return bar0 + 8u * (2 * C::STAGES + 2 * C::W_STAGES + 4 + C::MAX_X_STAGES + q); };
 
-    const uint32_t peers_ready = bar0 + 8u * (C::BARRIERS - 2); // every pair of the cluster has multiplied: its rings are free
+    const uint32_t peers_ready = bar0 + 8u * (C::BARRIERS - 2); // every pair of the cluster has multiplied: the rings are free
     const uint32_t parts_here = bar0 + 8u * (C::BARRIERS - 1);  // every pair's sums of this CTA's batch rows have arrived
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -614,6 +615,11 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                     tcgen05_commit_pair(acc_full(b), pair_mask, issue);
                 si++;
             }
+            // K shared by the cluster's pairs: their plain stores follow where this pair's rings were.  The same kind of
+            // arrival that hands a stage back to its producer announces that, here to every CTA of the cluster.  (A release
+            // at cluster scope by the epilogue warps cost 0.3 us of 19.4 at 48 x 4096 x 11008.)
+            if (ok && p.ksplit > 1)
+                tcgen05_commit_pair(peers_ready, (uint16_t)((1u << (2 * p.ksplit)) - 1u), issue);
         }
     }
     else if (warp < C::DQ_WARPS)
@@ -999,9 +1005,7 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                 fine = fine && wait_warp<100>(acc_full(set), 0u, abort_flag);
             tcgen05_fence_after();
             const int pair = blockIdx.x >> 1, part = pair % p.ksplit, tile = pair / p.ksplit;
-            if (fine && ew == 0 && lane < p.ksplit)
-                mbar_arrive_cluster(map_to_rank(peers_ready, 2u * (uint32_t)lane + rank));
-            fine = fine && wait_warp<0>(peers_ready, 0u, abort_flag);
+            fine = fine && wait_warp<0, true>(peers_ready, 0u, abort_flag);
             const uint32_t buf = smem_u32(xs); // [set][part][batch row of the slice][128] floats
             if (fine)
             {

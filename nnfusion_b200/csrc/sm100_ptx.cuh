@@ -213,13 +213,13 @@ __device__ __forceinline__ void tcgen05_wait_st()
 }
 // Both are issued by the one lane whose `issue` is set; as a predicate and not as a branch around them, so that the warp stays
 // together and addresses stay in uniform registers (in a branch of its own every multiply took about 100 clocks to issue).
-// The barrier at this offset in both CTAs of the pair gets one arrival once every tcgen05.mma issued so far by this
-// thread has completed.
-__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar, uint16_t pair_mask, uint32_t issue)
+// The barrier at this offset in every CTA of the cluster that the mask names (both of the pair, mostly) gets one arrival
+// once every tcgen05.mma issued so far by this thread has completed.
+__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar, uint16_t mask, uint32_t issue)
 {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
                  "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar),
-                 "h"(pair_mask), "r"(issue)
+                 "h"(mask), "r"(issue)
                  : "memory");
 }
 // D[tmem] (+)= A[tmem] . B[smem descriptor]; kind::f16.  Each CTA holds its half of A's and D's rows and its half of B's.

@@ -45,3 +45,18 @@ def test_splits(M, N, K, bits, dual):
         err = orc.max_rel_err(y.float().cpu().numpy(), want)
         # fp16 scale products and, with SiLU, one rounding of the gate to y's type: the kernel's other tests' bounds
         assert err <= min(TOL_F16, 3e-3 if dual else 2e-3), (y_dtype, add, err)
+
+
+@pytest.mark.parametrize("M,N,K,dual", [(48, 4096, 11008, False), (100, 1000, 4096, True), (17, 2560, 2048, False)])
+def test_pairs_that_share_k_repeat_back_to_back(M, N, K, dual):
+    """Partial sums land where the peers' rings were: launch after launch without a pause must give the same bits."""
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(M))
+    op = DequantDot(*[DeviceWeight.from_host(synth.make_weights(rng, N, K, 4, 128)) for _ in range(1 + dual)])
+    x = torch.from_numpy(synth.make_x(rng, M, K, np.float16)).cuda()
+    first = op(x).clone()
+    outs = [op(x) for _ in range(300)]
+    torch.cuda.synchronize()
+    op.ctx.device_status()
+    assert not [i for i, y in enumerate(outs) if not torch.equal(y, first)]
