@@ -30,6 +30,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <mutex>
 #include <string>
@@ -243,7 +244,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) decode_attention_kernel(const A
         qh[c] = *reinterpret_cast<const uint4*>(&qh_s[g][32 * c + 8 * t]), ql[c] = *reinterpret_cast<const uint4*>(&ql_s[g][32 * c + 8 * t]);
 
     // ---- running softmax over the warp's blocks of rows; this lane's columns are queries 2t and 2t + 1
-    float m_ref[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    // (m_ref starts at the lowest finite number: rows of score -inf weigh nothing, also before the first finite one)
+    float m_ref[2] = {-FLT_MAX, -FLT_MAX}, l_run[2] = {0.f, 0.f};
     float o[2][4][4]; // [64 dimensions][pair of dimensions][dimension 8g + 2j: queries 2t, 2t + 1; 8g + 2j + 1: likewise]
 #pragma unroll
     for (int h = 0; h < 2; h++)
@@ -285,9 +287,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) decode_attention_kernel(const A
         const int next = row0 + kPass;
         if (next < end)
             load_k(next);
+        // (A score whose hi part is infinite already - a key that left the fp16 range, a row masked by infinities - is that: lo
+        // is of either sign or zero, and its product with the infinity would make a NaN of it.)
 #pragma unroll
         for (int e = 0; e < 4; e++)
-            s4[e] = row0 + g + 8 * (e >> 1) < end ? ((s4[e] + sb[e]) + (sc[e] + sd[e])) * p.scale : -INFINITY;
+        {
+            const float hi = s4[e] + sb[e], sum = fabsf(hi) == INFINITY ? hi : hi + (sc[e] + sd[e]);
+            s4[e] = row0 + g + 8 * (e >> 1) < end ? sum * p.scale : -INFINITY;
+        }
         // Largest score per query over the block.  The reference value that the exponents are taken against follows only
         // when a score exceeds it by more than 2^8: until then nothing has to be rescaled, and the weights (at most 256)
         // stay well inside fp16.
@@ -376,9 +383,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) decode_attention_kernel(const A
 #pragma unroll
         for (int w = 1; w < WARPS; w++)
             m = fmaxf(m, m_s[w][qi]);
-        // an empty range has m = -inf everywhere: weights of zero
-        const float f = m > -INFINITY ? exp2f(m_s[tid / kQ][qi] - m) : 0.f;
-        f_s[tid / kQ][qi] = f;
+        f_s[tid / kQ][qi] = exp2f(m_s[tid / kQ][qi] - m); // (a warp without rows has sums of zero)
         if (tid < kQ)
             mcta_s[qi] = m;
     }
