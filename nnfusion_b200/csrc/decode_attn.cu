@@ -107,6 +107,37 @@ __device__ __forceinline__ uint32_t word(const uint4& v, int i)
     return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
 }
 
+// A query's sums over the rows [begin, end) once more, four dimensions a lane: an infinite value (one that left the fp16
+// range) times a weight's lo half is of either sign or NaN.  Here scores and weights are fp32, so that the sums are infinite,
+// or NaN if they have to be.  m: what the weights are taken against; qh, ql: the query's halves; knew: the new key.
+// Called by a whole warp, and rarely.
+__device__ __forceinline__ float4 sum_infinite_values(const AttnParams& p, int kvh, int begin, int end, float m, const __half* qh,
+                                                      const __half* ql, const __half* knew)
+{
+    const int d = 4 * (threadIdx.x & 31);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int row = begin; row < end; row++)
+    {
+        const size_t at = ((size_t)kvh * p.capacity + row) * kD + d;
+        const bool is_new = row == p.position;
+        const __half* const k = is_new ? knew + d : p.k_cache + at;
+        const __half* const v = is_new ? p.v_new + (size_t)kvh * kD + d : p.v_cache + at;
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            s = fmaf(__half2float(qh[d + j]) + __half2float(ql[d + j]), __half2float(k[j]), s);
+#pragma unroll
+        for (int x = 1; x < 32; x <<= 1)
+            s += __shfl_xor_sync(0xffffffffu, s, x);
+        const float w = exp2f(s * p.scale - m);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            acc[j] = fmaf(w, __half2float(v[j]), acc[j]);
+    }
+    return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) decode_attention_kernel(const AttnParams p)
 {
@@ -410,6 +441,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) decode_attention_kernel(const A
             const float4 x = *reinterpret_cast<const float4*>(part_s + (w * kQ + qi) * kD + 4 * d4);
             l = fmaf(l_s[w][qi], f, l);
             v.x = fmaf(x.x, f, v.x), v.y = fmaf(x.y, f, v.y), v.z = fmaf(x.z, f, v.z), v.w = fmaf(x.w, f, v.w);
+        }
+        if (__any_sync(0xffffffffu, isnan((v.x + v.y) + (v.z + v.w)))) // (a warp has the 32 pieces of one query)
+        {
+            const float4 e = sum_infinite_values(p, kvh, begin, end, mcta_s[qi], qh_s[qi], ql_s[qi], knew_s);
+            v.x = isnan(v.x) ? e.x : v.x, v.y = isnan(v.y) ? e.y : v.y, v.z = isnan(v.z) ? e.z : v.z, v.w = isnan(v.w) ? e.w : v.w;
         }
         if (p.splits == 1)
         {

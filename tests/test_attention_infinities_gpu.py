@@ -55,3 +55,21 @@ def test_an_infinite_score_leaves_nothing_finite(H, Hkv, pos):
         kc[:, 3, 5] = np.inf
     y, ref = _run(H, Hkv, pos, 70 + pos, change)
     assert np.isnan(ref).all() and np.isnan(y).all()  # inf - inf
+
+
+@pytest.mark.parametrize("H,Hkv,pos", _SHAPES)
+@pytest.mark.parametrize("sign", [1, -1])
+def test_infinite_values_stay_infinities(H, Hkv, pos, sign):
+    """A value beyond the fp16 range is infinite in its own dimension for every query that looks at its row, and nowhere
+    else; opposite infinities and a masked row's infinity have no value."""
+    def change(q, kc, vc):
+        vc[:, 3, 7], vc[:, pos // 2, 64] = sign * np.inf, -sign * np.inf
+        vc[:, pos - 1, 100], vc[:, pos - 2, 100] = np.inf, -np.inf
+        kc[:, 9, 5], vc[:, 9, 30] = -np.inf, np.inf
+        q *= np.float16(0.25)  # weights of one order of magnitude: none underflows
+    y, ref = _run(H, Hkv, pos, 80 + pos, change)
+    assert np.isinf(ref[:, 7]).all() and np.isinf(ref[:, 64]).all() and np.isnan(ref[:, [30, 100]]).all()
+    np.testing.assert_array_equal(np.isnan(y), np.isnan(ref))
+    np.testing.assert_array_equal(y[np.isinf(ref)], ref[np.isinf(ref)])
+    ok = np.isfinite(ref)
+    assert ok.sum() == H * 124 and np.abs(y[ok] - ref[ok]).max() <= TOL_F16 * np.abs(ref[ok]).max()
