@@ -11,11 +11,14 @@
 // return None, and the Python method runs its full path, which checks, raises and prepares as it always did.
 //
 // Entries are registered and looked up under the interpreter lock.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "nnf_b200.h"
@@ -111,7 +114,7 @@ PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* p
     }
     else
         bias = address_of(self->bias);
-    PyObject* out;
+    THPObjectPtr out;
     if (pout == Py_None)
     {
         if (lead)
@@ -130,10 +133,9 @@ PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* p
         const at::Tensor* o = plain_cuda(pout);
         if (!o || o->dim() != 2 || o->size(0) != M || o->size(1) != N || o->scalar_type() != yt)
             Py_RETURN_NONE;
-        out = pout;
-        Py_INCREF(out);
+        out = THPObjectPtr::dup(pout);
     }
-    void* y = THPVariable_Unpack(out).mutable_data_ptr();
+    void* y = THPVariable_Unpack(out.get()).mutable_data_ptr();
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     const void *px_data = x->const_data_ptr(), *gain = address_of(self->gain);
     int rc;
@@ -142,24 +144,17 @@ PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* p
                   e.ws_bytes);
     Py_END_ALLOW_THREADS
     if (rc != NNF_B200_OK)
-    {
-        Py_DECREF(out);
         return PyObject_CallFunction(self->check, "i", rc);
-    }
-    return out;
+    return out.release();
 }
 
-PyObject* guarded(PyObject* (*body)(PyObject*, PyObject* const*), PyObject* self, PyObject* const* args)
+// C++ exceptions leave as torch's own bindings would raise them (OutOfMemoryError for an allocation that failed, ...).
+template <typename Body>
+PyObject* guarded(Body&& body)
 {
-    try
-    {
-        return body(self, args);
-    }
-    catch (const std::exception& e) // an allocation that failed, a CUDA error
-    {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
-    }
+    HANDLE_TH_ERRORS
+    return body();
+    END_HANDLE_TH_ERRORS
 }
 
 // call(x, out, addend) -> tensor or None
@@ -167,9 +162,7 @@ PyObject* linear_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
 {
     if (n != 3)
         return PyErr_Format(PyExc_TypeError, "call(x, out, addend)");
-    return guarded([](PyObject* s, PyObject* const* a) {
-        return linear_run(reinterpret_cast<LinearCall*>(s), a[0], a[1], a[2], false);
-    }, self, args);
+    return guarded([&] { return linear_run(reinterpret_cast<LinearCall*>(self), args[0], args[1], args[2], false); });
 }
 
 // call_lead(x, wq) -> tensor or None: any leading dimensions; None too when wq is no longer the tensor the node was
@@ -178,12 +171,12 @@ PyObject* linear_call_lead(PyObject* self, PyObject* const* args, Py_ssize_t n)
 {
     if (n != 2)
         return PyErr_Format(PyExc_TypeError, "call_lead(x, wq)");
-    return guarded([](PyObject* s, PyObject* const* a) -> PyObject* {
-        LinearCall* self = reinterpret_cast<LinearCall*>(s);
-        if (!THPVariable_Check(a[1]) || THPVariable_Unpack(a[1]).const_data_ptr() != self->w.wq)
+    return guarded([&]() -> PyObject* {
+        LinearCall* c = reinterpret_cast<LinearCall*>(self);
+        if (!THPVariable_Check(args[1]) || THPVariable_Unpack(args[1]).const_data_ptr() != c->w.wq)
             Py_RETURN_NONE;
-        return linear_run(self, a[0], Py_None, Py_None, true);
-    }, self, args);
+        return linear_run(c, args[0], Py_None, Py_None, true);
+    });
 }
 
 // register(desc bytes, workspace address, workspace bytes)
@@ -205,13 +198,15 @@ PyObject* linear_register(PyObject* self, PyObject* args)
         for (LinearEntry& q : *c->entries)
             if (q.desc.M == e.desc.M && q.desc.x_dtype == e.desc.x_dtype)
                 q = e, known = true;
-        if (!known)
-            c->entries->push_back(e);
+        PyBuffer_Release(&desc);
+        return guarded([&]() -> PyObject* {
+            if (!known)
+                c->entries->push_back(e);
+            Py_RETURN_NONE;
+        });
     }
     PyBuffer_Release(&desc);
-    if (!ok)
-        return PyErr_Format(PyExc_ValueError, "descriptor size");
-    Py_RETURN_NONE;
+    return PyErr_Format(PyExc_ValueError, "descriptor size");
 }
 
 PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
@@ -223,7 +218,15 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
     w2.buf = nullptr;
     if (!PyArg_ParseTuple(args, "KKy*z*iOOO", &fn, &ctx, &w, &w2, &add, &gain, &bias, &check))
         return nullptr;
-    LinearCall* c = reinterpret_cast<LinearCall*>(type->tp_alloc(type, 0));
+    const bool sizes = w.len == (Py_ssize_t)sizeof(nnf_b200_qweight) && (!w2.buf || w2.len == (Py_ssize_t)sizeof(nnf_b200_qweight));
+    auto* entries = sizes ? new (std::nothrow) std::vector<LinearEntry>() : nullptr;
+    LinearCall* c = entries ? reinterpret_cast<LinearCall*>(type->tp_alloc(type, 0)) : nullptr;
+    if (!c)
+        delete entries;
+    if (!sizes)
+        PyErr_SetString(PyExc_ValueError, "weight set size");
+    else if (!entries)
+        PyErr_NoMemory();
     if (c)
     {
         c->fn = reinterpret_cast<LinearFn>(fn);
@@ -234,7 +237,7 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
             memcpy(&c->w2, w2.buf, sizeof c->w2);
         c->add = add;
         c->gain = Py_NewRef(gain), c->bias = Py_NewRef(bias), c->check = Py_NewRef(check);
-        c->entries = new std::vector<LinearEntry>();
+        c->entries = entries;
     }
     PyBuffer_Release(&w);
     if (w2.buf)
@@ -283,8 +286,9 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
 {
     if (n != 7)
         return PyErr_Format(PyExc_TypeError, "call(q, k_new, v_new, k_cache, v_cache, position, out)");
-    return guarded([](PyObject* s, PyObject* const* a) -> PyObject* {
-        AttnCall* c = reinterpret_cast<AttnCall*>(s);
+    return guarded([&]() -> PyObject* {
+        PyObject* const* a = args;
+        AttnCall* c = reinterpret_cast<AttnCall*>(self);
         const int64_t hd = (int64_t)c->desc.heads * c->desc.head_dim, kd = (int64_t)c->desc.kv_heads * c->desc.head_dim;
         const at::Tensor *q = half_of(a[0], hd), *k = half_of(a[1], kd), *v = half_of(a[2], kd);
         const at::Tensor *kc = half_of(a[3], kd * c->desc.capacity), *vc = half_of(a[4], kd * c->desc.capacity);
@@ -301,7 +305,7 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         const size_t need = c->ws_fn(c->ctx, &d);
         if (need > c->ws_bytes)
             Py_RETURN_NONE;
-        PyObject* out;
+        THPObjectPtr out;
         if (a[6] == Py_None)
         {
             out = wrapped_empty({1, hd}, at::kHalf, q->device());
@@ -312,23 +316,20 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         {
             if (!half_of(a[6], hd))
                 Py_RETURN_NONE;
-            out = Py_NewRef(a[6]);
+            out = THPObjectPtr::dup(a[6]);
         }
         cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
         const void *qp = q->const_data_ptr(), *kp = k->const_data_ptr(), *vp = v->const_data_ptr();
         void *kcp = kc->mutable_data_ptr(), *vcp = vc->mutable_data_ptr();
-        void* op = THPVariable_Unpack(out).mutable_data_ptr();
+        void* op = THPVariable_Unpack(out.get()).mutable_data_ptr();
         int rc;
         Py_BEGIN_ALLOW_THREADS
         rc = c->fn(c->ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? c->ws : nullptr, need ? c->ws_bytes : 0);
         Py_END_ALLOW_THREADS
         if (rc != NNF_B200_OK)
-        {
-            Py_DECREF(out);
             return PyObject_CallFunction(c->check, "i", rc);
-        }
-        return out;
-    }, self, args);
+        return out.release();
+    });
 }
 
 PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
@@ -338,6 +339,11 @@ PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
     PyObject* check;
     if (!PyArg_ParseTuple(args, "KKKy*KKO", &fn, &ws_fn, &ctx, &desc, &ws, &ws_bytes, &check))
         return nullptr;
+    if (desc.len != (Py_ssize_t)sizeof(nnf_b200_attn_desc))
+    {
+        PyBuffer_Release(&desc);
+        return PyErr_Format(PyExc_ValueError, "descriptor size");
+    }
     AttnCall* c = reinterpret_cast<AttnCall*>(type->tp_alloc(type, 0));
     if (c)
     {

@@ -63,3 +63,23 @@ def test_a_node_whose_kernel_and_split_change():
             y = torch.full((8, 512), float("nan"), dtype=torch.float16, device="cuda")  # rows nobody writes stay NaN
             op(tx, out=y)
             assert orc.max_rel_err(y.cpu().numpy(), want) <= min(TOL_F16, 2e-3), (kernel, split_k)
+
+
+def test_an_allocation_that_fails_keeps_its_type():
+    """A repeated call whose output does not fit raises torch's out-of-memory error, like the first one."""
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    x, w = synth.u4g128(14, 4096, 65536, 256)
+    op = DequantDot(DeviceWeight.from_host(w))
+    tx = torch.from_numpy(x).cuda()
+    op(tx)  # 512 MB
+    assert op._native is not None
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            op(tx)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert op(tx).shape == (4096, 65536)

@@ -40,3 +40,12 @@ def test_a_workspace_serves_one_descriptor(node, name, value):
     assert other is not first and other.data_ptr() != first.data_ptr()
     setattr(node, name, before)
     assert node.workspace(node.desc(8, torch.float16)) is first
+
+
+def test_prepared_calls_refuse_descriptors_of_another_size():
+    """Sizes are checked before anything is copied out of the buffers."""
+    host = L.host_calls()
+    with pytest.raises(ValueError):
+        host.LinearCall(0, 0, b"\0" * 8, None, 0, None, None, None)
+    with pytest.raises(ValueError):
+        host.AttnCall(0, 0, 0, b"\0" * 8, 0, 0, None)
