@@ -65,7 +65,7 @@ struct LinearCall
 {
     PyObject_HEAD
     LinearFn fn;
-    nnf_b200_ctx* ctx;
+    Py_buffer handle;
     nnf_b200_qweight w, w2;
     int has_w2, add;
     PyObject* gain;  // tensors or None: their addresses are read at every call
@@ -73,6 +73,24 @@ struct LinearCall
     PyObject* check; // Context.check: raises for a status that is not OK
     std::vector<LinearEntry>* entries;
 };
+
+// The library's context, as the node's Context holds it now: null once that has been closed (the C ABI then refuses).
+nnf_b200_ctx* context(const Py_buffer& handle)
+{
+    return *static_cast<nnf_b200_ctx* const*>(handle.buf);
+}
+
+// Takes a Context's handle (a ctypes.c_void_p; its storage is read at every call).
+bool hold_handle(PyObject* o, Py_buffer* handle)
+{
+    if (PyObject_GetBuffer(o, handle, PyBUF_SIMPLE) < 0)
+        return false;
+    if (handle->len == (Py_ssize_t)sizeof(void*))
+        return true;
+    PyBuffer_Release(handle);
+    PyErr_SetString(PyExc_ValueError, "handle size");
+    return false;
+}
 
 const void* address_of(PyObject* o)
 {
@@ -138,9 +156,10 @@ PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* p
     void* y = THPVariable_Unpack(out.get()).mutable_data_ptr();
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     const void *px_data = x->const_data_ptr(), *gain = address_of(self->gain);
+    nnf_b200_ctx* const ctx = context(self->handle);
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = self->fn(self->ctx, stream, &e.desc, px_data, &self->w, self->has_w2 ? &self->w2 : nullptr, gain, bias, y, e.ws,
+    rc = self->fn(ctx, stream, &e.desc, px_data, &self->w, self->has_w2 ? &self->w2 : nullptr, gain, bias, y, e.ws,
                   e.ws_bytes);
     Py_END_ALLOW_THREADS
     if (rc != NNF_B200_OK)
@@ -211,26 +230,31 @@ PyObject* linear_register(PyObject* self, PyObject* args)
 
 PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
 {
-    unsigned long long fn, ctx;
-    Py_buffer w, w2;
+    unsigned long long fn;
+    Py_buffer w, w2, handle;
     int add;
-    PyObject *gain, *bias, *check;
+    PyObject *hobj, *gain, *bias, *check;
     w2.buf = nullptr;
-    if (!PyArg_ParseTuple(args, "KKy*z*iOOO", &fn, &ctx, &w, &w2, &add, &gain, &bias, &check))
+    if (!PyArg_ParseTuple(args, "KOy*z*iOOO", &fn, &hobj, &w, &w2, &add, &gain, &bias, &check))
         return nullptr;
     const bool sizes = w.len == (Py_ssize_t)sizeof(nnf_b200_qweight) && (!w2.buf || w2.len == (Py_ssize_t)sizeof(nnf_b200_qweight));
-    auto* entries = sizes ? new (std::nothrow) std::vector<LinearEntry>() : nullptr;
+    const bool held = sizes && hold_handle(hobj, &handle);
+    auto* entries = held ? new (std::nothrow) std::vector<LinearEntry>() : nullptr;
     LinearCall* c = entries ? reinterpret_cast<LinearCall*>(type->tp_alloc(type, 0)) : nullptr;
-    if (!c)
-        delete entries;
     if (!sizes)
         PyErr_SetString(PyExc_ValueError, "weight set size");
-    else if (!entries)
+    else if (held && !entries)
         PyErr_NoMemory();
+    if (!c)
+    {
+        delete entries;
+        if (held)
+            PyBuffer_Release(&handle);
+    }
     if (c)
     {
         c->fn = reinterpret_cast<LinearFn>(fn);
-        c->ctx = reinterpret_cast<nnf_b200_ctx*>(ctx);
+        c->handle = handle;
         memcpy(&c->w, w.buf, sizeof c->w);
         c->has_w2 = w2.buf != nullptr;
         if (c->has_w2)
@@ -248,6 +272,7 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
 void linear_dealloc(PyObject* self)
 {
     LinearCall* c = reinterpret_cast<LinearCall*>(self);
+    PyBuffer_Release(&c->handle);
     Py_XDECREF(c->gain);
     Py_XDECREF(c->bias);
     Py_XDECREF(c->check);
@@ -268,7 +293,7 @@ struct AttnCall
     PyObject_HEAD
     AttnFn fn;
     AttnWsFn ws_fn;
-    nnf_b200_ctx* ctx;
+    Py_buffer handle;
     nnf_b200_attn_desc desc;
     void* ws;
     size_t ws_bytes;
@@ -302,7 +327,8 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         }
         nnf_b200_attn_desc d = c->desc;
         d.position = (int32_t)position;
-        const size_t need = c->ws_fn(c->ctx, &d);
+        nnf_b200_ctx* const ctx = context(c->handle);
+        const size_t need = c->ws_fn(ctx, &d);
         if (need > c->ws_bytes)
             Py_RETURN_NONE;
         THPObjectPtr out;
@@ -324,7 +350,7 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         void* op = THPVariable_Unpack(out.get()).mutable_data_ptr();
         int rc;
         Py_BEGIN_ALLOW_THREADS
-        rc = c->fn(c->ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? c->ws : nullptr, need ? c->ws_bytes : 0);
+        rc = c->fn(ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? c->ws : nullptr, need ? c->ws_bytes : 0);
         Py_END_ALLOW_THREADS
         if (rc != NNF_B200_OK)
             return PyObject_CallFunction(c->check, "i", rc);
@@ -334,21 +360,28 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
 
 PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
 {
-    unsigned long long fn, ws_fn, ctx, ws, ws_bytes;
-    Py_buffer desc;
-    PyObject* check;
-    if (!PyArg_ParseTuple(args, "KKKy*KKO", &fn, &ws_fn, &ctx, &desc, &ws, &ws_bytes, &check))
+    unsigned long long fn, ws_fn, ws, ws_bytes;
+    Py_buffer desc, handle;
+    PyObject *hobj, *check;
+    if (!PyArg_ParseTuple(args, "KKOy*KKO", &fn, &ws_fn, &hobj, &desc, &ws, &ws_bytes, &check))
         return nullptr;
     if (desc.len != (Py_ssize_t)sizeof(nnf_b200_attn_desc))
     {
         PyBuffer_Release(&desc);
         return PyErr_Format(PyExc_ValueError, "descriptor size");
     }
+    if (!hold_handle(hobj, &handle))
+    {
+        PyBuffer_Release(&desc);
+        return nullptr;
+    }
     AttnCall* c = reinterpret_cast<AttnCall*>(type->tp_alloc(type, 0));
-    if (c)
+    if (!c)
+        PyBuffer_Release(&handle);
+    else
     {
         c->fn = reinterpret_cast<AttnFn>(fn), c->ws_fn = reinterpret_cast<AttnWsFn>(ws_fn);
-        c->ctx = reinterpret_cast<nnf_b200_ctx*>(ctx);
+        c->handle = handle;
         memcpy(&c->desc, desc.buf, sizeof c->desc);
         c->ws = reinterpret_cast<void*>(ws), c->ws_bytes = ws_bytes;
         c->check = Py_NewRef(check);
@@ -359,6 +392,7 @@ PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
 
 void attn_dealloc(PyObject* self)
 {
+    PyBuffer_Release(&reinterpret_cast<AttnCall*>(self)->handle);
     Py_XDECREF(reinterpret_cast<AttnCall*>(self)->check);
     Py_TYPE(self)->tp_free(self);
 }

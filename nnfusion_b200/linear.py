@@ -57,7 +57,7 @@ class Context:
     def close(self) -> None:
         if self.handle:
             self.lib.nnf_b200_free(self.handle)
-            self.handle = ctypes.c_void_p()
+            self.handle.value = None  # in place: prepared calls read it there
 
     def __del__(self):  # pragma: no cover
         try:
@@ -187,7 +187,7 @@ class DequantDot:
         if self._native is None:
             fn = ctypes.cast(self.ctx.lib.nnf_b200_linear, ctypes.c_void_p).value
             self._native = L.host_calls().LinearCall(
-                fn, self.ctx.handle.value, bytes(self._abi_w), bytes(self._abi_w2) if self._abi_w2 is not None else None,
+                fn, self.ctx.handle, bytes(self._abi_w), bytes(self._abi_w2) if self._abi_w2 is not None else None,
                 int(self.add), self.gain, self.bias, self.ctx.check)
         self._native.register(bytes(d), ws.data_ptr() if ws is not None else 0, ws.numel() if ws is not None else 0)
 

@@ -83,3 +83,25 @@ def test_an_allocation_that_fails_keeps_its_type():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert op(tx).shape == (4096, 65536)
+
+
+def test_calls_after_the_context_was_closed_are_refused():
+    """A prepared call must not use the context that its node's Context has given back."""
+    import torch
+    from nnfusion_b200.attention import DecodeAttention
+    from nnfusion_b200.linear import Context, DequantDot, DeviceWeight, NNFB200Error
+    ctx = Context(0)
+    x, w = synth.u4g128(15, 2, 64, 512)
+    op, at = DequantDot(DeviceWeight.from_host(w), ctx=ctx), DecodeAttention(2, 2, 128, 64, ctx=ctx)
+    tx, q = torch.from_numpy(x).cuda(), torch.zeros(256, dtype=torch.float16, device="cuda")
+    for _ in range(2):
+        op(tx)
+        at(q, q, q, 3)
+    assert op._native is not None and at._native is not None
+    torch.cuda.synchronize()
+    ctx.close()
+    for _ in range(2):
+        with pytest.raises(NNFB200Error):
+            op(tx)
+        with pytest.raises(NNFB200Error):
+            at(q, q, q, 3)

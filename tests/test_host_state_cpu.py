@@ -1,4 +1,5 @@
 """What a node keeps between calls, without a device: a stand-in for the library answers size queries."""
+import ctypes
 import types
 
 import pytest
@@ -46,6 +47,8 @@ def test_prepared_calls_refuse_descriptors_of_another_size():
     """Sizes are checked before anything is copied out of the buffers."""
     host = L.host_calls()
     with pytest.raises(ValueError):
-        host.LinearCall(0, 0, b"\0" * 8, None, 0, None, None, None)
+        host.LinearCall(0, ctypes.c_void_p(), b"\0" * 8, None, 0, None, None, None)
     with pytest.raises(ValueError):
-        host.AttnCall(0, 0, 0, b"\0" * 8, 0, 0, None)
+        host.AttnCall(0, 0, ctypes.c_void_p(), b"\0" * 8, 0, 0, None)
+    with pytest.raises(ValueError):
+        host.LinearCall(0, b"four", b"\0" * 24, None, 0, None, None, None)
