@@ -43,10 +43,7 @@ class DecodeAttention:
         lib = self.ctx.lib
         fn, ws_fn = (ctypes.cast(f, ctypes.c_void_p).value
                      for f in (lib.nnf_b200_decode_attention, lib.nnf_b200_decode_attention_workspace_bytes))
-        ws = self._ws.get("ws")
-        self._native = L.host_calls().AttnCall(fn, ws_fn, self.ctx.handle, bytes(d),
-                                               ws.data_ptr() if ws is not None else 0,
-                                               ws.numel() if ws is not None else 0, self.ctx.check)
+        self._native = L.host_calls().AttnCall(fn, ws_fn, self.ctx.handle, bytes(d), self._ws.get("ws"), self.ctx.check)
 
     def desc(self, position: int) -> L.AttnDesc:
         d = L.AttnDesc()

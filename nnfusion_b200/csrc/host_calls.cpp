@@ -57,8 +57,7 @@ PyObject* wrapped_empty(at::IntArrayRef sizes, c10::ScalarType dtype, c10::Devic
 struct LinearEntry
 {
     nnf_b200_linear_desc desc;
-    void* ws;
-    size_t ws_bytes;
+    PyObject* ws; // the workspace, a tensor that this entry keeps alive, or None
 };
 
 struct LinearCall
@@ -97,6 +96,17 @@ const void* address_of(PyObject* o)
     return o == Py_None ? nullptr : THPVariable_Unpack(o).const_data_ptr();
 }
 
+// A workspace: a tensor of bytes, or None.
+bool is_workspace(PyObject* o)
+{
+    return o == Py_None || (THPVariable_Check(o) && THPVariable_Unpack(o).is_contiguous() && THPVariable_Unpack(o).itemsize() == 1);
+}
+
+size_t bytes_of(PyObject* ws)
+{
+    return ws == Py_None ? 0 : (size_t)THPVariable_Unpack(ws).numel();
+}
+
 // y = node(x) with x [..., K]; lead: the output takes x's leading dimensions instead of [M, N].
 PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* paddend, bool lead)
 {
@@ -111,15 +121,15 @@ PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* p
     if (x->size(dims - 1) != K)
         Py_RETURN_NONE;
     const int64_t M = x->numel() / K;
-    LinearEntry e; // a copy: the call below runs without the interpreter lock
-    bool found = false;
+    LinearEntry e; // a copy, and a reference to its workspace: the call below runs without the interpreter lock
+    THPObjectPtr ws;
     for (const LinearEntry& c : *self->entries)
         if (c.desc.M == M && c.desc.x_dtype == xd)
         {
-            e = c, found = true;
+            e = c, ws = THPObjectPtr::dup(c.ws);
             break;
         }
-    if (!found || (self->add != 0) != (paddend != Py_None))
+    if (!ws || (self->add != 0) != (paddend != Py_None))
         Py_RETURN_NONE;
     const c10::ScalarType yt = e.desc.y_dtype == NNF_B200_F16 ? at::kHalf : at::kFloat;
     const void* bias = nullptr;
@@ -157,10 +167,12 @@ PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* p
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     const void *px_data = x->const_data_ptr(), *gain = address_of(self->gain);
     nnf_b200_ctx* const ctx = context(self->handle);
+    void* const ws_data = const_cast<void*>(address_of(ws.get()));
+    const size_t ws_bytes = bytes_of(ws.get());
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = self->fn(ctx, stream, &e.desc, px_data, &self->w, self->has_w2 ? &self->w2 : nullptr, gain, bias, y, e.ws,
-                  e.ws_bytes);
+    rc = self->fn(ctx, stream, &e.desc, px_data, &self->w, self->has_w2 ? &self->w2 : nullptr, gain, bias, y,
+                  ws_data, ws_bytes);
     Py_END_ALLOW_THREADS
     if (rc != NNF_B200_OK)
         return PyObject_CallFunction(self->check, "i", rc);
@@ -198,34 +210,35 @@ PyObject* linear_call_lead(PyObject* self, PyObject* const* args, Py_ssize_t n)
     });
 }
 
-// register(desc bytes, workspace address, workspace bytes)
+// register(desc bytes, workspace tensor or None)
 PyObject* linear_register(PyObject* self, PyObject* args)
 {
     Py_buffer desc;
-    unsigned long long ws, bytes;
-    if (!PyArg_ParseTuple(args, "y*KK", &desc, &ws, &bytes))
+    PyObject* ws;
+    if (!PyArg_ParseTuple(args, "y*O", &desc, &ws))
         return nullptr;
     LinearCall* c = reinterpret_cast<LinearCall*>(self);
-    const bool ok = desc.len == (Py_ssize_t)sizeof(nnf_b200_linear_desc);
+    const bool ok = desc.len == (Py_ssize_t)sizeof(nnf_b200_linear_desc) && is_workspace(ws);
+    LinearEntry e;
     if (ok)
-    {
-        LinearEntry e;
         memcpy(&e.desc, desc.buf, sizeof e.desc);
-        e.ws = reinterpret_cast<void*>(ws);
-        e.ws_bytes = bytes;
-        bool known = false;
+    PyBuffer_Release(&desc);
+    if (!ok)
+        return PyErr_Format(PyExc_ValueError, "register(descriptor bytes, workspace)");
+    return guarded([&]() -> PyObject* {
+        THPObjectPtr mine = THPObjectPtr::dup(ws), before;
+        e.ws = ws;
+        LinearEntry* known = nullptr;
         for (LinearEntry& q : *c->entries)
             if (q.desc.M == e.desc.M && q.desc.x_dtype == e.desc.x_dtype)
-                q = e, known = true;
-        PyBuffer_Release(&desc);
-        return guarded([&]() -> PyObject* {
-            if (!known)
-                c->entries->push_back(e);
-            Py_RETURN_NONE;
-        });
-    }
-    PyBuffer_Release(&desc);
-    return PyErr_Format(PyExc_ValueError, "descriptor size");
+                known = &q;
+        if (known)
+            before = known->ws, *known = e;
+        else
+            c->entries->push_back(e);
+        mine.release();
+        Py_RETURN_NONE;
+    });
 }
 
 PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
@@ -276,6 +289,8 @@ void linear_dealloc(PyObject* self)
     Py_XDECREF(c->gain);
     Py_XDECREF(c->bias);
     Py_XDECREF(c->check);
+    for (LinearEntry& e : *c->entries)
+        Py_DECREF(e.ws);
     delete c->entries;
     Py_TYPE(self)->tp_free(self);
 }
@@ -295,8 +310,7 @@ struct AttnCall
     AttnWsFn ws_fn;
     Py_buffer handle;
     nnf_b200_attn_desc desc;
-    void* ws;
-    size_t ws_bytes;
+    PyObject* ws; // the workspace, kept alive, or None
     PyObject* check;
 };
 
@@ -329,7 +343,8 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         d.position = (int32_t)position;
         nnf_b200_ctx* const ctx = context(c->handle);
         const size_t need = c->ws_fn(ctx, &d);
-        if (need > c->ws_bytes)
+        const size_t ws_bytes = bytes_of(c->ws);
+        if (need > ws_bytes)
             Py_RETURN_NONE;
         THPObjectPtr out;
         if (a[6] == Py_None)
@@ -348,9 +363,10 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         const void *qp = q->const_data_ptr(), *kp = k->const_data_ptr(), *vp = v->const_data_ptr();
         void *kcp = kc->mutable_data_ptr(), *vcp = vc->mutable_data_ptr();
         void* op = THPVariable_Unpack(out.get()).mutable_data_ptr();
+        void* const ws_data = const_cast<void*>(address_of(c->ws));
         int rc;
         Py_BEGIN_ALLOW_THREADS
-        rc = c->fn(ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? c->ws : nullptr, need ? c->ws_bytes : 0);
+        rc = c->fn(ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? ws_data : nullptr, need ? ws_bytes : 0);
         Py_END_ALLOW_THREADS
         if (rc != NNF_B200_OK)
             return PyObject_CallFunction(c->check, "i", rc);
@@ -360,15 +376,15 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
 
 PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
 {
-    unsigned long long fn, ws_fn, ws, ws_bytes;
+    unsigned long long fn, ws_fn;
     Py_buffer desc, handle;
-    PyObject *hobj, *check;
-    if (!PyArg_ParseTuple(args, "KKOy*KKO", &fn, &ws_fn, &hobj, &desc, &ws, &ws_bytes, &check))
+    PyObject *hobj, *ws, *check;
+    if (!PyArg_ParseTuple(args, "KKOy*OO", &fn, &ws_fn, &hobj, &desc, &ws, &check))
         return nullptr;
-    if (desc.len != (Py_ssize_t)sizeof(nnf_b200_attn_desc))
+    if (desc.len != (Py_ssize_t)sizeof(nnf_b200_attn_desc) || !is_workspace(ws))
     {
         PyBuffer_Release(&desc);
-        return PyErr_Format(PyExc_ValueError, "descriptor size");
+        return PyErr_Format(PyExc_ValueError, "descriptor size, or no workspace");
     }
     if (!hold_handle(hobj, &handle))
     {
@@ -383,7 +399,7 @@ PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
         c->fn = reinterpret_cast<AttnFn>(fn), c->ws_fn = reinterpret_cast<AttnWsFn>(ws_fn);
         c->handle = handle;
         memcpy(&c->desc, desc.buf, sizeof c->desc);
-        c->ws = reinterpret_cast<void*>(ws), c->ws_bytes = ws_bytes;
+        c->ws = Py_NewRef(ws);
         c->check = Py_NewRef(check);
     }
     PyBuffer_Release(&desc);
@@ -393,6 +409,7 @@ PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
 void attn_dealloc(PyObject* self)
 {
     PyBuffer_Release(&reinterpret_cast<AttnCall*>(self)->handle);
+    Py_XDECREF(reinterpret_cast<AttnCall*>(self)->ws);
     Py_XDECREF(reinterpret_cast<AttnCall*>(self)->check);
     Py_TYPE(self)->tp_free(self);
 }

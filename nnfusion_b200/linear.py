@@ -177,7 +177,7 @@ class DequantDot:
     def __setattr__(self, name, value):
         """Calls that are already prepared (``_native``) hold what the attributes said: a change makes them stale."""
         object.__setattr__(self, name, value)
-        if name not in ("_native", "_ws"):
+        if name != "_native":
             object.__setattr__(self, "_native", None)
 
     def _prepared(self, d: L.LinearDesc, ws: Optional[torch.Tensor]) -> None:
@@ -189,7 +189,7 @@ class DequantDot:
             self._native = L.host_calls().LinearCall(
                 fn, self.ctx.handle, bytes(self._abi_w), bytes(self._abi_w2) if self._abi_w2 is not None else None,
                 int(self.add), self.gain, self.bias, self.ctx.check)
-        self._native.register(bytes(d), ws.data_ptr() if ws is not None else 0, ws.numel() if ws is not None else 0)
+        self._native.register(bytes(d), ws)
 
     def desc(self, M: int, x_dtype: torch.dtype) -> L.LinearDesc:
         d = L.LinearDesc()

@@ -105,3 +105,25 @@ def test_calls_after_the_context_was_closed_are_refused():
             op(tx)
         with pytest.raises(NNFB200Error):
             at(q, q, q, 3)
+
+
+def test_a_workspace_that_the_node_lets_go_is_not_used_after():
+    """The buffers of prepared calls belong to them: calls give the same result when the node's own table is emptied and
+    the memory is asked for by somebody else."""
+    import torch
+    from nnfusion_b200.attention import DecodeAttention
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    x, w = synth.u4g128(16, 8, 512, 10240)
+    op, at = DequantDot(DeviceWeight.from_host(w), split_k=4), DecodeAttention(8, 1, 128, 8192)
+    at.k_cache.normal_()
+    at.v_cache.normal_()
+    tx, q = torch.from_numpy(x).cuda(), torch.ones(1024, dtype=torch.float16, device="cuda")
+    first = op(tx), at(q, q[:128], q[:128], 8000)
+    sizes = [t.numel() for t in (*op._ws.values(), *at._ws.values())]
+    assert min(sizes) > 0
+    op._ws.clear()
+    at._ws.clear()
+    others = [torch.full((n + 256,), 0xAB, dtype=torch.uint8, device="cuda") for n in sizes for _ in range(3)]
+    for _ in range(2):
+        assert torch.equal(op(tx), first[0]) and torch.equal(at(q, q[:128], q[:128], 8000), first[1])
+    assert all(bool((t == 0xAB).all()) for t in others)
