@@ -127,3 +127,15 @@ def test_a_workspace_that_the_node_lets_go_is_not_used_after():
     for _ in range(2):
         assert torch.equal(op(tx), first[0]) and torch.equal(at(q, q[:128], q[:128], 8000), first[1])
     assert all(bool((t == 0xAB).all()) for t in others)
+
+
+def test_module_whose_weights_became_a_parameter():
+    import torch
+    from nnfusion_b200.jit import QuantLinear, jit
+    x, w = synth.u4g128(17, 2, 48, 256)
+    m = jit(QuantLinear.from_host(w).cuda())
+    tx = torch.from_numpy(x).cuda()
+    first = m(tx)
+    m.wq = torch.nn.Parameter(m.wq.clone(), requires_grad=False)  # no longer among the buffers
+    assert "wq" not in m._buffers
+    assert torch.equal(m(tx), first) and torch.equal(m(tx), first)
