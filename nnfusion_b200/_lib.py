@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libnnf_b200.so")
@@ -65,16 +66,18 @@ _host_calls = None
 
 
 def host_calls():
-    """The extension module behind repeated calls of a node (``csrc/host_calls.cpp``); raises if it has not been built."""
+    """The extension module behind repeated calls of a node (``csrc/host_calls.cpp``), or None where it cannot be loaded:
+    it saves host time only, every call works through ctypes as well.  Says so once."""
     global _host_calls
     if _host_calls is None:
         try:
             from . import _host_calls as module
+            _host_calls = module
         except ImportError as e:
-            raise RuntimeError("nnfusion_b200/_host_calls.so cannot be loaded: build it with "
-                               f"`python -m nnfusion_b200.build` ({e})") from e
-        _host_calls = module
-    return _host_calls
+            _host_calls = False
+            warnings.warn("nnfusion_b200/_host_calls.so cannot be loaded, calls take about 10 us more host time: build it "
+                          f"with `python -m nnfusion_b200.build` ({e})", RuntimeWarning, stacklevel=3)
+    return _host_calls or None
 
 
 def load() -> ctypes.CDLL:

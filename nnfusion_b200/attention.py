@@ -40,10 +40,13 @@ class DecodeAttention:
 
     def _prepared(self, d: L.AttnDesc) -> None:
         """Later calls skip ``__call__``'s Python path (``csrc/host_calls.cpp``)."""
+        host = L.host_calls()
+        if host is None:
+            return
         lib = self.ctx.lib
         fn, ws_fn = (ctypes.cast(f, ctypes.c_void_p).value
                      for f in (lib.nnf_b200_decode_attention, lib.nnf_b200_decode_attention_workspace_bytes))
-        self._native = L.host_calls().AttnCall(fn, ws_fn, self.ctx.handle, bytes(d), self._ws.get("ws"), self.ctx.check)
+        self._native = host.AttnCall(fn, ws_fn, self.ctx.handle, bytes(d), self._ws.get("ws"), self.ctx.check)
 
     def desc(self, position: int) -> L.AttnDesc:
         d = L.AttnDesc()

@@ -184,9 +184,12 @@ class DequantDot:
         """Later calls with this row count and type skip ``__call__``'s Python path (``csrc/host_calls.cpp``)."""
         if self.kernel_db is not None:
             return  # the launch choice is looked up at every call
+        host = L.host_calls()
+        if host is None:
+            return
         if self._native is None:
             fn = ctypes.cast(self.ctx.lib.nnf_b200_linear, ctypes.c_void_p).value
-            self._native = L.host_calls().LinearCall(
+            self._native = host.LinearCall(
                 fn, self.ctx.handle, bytes(self._abi_w), bytes(self._abi_w2) if self._abi_w2 is not None else None,
                 int(self.add), self.gain, self.bias, self.ctx.check)
         self._native.register(bytes(d), ws)

@@ -139,3 +139,18 @@ def test_module_whose_weights_became_a_parameter():
     m.wq = torch.nn.Parameter(m.wq.clone(), requires_grad=False)  # no longer among the buffers
     assert "wq" not in m._buffers
     assert torch.equal(m(tx), first) and torch.equal(m(tx), first)
+
+
+def test_calls_without_the_extension(monkeypatch):
+    import torch
+    from nnfusion_b200 import _lib as L
+    from nnfusion_b200.attention import DecodeAttention
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    x, w = synth.u4g128(18, 2, 64, 512)
+    tx, q = torch.from_numpy(x).cuda(), torch.ones(256, dtype=torch.float16, device="cuda")
+    want = DequantDot(DeviceWeight.from_host(w))(tx), DecodeAttention(2, 2, 128, 64)(q, q, q, 0)
+    monkeypatch.setattr(L, "_host_calls", False)
+    op, at = DequantDot(DeviceWeight.from_host(w)), DecodeAttention(2, 2, 128, 64)
+    for _ in range(2):
+        assert torch.equal(op(tx), want[0]) and torch.equal(at(q, q, q, 0), want[1])
+    assert op._native is None and at._native is None
