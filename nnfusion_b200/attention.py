@@ -30,23 +30,28 @@ class DecodeAttention:
         self.k_cache = torch.zeros((kv_heads, capacity, head_dim), dtype=torch.float16, device=dev)
         self.v_cache = torch.zeros((kv_heads, capacity, head_dim), dtype=torch.float16, device=dev)
         self._ws: dict = {}
-        self._native = None
+
+    _native = None  # what calls go through (``csrc/host_calls.cpp``), made by the first one
 
     def __setattr__(self, name, value):
-        """The prepared call (``_native``) holds what the attributes said: a change makes it stale."""
+        """``_native`` holds what the attributes said: a change makes it stale."""
         object.__setattr__(self, name, value)
-        if name != "_native":
+        if name != "_native" and self._native is not None:
             object.__setattr__(self, "_native", None)
 
-    def _prepared(self, d: L.AttnDesc) -> None:
-        """Later calls skip ``__call__``'s Python path (``csrc/host_calls.cpp``)."""
+    def _prepare(self):
+        """The native side of ``__call__``, or None where its extension is missing."""
         host = L.host_calls()
-        if host is None:
-            return
-        lib = self.ctx.lib
-        fn, ws_fn = (ctypes.cast(f, ctypes.c_void_p).value
-                     for f in (lib.nnf_b200_decode_attention, lib.nnf_b200_decode_attention_workspace_bytes))
-        self._native = host.AttnCall(fn, ws_fn, self.ctx.handle, bytes(d), self._ws.get("ws"), self.ctx.check)
+        if host is not None:
+            ws = self._ws.get((self.heads, self.kv_heads))
+            self._native = host.AttnCall(self.ctx.entry_point("nnf_b200_decode_attention"),
+                                         self.ctx.entry_point("nnf_b200_decode_attention_workspace_bytes"),
+                                         self.ctx.handle, bytes(self.desc(0)), ws, self.ctx.check)
+        return self._native
+
+    def _grown(self, position: int) -> Optional[torch.Tensor]:
+        """A workspace for ``position`` (asked for by the native side when the one it has is too small)."""
+        return self.workspace(self.desc(position))
 
     def desc(self, position: int) -> L.AttnDesc:
         d = L.AttnDesc()
@@ -62,7 +67,8 @@ class DecodeAttention:
         n = int(self.ctx.lib.nnf_b200_decode_attention_workspace_bytes(self.ctx.handle, ctypes.byref(d)))
         if n == 0:
             return None
-        ws = self._ws.get("ws")
+        key = (self.heads, self.kv_heads)  # the counters' layout
+        ws = self._ws.get(key)
         if ws is None or ws.numel() < n:
             # sized for the longest sequence the caches can hold, zeroed once
             full = self.desc(self.capacity - 1)
@@ -73,13 +79,14 @@ class DecodeAttention:
             ws = raw[off:off + cap]
             stream = torch.cuda.current_stream().cuda_stream
             self.ctx.check(self.ctx.lib.nnf_b200_workspace_reset(self.ctx.handle, stream, ws.data_ptr(), cap))
-            self._ws["ws"] = ws
+            self._ws[key] = ws
         return ws
 
     def __call__(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, position: int,
                  out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        if self._native is not None:
-            y = self._native.call(q, k_new, v_new, self.k_cache, self.v_cache, position, out)
+        native = self._native or self._prepare()
+        if native is not None:
+            y = native.call(self, q, k_new, v_new, self.k_cache, self.v_cache, position, out)
             if y is not None:
                 return y
         hd, kd = self.heads * self.head_dim, self.kv_heads * self.head_dim
@@ -96,5 +103,4 @@ class DecodeAttention:
             self.k_cache.data_ptr(), self.v_cache.data_ptr(), out.data_ptr(),
             ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0)
         self.ctx.check(rc)
-        self._prepared(d)
         return out

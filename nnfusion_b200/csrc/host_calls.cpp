@@ -1,16 +1,18 @@
-// The host side of a node's repeated call, as a CPython extension: what DequantDot / DecodeAttention do between "the
-// user has a tensor" and "the C ABI is called" once a call of the same shape has been seen.
+// The host side of a node's call, as a CPython extension: what DequantDot / DecodeAttention do between "the user has a
+// tensor" and "the C ABI is called".
 //
 // A decode step is a chain of launches of a few microseconds each, so the time the host spends per launch is part of
 // the step: through ctypes and torch's Python wrappers (descriptor fields, workspace lookup, current stream, nine
 // converted arguments) a call took 13 to 19 us of host time for 4 to 8 us of GPU time.  Here a call is: look at the
-// tensor, find the entry for its row count and type, allocate the output, take the current stream, call the C ABI.
+// tensor, find the entry for its row count and type, allocate the output, take the current stream, call the C ABI.  A row
+// count and type that has not been seen asks the node for its descriptor and workspace first (a prompt's length is new more
+// often than not: 20 us where the Python path takes 28).
 //
-// The objects here never decide anything on their own.  Whatever is not the plain, already prepared case (a new row
-// count, a tensor that is not a contiguous CUDA tensor of the right shape, an addend that is missing) makes the call
-// return None, and the Python method runs its full path, which checks, raises and prepares as it always did.
+// The objects here never decide anything on their own.  Whatever is not the plain case (a tensor that is not a contiguous
+// CUDA tensor of the right shape, an addend that is missing) makes the call return None, and the Python method runs its full
+// path, which checks and raises.
 //
-// Entries are registered and looked up under the interpreter lock.
+// Entries are added and looked up under the interpreter lock.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
@@ -19,7 +21,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <cstring>
 #include <new>
-#include <vector>
+#include <unordered_map>
 
 #include "nnf_b200.h"
 
@@ -52,12 +54,23 @@ PyObject* wrapped_empty(at::IntArrayRef sizes, c10::ScalarType dtype, c10::Devic
     return THPVariable_Wrap(at::Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt)));
 }
 
+// A workspace: a tensor of bytes, or None.
+bool is_workspace(PyObject* o)
+{
+    return o == Py_None || (THPVariable_Check(o) && THPVariable_Unpack(o).is_contiguous() && THPVariable_Unpack(o).itemsize() == 1);
+}
+
+size_t bytes_of(PyObject* ws)
+{
+    return ws == Py_None ? 0 : (size_t)THPVariable_Unpack(ws).numel();
+}
+
 // ---------------------------------------------------------------------------------------------------- linear
 
 struct LinearEntry
 {
     nnf_b200_linear_desc desc;
-    PyObject* ws; // the workspace, a tensor that this entry keeps alive, or None
+    PyObject* ws = nullptr; // the workspace, a tensor that this entry keeps alive, or None
 };
 
 struct LinearCall
@@ -70,8 +83,46 @@ struct LinearCall
     PyObject* gain;  // tensors or None: their addresses are read at every call
     PyObject* bias;
     PyObject* check; // Context.check: raises for a status that is not OK
-    std::vector<LinearEntry>* entries;
+    int64_t N, K;
+    std::unordered_map<uint64_t, LinearEntry>* entries; // by row count and type
 };
+constexpr size_t kMaxEntries = 4096; // beyond that they are all let go and made again
+
+void clear_entries(LinearCall* c)
+{
+    std::unordered_map<uint64_t, LinearEntry> old;
+    old.swap(*c->entries);
+    for (auto& e : old)
+        Py_DECREF(e.second.ws);
+}
+
+// Adds the entry that the node gives for a row count and type: (descriptor bytes, workspace or None).
+bool add_entry(LinearCall* c, PyObject* node, int64_t M, int xd, LinearEntry* e, THPObjectPtr* ws)
+{
+    THPObjectPtr plan(PyObject_CallMethod(node, "_plan", "Li", (long long)M, xd));
+    Py_buffer desc;
+    PyObject* w;
+    if (!plan || !PyArg_ParseTuple(plan.get(), "y*O", &desc, &w))
+        return false;
+    const bool ok = desc.len == (Py_ssize_t)sizeof e->desc && is_workspace(w);
+    if (ok)
+        memcpy(&e->desc, desc.buf, sizeof e->desc);
+    PyBuffer_Release(&desc);
+    if (!ok)
+    {
+        PyErr_SetString(PyExc_ValueError, "_plan: (descriptor bytes, workspace)");
+        return false;
+    }
+    *ws = THPObjectPtr::dup(w);
+    e->ws = w;
+    if (c->entries->size() >= kMaxEntries)
+        clear_entries(c);
+    LinearEntry& slot = (*c->entries)[(uint64_t)M << 1 | (uint64_t)xd];
+    THPObjectPtr before(slot.ws); // (another thread may have been here meanwhile)
+    slot = *e;
+    Py_INCREF(w);
+    return true;
+}
 
 // The library's context, as the node's Context holds it now: null once that has been closed (the C ABI then refuses).
 nnf_b200_ctx* context(const Py_buffer& handle)
@@ -96,41 +147,27 @@ const void* address_of(PyObject* o)
     return o == Py_None ? nullptr : THPVariable_Unpack(o).const_data_ptr();
 }
 
-// A workspace: a tensor of bytes, or None.
-bool is_workspace(PyObject* o)
-{
-    return o == Py_None || (THPVariable_Check(o) && THPVariable_Unpack(o).is_contiguous() && THPVariable_Unpack(o).itemsize() == 1);
-}
-
-size_t bytes_of(PyObject* ws)
-{
-    return ws == Py_None ? 0 : (size_t)THPVariable_Unpack(ws).numel();
-}
-
 // y = node(x) with x [..., K]; lead: the output takes x's leading dimensions instead of [M, N].
-PyObject* linear_run(LinearCall* self, PyObject* px, PyObject* pout, PyObject* paddend, bool lead)
+PyObject* linear_run(LinearCall* self, PyObject* node, PyObject* px, PyObject* pout, PyObject* paddend, bool lead)
 {
     const at::Tensor* x = plain_cuda(px);
     if (!x)
         Py_RETURN_NONE;
     const int xd = dtype_code(x->scalar_type());
     const int64_t dims = x->dim();
-    if (xd < 0 || (lead ? dims < 1 : dims != 2) || self->entries->empty())
-        Py_RETURN_NONE;
-    const int64_t K = self->entries->front().desc.K, N = self->entries->front().desc.N;
-    if (x->size(dims - 1) != K)
+    const int64_t K = self->K, N = self->N;
+    if (xd < 0 || (lead ? dims < 1 : dims != 2) || x->size(dims - 1) != K || (self->add != 0) != (paddend != Py_None))
         Py_RETURN_NONE;
     const int64_t M = x->numel() / K;
+    if (M < 1 || M > INT32_MAX)
+        Py_RETURN_NONE;
     LinearEntry e; // a copy, and a reference to its workspace: the call below runs without the interpreter lock
     THPObjectPtr ws;
-    for (const LinearEntry& c : *self->entries)
-        if (c.desc.M == M && c.desc.x_dtype == xd)
-        {
-            e = c, ws = THPObjectPtr::dup(c.ws);
-            break;
-        }
-    if (!ws || (self->add != 0) != (paddend != Py_None))
-        Py_RETURN_NONE;
+    const auto known = self->entries->find((uint64_t)M << 1 | (uint64_t)xd);
+    if (known != self->entries->end())
+        e = known->second, ws = THPObjectPtr::dup(e.ws);
+    else if (!add_entry(self, node, M, xd, &e, &ws))
+        return nullptr;
     const c10::ScalarType yt = e.desc.y_dtype == NNF_B200_F16 ? at::kHalf : at::kFloat;
     const void* bias = nullptr;
     if (paddend != Py_None)
@@ -188,56 +225,25 @@ PyObject* guarded(Body&& body)
     END_HANDLE_TH_ERRORS
 }
 
-// call(x, out, addend) -> tensor or None
+// call(node, x, out, addend) -> tensor or None
 PyObject* linear_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
 {
-    if (n != 3)
-        return PyErr_Format(PyExc_TypeError, "call(x, out, addend)");
-    return guarded([&] { return linear_run(reinterpret_cast<LinearCall*>(self), args[0], args[1], args[2], false); });
+    if (n != 4)
+        return PyErr_Format(PyExc_TypeError, "call(node, x, out, addend)");
+    return guarded([&] { return linear_run(reinterpret_cast<LinearCall*>(self), args[0], args[1], args[2], args[3], false); });
 }
 
-// call_lead(x, wq) -> tensor or None: any leading dimensions; None too when wq is no longer the tensor the node was
+// call_lead(node, x, wq) -> tensor or None: any leading dimensions; None too when wq is no longer the tensor the node was
 // built for.
 PyObject* linear_call_lead(PyObject* self, PyObject* const* args, Py_ssize_t n)
 {
-    if (n != 2)
-        return PyErr_Format(PyExc_TypeError, "call_lead(x, wq)");
+    if (n != 3)
+        return PyErr_Format(PyExc_TypeError, "call_lead(node, x, wq)");
     return guarded([&]() -> PyObject* {
         LinearCall* c = reinterpret_cast<LinearCall*>(self);
-        if (!THPVariable_Check(args[1]) || THPVariable_Unpack(args[1]).const_data_ptr() != c->w.wq)
+        if (!THPVariable_Check(args[2]) || THPVariable_Unpack(args[2]).const_data_ptr() != c->w.wq)
             Py_RETURN_NONE;
-        return linear_run(c, args[0], Py_None, Py_None, true);
-    });
-}
-
-// register(desc bytes, workspace tensor or None)
-PyObject* linear_register(PyObject* self, PyObject* args)
-{
-    Py_buffer desc;
-    PyObject* ws;
-    if (!PyArg_ParseTuple(args, "y*O", &desc, &ws))
-        return nullptr;
-    LinearCall* c = reinterpret_cast<LinearCall*>(self);
-    const bool ok = desc.len == (Py_ssize_t)sizeof(nnf_b200_linear_desc) && is_workspace(ws);
-    LinearEntry e;
-    if (ok)
-        memcpy(&e.desc, desc.buf, sizeof e.desc);
-    PyBuffer_Release(&desc);
-    if (!ok)
-        return PyErr_Format(PyExc_ValueError, "register(descriptor bytes, workspace)");
-    return guarded([&]() -> PyObject* {
-        THPObjectPtr mine = THPObjectPtr::dup(ws), before;
-        e.ws = ws;
-        LinearEntry* known = nullptr;
-        for (LinearEntry& q : *c->entries)
-            if (q.desc.M == e.desc.M && q.desc.x_dtype == e.desc.x_dtype)
-                known = &q;
-        if (known)
-            before = known->ws, *known = e;
-        else
-            c->entries->push_back(e);
-        mine.release();
-        Py_RETURN_NONE;
+        return linear_run(c, args[0], args[1], Py_None, Py_None, true);
     });
 }
 
@@ -246,16 +252,17 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
     unsigned long long fn;
     Py_buffer w, w2, handle;
     int add;
+    long long N, K;
     PyObject *hobj, *gain, *bias, *check;
     w2.buf = nullptr;
-    if (!PyArg_ParseTuple(args, "KOy*z*iOOO", &fn, &hobj, &w, &w2, &add, &gain, &bias, &check))
+    if (!PyArg_ParseTuple(args, "KOy*z*iOOOLL", &fn, &hobj, &w, &w2, &add, &gain, &bias, &check, &N, &K))
         return nullptr;
-    const bool sizes = w.len == (Py_ssize_t)sizeof(nnf_b200_qweight) && (!w2.buf || w2.len == (Py_ssize_t)sizeof(nnf_b200_qweight));
+    const bool sizes = N > 0 && K > 0 && w.len == (Py_ssize_t)sizeof(nnf_b200_qweight) && (!w2.buf || w2.len == (Py_ssize_t)sizeof(nnf_b200_qweight));
     const bool held = sizes && hold_handle(hobj, &handle);
-    auto* entries = held ? new (std::nothrow) std::vector<LinearEntry>() : nullptr;
+    auto* entries = held ? new (std::nothrow) std::unordered_map<uint64_t, LinearEntry>() : nullptr;
     LinearCall* c = entries ? reinterpret_cast<LinearCall*>(type->tp_alloc(type, 0)) : nullptr;
     if (!sizes)
-        PyErr_SetString(PyExc_ValueError, "weight set size");
+        PyErr_SetString(PyExc_ValueError, "weight set or matrix size");
     else if (held && !entries)
         PyErr_NoMemory();
     if (!c)
@@ -274,6 +281,7 @@ PyObject* linear_new(PyTypeObject* type, PyObject* args, PyObject*)
             memcpy(&c->w2, w2.buf, sizeof c->w2);
         c->add = add;
         c->gain = Py_NewRef(gain), c->bias = Py_NewRef(bias), c->check = Py_NewRef(check);
+        c->N = N, c->K = K;
         c->entries = entries;
     }
     PyBuffer_Release(&w);
@@ -289,8 +297,7 @@ void linear_dealloc(PyObject* self)
     Py_XDECREF(c->gain);
     Py_XDECREF(c->bias);
     Py_XDECREF(c->check);
-    for (LinearEntry& e : *c->entries)
-        Py_DECREF(e.ws);
+    clear_entries(c);
     delete c->entries;
     Py_TYPE(self)->tp_free(self);
 }
@@ -298,7 +305,6 @@ void linear_dealloc(PyObject* self)
 PyMethodDef linear_methods[] = {
     {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(linear_call)), METH_FASTCALL, nullptr},
     {"call_lead", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(linear_call_lead)), METH_FASTCALL, nullptr},
-    {"register", linear_register, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
 // ---------------------------------------------------------------------------------------------------- attention
@@ -320,13 +326,13 @@ const at::Tensor* half_of(PyObject* o, int64_t numel)
     return t && t->scalar_type() == at::kHalf && t->numel() == numel ? t : nullptr;
 }
 
-// call(q, k_new, v_new, k_cache, v_cache, position, out) -> tensor or None
+// call(node, q, k_new, v_new, k_cache, v_cache, position, out) -> tensor or None
 PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
 {
-    if (n != 7)
-        return PyErr_Format(PyExc_TypeError, "call(q, k_new, v_new, k_cache, v_cache, position, out)");
+    if (n != 8)
+        return PyErr_Format(PyExc_TypeError, "call(node, q, k_new, v_new, k_cache, v_cache, position, out)");
     return guarded([&]() -> PyObject* {
-        PyObject* const* a = args;
+        PyObject* const* a = args + 1;
         AttnCall* c = reinterpret_cast<AttnCall*>(self);
         const int64_t hd = (int64_t)c->desc.heads * c->desc.head_dim, kd = (int64_t)c->desc.kv_heads * c->desc.head_dim;
         const at::Tensor *q = half_of(a[0], hd), *k = half_of(a[1], kd), *v = half_of(a[2], kd);
@@ -343,9 +349,20 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         d.position = (int32_t)position;
         nnf_b200_ctx* const ctx = context(c->handle);
         const size_t need = c->ws_fn(ctx, &d);
-        const size_t ws_bytes = bytes_of(c->ws);
-        if (need > ws_bytes)
-            Py_RETURN_NONE;
+        if (need > bytes_of(c->ws))
+        {
+            THPObjectPtr grown(PyObject_CallMethod(args[0], "_grown", "l", position));
+            if (!grown)
+                return nullptr;
+            if (!is_workspace(grown.get()) || bytes_of(grown.get()) < need)
+                Py_RETURN_NONE;
+            PyObject* const before = c->ws;
+            c->ws = grown.release();
+            Py_DECREF(before);
+        }
+        // (referenced: the call below runs without the interpreter lock)
+        THPObjectPtr ws = THPObjectPtr::dup(c->ws);
+        const size_t ws_bytes = bytes_of(ws.get());
         THPObjectPtr out;
         if (a[6] == Py_None)
         {
@@ -363,7 +380,7 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         const void *qp = q->const_data_ptr(), *kp = k->const_data_ptr(), *vp = v->const_data_ptr();
         void *kcp = kc->mutable_data_ptr(), *vcp = vc->mutable_data_ptr();
         void* op = THPVariable_Unpack(out.get()).mutable_data_ptr();
-        void* const ws_data = const_cast<void*>(address_of(c->ws));
+        void* const ws_data = const_cast<void*>(address_of(ws.get()));
         int rc;
         Py_BEGIN_ALLOW_THREADS
         rc = c->fn(ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? ws_data : nullptr, need ? ws_bytes : 0);

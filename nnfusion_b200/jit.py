@@ -75,8 +75,9 @@ class QuantLinear(torch.nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         node = self._node
-        if node is not None and node._native is not None:
-            y = node._native.call_lead(x, self._buffers.get("wq"))
+        native = (node._native or node._prepare()) if node is not None else None
+        if native is not None:
+            y = native.call_lead(node, x, self._buffers.get("wq"))
             if y is not None:
                 return y
         lead = x.shape[:-1]

@@ -33,6 +33,7 @@ class Context:
         self.lib = L.load()
         self.handle = ctypes.c_void_p()
         self.device = device
+        self._entry_points: dict = {}
         rc = self.lib.nnf_b200_init(device, ctypes.byref(self.handle))
         if rc != L.OK:
             raise NNFB200Error(rc, self.lib.nnf_b200_strerror(rc).decode(), "nnf_b200_init")
@@ -41,6 +42,12 @@ class Context:
         if rc != L.OK:
             raise NNFB200Error(rc, self.lib.nnf_b200_strerror(rc).decode(),
                                self.lib.nnf_b200_last_error(self.handle).decode())
+
+    def entry_point(self, name: str) -> int:
+        """Address of a function of the library."""
+        if name not in self._entry_points:
+            self._entry_points[name] = ctypes.cast(getattr(self.lib, name), ctypes.c_void_p).value
+        return self._entry_points[name]
 
     @property
     def sm_count(self) -> int:
@@ -76,6 +83,7 @@ def default_context(device: int = 0) -> Context:
 
 
 _DT = {torch.float32: L.F32, torch.float16: L.F16}
+_TORCH = {code: dtype for dtype, code in _DT.items()}
 
 
 @dataclass
@@ -172,27 +180,29 @@ class DequantDot:
         self._ws: dict = {}
         self._abi_w = weight.abi()
         self._abi_w2 = weight2.abi() if weight2 is not None else None
-        self._native = None
+
+    _native = None  # what calls go through (``csrc/host_calls.cpp``), made by the first one
 
     def __setattr__(self, name, value):
-        """Calls that are already prepared (``_native``) hold what the attributes said: a change makes them stale."""
+        """``_native`` holds what the attributes said: a change makes it stale."""
         object.__setattr__(self, name, value)
-        if name != "_native":
+        if name != "_native" and self._native is not None:
             object.__setattr__(self, "_native", None)
 
-    def _prepared(self, d: L.LinearDesc, ws: Optional[torch.Tensor]) -> None:
-        """Later calls with this row count and type skip ``__call__``'s Python path (``csrc/host_calls.cpp``)."""
-        if self.kernel_db is not None:
-            return  # the launch choice is looked up at every call
-        host = L.host_calls()
-        if host is None:
-            return
-        if self._native is None:
-            fn = ctypes.cast(self.ctx.lib.nnf_b200_linear, ctypes.c_void_p).value
+    def _prepare(self):
+        """The native side of ``__call__``, or None where every call takes the Python path."""
+        host = L.host_calls() if self.kernel_db is None else None  # (a launch choice is looked up at every call)
+        if host is not None:
             self._native = host.LinearCall(
-                fn, self.ctx.handle, bytes(self._abi_w), bytes(self._abi_w2) if self._abi_w2 is not None else None,
-                int(self.add), self.gain, self.bias, self.ctx.check)
-        self._native.register(bytes(d), ws)
+                self.ctx.entry_point("nnf_b200_linear"), self.ctx.handle, bytes(self._abi_w),
+                bytes(self._abi_w2) if self._abi_w2 is not None else None, int(self.add), self.gain, self.bias,
+                self.ctx.check, self.w.N, self.w.K)
+        return self._native
+
+    def _plan(self, M: int, x_dtype: int):
+        """Descriptor and workspace of calls with ``M`` rows (asked for by the native side when they are new)."""
+        d = self.desc(M, _TORCH[x_dtype])
+        return bytes(d), self.workspace(d)
 
     def desc(self, M: int, x_dtype: torch.dtype) -> L.LinearDesc:
         d = L.LinearDesc()
@@ -236,8 +246,9 @@ class DequantDot:
 
     def __call__(self, x: torch.Tensor, out: Optional[torch.Tensor] = None,
                  addend: Optional[torch.Tensor] = None) -> torch.Tensor:
-        if self._native is not None:
-            y = self._native.call(x, out, addend)
+        native = self._native or self._prepare()
+        if native is not None:
+            y = native.call(self, x, out, addend)
             if y is not None:
                 return y
         if x.dim() != 2 or x.shape[1] != self.w.K or not x.is_contiguous():
@@ -253,7 +264,6 @@ class DequantDot:
             raise ValueError("addend must be a contiguous [M, N] tensor of the output's dtype")
         ws = self.workspace(d)
         self.run_raw(d, x.data_ptr(), out.data_ptr(), ws, addend.data_ptr() if addend is not None else None)
-        self._prepared(d, ws)
         return out
 
     def host_entry(self, x_host: torch.Tensor, y_host: torch.Tensor) -> torch.Tensor:

@@ -1,5 +1,5 @@
-"""Repeated calls go through ``csrc/host_calls.cpp``: same bits as the first call's Python path, same errors, and no
-stale descriptor after an attribute of the node has changed."""
+"""Calls go through ``csrc/host_calls.cpp``: same bits and same errors as the Python path, and no stale descriptor after an
+attribute of the node has changed."""
 import numpy as np
 import pytest
 
@@ -154,3 +154,31 @@ def test_calls_without_the_extension(monkeypatch):
     for _ in range(2):
         assert torch.equal(op(tx), want[0]) and torch.equal(at(q, q, q, 0), want[1])
     assert op._native is None and at._native is None
+
+
+def test_new_row_counts_take_the_native_path(monkeypatch):
+    """A row count or a position that has not been seen costs its plan, not the Python path; and a node's table of row
+    counts is bounded."""
+    import torch
+    from nnfusion_b200.attention import DecodeAttention
+    from nnfusion_b200.jit import QuantLinear, jit
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    x, w = synth.u4g128(19, 40, 48, 256)
+    dw, tx = DeviceWeight.from_host(w), torch.from_numpy(x).cuda()
+    rows = [1, 2, 16, 17, 40]
+    with monkeypatch.context() as m:
+        m.setattr(DequantDot, "_prepare", lambda self: None)
+        want = [DequantDot(dw)(tx[:r]) for r in rows]
+    module = jit(QuantLinear.from_host(w).cuda())
+    op, at = DequantDot(dw), DecodeAttention(2, 1, 128, 2048)
+    monkeypatch.setattr(DequantDot, "run_raw", None)            # the Python path's launch
+    for r, y in zip(rows, want):
+        assert torch.equal(op(tx[:r]), y) and torch.equal(op(tx[:r]), y) and torch.equal(module(tx[None, :r])[0], y)
+    q = torch.ones(256, dtype=torch.float16, device="cuda")
+    for position in (0, 40, 500, 2000, 3):                      # no workspace, then one of growing size
+        y = at(q, q[:128], q[:128], position)
+        assert torch.equal(at(q, q[:128], q[:128], position), y)
+    tall = torch.zeros((5000, 256), dtype=torch.float16, device="cuda")
+    for r in range(200, 5000):                                  # more lengths than are kept
+        op(tall[:r])
+    assert torch.equal(op(tx), want[-1])

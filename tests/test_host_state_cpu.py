@@ -48,32 +48,24 @@ def test_prepared_calls_refuse_descriptors_of_another_size():
     """Sizes are checked before anything is copied out of the buffers."""
     host = L.host_calls()
     with pytest.raises(ValueError):
-        host.LinearCall(0, ctypes.c_void_p(), b"\0" * 8, None, 0, None, None, None)
+        host.LinearCall(0, ctypes.c_void_p(), b"\0" * 8, None, 0, None, None, None, 16, 128)
     with pytest.raises(ValueError):
         host.AttnCall(0, 0, ctypes.c_void_p(), b"\0" * 8, None, None)
     with pytest.raises(ValueError):
-        host.LinearCall(0, b"four", b"\0" * 24, None, 0, None, None, None)
+        host.LinearCall(0, b"four", b"\0" * 24, None, 0, None, None, None, 16, 128)
 
 
 def test_prepared_calls_keep_their_workspaces_alive():
     """Whatever becomes of the node's own reference, the address that a later call hands over stays that tensor's."""
     host = L.host_calls()
-    w, d, a = bytes(L.QWeight()), L.LinearDesc(M=3, N=16, K=128), L.AttnDesc()
-    linear = host.LinearCall(0, ctypes.c_void_p(), w, None, 0, None, None, None)
-
     t = torch.zeros(256, dtype=torch.uint8)
     held = sys.getrefcount(t)
-    linear.register(bytes(d), t)
+    attention = host.AttnCall(0, 0, ctypes.c_void_p(), bytes(L.AttnDesc()), t, None)
     assert sys.getrefcount(t) == held + 1
-    linear.register(bytes(d), None)     # another one for the same rows
-    assert sys.getrefcount(t) == held
-    linear.register(bytes(d), t)
-    attention = host.AttnCall(0, 0, ctypes.c_void_p(), bytes(a), t, None)
-    assert sys.getrefcount(t) == held + 2
-    del linear, attention
+    del attention
     assert sys.getrefcount(t) == held
     with pytest.raises(ValueError):
-        host.AttnCall(0, 0, ctypes.c_void_p(), bytes(a), torch.zeros(8), None)  # not bytes
+        host.AttnCall(0, 0, ctypes.c_void_p(), bytes(L.AttnDesc()), torch.zeros(8), None)  # not bytes
 
 
 def test_a_missing_extension_costs_host_time_only(monkeypatch):
