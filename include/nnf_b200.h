@@ -165,7 +165,10 @@ NNF_B200_API int nnf_b200_sm_count(const nnf_b200_ctx* ctx);
  * or RMS-normalised activations).  The scratch must be zero-filled once before
  * its first use (nnf_b200_workspace_reset); every call leaves its counters zeroed
  * again, so calls of one descriptor can follow one another on the same buffer;
- * zero-fill it again before it serves another descriptor.  Calls that share one
+ * zero-fill it again before it serves another descriptor.  Above 16 rows a
+ * smaller buffer is taken too, as long as it holds the fp16 copy: the call then
+ * shares tiles through less of it or not at all (a program whose buffer was sized
+ * by another version of the library keeps running, slower perhaps).  Calls that share one
  * scratch buffer must not overlap on the device.  ctx may be NULL (a 148-SM device
  * is assumed), for sizing at code-generation time. */
 NNF_B200_API size_t nnf_b200_linear_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc* desc);

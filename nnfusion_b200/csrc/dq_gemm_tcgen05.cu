@@ -1252,8 +1252,8 @@ static bool needs_prepass(const nnf_b200_linear_desc& d)
     return d.x_dtype == NNF_B200_F32 || d.prologue == NNF_B200_PROLOGUE_RMSNORM;
 }
 
-// How a launch is laid out (see the top of this file); the workspace holds the arrival counters of the tiles' halves,
-// partial-sum slots of every CTA and, when needed, the fp16 copy of x.
+// How a launch is laid out (see the top of this file).  The workspace holds, for tiles shared through it, the arrival
+// counters of the tiles' halves and partial-sum slots of every CTA; and, when needed, the fp16 copy of x.
 struct GemmLayout
 {
     int bx, m_tiles, n_tiles, tiles, sets, cpt, pairs, whole_tiles, ksplit;
@@ -1261,7 +1261,19 @@ struct GemmLayout
     size_t total() const { return counter_bytes + slot_bytes + prepass_bytes; }
 };
 
-static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+// Tiles shared through the workspace: counters for both halves of every tile, and slots of 128 x BX for two tiles per CTA
+// and weight set.
+static size_t shared_counter_bytes(int tiles)
+{
+    return ((size_t)2 * tiles * sizeof(uint32_t) + 255) / 256 * 256;
+}
+static size_t shared_slot_bytes(int pairs, int sets, int bx)
+{
+    return (size_t)2 * pairs * 2 * sets * 128 * bx * sizeof(float);
+}
+
+// room: bytes that counters and slots may take.
+static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, size_t room = SIZE_MAX)
 {
     GemmLayout L{};
     const int sms = ctx ? ctx->sm_count : 148;
@@ -1279,6 +1291,9 @@ static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_des
     // clock under load.  Whole tiles cost whole waves.  Partial sums through the workspace (store, ticket, read back) cost
     // 9 to 26 us, inside a cluster 1 to 4 us.
     const double kb = (double)d.K / 64.0 * L.sets;
+    auto pairs_of = [&](int tiles, bool whole) {
+        return (int)std::min<long long>(whole ? tiles : (long long)tiles * L.sets * L.cpt, max_pairs);
+    };
     double best = 0;
     const int m_min = (d.M + 255) / 256;
     for (int mt = m_min; mt <= m_min * 2 + 2 && mt <= (d.M + 15) / 16; mt++)
@@ -1292,24 +1307,19 @@ static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_des
                 best = t, L.bx = bx, L.m_tiles = m_tiles, L.whole_tiles = whole, L.ksplit = ksplit;
         };
         take(std::ceil((double)tiles / max_pairs) * tile + 0.004 * out, 1, 1);
-        take(std::max((double)tiles / max_pairs, 1.0 / L.cpt) * tile + 6.0 + (tiles < max_pairs ? 0.08 : 0.05) * out, 0, 1);
+        if (shared_counter_bytes(tiles) + shared_slot_bytes(pairs_of(tiles, false), L.sets, bx) <= room)
+            take(std::max((double)tiles / max_pairs, 1.0 / L.cpt) * tile + 6.0 + (tiles < max_pairs ? 0.08 : 0.05) * out, 0, 1);
         for (int s = 2; s <= 4 && s <= L.cpt; s++)
             if (tiles <= held[s] && (L.sets == 1 || bx <= 128))
                 take((double)((L.cpt + s - 1) / s) * kb_per_chunk * L.sets * t_kb + 1.0 + 0.008 * out, 0, s);
     }
     L.tiles = L.m_tiles * L.n_tiles;
-    const long long units = (long long)L.tiles * L.sets * L.cpt;
-    L.pairs = L.ksplit > 1 ? L.tiles * L.ksplit : (int)std::min<long long>(L.whole_tiles ? L.tiles : units, max_pairs);
-    // Tiles shared through the workspace: counters for both halves of every tile, and slots of 128 x BX for two tiles per CTA
-    // (and weight set).  The size handed out is at least that of 128-row tiles of 64 or 256 batch rows, one counter each,
-    // with two slots per CTA.
-    const bool shared = !L.whole_tiles && L.ksplit == 1;
-    const int wide = d.M <= 64 ? 64 : 256;
-    const long long tiles128 = (long long)((d.M + wide - 1) / wide) * ((d.N + 127) / 128);
-    const long long ctas128 = std::min<long long>(tiles128 * L.cpt, sms);
-    L.counter_bytes = ((size_t)std::max<long long>(shared ? 2ll * L.tiles : 0, tiles128) * sizeof(uint32_t) + 255) / 256 * 256;
-    L.slot_bytes = std::max<size_t>(shared ? (size_t)2 * L.pairs * 2 * L.sets * 128 * L.bx * sizeof(float) : (size_t)0,
-                                    (size_t)2 * ctas128 * 128 * wide * sizeof(float));
+    L.pairs = L.ksplit > 1 ? L.tiles * L.ksplit : pairs_of(L.tiles, L.whole_tiles);
+    if (!L.whole_tiles && L.ksplit == 1)
+    {
+        L.counter_bytes = shared_counter_bytes(L.tiles);
+        L.slot_bytes = shared_slot_bytes(L.pairs, L.sets, L.bx);
+    }
     L.prepass_bytes = needs_prepass(d) ? ((size_t)d.M * d.K * sizeof(__half) + 255) / 256 * 256 : 0;
     return L;
 }
@@ -1347,11 +1357,14 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
                 const nnf_b200_qweight* w, const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y,
                 void* workspace, size_t workspace_bytes)
 {
-    const GemmLayout L = gemm_layout(ctx, d);
-    if (!workspace || workspace_bytes < L.total())
+    GemmLayout L = gemm_layout(ctx, d);
+    if (L.total() > 0 && (!workspace || workspace_bytes < L.prepass_bytes))
         return set_error(ctx, NNF_B200_EWORKSPACE,
                          "workspace of " + std::to_string(L.total()) +
                              " bytes required (tile counters, partial sums of shared tiles, fp16 copy of the activations)");
+    // A smaller one (a program that was generated when this shape asked for less) takes the best layout that it holds.
+    if (workspace_bytes < L.total())
+        L = gemm_layout(ctx, d, workspace_bytes - L.prepass_bytes);
     if (reinterpret_cast<uintptr_t>(workspace) & 15u)
         return set_error(ctx, NNF_B200_EALIGN, "the workspace must be 16-byte aligned");
     uint8_t* ws = static_cast<uint8_t*>(workspace);

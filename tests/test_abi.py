@@ -62,22 +62,22 @@ def test_pack_u4_host_helper(lib):
 
 
 def test_workspace_sizes_without_a_device(lib):
-    """Sizing at code-generation time (no context: a 148-SM device is assumed).  Large M: the tiles' arrival counters,
-    two fp32 tile slots per persistent CTA, and the fp16 copy of the activations when there is a pre-pass."""
-    def need(M, N, K, x=L.F16, prologue=0):
-        d = L.LinearDesc(M=M, N=N, K=K, w_bits=4, group_size=128, x_dtype=x, y_dtype=x, scale_dtype=L.F16,
-                         prologue=prologue)
+    """Sizing at code-generation time (no context: a 148-SM device is assumed).  Large M: nothing for whole tiles and for K
+    shared inside clusters; for tiles shared through the workspace two arrival counters a tile and slots of 128 rows for two
+    tiles per CTA and weight set; and the fp16 copy of the activations when there is a pre-pass."""
+    def need(M, N, K, x=L.F16, prologue=0, epilogue=0):
+        d = L.LinearDesc(M=M, N=N, K=K, w_bits=4, group_size=64, x_dtype=x, y_dtype=x, scale_dtype=L.F16,
+                         prologue=prologue, epilogue=epilogue)
         return int(lib.nnf_b200_linear_workspace_bytes(None, ctypes.byref(d)))
-    slots = 2 * 148 * 128 * 256 * 4
-    tiles = 16 * 86                                  # 4096 / 256 batch tiles x 11008 / 128 weight-row tiles
-    plain = need(4096, 11008, 4096)
-    assert plain == (tiles * 4 + 255) // 256 * 256 + slots
-    assert need(4096, 11008, 4096, x=L.F32) == plain + 4096 * 4096 * 2
-    assert need(4096, 11008, 4096, prologue=L.PROLOGUE_RMSNORM) == plain + 4096 * 4096 * 2
-    # a launch with fewer units of work than SMs uses fewer CTAs, hence fewer slots; up to 64 batch rows the tile
-    # (and with it a slot) is 64 rows wide instead of 256
-    assert need(32, 128, 256) == 256 + 2 * 1 * 128 * 64 * 4
-    assert need(65, 128, 256) == 256 + 2 * 1 * 128 * 256 * 4
+    assert need(4096, 11008, 4096) == 0                           # whole tiles
+    assert need(4096, 11008, 4096, x=L.F32) == 4096 * 4096 * 2
+    assert need(4096, 11008, 4096, prologue=L.PROLOGUE_RMSNORM) == 4096 * 4096 * 2
+    assert need(48, 4096, 11008) == need(32, 128, 256) == 0       # clusters that share K
+    # 75 tiles of 32 batch rows on 74 pairs: seam shares
+    slots = 74 * 2 * 2 * 128 * 32 * 4
+    assert need(18, 19001, 3136) == 768 + slots
+    assert need(18, 19001, 3136, epilogue=L.EPILOGUE_SILU_MUL) == 768 + 2 * slots
+    assert need(18, 19001, 3136, x=L.F32) == 768 + slots + (18 * 3136 * 2 + 255) // 256 * 256
     # small M: split-K scratch only
     assert need(1, 11008, 4096) < 1 << 20
 

@@ -60,3 +60,34 @@ def test_pairs_that_share_k_repeat_back_to_back(M, N, K, dual):
     torch.cuda.synchronize()
     op.ctx.device_status()
     assert not [i for i, y in enumerate(outs) if not torch.equal(y, first)]
+
+
+@pytest.mark.parametrize("M,N,K,dual,bias", [(17, 19, 5312, True, False), (18, 19001, 3136, False, True)])
+def test_smaller_workspaces_are_used_as_far_as_they_go(M, N, K, dual, bias):
+    """A program whose buffer was sized by another version of the library keeps running: the launch takes the best layout
+    that the buffer holds, writes nothing behind it, and only a missing buffer is refused."""
+    import ctypes
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight, NNFB200Error
+    rng = np.random.Generator(np.random.PCG64(M + K))
+    x = synth.make_x(rng, M, K, np.float16)
+    w = [synth.make_weights(rng, N, K, 4, 64) for _ in range(1 + dual)]
+    b = rng.standard_normal(N).astype(np.float32) if bias else None
+    op = DequantDot(*[DeviceWeight.from_host(v) for v in w], bias=torch.from_numpy(b).cuda() if bias else None)
+    tx, want = torch.from_numpy(x).cuda(), oracle_linear(x, *w, bias=b)
+    d = op.desc(M, tx.dtype)
+    need = int(op.ctx.lib.nnf_b200_linear_workspace_bytes(op.ctx.handle, ctypes.byref(d)))
+    assert need > 1 << 20
+    y = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    for size in (need, need - 256, need // 2, need // 4 // 256 * 256, 256):
+        guarded = torch.zeros(size + 4096, dtype=torch.uint8, device="cuda")
+        guarded[size:] = 0xAB
+        for _ in range(2):
+            y.fill_(float("nan"))
+            op.run_raw(d, tx.data_ptr(), y.data_ptr(), guarded[:size])
+            assert orc.max_rel_err(y.cpu().numpy(), want) <= min(TOL_F16, 3e-3 if dual else 2e-3), size
+        assert bool((guarded[size:] == 0xAB).all())
+    op.ctx.device_status()
+    with pytest.raises(NNFB200Error) as e:
+        op.run_raw(d, tx.data_ptr(), y.data_ptr(), None)
+    assert e.value.status == L.EWORKSPACE
