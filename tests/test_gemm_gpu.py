@@ -132,12 +132,12 @@ def test_prepass_needs_its_workspace():
 
 
 # ---------------------------------------------------------------------------------------------------------------
-# Persistent CTAs that share tiles: the work of a launch is cut evenly into raw-chunk units, so tiles at the seams
-# are computed by two or more CTAs and added in a fixed order by the last one to arrive.
+# Few tiles: the pairs of CTAs of a cluster share a tile's K and exchange their sums through shared memory.  (Tiles shared
+# through the workspace: test_gemm_splits_gpu.py.)
 
 @pytest.mark.parametrize("M,N,K,bits", [
-    (256, 1024, 4096, 4),     # 8 tiles of 16 chunks on 128 CTAs: every tile is shared by 16 CTAs
-    (300, 2000, 2048, 4),     # ragged M and N, 32 tiles of 8 chunks: seams inside most tiles
+    (256, 1024, 4096, 4),     # few tiles of 16 chunks
+    (300, 2000, 2048, 4),     # ragged M and N, tiles of 8 chunks
     (520, 1280, 1024, 8),     # uint8 weights (two k-blocks per chunk)
     (64, 128, 320, 4),        # K / 64 = 5: the tile's last chunk holds one k-block, which only one group converts
     (96, 256, 192, 8),        # the same for uint8: three k-blocks, two per chunk
@@ -162,8 +162,8 @@ def test_shared_tiles_silu_mul_and_bias():
 
 
 def test_repeated_calls_share_one_workspace_and_agree_bitwise():
-    """The arrival counters are left zeroed by every launch, and the order in which shared tiles are added does not
-    depend on which CTA arrives last: the same call twice on one workspace gives the same bits."""
+    """The order in which the parts of a shared tile are added does not depend on which CTA is done last: the same call
+    again gives the same bits."""
     import torch
     from nnfusion_b200.linear import DequantDot, DeviceWeight
     x, w = synth.u4g128(43, 256, 1024, 4096)
@@ -177,7 +177,7 @@ def test_repeated_calls_share_one_workspace_and_agree_bitwise():
 
 
 def test_shared_tiles_odd_n_scalar_stores():
-    """N not a multiple of four: the CTA that adds a shared tile's slots stores element by element."""
+    """N not a multiple of four: the CTA that adds a shared tile's parts stores element by element."""
     rng = np.random.Generator(np.random.PCG64(44))
     M, N, K = 300, 1001, 2048
     x = synth.make_x(rng, M, K, np.float16)
@@ -210,8 +210,8 @@ def test_shared_tiles_add_epilogue_in_place(N):
 
 
 def test_silu_mul_fp32_output_and_odd_n():
-    """SiLU(gate) * up as two launches that meet in y: fp32 y keeps the gate products in fp32; odd N takes the scalar
-    path of the CTA that adds a shared tile's slots."""
+    """SiLU(gate) * up: fp32 y keeps the gate products in fp32; odd N takes the scalar path of the CTA that adds a shared
+    tile's parts."""
     rng = np.random.Generator(np.random.PCG64(46))
     M, N, K = 130, 1001, 2048
     x = synth.make_x(rng, M, K, np.float16)
@@ -241,8 +241,8 @@ def test_output_padding_untouched_with_shared_tiles():
 
 
 @pytest.mark.parametrize("M,N,K,dual,launches", [
-    (4096, 11008, 4096, False, 60),     # 9 tiles per CTA
-    (256, 3584, 8192, True, 300),       # every tile shared by 6 CTAs, segments as short as one chunk, two passes
+    (4096, 11008, 4096, False, 60),     # 9 or 10 whole tiles per pair
+    (256, 3584, 8192, True, 300),       # gate and up behind one another in a tile
 ])
 def test_back_to_back_launches_repeat_bit_for_bit(M, N, K, dual, launches):
     """Many launches in a row, no host synchronisation in between, must all give the first launch's bits.  Two races
@@ -267,14 +267,13 @@ def test_back_to_back_launches_repeat_bit_for_bit(M, N, K, dual, launches):
 
 @pytest.mark.parametrize("M", [17, 48, 64, 65])
 @pytest.mark.parametrize("N,K,bits,dual", [
-    (1024, 4096, 4, False),    # 8 tiles of 16 chunks on 128 CTAs: every tile shared by 16 CTAs
-    (1001, 2048, 4, True),     # odd N (scalar stores), SiLU(gate) * up in two passes
+    (1024, 4096, 4, False),    # few tiles of 16 chunks: K shared in clusters
+    (1001, 2048, 4, True),     # odd N (scalar stores), SiLU(gate) * up
     (640, 1024, 8, False),     # uint8 weights
 ])
 def test_narrow_batch_tile(M, N, K, bits, dual):
-    """Up to 64 batch rows the tensor-core kernel works on tiles of 64 batch rows (a quarter of the accumulator, of
-    the activation tile and of a shared tile's slot); 65 rows are the first to take the 256-row tile again.  Both
-    against the oracle, and three calls in a row bit for bit."""
+    """Narrow batches (tiles are as wide as the batch, in steps of 16) against the oracle, and three calls in a row bit for
+    bit."""
     rng = np.random.Generator(np.random.PCG64(300 + M + N))
     x = synth.make_x(rng, M, K, np.float16)
     w = synth.make_weights(rng, N, K, bits, 128)

@@ -91,3 +91,42 @@ def test_smaller_workspaces_are_used_as_far_as_they_go(M, N, K, dual, bias):
     with pytest.raises(NNFB200Error) as e:
         op.run_raw(d, tx.data_ptr(), y.data_ptr(), None)
     assert e.value.status == L.EWORKSPACE
+
+
+def _seam_bytes(M, N, K, bits, sets, bx):
+    """Workspace of a launch whose tiles of bx batch rows are shared through it (148 SMs: 74 pairs)."""
+    tiles = (M + bx - 1) // bx * ((N + 255) // 256)
+    chunks = (K // 64 + (3 if bits == 4 else 1)) // (4 if bits == 4 else 2)
+    return (2 * tiles * 4 + 255) // 256 * 256 + min(tiles * sets * chunks, 74) * 2 * 2 * sets * 128 * bx * 4
+
+
+@pytest.mark.parametrize("M,N,K,bx,dual", [
+    (23, 17, 5696, 16, True),       # 2 tiles on 74 pairs: one or two chunks a share, odd N
+    (141, 312, 10816, 48, True),    # 7 of a weight set's 43 chunks a share: shares that hold the end of the gate's chunks
+    (189, 306, 12864, 48, True),    # the same, N not a multiple of four
+    (646, 6156, 2944, 224, True),   # 75 tiles, above 128 batch rows: whole tiles between the seams
+    (686, 1281, 15040, 176, True),  # above 128 batch rows, odd N: several shares per weight set
+    (129, 338, 15872, 48, False),   # with a bias
+    (660, 6337, 3904, 224, False),  # with a bias, above 128 batch rows, odd N
+])
+def test_seam_shares_with_two_weight_sets_and_bias(M, N, K, bx, dual):
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(M * 7 + N))
+    x = synth.make_x(rng, M, K, np.float16)
+    w = [synth.make_weights(rng, N, K, 4, 64) for _ in range(1 + dual)]
+    bias = None if dual else rng.standard_normal(N).astype(np.float32)
+    rows = sorted({0, 1, 15, 16, bx - 1, min(bx, M - 1), M // 2, M - 2, M - 1} & set(range(M)))  # the oracle's rows are independent
+    r32 = oracle_linear(x[rows], *w, bias=bias, out_dtype=np.float32)
+    dev, tx = [DeviceWeight.from_host(v) for v in w], torch.from_numpy(x).cuda()
+    for y_dtype in (torch.float16, torch.float32):
+        op = DequantDot(*dev, bias=None if dual else torch.from_numpy(bias).cuda(), y_dtype=y_dtype)
+        y = torch.full((M, N), float("nan"), dtype=y_dtype, device="cuda")
+        op(tx, out=y)
+        (ws,) = op._ws.values()
+        assert ws.numel() == _seam_bytes(M, N, K, 4, 1 + dual, bx)      # this is the layout that the launch took
+        assert bool(torch.isfinite(y).all()) and torch.equal(op(tx), y)
+        op.ctx.device_status()
+        err = orc.max_rel_err(y[rows].float().cpu().numpy(), r32)
+        # fp16 scale products and, with SiLU, one rounding of the gate to y's type: the kernel's other tests' bounds
+        assert err <= min(TOL_F16, 3e-3 if dual else 2e-3), (y_dtype, err)
