@@ -572,6 +572,126 @@ __global__ void __launch_bounds__(WARPS * 32, 1) decode_attention_kernel(const A
     *reinterpret_cast<uint2*>(p.out + (size_t)(head0 + qi) * kD + 4 * d4) = pk;
 }
 
+// A sequence of up to 32 rows, one CTA of four warps per query head: a lane has 8 dimensions of one row per round, so that all
+// rows are in registers at once, the products are fp32, and the rows are added up in one go.  It is a chain of dependent
+// steps throughout, and this is the shortest one (the rows of shared key/value heads come from L2): 1 to 32 rows 1.5 us in a
+// chain of launches, where the kernel above takes 2.9 to 3.1.
+constexpr int kShortRows = 32;
+constexpr int kShortThreads = 128;
+__global__ void __launch_bounds__(kShortThreads) short_attention_kernel(const AttnParams p)
+{
+    constexpr int kRounds = kShortRows / 8; // a round is 8 rows: two a warp, 16 lanes each
+    __shared__ __align__(16) float q_s[kD]; // rotated query, times the softmax scale
+    __shared__ __align__(16) __half knew_s[kD];
+    __shared__ float red_s[4][kD], m_s[4], l_s[4];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int half = lane >> 4, dg = lane & 15; // which of the warp's two rows, which 8 dimensions
+    const int head = blockIdx.x, kvh = head / p.group;
+    const int rows = p.position + 1;
+    const size_t cache0 = (size_t)kvh * p.capacity * kD;
+    if (tid == 0)
+    {
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.k_cache + cache0), "r"(rows * kD * 2) : "memory");
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.v_cache + cache0), "r"(rows * kD * 2) : "memory");
+    }
+    float cs = 1.f, sn = 0.f; // of dimensions tid and tid ^ 64
+    if (p.rotary)
+        sincosf((float)p.position * exp2f(-(float)(2 * (tid & 63)) / (float)kD * p.log2_base), &sn, &cs);
+    if (tid < 64)
+        sn = -sn;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    const __half* const q = p.q + (size_t)head * kD;
+    const __half* const kx = p.k_new + (size_t)kvh * kD;
+    const __half* const vx = p.v_new + (size_t)kvh * kD;
+    const __half qa = q[tid], qb = q[tid ^ 64], ka = kx[tid], kb = kx[tid ^ 64], vn = vx[tid];
+    uint4 kr[kRounds], vr[kRounds];
+    auto row_of = [&](int r) { return r * 8 + warp * 2 + half; };
+#pragma unroll
+    for (int r = 0; r < kRounds; r++)
+    {
+        const size_t at = cache0 + (size_t)row_of(r) * kD + 8 * dg;
+        const bool live = row_of(r) < p.position; // (the new row is patched in below)
+        kr[r] = live ? load_once(p.k_cache + at) : make_uint4(0u, 0u, 0u, 0u);
+        vr[r] = live ? load_once(p.v_cache + at) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    auto rotated = [&](__half a, __half b) {
+        return p.rotary ? fmaf(__half2float(b), sn, __half2float(a) * cs) : __half2float(a);
+    };
+    q_s[tid] = rotated(qa, qb) * p.scale;
+    const __half kn = __float2half_rn(rotated(ka, kb));
+    knew_s[tid] = kn;
+    // append: every head of a group writes the same values
+    p.k_cache[cache0 + (size_t)p.position * kD + tid] = kn;
+    p.v_cache[cache0 + (size_t)p.position * kD + tid] = vn;
+    __syncthreads();
+    float qv[8];
+    *reinterpret_cast<float4*>(qv) = *reinterpret_cast<const float4*>(q_s + 8 * dg);
+    *reinterpret_cast<float4*>(qv + 4) = *reinterpret_cast<const float4*>(q_s + 8 * dg + 4);
+    float s[kRounds], m = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kRounds; r++)
+    {
+        if (row_of(r) == p.position)
+        {
+            kr[r] = *reinterpret_cast<const uint4*>(knew_s + 8 * dg);
+            vr[r] = *reinterpret_cast<const uint4*>(vx + 8 * dg);
+        }
+        const __half2* k = reinterpret_cast<const __half2*>(&kr[r]);
+        float d = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const float2 f = __half22float2(k[j]);
+            d = fmaf(qv[2 * j], f.x, d), d = fmaf(qv[2 * j + 1], f.y, d);
+        }
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1)
+            d += __shfl_xor_sync(0xffffffffu, d, x);
+        s[r] = row_of(r) < rows ? d : -INFINITY;
+        m = fmaxf(m, s[r]);
+    }
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+    if (lane == 0)
+        m_s[warp] = m;
+    __syncthreads();
+    m = fmaxf(fmaxf(m_s[0], m_s[1]), fmaxf(m_s[2], m_s[3]));
+    float l = 0.f, acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        acc[j] = 0.f;
+#pragma unroll
+    for (int r = 0; r < kRounds; r++)
+    {
+        const float w = exp2f(s[r] - m); // 0 for rows past the end
+        l += w;
+        const __half2* v = reinterpret_cast<const __half2*>(&vr[r]);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const float2 f = __half22float2(v[j]);
+            acc[2 * j] = fmaf(w, f.x, acc[2 * j]), acc[2 * j + 1] = fmaf(w, f.y, acc[2 * j + 1]);
+        }
+    }
+    // the two rows of a warp, then the four warps
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
+    if (half == 0)
+    {
+        *reinterpret_cast<float4*>(&red_s[warp][8 * dg]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        *reinterpret_cast<float4*>(&red_s[warp][8 * dg + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+    if (lane == 0)
+        l_s[warp] = l;
+    __syncthreads();
+    const float sum = (red_s[0][tid] + red_s[1][tid]) + (red_s[2][tid] + red_s[3][tid]);
+    p.out[(size_t)head * kD + tid] = __float2half_rn(sum / ((l_s[0] + l_s[1]) + (l_s[2] + l_s[3])));
+}
+
 int head_blocks(const nnf_b200_attn_desc& d)
 {
     return d.kv_heads * ((d.heads / d.kv_heads + kQ - 1) / kQ);
@@ -700,11 +820,12 @@ int attn_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_attn_desc
         return set_error(ctx, NNF_B200_ECUDA, std::string("decode_attention set-up: ") + cudaGetErrorString(e));
     (void)cudaGetLastError();
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.splits, head_blocks(d));
-    // an uncut sequence of up to two passes of four warps: 30 rows 3.7 -> 3.05 us, 61 rows 4.1 -> 3.5 us
+    const bool short_one = p.splits == 1 && rows <= kShortRows;
+    cfg.gridDim = short_one ? dim3(d.heads) : dim3(p.splits, head_blocks(d));
+    // an uncut sequence of up to two passes of four warps: 61 rows 4.1 -> 3.5 us
     const bool few = p.splits == 1 && rows <= 2 * kFewWarps * kRows;
-    cfg.blockDim = dim3((few ? kFewWarps : kWarps) * 32);
-    cfg.dynamicSmemBytes = few ? kFewWarps * kQ * kD * sizeof(float) : kSmemBytes;
+    cfg.blockDim = dim3(short_one ? kShortThreads : (few ? kFewWarps : kWarps) * 32);
+    cfg.dynamicSmemBytes = short_one ? 0 : few ? kFewWarps * kQ * kD * sizeof(float) : kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     overlap_attribute(attr, &cfg.numAttrs);
@@ -718,8 +839,9 @@ int attn_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_attn_desc
         cfg.numAttrs++;
     }
     cfg.attrs = attr;
-    e = few ? cudaLaunchKernelEx(&cfg, decode_attention_kernel<kFewWarps>, p)
-            : cudaLaunchKernelEx(&cfg, decode_attention_kernel<kWarps>, p);
+    e = short_one ? cudaLaunchKernelEx(&cfg, short_attention_kernel, p)
+        : few     ? cudaLaunchKernelEx(&cfg, decode_attention_kernel<kFewWarps>, p)
+                  : cudaLaunchKernelEx(&cfg, decode_attention_kernel<kWarps>, p);
     if (e != cudaSuccess)
         return set_error(ctx, NNF_B200_ECUDA, std::string("decode_attention launch: ") + cudaGetErrorString(e));
     ctx->launches++;

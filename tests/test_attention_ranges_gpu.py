@@ -23,3 +23,15 @@ def test_long_sequences_on_few_heads(H, Hkv, pos):
     outs, ref, _, _ = _run(H, Hkv, pos + 1, pos, seed=300 + H, calls=2)
     _check(outs[0], ref)
     np.testing.assert_array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("rotary", [True, False])
+@pytest.mark.parametrize("H,Hkv", [(1, 1), (9, 3), (32, 32), (64, 8)])
+@pytest.mark.parametrize("pos", [0, 1, 7, 8, 15, 16, 30, 31, 32])
+def test_short_sequences(H, Hkv, pos, rotary):
+    """Up to 32 rows one CTA takes a query head (33: the first that does not), whatever shares its key/value head."""
+    outs, ref, caches, caches_ref = _run(H, Hkv, 40, pos, seed=400 + pos, rotary=rotary, calls=2)
+    _check(outs[0], ref)
+    np.testing.assert_array_equal(outs[0], outs[1])
+    np.testing.assert_array_equal(caches[1], caches_ref[1])
+    np.testing.assert_allclose(caches[0].astype(np.float32), caches_ref[0].astype(np.float32), rtol=2e-3, atol=2e-3)
