@@ -698,7 +698,8 @@ int head_blocks(const nnf_b200_attn_desc& d)
 }
 
 // Ranges per head block, one CTA per SM.  Up to 8 ranges meet in the shared memory of a cluster (about 1 us), more in the
-// workspace (about 3 us: store, fence, ticket, read back).  Measured: a sequence of up to 112 rows is fastest uncut; a
+// workspace (about 3 us: store, fence, ticket, read back).  Measured: a sequence of up to 128 rows is fastest uncut (128 rows,
+// 8 heads on 8: 4.20 us, 2 ranges 4.59, 3 ranges 4.40, 4 ranges 4.36; 64 on 8: 4.46, 4.92, 4.76, 4.77); a
 // range pays from 64 rows on (563 rows on 2 key/value heads: 3 ranges 6.2 us, 8 ranges 5.3 us, since one SM takes in no
 // more than about 85 GB/s); up to about 600 rows a range the cluster wins (4097 rows on 8 heads: 8 ranges 9.2 us, 16
 // through the workspace 9.6 us; 8192 rows: 16.0 and 13.1 us), beyond that as many ranges as one wave holds, of 256 rows at
@@ -710,7 +711,7 @@ int pick_splits(const nnf_b200_ctx* ctx, const nnf_b200_attn_desc& d)
     if (d.splits > 0)
         return std::min(std::min(d.splits, std::max(1, rows / 16)), kMaxSplits);
     const int wave = std::max(1, sms / head_blocks(d));
-    if (rows <= 112 || wave == 1)
+    if (rows <= 128 || wave == 1)
         return 1;
     // clusters of n one-per-SM CTAs that the 148 SMs hold at once (the occupancy calculator's answers; the launch asks
     // again and falls back to the workspace)

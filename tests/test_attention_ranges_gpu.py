@@ -8,7 +8,7 @@ from tests.test_attention_gpu import _check, _run
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("pos", [63, 64, 111, 112, 127, 128, 191, 192, 447, 448])
+@pytest.mark.parametrize("pos", [63, 64, 111, 112, 126, 127, 128, 129, 191, 192, 447, 448])
 @pytest.mark.parametrize("H,Hkv", [(2, 2), (9, 1)])
 def test_lengths_around_the_cuts(H, Hkv, pos):
     outs, ref, caches, caches_ref = _run(H, Hkv, 512, pos, seed=200 + pos, calls=2)
