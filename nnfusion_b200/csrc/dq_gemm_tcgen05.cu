@@ -547,7 +547,10 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
         // (the whole warp walks the loop, one elected lane issues)
         if (rank == 0)
         {
-            // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = BX, M = 256
+            // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = BX, M = 256.  (N: kind::f16 with
+            // cta_group::2 and M = 256 takes 16 to 256 in steps of 16.  The PTX ISA's table of tcgen05.mma shapes goes by kind,
+            // CTA group and M, not by whether A lies in shared or in tensor memory; every width is held against the oracle in
+            // the tests.)
             const uint32_t idesc = (1u << 4) | ((uint32_t)(p.bx >> 3) << 17) | ((uint32_t)((2 * kBN) >> 4) << 24);
             bool ok = true;
             uint32_t si = 0;
@@ -1298,7 +1301,7 @@ static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_des
     const int m_min = (d.M + 255) / 256;
     for (int mt = m_min; mt <= m_min * 2 + 2 && mt <= (d.M + 15) / 16; mt++)
     {
-        const int bx = ((d.M + mt - 1) / mt + 15) / 16 * 16;
+        const int bx = ((d.M + mt - 1) / mt + 15) / 16 * 16; // 16 to 256: m_min tiles are no wider
         const int m_tiles = (d.M + bx - 1) / bx, tiles = m_tiles * L.n_tiles;
         const double t_kb = bx <= 128 ? 0.19 + 0.0004 * bx : 0.25 + 0.00037 * bx, out = (double)bx * L.sets;
         const double tile = kb * t_kb + 0.5 + 3.0 * (L.sets - 1);

@@ -7,7 +7,7 @@ import pytest
 from nnfusion_b200 import _lib as L
 from nnfusion_b200 import synth
 from oracle import oracle as orc
-from tests.util import TOL_F16, oracle_linear
+from tests.util import TOL_F16, gpu_linear, oracle_linear
 
 pytestmark = pytest.mark.gpu
 
@@ -130,3 +130,15 @@ def test_seam_shares_with_two_weight_sets_and_bias(M, N, K, bx, dual):
         err = orc.max_rel_err(y[rows].float().cpu().numpy(), r32)
         # fp16 scale products and, with SiLU, one rounding of the gate to y's type: the kernel's other tests' bounds
         assert err <= min(TOL_F16, 3e-3 if dual else 2e-3), (y_dtype, err)
+
+
+@pytest.mark.parametrize("M", range(16, 257, 16))
+def test_every_tile_width(M):
+    """One batch tile of every width that the tensor core is given, with all its rows, and with one less."""
+    rng = np.random.Generator(np.random.PCG64(M))
+    w = synth.make_weights(rng, 300, 576, 4, 64)
+    x = synth.make_x(rng, M, 576, np.float16)
+    want = oracle_linear(x, w)
+    for rows in (M, M - 1):
+        y = gpu_linear(x[:rows], w, kernel=L.KERNEL_GEMM)
+        assert orc.max_rel_err(y, want[:rows]) <= min(TOL_F16, 2e-3)  # fp16 scale products: the kernel's other tests' bound
