@@ -1288,11 +1288,6 @@ void fill_params(GemvParams& p, const nnf_b200_linear_desc& d, const nnf::GemvPl
 
 namespace nnf
 {
-int gemv_configure(nnf_b200_ctx*)
-{
-    return NNF_B200_OK;
-}
-
 int gemv_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, GemvPlan* plan, std::string* why,
               bool allow_direct)
 {

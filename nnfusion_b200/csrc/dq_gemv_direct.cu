@@ -85,7 +85,7 @@ struct DirectParams
     int slot_floats;
     float eps;
     // shared-memory byte offsets (DirectSmem, computed once on the host)
-    int off_bars, off_red, off_ss, off_flags;
+    int off_red, off_ss, off_flags;
     // a 64-byte unit's quantisation group = unit / group_units, done as a multiplication
     int group_units;
     uint32_t group_magic; // ceil(2^32 / group_units); exact for units below 2^16
@@ -229,20 +229,19 @@ __host__ __device__ inline ParamRange param_range(int slice0, int slices, int sl
 // Shared-memory footprint, shared by host and device.  All sizes in bytes.
 struct DirectSmem
 {
-    size_t params, bars, red, ss, flags, xsm, cslots, total;
+    size_t params, red, ss, flags, xsm, cslots, total;
     __host__ __device__ DirectSmem(int sets, int mb, int warps, int batch, int tq, int pset_bytes, int xfrag_bytes,
                                    int nbuf = 2, int cluster_splits = 0)
     {
         // (scales, zero-points) of a batch per weight set; two batches take turns unless one holds all tiles
         params = (size_t)nbuf * batch * sets * pset_bytes;
-        bars = 0;
         red = sizeof(float) * (size_t)warps * batch * sets * mb * 8 * tq * 4;
         ss = sizeof(float) * ((size_t)warps * 8 * mb + 8 * mb);
         flags = sizeof(int) * (2 * kBatch + 4); // last-arriver flags, call numbers, "all peers answered"
         xsm = ((size_t)warps * xfrag_bytes + 15) / 16 * 16;
         // the splits' sums of a batch, in the first CTA of a cluster: [split][tile][sets * mb * 128 + 8 * mb] floats
         cslots = sizeof(float) * (size_t)cluster_splits * batch * ((size_t)sets * mb * 128 + 8 * mb);
-        total = params + bars + red + ss + flags + xsm + cslots;
+        total = params + red + ss + flags + xsm + cslots;
     }
 };
 
@@ -1433,23 +1432,31 @@ cudaError_t launch(const DirectParams& p_in, const nnf::GemvPlan& plan, cudaStre
     X(8, 2, true, false, 2)                                                                                       \
     X(8, 2, true, true, 2)
 
+// The specialised parameter paths exist where they matter: side-by-side pairs for uint4 (with a form of its own for one
+// batch row, the decode case), one group per slice for uint8.
+template <int WBITS, int MB, bool XSPLIT, bool DUAL, int PD>
+cudaError_t launch_pmode(const DirectParams& p, const nnf::GemvPlan& plan, cudaStream_t stream)
+{
+    if constexpr (WBITS == 4)
+    {
+        if (p.pmode == 1)
+        {
+            if constexpr (MB == 1 && !XSPLIT)
+                if (p.M == 1)
+                    return launch<WBITS, MB, XSPLIT, DUAL, PD, 1, true>(p, plan, stream);
+            return launch<WBITS, MB, XSPLIT, DUAL, PD, 1, false>(p, plan, stream);
+        }
+    }
+    else if (p.pmode == 2)
+        return launch<WBITS, MB, XSPLIT, DUAL, PD, 2, false>(p, plan, stream);
+    return launch<WBITS, MB, XSPLIT, DUAL, PD, 0, false>(p, plan, stream);
+}
+
 cudaError_t dispatch(int wbits, const nnf::GemvPlan& plan, const DirectParams& p, cudaStream_t stream)
 {
-    // the specialised parameter paths exist where they matter: side-by-side pairs for uint4, one group per slice
-    // for uint8
 #define NNF_X(WB, MBV, XSP, DU, PDV)                                                                              \
     if (wbits == WB && plan.mb == MBV && plan.xsplit == XSP && plan.dual == DU)                                   \
-    {                                                                                                             \
-        if (p.pmode == 1 && WB == 4)                                                                              \
-        {                                                                                                         \
-            if (p.M == 1 && MBV == 1 && !XSP) /* the decode case gets its own instantiation */                    \
-                return launch<WB, MBV, XSP, DU, PDV, (WB == 4 ? 1 : 0), (MBV == 1 && !XSP)>(p, plan, stream);     \
-            return launch<WB, MBV, XSP, DU, PDV, (WB == 4 ? 1 : 0), false>(p, plan, stream);                      \
-        }                                                                                                         \
-        if (p.pmode == 2 && WB == 8)                                                                              \
-            return launch<WB, MBV, XSP, DU, PDV, (WB == 8 ? 2 : 0), false>(p, plan, stream);                      \
-        return launch<WB, MBV, XSP, DU, PDV, 0, false>(p, plan, stream);                                          \
-    }
+        return launch_pmode<WB, MBV, XSP, DU, PDV>(p, plan, stream);
     NNF_DIRECT_FOR_EACH_VARIANT(NNF_X)
 #undef NNF_X
     return cudaErrorInvalidValue;
@@ -1560,7 +1567,6 @@ bool gemv_direct_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, Ge
     // one-per-SM CTAs but only 45 of 3, 33 of 4, 26 of 5, 22 of 6 and 15 of 7 or 8 (the occupancy calculator's
     // answers), so in practice halves of K meet in shared memory and finer splits do when a split has few CTAs.
     pl.cluster = 0;
-#ifndef NNF_NO_CLUSTER
     if (pl.splits >= 2 && pl.splits <= 8)
     {
         const size_t with = DirectSmem(sets, pl.mb, pl.warps, pl.batch, pl.tq, pl.pset_sm, pl.xfrag_bytes, pl.param_bufs,
@@ -1568,7 +1574,6 @@ bool gemv_direct_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, Ge
         if ((int)with + 1024 <= smem_cap / best_res)
             pl.cluster = 1, pl.smem_bytes = with;
     }
-#endif
     // L2 window ahead of the register pipeline: about 192 KB per CTA (whole tiles, shared by the K splits)
     const int row_bytes = d.w_bits == 4 ? d.K / 2 : d.K;
     pl.prefetch_tiles = std::max(1, std::min(64, (192 * 1024 * pl.splits) / (sets * 16 * row_bytes)));
@@ -1658,8 +1663,7 @@ cudaError_t gemv_direct_dispatch(const nnf_b200_linear_desc& d, const GemvPlan& 
         const DirectSmem lay(plan.dual ? 2 : 1, plan.mb, plan.warps, plan.batch, plan.tq,
                              p.bulk_params ? plan.pset_sm : 0, plan.xfrag_bytes, plan.param_bufs,
                              plan.cluster ? plan.splits : 0);
-        p.off_bars = (int)lay.params;
-        p.off_red = p.off_bars + (int)lay.bars;
+        p.off_red = (int)lay.params;
         p.off_ss = p.off_red + (int)lay.red;
         p.off_flags = p.off_ss + (int)lay.ss;
         p.off_cslots = p.off_flags + (int)lay.flags + (int)lay.xsm;

@@ -215,14 +215,6 @@ int nnf_b200_init(int device, nnf_b200_ctx** out)
         delete ctx;
         return NNF_B200_ECUDA;
     }
-    int rc = nnf::gemv_configure(ctx);
-    if (rc == NNF_B200_OK)
-        rc = nnf::gemm_configure(ctx);
-    if (rc != NNF_B200_OK)
-    {
-        delete ctx;
-        return rc;
-    }
     *out = ctx;
     return NNF_B200_OK;
 }

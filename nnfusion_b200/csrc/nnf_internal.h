@@ -89,14 +89,12 @@ cudaError_t gemv_direct_dispatch(const nnf_b200_linear_desc& d, const GemvPlan& 
 int gemv_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const GemvPlan& plan,
                 const void* x, const nnf_b200_qweight* w, const nnf_b200_qweight* w2, const void* gain,
                 const void* bias, void* y, void* workspace, const nnf_b200_peers* peers = nullptr);
-int gemv_configure(nnf_b200_ctx* ctx);
 
 size_t gemm_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d);
 int gemm_supported(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, std::string* why);
 int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const void* x,
                 const nnf_b200_qweight* w, const nnf_b200_qweight* w2, const void* gain, const void* bias,
                 void* y, void* workspace, size_t workspace_bytes);
-int gemm_configure(nnf_b200_ctx* ctx);
 
 size_t allreduce_flag_bytes(size_t count);
 int allreduce_launch(nnf_b200_ctx* ctx, cudaStream_t stream, int rank, int world, const void* const* bufs,
