@@ -11,8 +11,11 @@
  * device pointers, and never allocate device memory: like every kernel of the
  * generated runtime they receive tensors that live in the runtime's own memory
  * pool.  Kernels are launched as programmatic dependents of whatever precedes
- * them on the stream (they wait for it before touching anything it may have
- * written).
+ * them on the stream: they wait for it before touching activations, gain, bias,
+ * addend, outputs, caches and workspaces, which it may have written.  Weight sets
+ * (wq, scale, zp) are constants and are read ahead of that wait: neither the
+ * launch directly ahead nor another launch of this library that may still be
+ * running may write them.
  *
  * Each declaration names the reference interface it stands in for (paths are
  * relative to the reference project root).

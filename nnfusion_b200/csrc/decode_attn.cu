@@ -24,9 +24,11 @@
 // be running.
 // What bounds it: the chain wait -> queries (1 us) -> rows -> meeting (0.5 us) -> ranges (1 to 3 us); the rows themselves
 // come at 85 GB/s per SM.
-// (64 query heads on 8 key/value heads, 8192 rows, 33.6 MB: 47.7 us with one CTA per query head and FFMA dot products,
-// which read every row eight times and were bound by instructions; 13.2 us now.  32 heads of their own, 2049 rows,
-// 33.6 MB: 12.0 -> 11.1 us.)
+// (64 query heads on 8 key/value heads, 8192 rows, 33.6 MB, in a chain of launches: 45.0 us with one CTA per query head and
+// FFMA dot products, which read every row eight times and were bound by instructions; 11.4 us now.  32 heads of their own,
+// 2049 rows, 33.6 MB: 11.5 -> 9.1 us.)
+// Infinities: an infinite key makes its score infinite, an infinite value its dimension of the result; the lo halves are kept
+// from making NaN of either (where scores are formed, and sum_infinite_values).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <algorithm>

@@ -1244,11 +1244,6 @@ cudaError_t dispatch(int wbits, bool one_group, const GemmParams& p, const CUten
 
 namespace nnf
 {
-int gemm_configure(nnf_b200_ctx*)
-{
-    return NNF_B200_OK;
-}
-
 // fp32 activations and the RMSNorm prologue go through a pre-pass that writes fp16 [M,K] into the workspace.
 static bool needs_prepass(const nnf_b200_linear_desc& d)
 {
@@ -1288,11 +1283,12 @@ static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_des
     L.sets = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL ? 2 : 1;
     const int kb_per_chunk = d.w_bits == 4 ? 4 : 2;
     L.cpt = (d.K / 64 + kb_per_chunk - 1) / kb_per_chunk;
-    // Batch tiles of equal width and how K is shared, by an estimate in microseconds fitted to 20 shapes of 32 to 4096 batch
-    // rows times every choice.  What a k-block takes: up to 128 batch rows the conversion of the weights (and handing it
-    // over), 0.21 to 0.24; above, where two groups of warps convert, 0.31 to 0.345, at 256 rows the tensor core at its
-    // clock under load.  Whole tiles cost whole waves.  Partial sums through the workspace (store, ticket, read back) cost
-    // 9 to 26 us, inside a cluster 1 to 4 us.
+    // Batch tiles of equal width and how K is shared, by an estimate that ranks the choices: its constants were fitted to 20
+    // shapes of 32 to 4096 batch rows times every choice, without what all choices share (the launch, the first loads, the
+    // last stores), so that the microseconds themselves come out 20 to 40 % low (4096 x 11008 x 4096: 227 for 320 measured;
+    // 48 x 4096 x 11008: 13.9 for 18.9).  What a k-block takes: up to 128 batch rows the conversion of the weights (and
+    // handing it over), 0.21 to 0.24; above, where two groups of warps convert, 0.31 to 0.345.  Whole tiles cost whole waves.
+    // Partial sums through the workspace (store, ticket, read back) cost 9 to 26 us, inside a cluster 1 to 4 us.
     const double kb = (double)d.K / 64.0 * L.sets;
     auto pairs_of = [&](int tiles, bool whole) {
         return (int)std::min<long long>(whole ? tiles : (long long)tiles * L.sets * L.cpt, max_pairs);
