@@ -36,7 +36,7 @@ if ROOT not in sys.path:
 L2_BYTES = 126e6
 # DRAM bytes (read + written) of one launch of the small-M kernel on the decode_gemv workload, from one ncu capture
 # of that launch (dram__bytes_read.sum + dram__bytes_write.sum; the output stays in L2).
-NCU_TRAFFIC_DECODE_GEMV = 23_499_008
+NCU_TRAFFIC_DECODE_GEMV = 23_500_800
 
 
 def measured_peaks():
@@ -358,7 +358,7 @@ def run_decode_gemv(args, torch, sampler_index):
                    "launch": "CUDA graph replay of the C-ABI calls"},
         "roofline": {"bound": "hbm", "achieved": round(value, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": round(value / peaks["hbm_gbs"], 4), "traffic": NCU_TRAFFIC_DECODE_GEMV,
-                     "peak_source": f"of {peaks['source']}", "kernel": "dq_gemv_direct_kernel<4,1,false,false,2,1,true>"},
+                     "peak_source": f"of {peaks['source']}", "kernel": "dq_gemv_direct_kernel<4,1,false,false,2,1,true,false>"},
         "e2e": {"value": round(e2e_value, 2), "unit": "GB/s", "h2d_bytes_per_step": M * K * 2,
                 "d2h_bytes_per_step": M * N * 2, "ms_per_step": ms_e2e / e2e_steps, "steps": e2e_steps,
                 "path": e2e_path},
@@ -398,7 +398,7 @@ def run_config1_gemv(args, torch, sampler_index):
                    "launch": "CUDA graph replay of the C-ABI calls"},
         "roofline": {"bound": "hbm", "achieved": round(value, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": round(value / peaks["hbm_gbs"], 4), "traffic": None,
-                     "peak_source": f"of {peaks['source']}", "kernel": "dq_gemv_direct_kernel<8,2,true,false,2,2,false>"},
+                     "peak_source": f"of {peaks['source']}", "kernel": "dq_gemv_direct_kernel<8,2,true,false,2,2,false,false>"},
         "e2e": {"value": round(bytes_step * e2e_steps / (ms_e2e * 1e-3) / 1e9, 2), "unit": "GB/s",
                 "h2d_bytes_per_step": M * K * 4, "d2h_bytes_per_step": M * N * 4, "ms_per_step": ms_e2e / e2e_steps,
                 "steps": e2e_steps, "path": "DequantDot.host_entry: pinned host x -> device, nnf_b200_linear, device y -> "
@@ -556,7 +556,7 @@ def extra_measurements(torch, budget_s=90.0):
     attention("decode_attention_32x2048x128")
     layer7b("layer7b_decode_pos2048")
     mlp70b_one_gpu("mlp70b_decode_whole_mlp_m1_one_gpu")
-    for M in (32, 256, 1024, 4096):     # 32: the 64-row batch tile of the tensor-core kernel
+    for M in (32, 256, 1024, 4096):     # 32: clusters of pairs that share K
         gemm(f"prefill_gemm_up_m{M}_11008x4096", M, 11008, 4096)
     gemm("prefill_gemm_down_m4096_4096x11008", 4096, 4096, 11008)
     return also
@@ -592,7 +592,7 @@ def run_prefill_gemm(args, torch, sampler_index):
                    "l2": "x (33.6 MB) + y (90 MB) + weights (23 MB) per step exceed L2"},
         "roofline": {"bound": "tensor", "achieved": round(tf, 1), "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
                      "frac": round(tf / peaks["bf16_tflops_sustained"], 4), "traffic": None,
-                     "peak_source": f"of {peaks['source']} (sustained)", "kernel": "dq_gemm_kernel<4,false>"},
+                     "peak_source": f"of {peaks['source']} (sustained)", "kernel": "dq_gemm_kernel<4,true,false>"},
         "e2e": {"value": round(2.0 * M * N * K * e2e_steps / (ms_e2e * 1e-3) / 1e12, 1), "unit": "TFLOP/s",
                 "h2d_bytes_per_step": M * K * 2, "d2h_bytes_per_step": M * N * 2},
         "gpu_launches": args.steps, "clocks": cs.summary(),
@@ -644,7 +644,7 @@ def run_layer7b(args, torch, sampler_index):
                    "launch": "CUDA graph replay of the C-ABI calls"},
         "roofline": {"bound": "hbm", "achieved": round(value, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": round(value / peaks["hbm_gbs"], 4), "traffic": None,
-                     "peak_source": f"of {peaks['source']}", "kernel": "dq_gemv_kernel x4, decode_attention_kernel"},
+                     "peak_source": f"of {peaks['source']}", "kernel": "dq_gemv_direct_kernel x4, decode_attention_kernel<12>"},
         "e2e": {"value": round(b * e2e_steps / (ms_e2e * 1e-3) / 1e9, 1), "unit": "GB/s",
                 "h2d_bytes_per_step": H * 2, "d2h_bytes_per_step": H * 2},
         "gpu_launches": layers[0].launches * args.steps,
