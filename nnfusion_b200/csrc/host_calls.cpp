@@ -54,6 +54,11 @@ PyObject* wrapped_empty(at::IntArrayRef sizes, c10::ScalarType dtype, c10::Devic
     return THPVariable_Wrap(at::Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt)));
 }
 
+const void* address_of(PyObject* o)
+{
+    return o == Py_None ? nullptr : THPVariable_Unpack(o).const_data_ptr();
+}
+
 // A workspace: a tensor of bytes, or None.
 bool is_workspace(PyObject* o)
 {
@@ -71,6 +76,8 @@ struct LinearEntry
 {
     nnf_b200_linear_desc desc;
     PyObject* ws = nullptr; // the workspace, a tensor that this entry keeps alive, or None
+    void* ws_data = nullptr;
+    size_t ws_bytes = 0;
 };
 
 struct LinearCall
@@ -85,6 +92,8 @@ struct LinearCall
     PyObject* check; // Context.check: raises for a status that is not OK
     int64_t N, K;
     std::unordered_map<uint64_t, LinearEntry>* entries; // by row count and type
+    const LinearEntry* last; // ... the one found last, and its key
+    uint64_t last_key;
 };
 constexpr size_t kMaxEntries = 4096; // beyond that they are all let go and made again
 
@@ -92,6 +101,7 @@ void clear_entries(LinearCall* c)
 {
     std::unordered_map<uint64_t, LinearEntry> old;
     old.swap(*c->entries);
+    c->last = nullptr;
     for (auto& e : old)
         Py_DECREF(e.second.ws);
 }
@@ -114,7 +124,7 @@ bool add_entry(LinearCall* c, PyObject* node, int64_t M, int xd, LinearEntry* e,
         return false;
     }
     *ws = THPObjectPtr::dup(w);
-    e->ws = w;
+    e->ws = w, e->ws_data = const_cast<void*>(address_of(w)), e->ws_bytes = bytes_of(w);
     if (c->entries->size() >= kMaxEntries)
         clear_entries(c);
     LinearEntry& slot = (*c->entries)[(uint64_t)M << 1 | (uint64_t)xd];
@@ -142,11 +152,6 @@ bool hold_handle(PyObject* o, Py_buffer* handle)
     return false;
 }
 
-const void* address_of(PyObject* o)
-{
-    return o == Py_None ? nullptr : THPVariable_Unpack(o).const_data_ptr();
-}
-
 // y = node(x) with x [..., K]; lead: the output takes x's leading dimensions instead of [M, N].
 PyObject* linear_run(LinearCall* self, PyObject* node, PyObject* px, PyObject* pout, PyObject* paddend, bool lead)
 {
@@ -163,11 +168,17 @@ PyObject* linear_run(LinearCall* self, PyObject* node, PyObject* px, PyObject* p
         Py_RETURN_NONE;
     LinearEntry e; // a copy, and a reference to its workspace: the call below runs without the interpreter lock
     THPObjectPtr ws;
-    const auto known = self->entries->find((uint64_t)M << 1 | (uint64_t)xd);
-    if (known != self->entries->end())
-        e = known->second, ws = THPObjectPtr::dup(e.ws);
-    else if (!add_entry(self, node, M, xd, &e, &ws))
-        return nullptr;
+    const uint64_t key = (uint64_t)M << 1 | (uint64_t)xd;
+    if (!self->last || self->last_key != key)
+    {
+        const auto known = self->entries->find(key);
+        if (known != self->entries->end())
+            self->last = &known->second, self->last_key = key; // (stays where it is until the table is cleared)
+        else if (!add_entry(self, node, M, xd, &e, &ws))
+            return nullptr;
+    }
+    if (!ws)
+        e = *self->last, ws = THPObjectPtr::dup(e.ws);
     const c10::ScalarType yt = e.desc.y_dtype == NNF_B200_F16 ? at::kHalf : at::kFloat;
     const void* bias = nullptr;
     if (paddend != Py_None)
@@ -204,12 +215,10 @@ PyObject* linear_run(LinearCall* self, PyObject* node, PyObject* px, PyObject* p
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     const void *px_data = x->const_data_ptr(), *gain = address_of(self->gain);
     nnf_b200_ctx* const ctx = context(self->handle);
-    void* const ws_data = const_cast<void*>(address_of(ws.get()));
-    const size_t ws_bytes = bytes_of(ws.get());
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = self->fn(ctx, stream, &e.desc, px_data, &self->w, self->has_w2 ? &self->w2 : nullptr, gain, bias, y,
-                  ws_data, ws_bytes);
+                  e.ws_data, e.ws_bytes);
     Py_END_ALLOW_THREADS
     if (rc != NNF_B200_OK)
         return PyObject_CallFunction(self->check, "i", rc);
@@ -220,9 +229,15 @@ PyObject* linear_run(LinearCall* self, PyObject* node, PyObject* px, PyObject* p
 template <typename Body>
 PyObject* guarded(Body&& body)
 {
-    HANDLE_TH_ERRORS
-    return body();
-    END_HANDLE_TH_ERRORS
+    try
+    {
+        return body();
+    }
+    catch (...)
+    {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
 }
 
 // call(node, x, out, addend) -> tensor or None
@@ -317,6 +332,8 @@ struct AttnCall
     Py_buffer handle;
     nnf_b200_attn_desc desc;
     PyObject* ws; // the workspace, kept alive, or None
+    void* ws_data;
+    size_t ws_bytes;
     PyObject* check;
 };
 
@@ -349,7 +366,7 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         d.position = (int32_t)position;
         nnf_b200_ctx* const ctx = context(c->handle);
         const size_t need = c->ws_fn(ctx, &d);
-        if (need > bytes_of(c->ws))
+        if (need > c->ws_bytes)
         {
             THPObjectPtr grown(PyObject_CallMethod(args[0], "_grown", "l", position));
             if (!grown)
@@ -358,11 +375,13 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
                 Py_RETURN_NONE;
             PyObject* const before = c->ws;
             c->ws = grown.release();
+            c->ws_data = const_cast<void*>(address_of(c->ws)), c->ws_bytes = bytes_of(c->ws);
             Py_DECREF(before);
         }
         // (referenced: the call below runs without the interpreter lock)
         THPObjectPtr ws = THPObjectPtr::dup(c->ws);
-        const size_t ws_bytes = bytes_of(ws.get());
+        const size_t ws_bytes = c->ws_bytes;
+        void* const ws_data = c->ws_data;
         THPObjectPtr out;
         if (a[6] == Py_None)
         {
@@ -380,7 +399,6 @@ PyObject* attn_call(PyObject* self, PyObject* const* args, Py_ssize_t n)
         const void *qp = q->const_data_ptr(), *kp = k->const_data_ptr(), *vp = v->const_data_ptr();
         void *kcp = kc->mutable_data_ptr(), *vcp = vc->mutable_data_ptr();
         void* op = THPVariable_Unpack(out.get()).mutable_data_ptr();
-        void* const ws_data = const_cast<void*>(address_of(ws.get()));
         int rc;
         Py_BEGIN_ALLOW_THREADS
         rc = c->fn(ctx, stream, &d, qp, kp, vp, kcp, vcp, op, need ? ws_data : nullptr, need ? ws_bytes : 0);
@@ -417,6 +435,7 @@ PyObject* attn_new(PyTypeObject* type, PyObject* args, PyObject*)
         c->handle = handle;
         memcpy(&c->desc, desc.buf, sizeof c->desc);
         c->ws = Py_NewRef(ws);
+        c->ws_data = const_cast<void*>(address_of(ws)), c->ws_bytes = bytes_of(ws);
         c->check = Py_NewRef(check);
     }
     PyBuffer_Release(&desc);
