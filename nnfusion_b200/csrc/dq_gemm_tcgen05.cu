@@ -53,32 +53,40 @@ constexpr int kBK = 64;                       // k-block: one 128-byte swizzle r
 constexpr int kWStageBytes = kBN * 128;       // one raw chunk
 constexpr int kTmemCols = 512;                // all of it: it starts at column 0
 constexpr int kASlotCols = 32;                // a converted k-block in tensor memory: 64 fp16 per lane
-constexpr int kASlots = 8;
 constexpr int kMaxPairs = 128;                // pairs of a launch, at most
 constexpr int kEpiBarrier = 1;                // named barrier of the epilogue warps
 
+// BX: the most batch rows of a tile, 64, 128 or 256.
 // SMALL: tiles of up to 128 batch rows, whose multiplication takes no longer than the conversion of the weights: four
 // groups of conversion warps instead of two (about 220 clocks per k-block instead of 380; a k-block of 128 batch rows takes
 // the tensor core 256) and a raw ring of 128 KB (HBM's latency at full rate is about 100 KB per SM), paid for with half of
 // the epilogue warps and a smaller x ring.
-template <bool SMALL>
+// Up to 64 batch rows the two accumulators leave room for 12 converted k-blocks instead of 8, three stages instead of two: a
+// stage's conversion, its multiplies and the handing over between them follow one another, and what bounds these tiles is how
+// many stages are at it side by side.  With the quantisation parameters hoisted out of the conversion's loop: 48 x 11008 x 4096
+// 18.9 -> 17.6 us, the gate/up pair of that shape 35.6 -> 33.2, 48 x 4096 x 11008 19.3 -> 18.8 (graph replay, weights beyond L2).
+// Where the line lies: 65 rows would need accumulators of 80 columns, and 11 k-blocks are two whole stages again.
+template <int BX>
 struct Cfg
 {
-    static constexpr int MAX_BX = SMALL ? 128 : 256;
+    static constexpr bool SMALL = BX <= 128;
+    static constexpr int MAX_BX = BX;
+    static constexpr int ACC_COLS = SMALL ? BX : 128;    // TMEM columns from one accumulator to the next
     static constexpr int DQ_GROUPS = SMALL ? 4 : 2, DQ_WARPS = 4 * DQ_GROUPS;
     static constexpr int EPI_WARPS = SMALL ? 4 : 8;
     static constexpr int X_WARP = DQ_WARPS + EPI_WARPS, MMA_WARP = X_WARP + 1, W_WARP = X_WARP + 2;
     static constexpr int THREADS = (X_WARP + 4) * 32;    // whole warpgroups: registers are moved between them
-    static constexpr int X_BYTES = (SMALL ? 96 : 128) * 1024; // ring of x tiles: as many stages as fit
+    static constexpr int X_BYTES = (BX <= 64 ? 64 : SMALL ? 96 : 128) * 1024; // ring of x tiles: as many stages as fit
     static constexpr int MAX_X_STAGES = 16;
-    static constexpr int W_STAGES = SMALL ? 8 : 6;       // ring of raw chunks
+    static constexpr int W_STAGES = BX <= 64 ? 10 : SMALL ? 8 : 6;       // ring of raw chunks
     // A stage is what the tensor core is handed at a time: waits, commits and bookkeeping cost its warp about 500 clocks a
     // stage, whatever the stage holds (with two k-blocks of up to 128 batch rows they set the pace: 445 clocks a k-block).
     static constexpr int STAGE_KB = SMALL ? 4 : 2;       // k-blocks per stage
-    static constexpr int STAGES = kASlots / STAGE_KB;    // ring of stages of converted weights
+    static constexpr int A_SLOTS = (kTmemCols - 2 * ACC_COLS) / kASlotCols; // converted k-blocks
+    static constexpr int STAGES = A_SLOTS / STAGE_KB;    // ring of stages of converted weights
     // Large tiles: a group converts whole stages, in turn.  Small ones: every group converts one k-block of every stage.
     static constexpr int VISIT_KB = 2, VISIT_STAGES = 2;
-    static constexpr int A_COL0 = 256;                   // first TMEM column of the A stages; the accumulators are below
+    static constexpr int A_COL0 = 2 * ACC_COLS;                   // first TMEM column of the A stages; the accumulators are below
     static constexpr int PACKED = MAX_BX / (EPI_WARPS / 4) / 2; // registers for an epilogue thread's fp16 results
     // full / empty per stage of weights, of x and per raw chunk, full / empty per accumulator, exchange ready / complete
     static constexpr int BARRIERS = 2 * STAGES + 2 * MAX_X_STAGES + 2 * W_STAGES + 6;
@@ -89,7 +97,7 @@ struct Cfg
     static constexpr int DQ_REGS = 72, EPI_REGS = SMALL ? 136 : 144, ISSUE_REGS = SMALL ? 56 : 48;
     static_assert(DQ_GROUPS * DQ_REGS + EPI_WARPS / 4 * EPI_REGS + ISSUE_REGS <= THREADS / 128 * LAUNCH_REGS, "registers the CTA has");
     static_assert(LAUNCH_REGS * THREADS <= 65536, "registers the SM has");
-    static_assert(A_COL0 + kASlots * kASlotCols <= kTmemCols, "tensor memory budget");
+    static_assert(A_COL0 + A_SLOTS * kASlotCols <= kTmemCols, "tensor memory budget");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
 
@@ -366,12 +374,12 @@ __device__ __forceinline__ void add_parts(const GemmParams& p, Load load, int pa
 }
 
 // ONE_GROUP: two neighbouring k-blocks (of a raw chunk) always lie in one quantisation group.
-template <int WBITS, bool ONE_GROUP, bool SMALL>
-__global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
+template <int WBITS, bool ONE_GROUP, int BX>
+__global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
     dq_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
                    const __grid_constant__ CUtensorMap tmap_w1)
 {
-    using C = Cfg<SMALL>;
+    using C = Cfg<BX>;
     constexpr int KBC = (WBITS == 4) ? 4 : 2;           // k-blocks per raw chunk
     constexpr int RAW_BYTES = (WBITS == 4) ? 32 : 64;   // raw bytes per row and k-block
     extern __shared__ uint8_t smem_raw[];
@@ -573,7 +581,7 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                 if (!ok)
                     break;
                 tcgen05_fence_after();
-                const uint32_t d_tmem = tmem_base + b * 128u;
+                const uint32_t d_tmem = tmem_base + b * (uint32_t)C::ACC_COLS;
                 uint32_t accumulate = 0u; // the segment's first MMA overwrites D
                 const int kb_end = min(KB, sg.c1 * KBC);
                 for (int kb = sg.c0 * KBC; kb < kb_end; kb += C::STAGE_KB)
@@ -698,61 +706,70 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                 if (!ok)
                     break;
                 tcgen05_fence_after();
-                // Half a k-block at a time: raw bytes -> 32 fp16 (q - zp) * scale in k order (register i holds k = 2i in its
-                // low half and k = 2i + 1 in its high half).  (A loop: unrolled over the visit, a fifth of the issue slots
-                // went to instruction fetch.)
+                // A k-block at a time, in halves: raw bytes -> 32 fp16 (q - zp) * scale in k order (register i holds k = 2i in its low
+                // half and k = 2i + 1 in its high half).  (A loop: unrolled over the visit, a fifth of the issue slots went to
+                // instruction fetch; half a k-block per trip, and the quantisation parameters made anew in each, were a sixth of
+                // the conversion's instructions.)
+                __half2 scale2, zc; // scale; uint4: (1024 + zp, 64 + zp), uint8: 1024 + zp in both halves
+                auto set_params = [&](int j) {
+                    const uint32_t sraw = s_now[j], zraw = z_now[j];
+                    const __half2 from_f32 = __float2half2_rn(__uint_as_float(sraw));
+                    const uint32_t s2 = p.scale_f32 ? *reinterpret_cast<const uint32_t*>(&from_f32) : __byte_perm(sraw, 0u, 0x1010);
+                    scale2 = *reinterpret_cast<const __half2*>(&s2);
+                    const uint32_t zq = WBITS == 4 ? (zraw >> (4 * (g_now[j] & 1))) & 0xFu : zraw;
+                    const uint32_t z2 = WBITS == 4 ? (0x6400u | zq) | ((0x5400u | (zq << 4)) << 16) : (0x6400u | zq) * 0x00010001u;
+                    zc = *reinterpret_cast<const __half2*>(&z2);
+                };
+                set_params(0);
 #pragma unroll 1
-                for (int hb = 0; hb < 2 * nkb; hb++)
+                for (int kbi = 0; kbi < nkb; kbi++)
                 {
-                    constexpr int NV = RAW_BYTES / 32;
+                    constexpr int NV = RAW_BYTES / 16;
                     uint4 raw[NV];
 #pragma unroll
                     for (int v = 0; v < NV; v++)
-                        raw[v] = lds128(row + (uint32_t)((((2 * in_chunk + hb) * NV + v) ^ (r & 7)) * 16));
-                    const bool second = !ONE_GROUP && hb >= 2;
-                    const uint32_t sraw = second ? s_now[NP - 1] : s_now[0], zraw = second ? z_now[NP - 1] : z_now[0];
-                    const uint32_t zq = WBITS == 4 ? (zraw >> (4 * ((second ? g_now[NP - 1] : g_now[0]) & 1))) & 0xFu : zraw;
-                    const __half2 from_f32 = __float2half2_rn(__uint_as_float(sraw));
-                    const uint32_t s2 = p.scale_f32 ? *reinterpret_cast<const uint32_t*>(&from_f32) : __byte_perm(sraw, 0u, 0x1010);
-                    const __half2 scale2 = *reinterpret_cast<const __half2*>(&s2);
-                    uint32_t a[16];
-                    if (WBITS == 4)
+                        raw[v] = lds128(row + (uint32_t)((((in_chunk + kbi) * NV + v) ^ (r & 7)) * 16));
+                    if (!ONE_GROUP && kbi > 0)
+                        set_params(NP - 1);
+#pragma unroll
+                    for (int half = 0; half < 2; half++)
                     {
-                        const uint32_t zc = (0x6400u | zq) | ((0x5400u | (zq << 4)) << 16); // (1024 + zp, 64 + zp)
-                        const uint32_t w4[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
-#pragma unroll
-                        for (int wi = 0; wi < 4; wi++)
-#pragma unroll
-                            for (int b = 0; b < 4; b++)
-                            {
-                                // byte b of the word holds elements 2b (bits 0-3) and 2b+1 (bits 4-7)
-                                uint32_t t = __byte_perm(w4[wi], 0u, 0x1111u * b);
-                                asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(t) : "r"(t), "n"(0x00F0000Fu), "n"(0x54006400u));
-                                __half2 h = __hsub2(*reinterpret_cast<__half2*>(&t), *reinterpret_cast<const __half2*>(&zc));
-                                h = __hmul2(h, scale2);
-                                a[wi * 4 + b] = *reinterpret_cast<uint32_t*>(&h);
-                            }
-                    }
-                    else
-                    {
-                        const uint32_t zc = (0x6400u | zq) * 0x00010001u; // 1024 + zp in both halves
-#pragma unroll
-                        for (int v = 0; v < NV; v++)
+                        uint32_t a[16];
+                        if (WBITS == 4)
                         {
-                            const uint32_t w4[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
+                            const uint32_t w4[4] = {raw[half].x, raw[half].y, raw[half].z, raw[half].w};
 #pragma unroll
                             for (int wi = 0; wi < 4; wi++)
 #pragma unroll
-                                for (int b = 0; b < 2; b++)
+                                for (int b = 0; b < 4; b++)
                                 {
-                                    uint32_t t = __byte_perm(w4[wi], 0x64646464u, b ? 0x4342 : 0x4140); // 1024 + (b0, b1)
-                                    __half2 h = __hsub2(*reinterpret_cast<__half2*>(&t), *reinterpret_cast<const __half2*>(&zc));
-                                    h = __hmul2(h, scale2);
-                                    a[(v * 4 + wi) * 2 + b] = *reinterpret_cast<uint32_t*>(&h);
+                                    // byte b of the word holds elements 2b (bits 0-3) and 2b+1 (bits 4-7)
+                                    uint32_t t = __byte_perm(w4[wi], 0u, 0x1111u * b);
+                                    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(t) : "r"(t), "n"(0x00F0000Fu), "n"(0x54006400u));
+                                    const __half2 h = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&t), zc), scale2);
+                                    a[wi * 4 + b] = *reinterpret_cast<const uint32_t*>(&h);
                                 }
                         }
+                        else
+                        {
+#pragma unroll
+                            for (int v = 0; v < 2; v++)
+                            {
+                                const uint4 q = raw[(2 * half + v) % NV];
+                                const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                                for (int wi = 0; wi < 4; wi++)
+#pragma unroll
+                                    for (int b = 0; b < 2; b++)
+                                    {
+                                        const uint32_t t = __byte_perm(w4[wi], 0x64646464u, b ? 0x4342 : 0x4140); // 1024 + (b0, b1)
+                                        const __half2 h = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&t), zc), scale2);
+                                        a[(v * 4 + wi) * 2 + b] = *reinterpret_cast<const uint32_t*>(&h);
+                                    }
+                            }
+                        }
+                        tmem_st_32x16(col + (uint32_t)(kbi * kASlotCols + half * 16), a);
                     }
-                    tmem_st_32x16(col + (uint32_t)(hb * 16), a);
                 }
                 tcgen05_wait_st();
                 tcgen05_fence_before();
@@ -803,7 +820,7 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
             const int m_end = min(p.bx, p.M - m0); // columns that exist
             const float bias = p.has_bias && row_ok ? p.bias[n] : 0.f;
             const bool gated = sg.set == 1 && sg.whole;
-            const uint32_t d_addr = tmem_base + lane_addr + b * 128u;
+            const uint32_t d_addr = tmem_base + lane_addr + b * (uint32_t)C::ACC_COLS;
             const long long U = (long long)p.tiles * p.sets * p.cpt;
             const int G = (int)(gridDim.x >> 1);
             auto release = [&] { // this warp's last read of D: a later segment may overwrite it
@@ -1017,7 +1034,7 @@ __global__ void __launch_bounds__(Cfg<SMALL>::THREADS, 1)
                     {
                         const int dst = col / p.slice; // (slices are multiples of 16 batch rows)
                         uint32_t d[16];
-                        tmem_ld_32x16(tmem_base + lane_addr + (uint32_t)(set * 128 + col), d);
+                        tmem_ld_32x16(tmem_base + lane_addr + (uint32_t)(set * C::ACC_COLS + col), d);
                         const uint32_t to = map_to_rank(buf + (uint32_t)(((set * p.ksplit + part) * p.slice + col - dst * p.slice) * kBN + r) * 4u,
                                                         2u * (uint32_t)dst + rank);
                         tcgen05_wait_ld();
@@ -1196,11 +1213,11 @@ cudaError_t launch_prep(const void* x, const float* gain, __half* out, int M, in
     return cudaLaunchKernelEx(&cfg, prep_activations_kernel<XF32>, x, gain, out, K, eps);
 }
 
-template <int WBITS, bool ONE_GROUP, bool SMALL>
+template <int WBITS, bool ONE_GROUP, int BX>
 cudaError_t launch(const GemmParams& p, const CUtensorMap& tx, const CUtensorMap& tw0, const CUtensorMap& tw1, int pairs,
                    cudaStream_t stream)
 {
-    using C = Cfg<SMALL>;
+    using C = Cfg<BX>;
     static bool configured[nnf::kMaxDevices] = {}; // the attribute belongs to the device that is current
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1210,7 +1227,7 @@ cudaError_t launch(const GemmParams& p, const CUtensorMap& tx, const CUtensorMap
         return cudaErrorInvalidDevice;
     if (!configured[dev])
     {
-        e = cudaFuncSetAttribute(dq_gemm_kernel<WBITS, ONE_GROUP, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
+        e = cudaFuncSetAttribute(dq_gemm_kernel<WBITS, ONE_GROUP, BX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
         if (e != cudaSuccess)
             return e;
         configured[dev] = true;
@@ -1229,16 +1246,16 @@ cudaError_t launch(const GemmParams& p, const CUtensorMap& tx, const CUtensorMap
     attr[cfg.numAttrs].val.clusterDim.z = 1;
     cfg.numAttrs++;
     cfg.attrs = attr;
-    return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<WBITS, ONE_GROUP, SMALL>, p, tx, tw0, tw1);
+    return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<WBITS, ONE_GROUP, BX>, p, tx, tw0, tw1);
 }
 
-template <bool SMALL>
+template <int BX>
 cudaError_t dispatch(int wbits, bool one_group, const GemmParams& p, const CUtensorMap& tx, const CUtensorMap& tw0,
                      const CUtensorMap& tw1, int pairs, cudaStream_t stream)
 {
     if (wbits == 4)
-        return one_group ? launch<4, true, SMALL>(p, tx, tw0, tw1, pairs, stream) : launch<4, false, SMALL>(p, tx, tw0, tw1, pairs, stream);
-    return one_group ? launch<8, true, SMALL>(p, tx, tw0, tw1, pairs, stream) : launch<8, false, SMALL>(p, tx, tw0, tw1, pairs, stream);
+        return one_group ? launch<4, true, BX>(p, tx, tw0, tw1, pairs, stream) : launch<4, false, BX>(p, tx, tw0, tw1, pairs, stream);
+    return one_group ? launch<8, true, BX>(p, tx, tw0, tw1, pairs, stream) : launch<8, false, BX>(p, tx, tw0, tw1, pairs, stream);
 }
 } // namespace
 
@@ -1380,7 +1397,7 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     }
     const bool silu_mul = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
     const int row_bytes = d.w_bits == 4 ? d.K / 2 : d.K;
-    const bool small = L.bx <= Cfg<true>::MAX_BX;
+    const int cfg = L.bx <= 64 ? 64 : L.bx <= 128 ? 128 : 256;
     GemmParams p{};
     p.y = y;
     p.status = ctx->dev_status;
@@ -1391,8 +1408,8 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     p.y_f32 = d.y_dtype == NNF_B200_F32;
     p.scale_f32 = d.scale_dtype == NNF_B200_F32;
     p.bx = L.bx;
-    p.x_stages = std::min(Cfg<true>::MAX_X_STAGES, small ? Cfg<true>::X_BYTES / (L.bx * 64 * Cfg<true>::STAGE_KB)
-                                                         : Cfg<false>::X_BYTES / (L.bx * 64 * Cfg<false>::STAGE_KB));
+    const int x_ring = cfg == 64 ? Cfg<64>::X_BYTES : cfg == 128 ? Cfg<128>::X_BYTES : Cfg<256>::X_BYTES;
+    p.x_stages = std::min(Cfg<64>::MAX_X_STAGES, x_ring / (L.bx * 64 * (cfg <= 128 ? Cfg<128>::STAGE_KB : Cfg<256>::STAGE_KB)));
     p.m_tiles = L.m_tiles;
     p.tiles = L.tiles;
     p.sets = L.sets;
@@ -1431,8 +1448,9 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
             return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the weight tensor");
         tw[i] = *m;
     }
-    const cudaError_t e = small ? dispatch<true>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream)
-                                : dispatch<false>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream);
+    const cudaError_t e = cfg == 64    ? dispatch<64>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream)
+                          : cfg == 128 ? dispatch<128>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream)
+                                       : dispatch<256>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream);
     if (e != cudaSuccess)
         return set_error(ctx, NNF_B200_ECUDA, std::string("dq_gemm launch: ") + cudaGetErrorString(e));
     ctx->launches++;
