@@ -184,7 +184,10 @@ NNF_B200_API size_t nnf_b200_linear_workspace_bytes(const nnf_b200_ctx* ctx, con
  * meet in shared memory; the launch falls back to the workspace when the device
  * cannot hold every cluster at once), 2 weight loads take lines in L1, 4 only the
  * scale / zero-point columns of a CTA's own K range are kept in shared memory,
- * 8 one batch holds every tile of a CTA.  out[6..7] are zero for the tensor-core
+ * 8 one batch holds every tile of a CTA, 16 the call takes the form that streams the
+ * weights through shared memory when its workspace holds it (9 to 16 rows; the other
+ * fields then describe the split form, which serves smaller workspaces, the sum over
+ * ranks and the static scratch).  out[6..7] are zero for the tensor-core
  * kernel.  ctx may be NULL (a 148-SM device is assumed).  No reference
  * counterpart: the reference leaves such choices to cuBLAS. */
 NNF_B200_API int nnf_b200_linear_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc* desc, int32_t out[8]);

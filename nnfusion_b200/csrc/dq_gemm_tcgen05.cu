@@ -126,45 +126,6 @@ struct GemmParams
     int cpt;         // raw chunks (the unit of work) per tile and weight set
 };
 
-constexpr uint32_t kGemmSpin = 1u << 21;
-
-// Bounded waits that also give up as soon as another role of the CTA has raised the abort flag.  SLEEP: nanoseconds between
-// polls; a waiting role should not compete with the working ones for issue slots.
-// One thread:
-template <int SLEEP>
-__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag)
-{
-    for (uint32_t i = 0; i < kGemmSpin; i++)
-    {
-        if (mbar_try_wait(bar, parity))
-            return true;
-        if constexpr (SLEEP > 0)
-            __nanosleep(SLEEP);
-        if ((i & 255u) == 255u && *abort_flag)
-            return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
-// A whole warp.  Every decision is a vote, which the compiler knows to be the same for all lanes: the warp stays together
-// for the warp-wide tensor-memory instructions that follow, and what follows may use uniform registers.  CLUSTER: what was
-// announced happened in another CTA of the cluster.
-template <int SLEEP, bool CLUSTER = false>
-__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
-{
-    for (uint32_t i = 0; i < kGemmSpin; i++)
-    {
-        if (__all_sync(0xffffffffu, CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)))
-            return true;
-        if constexpr (SLEEP > 0)
-            __nanosleep(SLEEP);
-        if ((i & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0))
-            return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
-
 // UMMA shared-memory descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_k_sw128(uint32_t smem_addr)
 {
@@ -1046,7 +1007,7 @@ __global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
                 if (lane < p.ksplit)
                     mbar_arrive_cluster_release(map_to_rank(parts_here, 2u * (uint32_t)lane + rank));
                 bool here = false;
-                for (uint32_t i = 0; i < kGemmSpin && !here && !*abort_flag; i++)
+                for (uint32_t i = 0; i < kRoleSpin && !here && !*abort_flag; i++)
                     here = mbar_try_wait_cluster(parts_here, 0u);
                 fine = __all_sync(0xffffffffu, here);
             }

@@ -1,0 +1,659 @@
+// Dequantize-fused linear for 9 to 16 batch rows and much weight on sm_100a, weights streamed through shared memory:
+//     y[M,N] = epi(pro(x)[M,K] . dequant(W)[N,K]^T),  fp16 x, uint4 W
+//
+// Replaces the same launches of the reference as its neighbours do (Convert -> Subtract -> Multiply,
+// src/nnfusion/core/kernels/cuda_gpu/kernels/elementwise.hpp:33-157, and the Dot,
+// src/nnfusion/core/kernels/cuda_gpu/kernels/dot.cpp:27-372).
+//
+// Why a form of its own: with 16 rows the small-M kernel (dq_gemv_direct.cu) spills, keeps half of the activation fragments in
+// shared memory per warp, meets over its 16 warps once per batch of tiles and cuts a K beyond 4096 over CTAs.  Two launches
+// instead.  The first (stream_prep_kernel) brings the activations, a few hundred KB, into the order in which the second one's
+// lanes want them, normalised and rounded to fp16, with the sums that take the unpacking's offsets and the zero-points out of
+// the products.  The second:
+//   * work is counted in units of 128 weight rows x 128 elements of K; the units, tile by tile, are dealt out to the CTAs in
+//     equal contiguous shares, so that a narrow matrix with a long K and a wide one load the SMs alike;
+//   * the lanes of one warp keep a ring of units filled by TMA: 8 KB of packed weights, which leave before the launch ahead has
+//     ended, and the unit's 4 KB of prepared activations by a bulk copy;
+//   * eight warps consume it.  A warp owns 16 rows of the tile for all of the share's K: its sums stay in its registers, scaled
+//     in fp32 after every unit, and no warp ever meets another.  Weights become exact fp16 integers by the exponent trick (five
+//     instructions per eight weights) and multiply by mma.sync.m16n8k16;
+//   * a tile that several CTAs share goes through the workspace, warp by warp: each stores its sums and takes a ticket, the last
+//     one adds them in the order of their K ranges (bitwise repeatable; nobody waits for another CTA);
+//   * two weight sets (SiLU(gate) * up): a tile is 64 gate rows and the same 64 rows of the up projection, and a warp's 16 rows
+//     are 8 of each, so that a lane holds both sums of an output.
+// A CTA takes half an SM (113 KB, 288 threads), two are resident.
+// What bounds it: about 150 instructions a warp and unit at half of the issue rate (so are its neighbours), and a fixed cost of
+// some 8 us (two launches' hand-over, the shared tiles' ticket and sums), which is why small weights stay with the small-M kernel.
+// Every mbarrier wait is bounded; on a time-out the CTA raises a status flag and stores nothing more, after its copies have
+// landed.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <algorithm>
+
+#include "nnf_internal.h"
+#include "sm100_ptx.cuh"
+
+namespace
+{
+using namespace nnf::ptx;
+
+constexpr int kRows = 128;      // weight rows of a tile
+constexpr int kUnitK = 128;     // elements of K per unit
+constexpr int kBatch = 16;      // batch rows of a block of activations
+constexpr int MB = kBatch / 8;
+constexpr int kConsumers = 8;   // warps, 16 weight rows of a tile each
+constexpr int kThreads = (kConsumers + 1) * 32;
+constexpr int kWBytes = kRows * kUnitK / 2;              // packed weights of a unit
+constexpr int kBlockBytes = kBatch * (2 * kUnitK + 8);   // prepared activations of a unit
+constexpr int kStages = 9;                               // ring of units
+constexpr int kSums = MB * 4 * 32;                       // a warp's sums of a tile
+constexpr int kSmem = kStages * (kWBytes + kBlockBytes) + 2 * kStages * 8 + 16;
+constexpr int kPrepThreads = 128, kPrepSteps = 4;
+static_assert(kSmem <= 113 * 1024, "two CTAs an SM");
+static_assert(kStages <= 32, "a lane per stage");
+
+struct StreamParams
+{
+    const void* scale[2];
+    const uint8_t* zp[2];
+    const void* bias;        // fp32 [N], or (has_addend) [M,N] of y's type, or null
+    void* y;
+    int* status;
+    uint32_t* counters;      // [tiles][warps] arrivals at shared tiles; zero before and after
+    float* slots;            // [CTAs][2][warps][kSums] partial sums of shared tiles
+    const uint8_t* xblocks;  // [units of K][kBlockBytes] prepared activations
+    int M, N, KU;            // KU: units of K
+    int units_lo, units_rem; // a CTA's share: tiles x KU / CTAs and its remainder (the first units_rem CTAs have one more)
+    int dual;
+    int G, zp_row_bytes;
+    int group_units;         // units per quantisation group
+    uint32_t group_magic;    // ceil(2^32 / group_units)
+    int y_f32, scale_f32, has_addend;
+};
+
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Same, starting a sum: the addend is zero.
+__device__ __forceinline__ void mma16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// (w & MASK) | orv, the OR-ed constant in a register that the caller fills once
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t orv)
+{
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(orv));
+    return r;
+}
+__device__ __forceinline__ uint32_t held(uint32_t v)
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+// 16-byte aligned addresses, a size that is a multiple of 16
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    dq_stream_kernel(const StreamParams p, const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1)
+{
+    extern __shared__ __align__(1024) uint8_t smem[]; // [stages][weights], [stages][activations], barriers, abort flag
+    // The next launch on the stream may start as soon as there is room (it waits for this grid's results itself).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t smem_s = smem_u32(smem);
+    const uint32_t x_ring = smem_s + kStages * kWBytes;
+    const uint32_t bar0 = x_ring + kStages * kBlockBytes;
+    auto full = [&](int s) { return bar0 + 8u * s; };              // weights and activations of a unit have landed
+    auto empty = [&](int s) { return bar0 + 8u * (kStages + s); }; // ... and have been read by every warp
+    volatile int* const abort_flag = reinterpret_cast<volatile int*>(smem + kStages * (kWBytes + kBlockBytes) + 2 * kStages * 8);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int KU = p.KU;
+    auto share_begin = [&](int cta) { return cta * p.units_lo + min(cta, p.units_rem); };
+    const int u_begin = share_begin((int)blockIdx.x);
+    const int n_units = p.units_lo + ((int)blockIdx.x < p.units_rem ? 1 : 0);
+    const int tile_begin = u_begin / KU, ku_begin = u_begin - tile_begin * KU;
+
+    // (the producer's lanes each ask for a unit: the four instructions and the wait of a unit take one thread several hundred clocks)
+    auto ask_weights = [&](int st, int unit) {
+        const int at = ku_begin + unit, tile = tile_begin + at / KU, col = at % KU * (kUnitK / 2);
+        const uint32_t dst = smem_s + (uint32_t)(st * kWBytes);
+        mbar_arrive_expect_tx(full(st), kWBytes);
+        if (p.dual)
+        {
+            tma_load_2d(dst, &tmap_w0, full(st), col, tile * 64);
+            tma_load_2d(dst + kWBytes / 2, &tmap_w1, full(st), col, tile * 64);
+        }
+        else
+            tma_load_2d(dst, &tmap_w0, full(st), col, tile * kRows);
+    };
+    const int first_round = min(n_units, kStages);
+    if (warp == kConsumers)
+    {
+        if (lane < kStages)
+        {
+            mbar_init(full(lane), 2); // the weights' announcement and the activations'
+            mbar_init(empty(lane), kConsumers);
+        }
+        if (lane == 0)
+            *abort_flag = (smem_s & 1023u) != 0u; // (the swizzle counts on an aligned window)
+        fence_barrier_init();
+        __syncwarp();
+        if (lane < first_round) // weights are constants: they leave before anything else
+            ask_weights(lane, lane);
+    }
+    __syncthreads();
+
+    if (warp == kConsumers)
+    {
+        // ------------------------------------------------------------ producer
+        asm volatile("griddepcontrol.wait;" ::: "memory"); // the activations are what the launch ahead writes
+        auto ask_x = [&](int st, int unit) {
+            mbar_arrive_expect_tx(full(st), kBlockBytes);
+            bulk_load(x_ring + (uint32_t)(st * kBlockBytes), p.xblocks + (size_t)((ku_begin + unit) % KU) * kBlockBytes, kBlockBytes, full(st));
+        };
+        if (lane < first_round)
+            ask_x(lane, lane);
+        constexpr int batch = 4; // units at a time (fewer than stages: a lane per stage)
+        int i = first_round;
+        for (; i < n_units; i += batch)
+        {
+            const int unit = i + lane, st = unit % kStages;
+            const bool active = lane < batch && unit < n_units;
+            bool ok = false;
+            for (uint32_t tries = 0; tries < kRoleSpin; tries++)
+            {
+                ok = !active || mbar_try_wait(empty(st), ((unit / kStages) & 1u) ^ 1u);
+                if (__all_sync(0xffffffffu, ok) || ((tries & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0)))
+                    break;
+            }
+            if (!__all_sync(0xffffffffu, ok))
+            {
+                *abort_flag = 1;
+                break;
+            }
+            if (active)
+            {
+                ask_weights(st, unit);
+                ask_x(st, unit);
+            }
+        }
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) // copies in flight land before the CTA ends
+        {
+            const int last = min(n_units, i) - 1 - lane; // a lane per stage
+            if (lane < kStages && last >= 0)
+                for (int t = 0; t < 4096 && !mbar_test_wait(full(last % kStages), (last / kStages) & 1u); t++)
+                    __nanosleep(100);
+        }
+    }
+    else
+    {
+        // ------------------------------------------------------------ consumers
+        const int g = lane >> 2, t = lane & 3;
+        // rows of the tile (in shared memory) of accumulator rows g and g + 8
+        const int r0 = p.dual ? 8 * warp + g : 16 * warp + g, r1 = p.dual ? r0 + 64 : r0 + 8;
+        // raw bytes of a row: 16-byte piece j of row r lies at piece j ^ (r >> 1 & 3).  Lane t holds elements 32 t .. 32 t + 31 of
+        // the unit.
+        const uint32_t w_at[2] = {smem_s + (uint32_t)(r0 * 64 + ((t ^ ((r0 >> 1) & 3)) << 4)), smem_s + (uint32_t)(r1 * 64 + ((t ^ ((r1 >> 1) & 3)) << 4))};
+        const uint32_t x_at = x_ring + (uint32_t)(g * 64 + t * 16);
+        const uint32_t nc_at = x_ring + (uint32_t)(kBatch * 256 + t * 16);
+        const uint32_t k6400 = held(0x64006400u), k5400 = held(0x54005400u);
+
+        // Scales and zero-points: lane t of a row's four asks for those of unit 4 i + t, four units ahead; a unit's come round by
+        // shuffles.  (A warp's rows lie in as many lines: asked for unit by unit they would take the load unit's turns from shared
+        // memory's users.)
+        int s_tile = tile_begin, s_ku = ku_begin; // unit of this lane's next request
+        auto advance = [&](int by) {
+            for (s_ku += by; s_ku >= KU; s_ku -= KU)
+                s_tile++;
+        };
+        uint32_t s_raw[2] = {0u, 0u}, z_raw[2] = {0u, 0u}, s_cur[2], z_cur[2];
+        int z_shift = 0;
+        auto ask_params = [&] {
+            const int gr = p.group_units == 1 ? s_ku : (int)__umulhi((uint32_t)s_ku, p.group_magic);
+            z_shift = 4 * (gr & 1);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+            {
+                const int set = p.dual ? h : 0;
+                const size_t n = (size_t)min(p.dual ? s_tile * 64 + r0 : s_tile * kRows + (h == 0 ? r0 : r1), p.N - 1); // (rows past N are never stored)
+                s_raw[h] = p.scale_f32 ? __ldg(static_cast<const uint32_t*>(p.scale[set]) + n * p.G + gr)
+                                       : (uint32_t)__ldg(static_cast<const unsigned short*>(p.scale[set]) + n * p.G + gr);
+                z_raw[h] = (uint32_t)__ldg(p.zp[set] + n * p.zp_row_bytes + (gr >> 1));
+            }
+        };
+        advance(t);
+        if (t < n_units)
+            ask_params();
+
+        float tot[MB][4];
+#pragma unroll
+        for (int mb = 0; mb < MB; mb++)
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                tot[mb][c] = 0.f;
+        // y, the addend and the workspace may be the launch ahead's
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        int tile = tile_begin, ku = ku_begin, seg_ku0 = ku_begin, st = 0;
+        uint32_t phase = 0;
+        for (int i = 0; i < n_units; i++)
+        {
+            if ((i & 3) == 0)
+            {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    s_cur[h] = s_raw[h], z_cur[h] = (z_raw[h] >> z_shift) & 0xFu;
+                advance(4);
+                if (i + 4 + t < n_units)
+                    ask_params();
+            }
+            float sc[2], nz[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+            {
+                const uint32_t s = __shfl_sync(0xffffffffu, s_cur[h], (lane & ~3) | (i & 3));
+                sc[h] = p.scale_f32 ? __uint_as_float(s) : __half2float(__ushort_as_half((unsigned short)s));
+                nz[h] = (float)__shfl_sync(0xffffffffu, z_cur[h], (lane & ~3) | (i & 3));
+            }
+            if (!wait_warp<0>(full(st), phase, abort_flag))
+                break;
+            const uint32_t w_off = (uint32_t)(st * kWBytes), x_off = (uint32_t)(st * kBlockBytes);
+            const uint4 w[2] = {lds128(w_at[0] + w_off), lds128(w_at[1] + w_off)};
+            float acc[MB][4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                uint32_t a[2][4]; // [row half][pair]
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                {
+                    const uint32_t q = j == 0 ? w[h].x : (j == 1 ? w[h].y : (j == 2 ? w[h].z : w[h].w)), q8 = q >> 8;
+                    a[h][0] = and_or<0x000F000Fu>(q, k6400);  // 1024 + (n0, n4)
+                    a[h][1] = and_or<0x00F000F0u>(q, k5400);  //   64 + (n1, n5)
+                    a[h][2] = and_or<0x000F000Fu>(q8, k6400); // 1024 + (n2, n6)
+                    a[h][3] = and_or<0x00F000F0u>(q8, k5400); //   64 + (n3, n7)
+                }
+#pragma unroll
+                for (int mb = 0; mb < MB; mb++)
+                {
+                    const uint4 x = lds128(x_at + x_off + (uint32_t)((j * kBatch + 8 * mb) * 64));
+                    if (j == 0)
+                        mma16816_first(acc[mb], a[0][0], a[1][0], a[0][1], a[1][1], x.x, x.y);
+                    else
+                        mma16816(acc[mb], a[0][0], a[1][0], a[0][1], a[1][1], x.x, x.y);
+                    mma16816(acc[mb], a[0][2], a[1][2], a[0][3], a[1][3], x.z, x.w);
+                }
+            }
+#pragma unroll
+            for (int mb = 0; mb < MB; mb++)
+            {
+                const uint4 nc = lds128(nc_at + x_off + (uint32_t)(mb * 64));
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                {
+                    const float nc1 = __uint_as_float(c & 1 ? nc.z : nc.x), nc2 = __uint_as_float(c & 1 ? nc.w : nc.y);
+                    tot[mb][c] = fmaf(sc[c >> 1], acc[mb][c] + fmaf(nz[c >> 1], nc2, nc1), tot[mb][c]);
+                }
+            }
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(empty(st));
+            if (++st == kStages)
+                st = 0, phase ^= 1u;
+            if (ku != KU - 1 && i != n_units - 1)
+            {
+                ku++;
+                continue;
+            }
+            // ---- the end of this CTA's part of the tile
+            bool mine = true; // does this warp finish its rows?
+            if (seg_ku0 != 0 || ku != KU - 1)
+            {
+                auto owner = [&](int u) { // the CTA whose share holds unit u
+                    const int more = p.units_rem * (p.units_lo + 1); // units of the shares with one more
+                    return u < more ? u / (p.units_lo + 1) : p.units_rem + (u - more) / p.units_lo;
+                };
+                // a share's first tile has slot 0, another one that it shares (its last) slot 1
+                auto slot = [&](int cta) {
+                    return p.slots + (size_t)((2 * cta + (share_begin(cta) >= tile * KU ? 0 : 1)) * kConsumers + warp) * kSums + lane;
+                };
+                const int c_first = owner(tile * KU), c_last = owner(tile * KU + KU - 1);
+                float* const my = slot((int)blockIdx.x);
+#pragma unroll
+                for (int mb = 0; mb < MB; mb++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        __stcg(my + (mb * 4 + c) * 32, tot[mb][c]);
+                __threadfence();
+                __syncwarp();
+                uint32_t before = 0;
+                if (lane == 0)
+                {
+                    before = atomicAdd(p.counters + tile * kConsumers + warp, 1u);
+                    if (before == (uint32_t)(c_last - c_first))
+                        p.counters[tile * kConsumers + warp] = 0u; // leave the counter zeroed for the next call
+                }
+                before = __shfl_sync(0xffffffffu, before, 0);
+                mine = before == (uint32_t)(c_last - c_first);
+                if (mine)
+                {
+                    __threadfence();
+#pragma unroll
+                    for (int mb = 0; mb < MB; mb++)
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            tot[mb][c] = 0.f;
+#pragma unroll 1
+                    for (int c0 = c_first; c0 <= c_last; c0 += 4) // four parts' sums in flight
+                    {
+                        const float* part[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            part[e] = slot(min(c0 + e, c_last));
+#pragma unroll
+                        for (int mb = 0; mb < MB; mb++)
+                        {
+                            float v[4][4];
+#pragma unroll
+                            for (int e = 0; e < 4; e++)
+#pragma unroll
+                                for (int c = 0; c < 4; c++)
+                                    v[e][c] = __ldcg(part[e] + (mb * 4 + c) * 32);
+#pragma unroll
+                            for (int e = 0; e < 4; e++)
+                                if (c0 + e <= c_last)
+#pragma unroll
+                                    for (int c = 0; c < 4; c++)
+                                        tot[mb][c] += v[e][c];
+                        }
+                    }
+                }
+            }
+            if (mine)
+            {
+                const int n0 = p.dual ? tile * 64 + r0 : tile * kRows + r0;
+                const int y_shift = p.y_f32 ? 2 : 1;
+                auto store = [&](int m, int n, float v) {
+                    if (m >= p.M || n >= p.N)
+                        return;
+                    const size_t at = ((size_t)m * p.N + n) << y_shift;
+                    if (p.has_addend)
+                    {
+                        const char* add = static_cast<const char*>(p.bias) + at;
+                        v += p.y_f32 ? *reinterpret_cast<const float*>(add) : __half2float(*reinterpret_cast<const __half*>(add));
+                    }
+                    else if (p.bias != nullptr)
+                        v += static_cast<const float*>(p.bias)[n];
+                    char* y = static_cast<char*>(p.y) + at;
+                    if (p.y_f32)
+                        *reinterpret_cast<float*>(y) = v;
+                    else
+                        *reinterpret_cast<__half*>(y) = __float2half_rn(v);
+                };
+#pragma unroll
+                for (int mb = 0; mb < MB; mb++)
+#pragma unroll
+                    for (int c = 0; c < 2; c++)
+                    {
+                        const int m = 8 * mb + 2 * t + c;
+                        if (p.dual)
+                        {
+                            const float v = tot[mb][c];
+                            store(m, n0, v * (1.0f / (1.0f + expf(-v))) * tot[mb][2 + c]);
+                        }
+                        else
+                        {
+                            store(m, n0, tot[mb][c]);
+                            store(m, n0 + 8, tot[mb][2 + c]);
+                        }
+                    }
+            }
+#pragma unroll
+            for (int mb = 0; mb < MB; mb++)
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    tot[mb][c] = 0.f;
+            ku = 0, seg_ku0 = 0, tile++;
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && *abort_flag)
+        atomicExch(p.status, 1);
+}
+
+// The activations, normalised and rounded, as the blocks that dq_stream_kernel copies (rows past M are zeros).  A block is a unit
+// of K: [j][batch row][t] 16 bytes with elements 32 t + 8 j .. + 7 of the unit, in the order 0 4 1 5 2 6 3 7 that the unpacking
+// of the weights leaves, then per batch row -sum(offset_k x_k) and -sum(x_k), pairs of rows side by side.  A CTA takes one row,
+// all of it where the norm needs that (bound by one round trip to L2 and the launch); 128 threads, which fit beside two CTAs of
+// the linear.
+__global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half* x, const float* gain, uint8_t* blocks, int M, int K, float eps, int per_cta)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float part[kPrepThreads / 32];
+    const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int first = blockIdx.y * per_cta, K8 = min(K >> 3, first + per_cta); // this CTA's chunks of eight elements
+    auto load = [&](int k8) {
+        return m < M ? *reinterpret_cast<const uint4*>(x + (size_t)m * K + k8 * 8) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    auto floats = [&](const uint4& a, float (&v)[8]) {
+        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+            v[2 * j] = f.x, v[2 * j + 1] = f.y;
+        }
+    };
+    uint4 kept[kPrepSteps];
+#pragma unroll
+    for (int s = 0; s < kPrepSteps; s++)
+        if (first + tid + s * kPrepThreads < K8)
+            kept[s] = load(first + tid + s * kPrepThreads);
+    float r = 1.f;
+    if (gain != nullptr) // (then the CTA has the whole row)
+    {
+        float ss = 0.f;
+        auto add = [&](const uint4& a) {
+            float v[8];
+            floats(a, v);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                ss = fmaf(v[j], v[j], ss);
+        };
+#pragma unroll
+        for (int s = 0; s < kPrepSteps; s++)
+            if (tid + s * kPrepThreads < K8)
+                add(kept[s]);
+        for (int k8 = tid + kPrepSteps * kPrepThreads; k8 < K8; k8 += kPrepThreads)
+            add(load(k8));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0)
+            part[tid >> 5] = ss;
+        __syncthreads();
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < kPrepThreads / 32; w++) // fixed order: repeatable
+            sum += part[w];
+        r = 1.0f / sqrtf(sum / (float)K + eps);
+    }
+    const uint32_t half_warp = 0xFFFFu << (lane & 16); // the 16 lanes of a unit come together: K is a multiple of 128
+    auto put = [&](int k8, const uint4& raw) {
+        float v[8];
+        floats(raw, v);
+        if (gain != nullptr)
+        {
+            const float4 a = reinterpret_cast<const float4*>(gain + k8 * 8)[0], b = reinterpret_cast<const float4*>(gain + k8 * 8)[1];
+            const float gn[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                v[j] = __half2float(__float2half_rn(v[j] * r * gn[j]));
+        }
+        uint8_t* const block = blocks + (size_t)(k8 >> 4) * kBlockBytes;
+        uint32_t h[4];
+        float even = 0.f, odd = 0.f; // the unpacking leaves 1024 on even elements and 64 on odd ones
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            const __half2 a = __floats2half2_rn(v[2 * q], v[2 * q + 1]);
+            h[q] = *reinterpret_cast<const uint32_t*>(&a);
+            even += v[2 * q], odd += v[2 * q + 1];
+        }
+        *reinterpret_cast<uint4*>(block + ((k8 & 3) * kBatch + m) * 64 + ((k8 >> 2) & 3) * 16) =
+            make_uint4(__byte_perm(h[0], h[2], 0x5410), __byte_perm(h[0], h[2], 0x7632), __byte_perm(h[1], h[3], 0x5410), __byte_perm(h[1], h[3], 0x7632));
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1)
+        {
+            even += __shfl_xor_sync(half_warp, even, o);
+            odd += __shfl_xor_sync(half_warp, odd, o);
+        }
+        if ((lane & 15) == 0)
+            *reinterpret_cast<float2*>(block + kBatch * 256 + m * 8) = make_float2(-(1024.f * even + 64.f * odd), -(even + odd));
+    };
+#pragma unroll
+    for (int s = 0; s < kPrepSteps; s++)
+        if (first + tid + s * kPrepThreads < K8)
+            put(first + tid + s * kPrepThreads, kept[s]);
+    for (int k8 = first + tid + kPrepSteps * kPrepThreads; k8 < K8; k8 += kPrepThreads)
+        put(k8, load(k8));
+}
+} // namespace
+
+namespace nnf
+{
+struct StreamLayout
+{
+    int tiles, KU, ctas;
+    size_t counter_bytes, slot_bytes, block_bytes;
+    size_t total() const { return counter_bytes + slot_bytes + block_bytes; }
+};
+
+static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+{
+    StreamLayout L{};
+    const int sms = ctx ? ctx->sm_count : 148;
+    const bool dual = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
+    L.tiles = (d.N + (dual ? 63 : 127)) / (dual ? 64 : 128);
+    L.KU = d.K / kUnitK;
+    L.ctas = (int)std::min<long long>((long long)L.tiles * L.KU, 2 * sms);
+    if (L.tiles % L.ctas != 0) // some tile is shared
+    {
+        L.counter_bytes = ((size_t)L.tiles * kConsumers * sizeof(uint32_t) + 255) / 256 * 256;
+        L.slot_bytes = (size_t)2 * L.ctas * kConsumers * kSums * sizeof(float);
+    }
+    L.block_bytes = ((size_t)L.KU * kBlockBytes + 255) / 256 * 256;
+    return L;
+}
+
+// Whether this form serves a call with enough workspace.  Measured at 16 rows (us, small-M kernel / this; units per SM of 148):
+// 4096 x 4096 (7) 9.3 / 11.3 and 11008 x 4096 (19) 14.5 / 16.1, but 4096 x 11008 (19, K cut four ways there) 19.6 / 18.3, the
+// gate/up pair 11008 x 4096 (37) 25.4 / 21.9, with the norm 29.7 / 22.7, 8192 x 28672 (97) 68.8 / 48.5.  Up to 8 rows the small-M
+// kernel keeps all activations in registers and is faster nearly everywhere.
+bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+{
+    const int group = d.group_size > 0 ? d.group_size : d.K;
+    if (d.M < 9 || d.M > kBatch || d.w_bits != 4 || d.x_dtype != NNF_B200_F16 || d.split_k != 0 || (d.flags & NNF_B200_FLAG_EXACT_ZP) ||
+        d.kernel == NNF_B200_KERNEL_GEMM || d.K % kUnitK != 0 || group % kUnitK != 0 || d.K % group != 0)
+        return false;
+    const int sms = ctx ? ctx->sm_count : 148;
+    const long long KU = d.K / kUnitK, tiles = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL ? (d.N + 63ll) / 64 : (d.N + 127ll) / 128;
+    if (tiles * KU >= (1ll << 27) || KU >= (1 << 16)) // (counted in 32 bits)
+        return false;
+    return tiles * KU >= (d.K > 4096 ? 16 : 24) * (long long)sms;
+}
+
+size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+{
+    return stream_layout(ctx, d).total();
+}
+
+int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const void* x, const nnf_b200_qweight* w,
+                  const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y, void* workspace)
+{
+    static bool configured[kMaxDevices] = {}; // the attributes belong to the device that is current
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && (dev < 0 || dev >= kMaxDevices))
+        e = cudaErrorInvalidDevice;
+    if (e == cudaSuccess && !configured[dev])
+    {
+        e = cudaFuncSetAttribute(dq_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(dq_stream_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess) // (so that an SM need not drain before it can hold the linear's CTAs)
+            e = cudaFuncSetAttribute(stream_prep_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        configured[dev] = e == cudaSuccess;
+    }
+    if (e != cudaSuccess)
+        return set_error(ctx, NNF_B200_ECUDA, std::string("dq_stream set-up: ") + cudaGetErrorString(e));
+    const StreamLayout L = stream_layout(ctx, d);
+    uint8_t* const ws = static_cast<uint8_t*>(workspace);
+    uint8_t* const blocks = ws + L.counter_bytes + L.slot_bytes;
+
+    StreamParams p{};
+    p.dual = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
+    const nnf_b200_qweight* sets[2] = {w, p.dual ? w2 : w};
+    alignas(64) CUtensorMap tw[2];
+    for (int i = 0; i < 2; i++)
+    {
+        p.scale[i] = sets[i]->scale, p.zp[i] = static_cast<const uint8_t*>(sets[i]->zp);
+        // (copied by value at once: a later lookup may empty the context's cache)
+        const CUtensorMap* m = weight_tensor_map(ctx, sets[i]->wq, d.N, d.K / 2, kUnitK / 2, p.dual ? 64 : kRows);
+        if (!m)
+            return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the weight tensor");
+        tw[i] = *m;
+    }
+    p.bias = bias;
+    p.has_addend = d.epilogue == NNF_B200_EPILOGUE_ADD;
+    p.y = y;
+    p.status = ctx->dev_status;
+    p.counters = reinterpret_cast<uint32_t*>(ws);
+    p.slots = reinterpret_cast<float*>(ws + L.counter_bytes);
+    p.xblocks = blocks;
+    p.M = d.M, p.N = d.N, p.KU = L.KU;
+    p.units_lo = L.tiles * L.KU / L.ctas, p.units_rem = L.tiles * L.KU % L.ctas;
+    const int group = d.group_size > 0 ? d.group_size : d.K;
+    p.G = d.K / group;
+    p.zp_row_bytes = (p.G + 1) / 2;
+    p.group_units = group / kUnitK;
+    p.group_magic = p.group_units > 1 ? (uint32_t)((0x100000000ull + p.group_units - 1) / p.group_units) : 0u;
+    p.y_f32 = d.y_dtype == NNF_B200_F32, p.scale_f32 = d.scale_dtype == NNF_B200_F32;
+
+    (void)cudaGetLastError(); // do not inherit a stale error left behind by an unrelated earlier call
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    overlap_attribute(attr, &cfg.numAttrs);
+    cfg.attrs = attr;
+    cfg.stream = stream;
+    const int per_cta = gain != nullptr ? d.K / 8 : kPrepSteps * kPrepThreads; // (the norm needs its whole row)
+    cfg.gridDim = dim3(kBatch, (d.K / 8 + per_cta - 1) / per_cta);
+    cfg.blockDim = dim3(kPrepThreads);
+    e = cudaLaunchKernelEx(&cfg, stream_prep_kernel, static_cast<const __half*>(x), static_cast<const float*>(gain), blocks, (int)d.M, (int)d.K, d.rms_eps,
+                           per_cta);
+    if (e != cudaSuccess)
+        return set_error(ctx, NNF_B200_ECUDA, std::string("stream_prep launch: ") + cudaGetErrorString(e));
+    ctx->launches++;
+    cfg.gridDim = dim3(L.ctas);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    e = cudaLaunchKernelEx(&cfg, dq_stream_kernel, p, tw[0], tw[1]);
+    if (e != cudaSuccess)
+        return set_error(ctx, NNF_B200_ECUDA, std::string("dq_stream launch: ") + cudaGetErrorString(e));
+    ctx->launches++;
+    return NNF_B200_OK;
+}
+} // namespace nnf

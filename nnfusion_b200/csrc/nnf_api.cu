@@ -56,15 +56,14 @@ void overlap_attribute(cudaLaunchAttribute* attr, unsigned* count)
 const CUtensorMap* weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes,
                                      int box_rows)
 {
-    const int swz = box_bytes == 128 ? 1 : 0;
-    auto key = std::make_tuple(base, rows, row_bytes, box_bytes, box_rows, swz);
+    auto key = std::make_tuple(base, rows, row_bytes, box_bytes, box_rows);
     auto it = ctx->tensor_maps.find(key);
     if (it != ctx->tensor_maps.end())
         return &it->second;
     alignas(64) CUtensorMap map;
     if (!encode_tensor_map_2d(ctx->encode_tiled, &map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, (uint64_t)row_bytes,
                               (uint64_t)rows, (uint64_t)row_bytes, (uint32_t)box_bytes, (uint32_t)box_rows,
-                              swz ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE))
+                              box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))
         return nullptr;
     if (ctx->tensor_maps.size() > 4096) // callers that churn through weight buffers: start over
         ctx->tensor_maps.clear();
@@ -263,9 +262,13 @@ size_t nnf_b200_linear_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_l
         std::string why;
         if (nnf::gemv_plan(ctx, *desc, &plan, &why) != NNF_B200_OK)
             return 0;
-        if (nnf::gemv_plan(ctx, *desc, &ring, &why, false) != NNF_B200_OK)
-            return plan.workspace_bytes;
-        return plan.workspace_bytes > ring.workspace_bytes ? plan.workspace_bytes : ring.workspace_bytes;
+        size_t need = plan.workspace_bytes;
+        if (nnf::gemv_plan(ctx, *desc, &ring, &why, false) == NNF_B200_OK && ring.workspace_bytes > need)
+            need = ring.workspace_bytes;
+        // ... and the form that streams the weights through shared memory (a caller with less gets the former two)
+        if (nnf::stream_serves(ctx, *desc) && nnf::stream_workspace_bytes(ctx, *desc) > need)
+            need = nnf::stream_workspace_bytes(ctx, *desc);
+        return need;
     }
     return nnf::gemm_workspace_bytes(ctx, *desc);
 }
@@ -352,7 +355,7 @@ int nnf_b200_linear_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc* de
         out[5] = (int32_t)plan.smem_bytes;
         out[6] = plan.batch;
         out[7] = (plan.cluster ? 1 : 0) | (plan.l1_lines ? 2 : 0) | (plan.range_layout ? 4 : 0) |
-                 (plan.direct && plan.param_bufs == 1 ? 8 : 0);
+                 (plan.direct && plan.param_bufs == 1 ? 8 : 0) | (nnf::stream_serves(ctx, *desc) ? 16 : 0);
     }
     return NNF_B200_OK;
 }
@@ -434,6 +437,8 @@ static int linear_impl(nnf_b200_ctx* ctx, void* stream, const nnf_b200_linear_de
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (pick_kernel(d) == NNF_B200_KERNEL_GEMV)
     {
+        if (!peers && workspace && nnf::stream_serves(ctx, d) && workspace_bytes >= nnf::stream_workspace_bytes(ctx, d))
+            return nnf::stream_launch(ctx, s, d, x, w, w2, gain, bias, y, workspace);
         nnf::GemvPlan plan;
         std::string why;
         rc = cached_gemv_plan(ctx, d, &plan, &why);

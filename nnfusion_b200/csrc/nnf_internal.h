@@ -20,8 +20,8 @@ struct nnf_b200_ctx
     std::string last_error;
     void* encode_tiled = nullptr; // cuTensorMapEncodeTiled entry point (driver)
     int* dev_status = nullptr;    // device word set to non-zero when a bounded device-side wait gave up
-    // Tensor maps of weight tensors, keyed by (address, rows, row bytes, box bytes, box rows, swizzle).
-    std::map<std::tuple<const void*, int, int, int, int, int>, CUtensorMap> tensor_maps;
+    // Tensor maps of weight tensors, keyed by (address, rows, row bytes, box bytes, box rows).
+    std::map<std::tuple<const void*, int, int, int, int>, CUtensorMap> tensor_maps;
 };
 
 namespace nnf
@@ -73,8 +73,7 @@ int check_linear_call(const nnf_b200_linear_desc* d, const void* x, const nnf_b2
 // launch may have written.
 void overlap_attribute(cudaLaunchAttribute* attr, unsigned* count);
 
-// Cached 2-D byte tensor map [rows][row_bytes] with a box of box_rows x box_bytes (128-byte swizzle when
-// box_bytes == 128, none otherwise); nullptr if the driver refuses it.
+// Cached 2-D byte tensor map [rows][row_bytes] with a box of box_rows x box_bytes (swizzled over box_bytes, 64 or 128); nullptr if the driver refuses it.
 const CUtensorMap* weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes,
                                      int box_rows);
 
@@ -95,6 +94,11 @@ int gemm_supported(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, std::
 int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const void* x,
                 const nnf_b200_qweight* w, const nnf_b200_qweight* w2, const void* gain, const void* bias,
                 void* y, void* workspace, size_t workspace_bytes);
+
+bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d);
+size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d);
+int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const void* x, const nnf_b200_qweight* w,
+                  const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y, void* workspace);
 
 size_t allreduce_flag_bytes(size_t count);
 int allreduce_launch(nnf_b200_ctx* ctx, cudaStream_t stream, int rank, int world, const void* const* bufs,

@@ -249,6 +249,44 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
                  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                  : "memory");
 }
+constexpr uint32_t kRoleSpin = 1u << 21;
+
+// Waits of the roles of a CTA: bounded, and given up as soon as another role has raised the abort flag.  SLEEP: nanoseconds between
+// polls; a waiting role should not compete with the working ones for issue slots.
+// One thread:
+template <int SLEEP>
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag)
+{
+    for (uint32_t i = 0; i < kRoleSpin; i++)
+    {
+        if (mbar_try_wait(bar, parity))
+            return true;
+        if constexpr (SLEEP > 0)
+            __nanosleep(SLEEP);
+        if ((i & 255u) == 255u && *abort_flag)
+            return false;
+    }
+    *abort_flag = 1;
+    return false;
+}
+// A whole warp.  Every decision is a vote, which the compiler knows to be the same for all lanes: the warp stays together
+// for the warp-wide tensor-memory instructions that follow, and what follows may use uniform registers.  CLUSTER: what was
+// announced happened in another CTA of the cluster.
+template <int SLEEP, bool CLUSTER = false>
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
+{
+    for (uint32_t i = 0; i < kRoleSpin; i++)
+    {
+        if (__all_sync(0xffffffffu, CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)))
+            return true;
+        if constexpr (SLEEP > 0)
+            __nanosleep(SLEEP);
+        if ((i & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0))
+            return false;
+    }
+    *abort_flag = 1;
+    return false;
+}
 } // namespace ptx
 
 // Host: encode a 2-D row-major tensor map (inner dimension contiguous).  Returns false on failure.

@@ -1,0 +1,103 @@
+"""The small-M form that streams the weights through shared memory (``nnfusion_b200/csrc/dq_stream.cu``: 9 to 16 rows of fp16,
+uint4 weights, enough of them): both ends of its rows, ragged N, one unit of K and many, shares that begin and end inside a
+tile, every prologue and epilogue, both output and scale types, and the rule that chooses it, against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from nnfusion_b200 import _lib as L
+from nnfusion_b200 import synth
+from oracle import oracle as orc
+from tests.util import TOL_F16, oracle_linear
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan_bits(op, M, dtype):
+    d, out = op.desc(M, dtype), (ctypes.c_int32 * 8)()
+    assert op.ctx.lib.nnf_b200_linear_plan(op.ctx.handle, ctypes.byref(d), ctypes.byref(out)) == L.OK
+    return d, out
+
+
+@pytest.mark.parametrize("M,N,K,group,scale,norm,epilogue,y32", [
+    (9, 4100, 11008, 128, np.float16, False, "none", False),     # 33 tiles of 86 units on 296 CTAs, ragged N, odd groups a row
+    (16, 4096, 11008, 128, np.float16, False, "add", True),
+    (13, 3593, 8192, 128, np.float16, True, "silu", False),      # two weight sets, 57 tiles, odd N
+    (16, 7616, 4096, 256, np.float32, True, "silu", True),
+    (16, 30001, 2048, 128, np.float16, True, "bias", False),     # several tiles a CTA
+    (10, 9000, 6144, 0, np.float16, False, "bias", True),        # one group a row
+    (12, 151553, 384, 128, np.float16, False, "none", True),     # 3 units of K: four tiles a CTA
+    (16, 455000, 128, 128, np.float16, True, "none", False),     # one unit of K
+])
+def test_against_the_oracle(M, N, K, group, scale, norm, epilogue, y32):
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(M + N))
+    x = synth.make_x(rng, M, K, np.float16)
+    w = [synth.make_weights(rng, N, K, 4, group or K, scale) for _ in range(1 + (epilogue == "silu"))]
+    gain = rng.uniform(0.9, 1.1, K).astype(np.float32) if norm else None
+    bias = rng.standard_normal(N).astype(np.float32) if epilogue == "bias" else None
+    op = DequantDot(*[DeviceWeight.from_host(v) for v in w], gain=torch.from_numpy(gain).cuda() if norm else None,
+                    bias=torch.from_numpy(bias).cuda() if bias is not None else None, add=epilogue == "add",
+                    y_dtype=torch.float32 if y32 else None)
+    tx = torch.from_numpy(x).cuda()
+    d, out = _plan_bits(op, M, tx.dtype)
+    assert out[7] & 16
+    c = torch.randn(M, N, device="cuda").to(torch.float32 if y32 else torch.float16) if epilogue == "add" else None
+    kw = dict(addend=c) if c is not None else {}
+    y = torch.full((M, N), float("nan"), dtype=torch.float32 if y32 else torch.float16, device="cuda")
+    op(tx, out=y, **kw)
+    outs = [op(tx, **kw) for _ in range(20)]                     # back to back: the same bits, counters left zeroed
+    op.ctx.device_status()
+    assert all(torch.equal(o, y) for o in outs)
+    want = oracle_linear(x, *w, gain=gain, bias=bias, out_dtype=np.float32)
+    if c is not None:
+        want = want + c.float().cpu().numpy()
+    # exact integers, fp32 scales and sums: what is left is x's rounding behind the norm (2^-11 an element) and y's
+    assert orc.max_rel_err(y.float().cpu().numpy(), want) <= min(TOL_F16, 1.5e-3 if norm or not y32 else 1e-4)
+
+
+def test_a_smaller_workspace_takes_the_split_form():
+    """A program whose workspace was sized before this form existed keeps running, and nothing is written behind its buffer."""
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    x, w = synth.u4g128(3, 16, 4096, 11008)
+    op = DequantDot(DeviceWeight.from_host(w))
+    tx, want = torch.from_numpy(x).cuda(), oracle_linear(x, w)
+    d, _ = _plan_bits(op, 16, tx.dtype)
+    need = int(op.ctx.lib.nnf_b200_linear_workspace_bytes(op.ctx.handle, ctypes.byref(d)))
+    y = torch.empty((16, 4096), dtype=torch.float16, device="cuda")
+    d2 = op.desc(16, tx.dtype)
+    d2.split_k = 4                                               # what the split form asks for at the same cut
+    split = int(op.ctx.lib.nnf_b200_linear_workspace_bytes(op.ctx.handle, ctypes.byref(d2)))
+    assert split < need
+    for size in (need, split):
+        guarded = torch.zeros(size + 4096, dtype=torch.uint8, device="cuda")
+        guarded[size:] = 0xAB
+        for _ in range(2):
+            y.fill_(float("nan"))
+            op.run_raw(d, tx.data_ptr(), y.data_ptr(), guarded[:size])
+            assert orc.max_rel_err(y.cpu().numpy(), want) <= 1.5e-3
+        assert bool((guarded[size:] == 0xAB).all())
+
+
+def test_activations_gain_and_addend_written_by_the_launch_ahead():
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(5))
+    a = DequantDot(DeviceWeight.from_host(synth.make_weights(rng, 11008, 4096, 4, 128)), add=False)
+    b = DequantDot(DeviceWeight.from_host(synth.make_weights(rng, 4096, 11008, 4, 128)), add=True)
+    xs = [torch.from_numpy(synth.make_x(rng, 16, 4096, np.float16)).cuda() for _ in range(30)]
+    h, want = torch.empty((16, 11008), dtype=torch.float16, device="cuda"), []
+    for x in xs:
+        a(x, out=h)
+        torch.cuda.synchronize()
+        want.append(b(h, addend=x).clone())
+        torch.cuda.synchronize()
+    got = []
+    for x in xs:
+        a(x, out=h)
+        got.append(b(h, addend=x))
+    torch.cuda.synchronize()
+    assert not [i for i, (p, q) in enumerate(zip(got, want)) if not torch.equal(p, q)]
