@@ -1400,14 +1400,11 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     if (!encode_tensor_map_2d(ctx->encode_tiled, &tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)d.K,
                               (uint64_t)d.M, (uint64_t)d.K * 2, 64, (uint32_t)L.bx / 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the activations");
-    // (copied by value at once: a later lookup may empty the context's cache)
     alignas(64) CUtensorMap tw[2];
     for (int i = 0; i < 2; i++)
     {
-        const CUtensorMap* m = weight_tensor_map(ctx, sets[i]->wq, d.N, row_bytes, 128, 128);
-        if (!m)
+        if (!weight_tensor_map(ctx, sets[i]->wq, d.N, row_bytes, 128, 128, &tw[i]))
             return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the weight tensor");
-        tw[i] = *m;
     }
     const cudaError_t e = cfg == 64    ? dispatch<64>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream)
                           : cfg == 128 ? dispatch<128>(d.w_bits, one_group, p, tx, tw[0], tw[1], L.pairs, stream)

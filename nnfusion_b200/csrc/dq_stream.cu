@@ -560,9 +560,10 @@ static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear
 }
 
 // Whether this form serves a call with enough workspace.  Measured at 16 rows (us, small-M kernel / this; units per SM of 148):
-// 4096 x 4096 (7) 9.3 / 11.3 and 11008 x 4096 (19) 14.5 / 16.1, but 4096 x 11008 (19, K cut four ways there) 19.6 / 18.3, the
-// gate/up pair 11008 x 4096 (37) 25.4 / 21.9, with the norm 29.7 / 22.7, 8192 x 28672 (97) 68.8 / 48.5.  Up to 8 rows the small-M
-// kernel keeps all activations in registers and is faster nearly everywhere.
+// 4096 x 4096 (7) 9.3 / 11.3 and 11008 x 4096 (19) 14.5 / 16.1, but with a K that the small-M kernel cuts 4096 x 11008 (19) 19.6 /
+// 18.7, the gate/up pair 28672 x 8192 (388) 117 / 79, 8192 x 28672 (97) 68.8 / 44.6.  K up to 4096 stays there also where this
+// would be faster (gate/up pair 11008 x 4096 25.5 / 23.7): that kernel then needs no workspace, so that calls of one node on two
+// streams may overlap.  Up to 8 rows the small-M kernel keeps all activations in registers and is faster nearly everywhere.
 bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
 {
     const int group = d.group_size > 0 ? d.group_size : d.K;
@@ -573,7 +574,7 @@ bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
     const long long KU = d.K / kUnitK, tiles = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL ? (d.N + 63ll) / 64 : (d.N + 127ll) / 128;
     if (tiles * KU >= (1ll << 27) || KU >= (1 << 16)) // (counted in 32 bits)
         return false;
-    return tiles * KU >= (d.K > 4096 ? 16 : 24) * (long long)sms;
+    return d.K > 4096 && tiles * KU >= 16ll * sms;
 }
 
 size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
@@ -611,11 +612,8 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     for (int i = 0; i < 2; i++)
     {
         p.scale[i] = sets[i]->scale, p.zp[i] = static_cast<const uint8_t*>(sets[i]->zp);
-        // (copied by value at once: a later lookup may empty the context's cache)
-        const CUtensorMap* m = weight_tensor_map(ctx, sets[i]->wq, d.N, d.K / 2, kUnitK / 2, p.dual ? 64 : kRows);
-        if (!m)
+        if (!weight_tensor_map(ctx, sets[i]->wq, d.N, d.K / 2, kUnitK / 2, p.dual ? 64 : kRows, &tw[i]))
             return set_error(ctx, NNF_B200_ECUDA, "cuTensorMapEncodeTiled failed for the weight tensor");
-        tw[i] = *m;
     }
     p.bias = bias;
     p.has_addend = d.epilogue == NNF_B200_EPILOGUE_ADD;

@@ -53,21 +53,30 @@ void overlap_attribute(cudaLaunchAttribute* attr, unsigned* count)
     *count = 1;
 }
 
-const CUtensorMap* weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes,
-                                     int box_rows)
+bool weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes, int box_rows, CUtensorMap* out)
 {
-    auto key = std::make_tuple(base, rows, row_bytes, box_bytes, box_rows);
-    auto it = ctx->tensor_maps.find(key);
+    const auto key = std::make_tuple(base, rows, row_bytes, box_bytes, box_rows);
+    std::lock_guard<std::mutex> lock(ctx->tensor_maps_mutex);
+    const auto it = ctx->tensor_maps.find(key);
     if (it != ctx->tensor_maps.end())
-        return &it->second;
-    alignas(64) CUtensorMap map;
-    if (!encode_tensor_map_2d(ctx->encode_tiled, &map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, (uint64_t)row_bytes,
+    {
+        *out = it->second;
+        return true;
+    }
+    if (!encode_tensor_map_2d(ctx->encode_tiled, out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, (uint64_t)row_bytes,
                               (uint64_t)rows, (uint64_t)row_bytes, (uint32_t)box_bytes, (uint32_t)box_rows,
                               box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))
-        return nullptr;
-    if (ctx->tensor_maps.size() > 4096) // callers that churn through weight buffers: start over
-        ctx->tensor_maps.clear();
-    return &(ctx->tensor_maps[key] = map);
+        return false;
+    try
+    {
+        if (ctx->tensor_maps.size() > 4096) // callers that churn through weight buffers: start over
+            ctx->tensor_maps.clear();
+        ctx->tensor_maps[key] = *out;
+    }
+    catch (...) // (no memory for the entry: encoded again next time)
+    {
+    }
+    return true;
 }
 } // namespace nnf
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 
@@ -22,6 +23,7 @@ struct nnf_b200_ctx
     int* dev_status = nullptr;    // device word set to non-zero when a bounded device-side wait gave up
     // Tensor maps of weight tensors, keyed by (address, rows, row bytes, box bytes, box rows).
     std::map<std::tuple<const void*, int, int, int, int>, CUtensorMap> tensor_maps;
+    std::mutex tensor_maps_mutex;
 };
 
 namespace nnf
@@ -73,9 +75,9 @@ int check_linear_call(const nnf_b200_linear_desc* d, const void* x, const nnf_b2
 // launch may have written.
 void overlap_attribute(cudaLaunchAttribute* attr, unsigned* count);
 
-// Cached 2-D byte tensor map [rows][row_bytes] with a box of box_rows x box_bytes (swizzled over box_bytes, 64 or 128); nullptr if the driver refuses it.
-const CUtensorMap* weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes,
-                                     int box_rows);
+// Cached 2-D byte tensor map [rows][row_bytes] with a box of box_rows x box_bytes (swizzled over box_bytes, 64 or 128), copied
+// out under the cache's lock: threads may share a context; false if the driver refuses it.
+bool weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes, int box_rows, CUtensorMap* out);
 
 // allow_direct = false keeps the plan on the ring kernel (the one that takes the zero-points out before the multiply).
 int gemv_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, GemvPlan* plan, std::string* why,
