@@ -65,6 +65,7 @@ constexpr int kEpiBarrier = 1;                // named barrier of the epilogue w
 // stage's conversion, its multiplies and the handing over between them follow one another, and what bounds these tiles is how
 // many stages are at it side by side.  With the quantisation parameters hoisted out of the conversion's loop: 48 x 11008 x 4096
 // 18.9 -> 17.6 us, the gate/up pair of that shape 35.6 -> 33.2, 48 x 4096 x 11008 19.3 -> 18.8 (graph replay, weights beyond L2).
+// (uint4 only: with uint8 weights, whose conversion is shorter, the smaller x ring costs 1 to 3 % at 4096 x 4096.)
 // Where the line lies: 65 rows would need accumulators of 80 columns, and 11 k-blocks are two whole stages again.
 template <int BX>
 struct Cfg
@@ -1216,7 +1217,9 @@ cudaError_t dispatch(int wbits, bool one_group, const GemmParams& p, const CUten
 {
     if (wbits == 4)
         return one_group ? launch<4, true, BX>(p, tx, tw0, tw1, pairs, stream) : launch<4, false, BX>(p, tx, tw0, tw1, pairs, stream);
-    return one_group ? launch<8, true, BX>(p, tx, tw0, tw1, pairs, stream) : launch<8, false, BX>(p, tx, tw0, tw1, pairs, stream);
+    if constexpr (BX > 64)
+        return one_group ? launch<8, true, BX>(p, tx, tw0, tw1, pairs, stream) : launch<8, false, BX>(p, tx, tw0, tw1, pairs, stream);
+    return cudaErrorInvalidValue;
 }
 } // namespace
 
@@ -1358,7 +1361,7 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
     }
     const bool silu_mul = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
     const int row_bytes = d.w_bits == 4 ? d.K / 2 : d.K;
-    const int cfg = L.bx <= 64 ? 64 : L.bx <= 128 ? 128 : 256;
+    const int cfg = L.bx <= 64 && d.w_bits == 4 ? 64 : L.bx <= 128 ? 128 : 256;
     GemmParams p{};
     p.y = y;
     p.status = ctx->dev_status;
