@@ -559,12 +559,14 @@ static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear
     return L;
 }
 
-// Whether this form serves a call with enough workspace.  Measured at 16 rows (us, small-M kernel / this; units per SM of 148):
-// 4096 x 4096 (7) 9.3 / 11.3 and 11008 x 4096 (19) 14.5 / 16.1, but with a K that the small-M kernel cuts 4096 x 11008 (19) 19.6 /
-// 18.7, the gate/up pair 28672 x 8192 (388) 117 / 79, 8192 x 28672 (97) 68.8 / 44.6.  K up to 4096 stays there also where this
-// would be faster (gate/up pair 11008 x 4096 25.5 / 23.7): that kernel then needs no workspace, so that calls of one node on two
-// streams may overlap.  Up to 8 rows the small-M kernel keeps all activations in registers and is faster nearly everywhere.
-bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+// Whether this form serves a call with enough workspace.  `plan` is the small-M kernel's for the same descriptor: where that would
+// cut K into a cluster that the device holds (halves of K, in practice), its sums meet in shared memory and it touches no workspace,
+// so that calls of one node on two streams may overlap.  Those stay there, also where this would be faster, as does a K of up to
+// 4096, which is not cut (gate/up pair 11008 x 4096 at 16 rows 25.5 / 23.7 us, small-M kernel / this).
+// Otherwise, measured at 16 rows (us; units per SM of 148): 4096 x 11008 (19) 19.6 / 18.7, the gate/up pair 28672 x 8192 (388)
+// 117 / 79, 8192 x 28672 (97) 68.8 / 44.6.  Up to 8 rows the small-M kernel keeps all activations in registers and is faster nearly
+// everywhere.
+bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& plan)
 {
     const int group = d.group_size > 0 ? d.group_size : d.K;
     if (d.M < 9 || d.M > kBatch || d.w_bits != 4 || d.x_dtype != NNF_B200_F16 || d.split_k != 0 || (d.flags & NNF_B200_FLAG_EXACT_ZP) ||
@@ -574,6 +576,16 @@ bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
     const long long KU = d.K / kUnitK, tiles = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL ? (d.N + 63ll) / 64 : (d.N + 127ll) / 128;
     if (tiles * KU >= (1ll << 27) || KU >= (1 << 16)) // (counted in 32 bits)
         return false;
+    if (plan.splits <= 1)
+        return false;
+    if (plan.cluster)
+    {
+        // Clusters of 2 to 8 one-per-SM CTAs that 148 SMs hold at once (the occupancy calculator's answers, see gemv_direct_plan);
+        // CTAs of fewer warps may have twice or four times as many.
+        constexpr int held[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+        if (plan.ctas_per_split <= held[plan.splits] * std::max(1, std::min(4, 16 / plan.warps)))
+            return false;
+    }
     return d.K > 4096 && tiles * KU >= 16ll * sms;
 }
 

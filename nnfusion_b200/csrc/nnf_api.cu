@@ -275,7 +275,7 @@ size_t nnf_b200_linear_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_l
         if (nnf::gemv_plan(ctx, *desc, &ring, &why, false) == NNF_B200_OK && ring.workspace_bytes > need)
             need = ring.workspace_bytes;
         // ... and the form that streams the weights through shared memory (a caller with less gets the former two)
-        if (nnf::stream_serves(ctx, *desc) && nnf::stream_workspace_bytes(ctx, *desc) > need)
+        if (nnf::stream_serves(ctx, *desc, plan) && nnf::stream_workspace_bytes(ctx, *desc) > need)
             need = nnf::stream_workspace_bytes(ctx, *desc);
         return need;
     }
@@ -364,7 +364,7 @@ int nnf_b200_linear_plan(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc* de
         out[5] = (int32_t)plan.smem_bytes;
         out[6] = plan.batch;
         out[7] = (plan.cluster ? 1 : 0) | (plan.l1_lines ? 2 : 0) | (plan.range_layout ? 4 : 0) |
-                 (plan.direct && plan.param_bufs == 1 ? 8 : 0) | (nnf::stream_serves(ctx, *desc) ? 16 : 0);
+                 (plan.direct && plan.param_bufs == 1 ? 8 : 0) | (nnf::stream_serves(ctx, *desc, plan) ? 16 : 0);
     }
     return NNF_B200_OK;
 }
@@ -446,13 +446,13 @@ static int linear_impl(nnf_b200_ctx* ctx, void* stream, const nnf_b200_linear_de
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (pick_kernel(d) == NNF_B200_KERNEL_GEMV)
     {
-        if (!peers && workspace && nnf::stream_serves(ctx, d) && workspace_bytes >= nnf::stream_workspace_bytes(ctx, d))
-            return nnf::stream_launch(ctx, s, d, x, w, w2, gain, bias, y, workspace);
         nnf::GemvPlan plan;
         std::string why;
         rc = cached_gemv_plan(ctx, d, &plan, &why);
         if (rc != NNF_B200_OK)
             return nnf::set_error(ctx, rc, why);
+        if (!peers && workspace && nnf::stream_serves(ctx, d, plan) && workspace_bytes >= nnf::stream_workspace_bytes(ctx, d))
+            return nnf::stream_launch(ctx, s, d, x, w, w2, gain, bias, y, workspace);
         if (plan.workspace_bytes > 0 && (!workspace || workspace_bytes < plan.workspace_bytes))
             return nnf::set_error(ctx, NNF_B200_EWORKSPACE,
                                   "workspace of " + std::to_string(plan.workspace_bytes) + " bytes required");

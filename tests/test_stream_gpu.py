@@ -24,10 +24,14 @@ def _plan_bits(op, M, dtype):
     (9, 4100, 11008, 128, np.float16, False, "none", False),     # 33 tiles of 86 units on 296 CTAs, ragged N, odd groups a row
     (16, 4096, 11008, 128, np.float16, False, "add", True),
     (13, 3593, 8192, 128, np.float16, True, "silu", False),      # two weight sets, 57 tiles, odd N
-    (16, 4032, 5120, 256, np.float32, True, "silu", True),
-    (16, 9001, 4608, 128, np.float16, True, "bias", False),      # 71 tiles of 36 units
+    (16, 4032, 9216, 256, np.float32, True, "silu", True),
+    (16, 9001, 9088, 128, np.float16, True, "bias", False),      # 71 tiles of 71 units
     (11, 40000, 4224, 128, np.float16, False, "none", False),    # 313 tiles of 33 units, 35 a CTA: whole tiles too
-    (10, 9000, 6144, 0, np.float16, False, "bias", True),        # one group a row
+    (10, 9000, 8704, 0, np.float16, False, "bias", True),        # one group a row
+    # halves of K that meet in a cluster's shared memory: not this form, no workspace touched
+    (16, 4032, 5120, 256, np.float32, True, "silu", True),
+    (16, 9001, 4608, 128, np.float16, True, "bias", False),
+    (10, 9000, 6144, 0, np.float16, False, "bias", True),
 ])
 def test_against_the_oracle(M, N, K, group, scale, norm, epilogue, y32):
     import torch
@@ -42,7 +46,9 @@ def test_against_the_oracle(M, N, K, group, scale, norm, epilogue, y32):
                     y_dtype=torch.float32 if y32 else None)
     tx = torch.from_numpy(x).cuda()
     d, out = _plan_bits(op, M, tx.dtype)
-    assert out[7] & 16
+    halves = bool(out[2] == 2 and out[7] & 1)
+    assert halves == ((N, K) in ((4032, 5120), (9001, 4608), (9000, 6144)))
+    assert bool(out[7] & 16) == (not halves)
     c = torch.randn(M, N, device="cuda").to(torch.float32 if y32 else torch.float16) if epilogue == "add" else None
     kw = dict(addend=c) if c is not None else {}
     y = torch.full((M, N), float("nan"), dtype=torch.float32 if y32 else torch.float16, device="cuda")
@@ -100,3 +106,27 @@ def test_activations_gain_and_addend_written_by_the_launch_ahead():
         got.append(b(h, addend=x))
     torch.cuda.synchronize()
     assert not [i for i, (p, q) in enumerate(zip(got, want)) if not torch.equal(p, q)]
+
+
+@pytest.mark.parametrize("M,N,K,pair", [(16, 8192, 8192, False), (12, 4032, 5120, True), (16, 4096, 4096, False)])
+def test_one_node_on_two_streams(M, N, K, pair):
+    """Where K is not cut, or cut in halves that meet in a cluster, a call touches no workspace: overlapping calls of one node
+    give what calls one at a time give."""
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    rng = np.random.Generator(np.random.PCG64(N + K))
+    op = DequantDot(*[DeviceWeight.from_host(synth.make_weights(rng, N, K, 4, 128)) for _ in range(1 + pair)])
+    xs = [torch.from_numpy(synth.make_x(rng, M, K, np.float16)).cuda() for _ in range(2)]
+    want = [op(x).clone() for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = [[torch.empty_like(w) for _ in range(400)] for w in want]
+    for i in range(400):
+        for x, s, g in zip(xs, streams, got):
+            with torch.cuda.stream(s):
+                op(x, out=g[i])
+    torch.cuda.synchronize()
+    op.ctx.device_status()
+    for w, g in zip(want, got):
+        assert not [i for i, y in enumerate(g) if not torch.equal(y, w)]
+    assert all(torch.equal(op(x), w) for x, w in zip(xs, want))
