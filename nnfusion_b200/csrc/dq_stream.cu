@@ -49,7 +49,7 @@ constexpr int kBlockBytes = kBatch * (2 * kUnitK + 8);   // prepared activations
 constexpr int kStages = 9;                               // ring of units
 constexpr int kSums = MB * 4 * 32;                       // a warp's sums of a tile
 constexpr int kSmem = kStages * (kWBytes + kBlockBytes) + 2 * kStages * 8 + 16;
-constexpr int kPrepThreads = 128, kPrepSteps = 4;
+constexpr int kPrepThreads = 128, kPrepUnits = kPrepThreads / 4; // 32 elements a thread
 static_assert(kSmem <= 113 * 1024, "two CTAs an SM");
 static_assert(kStages <= 32, "a lane per stage");
 
@@ -435,18 +435,24 @@ __global__ void __launch_bounds__(kThreads, 2)
 
 // The activations, normalised and rounded, as the blocks that dq_stream_kernel copies (rows past M are zeros).  A block is a unit
 // of K: [j][batch row][t] 16 bytes with elements 32 t + 8 j .. + 7 of the unit, in the order 0 4 1 5 2 6 3 7 that the unpacking
-// of the weights leaves, then per batch row -sum(offset_k x_k) and -sum(x_k), pairs of rows side by side.  A CTA takes one row,
-// all of it where the norm needs that (bound by one round trip to L2 and the launch); 128 threads, which fit beside two CTAs of
-// the linear.
+// of the weights leaves, then per batch row -sum(offset_k x_k) and -sum(x_k), pairs of rows side by side.  These two are summed by
+// the tensor core, in the order and from the fragments of the products, with the offsets alone as the left operand: what the
+// accumulator rounds away of 1024 x then goes out with it (weights of q = zp = 0 give exactly 0; summed exactly instead, the error
+// of a result against 64 bits grew by an eighth, and by a third for activations of mean 1).  A warp takes eight units of a batch row,
+// a column of the accumulator each.  A CTA takes one row, all of it where the norm needs that (bound by one round trip to L2 and the
+// launch); 128 threads, which fit beside two CTAs of the linear.
 __global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half* x, const float* gain, uint8_t* blocks, int M, int K, float eps, int per_cta)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float part[kPrepThreads / 32];
-    const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-    const int first = blockIdx.y * per_cta, K8 = min(K >> 3, first + per_cta); // this CTA's chunks of eight elements
-    auto load = [&](int k8) {
-        return m < M ? *reinterpret_cast<const uint4*>(x + (size_t)m * K + k8 * 8) : make_uint4(0u, 0u, 0u, 0u);
+    const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int first = blockIdx.y * per_cta, end = min(K / kUnitK, first + per_cta); // this CTA's units
+    const int u0 = first + 8 * (tid >> 5);                                          // ... and this warp's first one
+    auto load = [&](int u, uint4 (&v)[4]) { // elements 32 t .. 32 t + 31 of a unit
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            v[j] = m < M && u < end ? *reinterpret_cast<const uint4*>(x + (size_t)m * K + u * kUnitK + 32 * t + 8 * j) : make_uint4(0u, 0u, 0u, 0u);
     };
     auto floats = [&](const uint4& a, float (&v)[8]) {
         const uint32_t w[4] = {a.x, a.y, a.z, a.w};
@@ -457,28 +463,30 @@ __global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half*
             v[2 * j] = f.x, v[2 * j + 1] = f.y;
         }
     };
-    uint4 kept[kPrepSteps];
-#pragma unroll
-    for (int s = 0; s < kPrepSteps; s++)
-        if (first + tid + s * kPrepThreads < K8)
-            kept[s] = load(first + tid + s * kPrepThreads);
+    uint4 kept[4];
+    load(u0 + g, kept);
     float r = 1.f;
     if (gain != nullptr) // (then the CTA has the whole row)
     {
         float ss = 0.f;
-        auto add = [&](const uint4& a) {
-            float v[8];
-            floats(a, v);
+        auto add = [&](const uint4 (&a)[4]) {
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                ss = fmaf(v[j], v[j], ss);
+            for (int j = 0; j < 4; j++)
+            {
+                float v[8];
+                floats(a[j], v);
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    ss = fmaf(v[e], v[e], ss);
+            }
         };
-#pragma unroll
-        for (int s = 0; s < kPrepSteps; s++)
-            if (tid + s * kPrepThreads < K8)
-                add(kept[s]);
-        for (int k8 = tid + kPrepSteps * kPrepThreads; k8 < K8; k8 += kPrepThreads)
-            add(load(k8));
+        add(kept);
+        for (int u = u0 + g + kPrepUnits; u < end; u += kPrepUnits)
+        {
+            uint4 more[4];
+            load(u, more);
+            add(more);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -491,45 +499,52 @@ __global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half*
             sum += part[w];
         r = 1.0f / sqrtf(sum / (float)K + eps);
     }
-    const uint32_t half_warp = 0xFFFFu << (lane & 16); // the 16 lanes of a unit come together: K is a multiple of 128
-    auto put = [&](int k8, const uint4& raw) {
-        float v[8];
-        floats(raw, v);
-        if (gain != nullptr)
-        {
-            const float4 a = reinterpret_cast<const float4*>(gain + k8 * 8)[0], b = reinterpret_cast<const float4*>(gain + k8 * 8)[1];
-            const float gn[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    auto put = [&](int ub, const uint4 (&raw)[4]) { // (the whole warp: units ub .. ub + 7)
+        const int u = ub + g;
+        float d[4]; // sums with the offsets / plain ones of units ub + 2t and ub + 2t + 1
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                v[j] = __half2float(__float2half_rn(v[j] * r * gn[j]));
-        }
-        uint8_t* const block = blocks + (size_t)(k8 >> 4) * kBlockBytes;
-        uint32_t h[4];
-        float even = 0.f, odd = 0.f; // the unpacking leaves 1024 on even elements and 64 on odd ones
-#pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int j = 0; j < 4; j++)
         {
-            const __half2 a = __floats2half2_rn(v[2 * q], v[2 * q + 1]);
-            h[q] = *reinterpret_cast<const uint32_t*>(&a);
-            even += v[2 * q], odd += v[2 * q + 1];
-        }
-        *reinterpret_cast<uint4*>(block + ((k8 & 3) * kBatch + m) * 64 + ((k8 >> 2) & 3) * 16) =
-            make_uint4(__byte_perm(h[0], h[2], 0x5410), __byte_perm(h[0], h[2], 0x7632), __byte_perm(h[1], h[3], 0x5410), __byte_perm(h[1], h[3], 0x7632));
+            uint32_t h[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
+            if (gain != nullptr && u < end)
+            {
+                float v[8];
+                floats(raw[j], v);
+                const float* const gj = gain + u * kUnitK + 32 * t + 8 * j;
+                const float4 a = reinterpret_cast<const float4*>(gj)[0], b = reinterpret_cast<const float4*>(gj)[1];
+                const float gn[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int o = 1; o < 16; o <<= 1)
-        {
-            even += __shfl_xor_sync(half_warp, even, o);
-            odd += __shfl_xor_sync(half_warp, odd, o);
+                for (int q = 0; q < 4; q++)
+                {
+                    const __half2 n = __floats2half2_rn(v[2 * q] * r * gn[2 * q], v[2 * q + 1] * r * gn[2 * q + 1]);
+                    h[q] = *reinterpret_cast<const uint32_t*>(&n);
+                }
+            }
+            const uint4 f = make_uint4(__byte_perm(h[0], h[2], 0x5410), __byte_perm(h[0], h[2], 0x7632), __byte_perm(h[1], h[3], 0x5410),
+                                       __byte_perm(h[1], h[3], 0x7632));
+            if (u < end)
+                *reinterpret_cast<uint4*>(blocks + (size_t)u * kBlockBytes + (j * kBatch + m) * 64 + t * 16) = f;
+            // rows 0-7 of the left operand: what the unpacking leaves, 1024 on even elements and 64 on odd ones; rows 8-15: ones
+            if (j == 0)
+                mma16816_first(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.x, f.y);
+            else
+                mma16816(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.x, f.y);
+            mma16816(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.z, f.w);
         }
-        if ((lane & 15) == 0)
-            *reinterpret_cast<float2*>(block + kBatch * 256 + m * 8) = make_float2(-(1024.f * even + 64.f * odd), -(even + odd));
+        if (g == 0)
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+                if (ub + 2 * t + c < end)
+                    *reinterpret_cast<float2*>(blocks + (size_t)(ub + 2 * t + c) * kBlockBytes + kBatch * 256 + m * 8) = make_float2(-d[c], -d[2 + c]);
     };
-#pragma unroll
-    for (int s = 0; s < kPrepSteps; s++)
-        if (first + tid + s * kPrepThreads < K8)
-            put(first + tid + s * kPrepThreads, kept[s]);
-    for (int k8 = first + tid + kPrepSteps * kPrepThreads; k8 < K8; k8 += kPrepThreads)
-        put(k8, load(k8));
+    if (u0 < end)
+        put(u0, kept);
+    for (int ub = u0 + kPrepUnits; ub < end; ub += kPrepUnits)
+    {
+        uint4 more[4];
+        load(ub + g, more);
+        put(ub, more);
+    }
 }
 } // namespace
 
@@ -649,8 +664,8 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     overlap_attribute(attr, &cfg.numAttrs);
     cfg.attrs = attr;
     cfg.stream = stream;
-    const int per_cta = gain != nullptr ? d.K / 8 : kPrepSteps * kPrepThreads; // (the norm needs its whole row)
-    cfg.gridDim = dim3(kBatch, (d.K / 8 + per_cta - 1) / per_cta);
+    const int per_cta = gain != nullptr ? L.KU : kPrepUnits; // (the norm needs its whole row)
+    cfg.gridDim = dim3(kBatch, (L.KU + per_cta - 1) / per_cta);
     cfg.blockDim = dim3(kPrepThreads);
     e = cudaLaunchKernelEx(&cfg, stream_prep_kernel, static_cast<const __half*>(x), static_cast<const float*>(gain), blocks, (int)d.M, (int)d.K, d.rms_eps,
                            per_cta);
