@@ -550,27 +550,29 @@ __global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half*
 
 namespace nnf
 {
+// The workspace: the split form's arrival counters, which this form leaves as they are (zero), the slots and the prepared activations
+// over that form's partial sums, and this form's counters behind all of what the split form uses.  So both find their counters
+// zeroed, in whatever order the calls of a descriptor take one form or the other (the sum over ranks takes the split form).
 struct StreamLayout
 {
     int tiles, KU, ctas;
-    size_t counter_bytes, slot_bytes, block_bytes;
-    size_t total() const { return counter_bytes + slot_bytes + block_bytes; }
+    size_t slots_at, blocks_at, counters_at, total;
 };
 
-static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& split)
 {
+    auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
     StreamLayout L{};
     const int sms = ctx ? ctx->sm_count : 148;
     const bool dual = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
     L.tiles = (d.N + (dual ? 63 : 127)) / (dual ? 64 : 128);
     L.KU = d.K / kUnitK;
     L.ctas = (int)std::min<long long>((long long)L.tiles * L.KU, 2 * sms);
-    if (L.tiles % L.ctas != 0) // some tile is shared
-    {
-        L.counter_bytes = ((size_t)L.tiles * kConsumers * sizeof(uint32_t) + 255) / 256 * 256;
-        L.slot_bytes = (size_t)2 * L.ctas * kConsumers * kSums * sizeof(float);
-    }
-    L.block_bytes = ((size_t)L.KU * kBlockBytes + 255) / 256 * 256;
+    const bool shared = L.tiles % L.ctas != 0; // some tile is
+    L.slots_at = up((size_t)split.row_tiles * sizeof(unsigned));
+    L.blocks_at = L.slots_at + (shared ? (size_t)2 * L.ctas * kConsumers * kSums * sizeof(float) : 0);
+    L.counters_at = up(std::max(L.blocks_at + (size_t)L.KU * kBlockBytes, split.workspace_bytes));
+    L.total = L.counters_at + (shared ? (size_t)L.tiles * kConsumers * sizeof(uint32_t) : 0);
     return L;
 }
 
@@ -604,13 +606,13 @@ bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const
     return d.K > 4096 && tiles * KU >= 16ll * sms;
 }
 
-size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d)
+size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& plan)
 {
-    return stream_layout(ctx, d).total();
+    return stream_layout(ctx, d, plan).total;
 }
 
-int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const void* x, const nnf_b200_qweight* w,
-                  const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y, void* workspace)
+int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const GemvPlan& plan, const void* x,
+                  const nnf_b200_qweight* w, const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y, void* workspace)
 {
     static bool configured[kMaxDevices] = {}; // the attributes belong to the device that is current
     int dev = 0;
@@ -628,9 +630,9 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     }
     if (e != cudaSuccess)
         return set_error(ctx, NNF_B200_ECUDA, std::string("dq_stream set-up: ") + cudaGetErrorString(e));
-    const StreamLayout L = stream_layout(ctx, d);
+    const StreamLayout L = stream_layout(ctx, d, plan);
     uint8_t* const ws = static_cast<uint8_t*>(workspace);
-    uint8_t* const blocks = ws + L.counter_bytes + L.slot_bytes;
+    uint8_t* const blocks = ws + L.blocks_at;
 
     StreamParams p{};
     p.dual = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
@@ -646,8 +648,8 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     p.has_addend = d.epilogue == NNF_B200_EPILOGUE_ADD;
     p.y = y;
     p.status = ctx->dev_status;
-    p.counters = reinterpret_cast<uint32_t*>(ws);
-    p.slots = reinterpret_cast<float*>(ws + L.counter_bytes);
+    p.counters = reinterpret_cast<uint32_t*>(ws + L.counters_at);
+    p.slots = reinterpret_cast<float*>(ws + L.slots_at);
     p.xblocks = blocks;
     p.M = d.M, p.N = d.N, p.KU = L.KU;
     p.units_lo = L.tiles * L.KU / L.ctas, p.units_rem = L.tiles * L.KU % L.ctas;

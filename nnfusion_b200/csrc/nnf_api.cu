@@ -275,8 +275,8 @@ size_t nnf_b200_linear_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_l
         if (nnf::gemv_plan(ctx, *desc, &ring, &why, false) == NNF_B200_OK && ring.workspace_bytes > need)
             need = ring.workspace_bytes;
         // ... and the form that streams the weights through shared memory (a caller with less gets the former two)
-        if (nnf::stream_serves(ctx, *desc, plan) && nnf::stream_workspace_bytes(ctx, *desc) > need)
-            need = nnf::stream_workspace_bytes(ctx, *desc);
+        if (nnf::stream_serves(ctx, *desc, plan) && nnf::stream_workspace_bytes(ctx, *desc, plan) > need)
+            need = nnf::stream_workspace_bytes(ctx, *desc, plan);
         return need;
     }
     return nnf::gemm_workspace_bytes(ctx, *desc);
@@ -451,8 +451,8 @@ static int linear_impl(nnf_b200_ctx* ctx, void* stream, const nnf_b200_linear_de
         rc = cached_gemv_plan(ctx, d, &plan, &why);
         if (rc != NNF_B200_OK)
             return nnf::set_error(ctx, rc, why);
-        if (!peers && workspace && nnf::stream_serves(ctx, d, plan) && workspace_bytes >= nnf::stream_workspace_bytes(ctx, d))
-            return nnf::stream_launch(ctx, s, d, x, w, w2, gain, bias, y, workspace);
+        if (!peers && workspace && nnf::stream_serves(ctx, d, plan) && workspace_bytes >= nnf::stream_workspace_bytes(ctx, d, plan))
+            return nnf::stream_launch(ctx, s, d, plan, x, w, w2, gain, bias, y, workspace);
         if (plan.workspace_bytes > 0 && (!workspace || workspace_bytes < plan.workspace_bytes))
             return nnf::set_error(ctx, NNF_B200_EWORKSPACE,
                                   "workspace of " + std::to_string(plan.workspace_bytes) + " bytes required");

@@ -98,9 +98,9 @@ int gemm_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_de
                 void* y, void* workspace, size_t workspace_bytes);
 
 bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& plan);
-size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d);
-int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const void* x, const nnf_b200_qweight* w,
-                  const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y, void* workspace);
+size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& plan);
+int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_desc& d, const GemvPlan& plan, const void* x,
+                  const nnf_b200_qweight* w, const nnf_b200_qweight* w2, const void* gain, const void* bias, void* y, void* workspace);
 
 size_t allreduce_flag_bytes(size_t count);
 int allreduce_launch(nnf_b200_ctx* ctx, cudaStream_t stream, int rank, int world, const void* const* bufs,

@@ -166,3 +166,46 @@ def test_offsets_leave_as_they_came(M, N, K, mean):
     want = x.astype(np.float64) @ dense.reshape(N, K).T
     err = [np.linalg.norm(y.double().cpu().numpy() - want) / np.linalg.norm(want) for y in (stream, split)]
     assert err[0] <= 1.05 * err[1]
+
+
+@pytest.mark.parametrize("M,N,K,pair", [(16, 37888, 9216, False), (9, 4100, 11008, False), (16, 5000, 11008, True)])
+def test_both_forms_on_one_buffer(M, N, K, pair):
+    """Calls of one descriptor follow one another on a buffer whichever form they take (the sum over ranks and smaller buffers take
+    the split form): each finds its arrival counters zeroed.  296 tiles, one a CTA, among them: none is shared."""
+    import torch
+    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    gen = torch.Generator(device="cuda").manual_seed(N)
+
+    def weight():
+        wq, zp = (torch.randint(0, 256, (N, n), dtype=torch.uint8, device="cuda", generator=gen) for n in (K // 2, (K // 128 + 1) // 2))
+        return DeviceWeight(N, K, 4, 128, wq, (torch.rand(N, K // 128, device="cuda", generator=gen) * 0.018 + 0.002).half(), zp)
+    op = DequantDot(*[weight() for _ in range(1 + pair)])
+    x = torch.randn(M, K, device="cuda", generator=gen).half()
+    d, plan = _plan_bits(op, M, x.dtype)
+    assert plan[7] & 16
+    need = int(op.ctx.lib.nnf_b200_linear_workspace_bytes(op.ctx.handle, ctypes.byref(d)))
+    d2 = op.desc(M, x.dtype)
+    d2.split_k = plan[2]
+    split = int(op.ctx.lib.nnf_b200_linear_workspace_bytes(op.ctx.handle, ctypes.byref(d2)))
+    counters = (N + 15) // 16 * 4                                # the split form's, in front
+    words = torch.zeros(16384, dtype=torch.int32, device="cuda")
+    peer = torch.zeros(2 * M * N, dtype=torch.float32, device="cuda")
+    peers = L.Peers(0, 1, (ctypes.c_void_p * 1)(peer.data_ptr()), (ctypes.c_void_p * 1)(words.data_ptr()), M * N * 4, 0)
+
+    def run(ws, streaming):
+        y = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        if streaming or pair:
+            op.run_raw(d, x.data_ptr(), y.data_ptr(), ws if streaming else ws[:split])
+        else:
+            op.ctx.check(op.ctx.lib.nnf_b200_linear_allreduce(
+                op.ctx.handle, torch.cuda.current_stream().cuda_stream, ctypes.byref(d), x.data_ptr(), ctypes.byref(op._abi_w), None,
+                y.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(peers)))
+        return y
+
+    fresh, ws = torch.zeros(need, dtype=torch.uint8, device="cuda"), torch.zeros(need, dtype=torch.uint8, device="cuda")
+    want = {False: run(torch.zeros_like(fresh), False), True: run(fresh, True)}
+    assert torch.linalg.vector_norm(want[True].double() - want[False].double()) <= 1e-3 * torch.linalg.vector_norm(want[False].double())
+    for streaming in (True, False, True, True, False, False, True):
+        assert torch.equal(run(ws, streaming), want[streaming])
+        assert int(ws[:counters].count_nonzero()) == 0
+    op.ctx.device_status()
