@@ -342,8 +342,10 @@ NNF_B200_API int nnf_b200_linear_allreduce(nnf_b200_ctx* ctx, void* stream, cons
                                            void* workspace, size_t workspace_bytes, const nnf_b200_peers* peers);
 
 /* Reads (and clears) the device-side status word: 0, or NNF_B200_ETIMEDOUT when a
- * bounded wait inside a kernel gave up since the last query.  Synchronises the
- * stream; meant for tests and debugging, not for the hot path. */
+ * bounded wait inside a kernel gave up since the last query.  Arrivals may then be
+ * half counted in the workspace of that call: zero-fill it before its next use
+ * (nnf_b200_workspace_reset).  Synchronises the stream; meant for tests and
+ * debugging, not for the hot path. */
 NNF_B200_API int nnf_b200_device_status(nnf_b200_ctx* ctx, void* stream);
 
 /* Number of kernels the library has launched on this context since init

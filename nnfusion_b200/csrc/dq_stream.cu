@@ -24,8 +24,9 @@
 // A CTA takes half an SM (113 KB, 288 threads), two are resident.
 // What bounds it: about 150 instructions a warp and unit at half of the issue rate (so are its neighbours), and a fixed cost of
 // some 8 us (two launches' hand-over, the shared tiles' ticket and sums), which is why small weights stay with the small-M kernel.
-// Every mbarrier wait is bounded; on a time-out the CTA raises a status flag and stores nothing more, after its copies have
-// landed.
+// Every mbarrier wait is bounded.  On a time-out the CTA raises the status flag; its warps store nothing and take no ticket at the
+// ends of tiles that they reach from then on, and it waits (bounded, too) for its copies.  What it has stored by then stays, and
+// tickets of shared tiles may be half counted: the workspace has to be zero-filled before its next use.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -190,12 +191,15 @@ __global__ void __launch_bounds__(kThreads, 2)
                 ask_x(st, unit);
             }
         }
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) // copies in flight land before the CTA ends
+        // The last copies of every stage land before the CTA ends, whether or not a consumer has waited for them.
+        const int last = min(n_units, i) - 1 - lane; // a lane per stage
+        if (lane < kStages && last >= 0)
         {
-            const int last = min(n_units, i) - 1 - lane; // a lane per stage
-            if (lane < kStages && last >= 0)
-                for (int t = 0; t < 4096 && !mbar_test_wait(full(last % kStages), (last / kStages) & 1u); t++)
-                    __nanosleep(100);
+            bool landed = false;
+            for (uint32_t tries = 0; tries < kRoleSpin && !landed; tries++)
+                landed = mbar_try_wait(full(last % kStages), (last / kStages) & 1u);
+            if (!landed)
+                *abort_flag = 1;
         }
     }
     else
@@ -318,6 +322,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                 continue;
             }
             // ---- the end of this CTA's part of the tile
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) // (a role gave up: no stores, no tickets from here on)
+                break;
             bool mine = true; // does this warp finish its rows?
             if (seg_ku0 != 0 || ku != KU - 1)
             {
