@@ -439,27 +439,36 @@ __global__ void __launch_bounds__(kThreads, 2)
         atomicExch(p.status, 1);
 }
 
+// 16 bytes that the launch ahead may have written; loads that follow one another stay together
+__device__ __forceinline__ uint4 load16(const void* p)
+{
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // The activations, normalised and rounded, as the blocks that dq_stream_kernel copies (rows past M are zeros).  A block is a unit
 // of K: [j][batch row][t] 16 bytes with elements 32 t + 8 j .. + 7 of the unit, in the order 0 4 1 5 2 6 3 7 that the unpacking
 // of the weights leaves, then per batch row -sum(offset_k x_k) and -sum(x_k), pairs of rows side by side.  These two are summed by
 // the tensor core, in the order and from the fragments of the products, with the offsets alone as the left operand: what the
 // accumulator rounds away of 1024 x then goes out with it (weights of q = zp = 0 give exactly 0; summed exactly instead, the error
-// of a result against 64 bits grew by an eighth, and by a third for activations of mean 1).  A warp takes eight units of a batch row,
-// a column of the accumulator each.  A CTA takes one row, all of it where the norm needs that (bound by one round trip to L2 and the
-// launch); 128 threads, which fit beside two CTAs of the linear.
-__global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half* x, const float* gain, uint8_t* blocks, int M, int K, float eps, int per_cta)
+// of a result against 64 bits grew by an eighth, and by a third for activations of mean 1).A warp takes eight units of a batch row,
+// a column of the accumulator each, a CTA 32 units; with the norm every CTA of a row sums up all of its squares, eight loads in
+// flight a thread (bound by a few round trips to L2 and the launch; a row whole to one CTA, a load at a time, took 25 us at
+// K = 28672).  128 threads, which fit beside two CTAs of the linear.
+__global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half* x, const float* gain, uint8_t* blocks, int M, int K, float eps)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float part[kPrepThreads / 32];
     const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int first = blockIdx.y * per_cta, end = min(K / kUnitK, first + per_cta); // this CTA's units
-    const int u0 = first + 8 * (tid >> 5);                                          // ... and this warp's first one
-    auto load = [&](int u, uint4 (&v)[4]) { // elements 32 t .. 32 t + 31 of a unit
+    const int KU = K / kUnitK;
+    const int ub = blockIdx.y * kPrepUnits + 8 * (tid >> 5), u = ub + g; // this warp's first unit and the lane's
+    const __half* const row = x + (size_t)m * K;
+    uint4 raw[4]; // elements 32 t .. 32 t + 31 of the unit
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-            v[j] = m < M && u < end ? *reinterpret_cast<const uint4*>(x + (size_t)m * K + u * kUnitK + 32 * t + 8 * j) : make_uint4(0u, 0u, 0u, 0u);
-    };
+    for (int j = 0; j < 4; j++)
+        raw[j] = m < M && u < KU ? load16(row + u * kUnitK + 32 * t + 8 * j) : make_uint4(0u, 0u, 0u, 0u);
     auto floats = [&](const uint4& a, float (&v)[8]) {
         const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
@@ -469,29 +478,28 @@ __global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half*
             v[2 * j] = f.x, v[2 * j + 1] = f.y;
         }
     };
-    uint4 kept[4];
-    load(u0 + g, kept);
     float r = 1.f;
-    if (gain != nullptr) // (then the CTA has the whole row)
+    if (gain != nullptr)
     {
         float ss = 0.f;
-        auto add = [&](const uint4 (&a)[4]) {
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-            {
-                float v[8];
-                floats(a[j], v);
-#pragma unroll
-                for (int e = 0; e < 8; e++)
-                    ss = fmaf(v[e], v[e], ss);
-            }
-        };
-        add(kept);
-        for (int u = u0 + g + kPrepUnits; u < end; u += kPrepUnits)
+        constexpr int in_flight = 8;
+        const int K8 = m < M ? K / 8 : 0;
+        for (int i = tid; i < K8; i += in_flight * kPrepThreads)
         {
-            uint4 more[4];
-            load(u, more);
-            add(more);
+            uint4 a[in_flight];
+#pragma unroll
+            for (int e = 0; e < in_flight; e++)
+                a[e] = load16(row + (size_t)min(i + e * kPrepThreads, K8 - 1) * 8);
+#pragma unroll
+            for (int e = 0; e < in_flight; e++)
+            {
+                float v[8], add = 0.f;
+                floats(a[e], v);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    add = fmaf(v[j], v[j], add);
+                ss += i + e * kPrepThreads < K8 ? add : 0.f;
+            }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -501,56 +509,45 @@ __global__ void __launch_bounds__(kPrepThreads) stream_prep_kernel(const __half*
         __syncthreads();
         float sum = 0.f;
 #pragma unroll
-        for (int w = 0; w < kPrepThreads / 32; w++) // fixed order: repeatable
+        for (int w = 0; w < kPrepThreads / 32; w++) // fixed order: repeatable, and the same in every CTA of the row
             sum += part[w];
         r = 1.0f / sqrtf(sum / (float)K + eps);
     }
-    auto put = [&](int ub, const uint4 (&raw)[4]) { // (the whole warp: units ub .. ub + 7)
-        const int u = ub + g;
-        float d[4]; // sums with the offsets / plain ones of units ub + 2t and ub + 2t + 1
+    float d[4]; // sums with the offsets / plain ones of units ub + 2t and ub + 2t + 1
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-        {
-            uint32_t h[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
-            if (gain != nullptr && u < end)
-            {
-                float v[8];
-                floats(raw[j], v);
-                const float* const gj = gain + u * kUnitK + 32 * t + 8 * j;
-                const float4 a = reinterpret_cast<const float4*>(gj)[0], b = reinterpret_cast<const float4*>(gj)[1];
-                const float gn[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                {
-                    const __half2 n = __floats2half2_rn(v[2 * q] * r * gn[2 * q], v[2 * q + 1] * r * gn[2 * q + 1]);
-                    h[q] = *reinterpret_cast<const uint32_t*>(&n);
-                }
-            }
-            const uint4 f = make_uint4(__byte_perm(h[0], h[2], 0x5410), __byte_perm(h[0], h[2], 0x7632), __byte_perm(h[1], h[3], 0x5410),
-                                       __byte_perm(h[1], h[3], 0x7632));
-            if (u < end)
-                *reinterpret_cast<uint4*>(blocks + (size_t)u * kBlockBytes + (j * kBatch + m) * 64 + t * 16) = f;
-            // rows 0-7 of the left operand: what the unpacking leaves, 1024 on even elements and 64 on odd ones; rows 8-15: ones
-            if (j == 0)
-                mma16816_first(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.x, f.y);
-            else
-                mma16816(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.x, f.y);
-            mma16816(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.z, f.w);
-        }
-        if (g == 0)
-#pragma unroll
-            for (int c = 0; c < 2; c++)
-                if (ub + 2 * t + c < end)
-                    *reinterpret_cast<float2*>(blocks + (size_t)(ub + 2 * t + c) * kBlockBytes + kBatch * 256 + m * 8) = make_float2(-d[c], -d[2 + c]);
-    };
-    if (u0 < end)
-        put(u0, kept);
-    for (int ub = u0 + kPrepUnits; ub < end; ub += kPrepUnits)
+    for (int j = 0; j < 4; j++)
     {
-        uint4 more[4];
-        load(ub + g, more);
-        put(ub, more);
+        uint32_t h[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
+        if (gain != nullptr && u < KU)
+        {
+            float v[8];
+            floats(raw[j], v);
+            const float* const gj = gain + u * kUnitK + 32 * t + 8 * j;
+            const float4 a = reinterpret_cast<const float4*>(gj)[0], b = reinterpret_cast<const float4*>(gj)[1];
+            const float gn[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+            {
+                const __half2 n = __floats2half2_rn(v[2 * q] * r * gn[2 * q], v[2 * q + 1] * r * gn[2 * q + 1]);
+                h[q] = *reinterpret_cast<const uint32_t*>(&n);
+            }
+        }
+        const uint4 f = make_uint4(__byte_perm(h[0], h[2], 0x5410), __byte_perm(h[0], h[2], 0x7632), __byte_perm(h[1], h[3], 0x5410),
+                                   __byte_perm(h[1], h[3], 0x7632));
+        if (u < KU)
+            *reinterpret_cast<uint4*>(blocks + (size_t)u * kBlockBytes + (j * kBatch + m) * 64 + t * 16) = f;
+        // rows 0-7 of the left operand: what the unpacking leaves, 1024 on even elements and 64 on odd ones; rows 8-15: ones
+        if (j == 0)
+            mma16816_first(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.x, f.y);
+        else
+            mma16816(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.x, f.y);
+        mma16816(d, 0x64006400u, 0x3C003C00u, 0x54005400u, 0x3C003C00u, f.z, f.w);
     }
+    if (g == 0)
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+            if (ub + 2 * t + c < KU)
+                *reinterpret_cast<float2*>(blocks + (size_t)(ub + 2 * t + c) * kBlockBytes + kBatch * 256 + m * 8) = make_float2(-d[c], -d[2 + c]);
 }
 } // namespace
 
@@ -672,11 +669,9 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     overlap_attribute(attr, &cfg.numAttrs);
     cfg.attrs = attr;
     cfg.stream = stream;
-    const int per_cta = gain != nullptr ? L.KU : kPrepUnits; // (the norm needs its whole row)
-    cfg.gridDim = dim3(kBatch, (L.KU + per_cta - 1) / per_cta);
+    cfg.gridDim = dim3(kBatch, (L.KU + kPrepUnits - 1) / kPrepUnits);
     cfg.blockDim = dim3(kPrepThreads);
-    e = cudaLaunchKernelEx(&cfg, stream_prep_kernel, static_cast<const __half*>(x), static_cast<const float*>(gain), blocks, (int)d.M, (int)d.K, d.rms_eps,
-                           per_cta);
+    e = cudaLaunchKernelEx(&cfg, stream_prep_kernel, static_cast<const __half*>(x), static_cast<const float*>(gain), blocks, (int)d.M, (int)d.K, d.rms_eps);
     if (e != cudaSuccess)
         return set_error(ctx, NNF_B200_ECUDA, std::string("stream_prep launch: ") + cudaGetErrorString(e));
     ctx->launches++;
