@@ -34,6 +34,7 @@
 
 #include "nnf_internal.h"
 #include "sm100_ptx.cuh"
+#include "stream_shares.h"
 
 namespace
 {
@@ -62,10 +63,10 @@ struct StreamParams
     void* y;
     int* status;
     uint32_t* counters;      // [tiles][warps] arrivals at shared tiles; zero before and after
-    float* slots;            // [CTAs][2][warps][kSums] partial sums of shared tiles
+    float* slots;            // [slots][warps][kSums] partial sums of shared tiles
     const uint8_t* xblocks;  // [units of K][kBlockBytes] prepared activations
-    int M, N, KU;            // KU: units of K
-    int units_lo, units_rem; // a CTA's share: tiles x KU / CTAs and its remainder (the first units_rem CTAs have one more)
+    int M, N;
+    nnf::StreamShares shares;
     int dual;
     int G, zp_row_bytes;
     int group_units;         // units per quantisation group
@@ -121,10 +122,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     volatile int* const abort_flag = reinterpret_cast<volatile int*>(smem + kStages * (kWBytes + kBlockBytes) + 2 * kStages * 8);
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int KU = p.KU;
-    auto share_begin = [&](int cta) { return cta * p.units_lo + min(cta, p.units_rem); };
-    const int u_begin = share_begin((int)blockIdx.x);
-    const int n_units = p.units_lo + ((int)blockIdx.x < p.units_rem ? 1 : 0);
+    const int KU = p.shares.KU;
+    const int u_begin = p.shares.begin((int)blockIdx.x);
+    const int n_units = p.shares.units((int)blockIdx.x);
     const int tile_begin = u_begin / KU, ku_begin = u_begin - tile_begin * KU;
 
     // (the producer's lanes each ask for a unit: the four instructions and the wait of a unit take one thread several hundred clocks)
@@ -327,15 +327,8 @@ __global__ void __launch_bounds__(kThreads, 2)
             bool mine = true; // does this warp finish its rows?
             if (seg_ku0 != 0 || ku != KU - 1)
             {
-                auto owner = [&](int u) { // the CTA whose share holds unit u
-                    const int more = p.units_rem * (p.units_lo + 1); // units of the shares with one more
-                    return u < more ? u / (p.units_lo + 1) : p.units_rem + (u - more) / p.units_lo;
-                };
-                // a share's first tile has slot 0, another one that it shares (its last) slot 1
-                auto slot = [&](int cta) {
-                    return p.slots + (size_t)((2 * cta + (share_begin(cta) >= tile * KU ? 0 : 1)) * kConsumers + warp) * kSums + lane;
-                };
-                const int c_first = owner(tile * KU), c_last = owner(tile * KU + KU - 1);
+                auto slot = [&](int cta) { return p.slots + (size_t)(p.shares.slot(cta, tile) * kConsumers + warp) * kSums + lane; };
+                const int c_first = p.shares.owner(tile * KU), c_last = p.shares.owner(tile * KU + KU - 1);
                 float* const my = slot((int)blockIdx.x);
 #pragma unroll
                 for (int mb = 0; mb < MB; mb++)
@@ -558,7 +551,7 @@ namespace nnf
 // zeroed, in whatever order the calls of a descriptor take one form or the other (the sum over ranks takes the split form).
 struct StreamLayout
 {
-    int tiles, KU, ctas;
+    StreamShares shares;
     size_t slots_at, blocks_at, counters_at, total;
 };
 
@@ -568,14 +561,11 @@ static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear
     StreamLayout L{};
     const int sms = ctx ? ctx->sm_count : 148;
     const bool dual = d.epilogue == NNF_B200_EPILOGUE_SILU_MUL;
-    L.tiles = (d.N + (dual ? 63 : 127)) / (dual ? 64 : 128);
-    L.KU = d.K / kUnitK;
-    L.ctas = (int)std::min<long long>((long long)L.tiles * L.KU, 2 * sms);
-    const bool shared = L.tiles % L.ctas != 0; // some tile is
+    L.shares.set((d.N + (dual ? 63 : 127)) / (dual ? 64 : 128), d.K / kUnitK, 2 * sms);
     L.slots_at = up((size_t)split.row_tiles * sizeof(unsigned));
-    L.blocks_at = L.slots_at + (shared ? (size_t)2 * L.ctas * kConsumers * kSums * sizeof(float) : 0);
-    L.counters_at = up(std::max(L.blocks_at + (size_t)L.KU * kBlockBytes, split.workspace_bytes));
-    L.total = L.counters_at + (shared ? (size_t)L.tiles * kConsumers * sizeof(uint32_t) : 0);
+    L.blocks_at = L.slots_at + (size_t)L.shares.slots() * kConsumers * kSums * sizeof(float);
+    L.counters_at = up(std::max(L.blocks_at + (size_t)L.shares.KU * kBlockBytes, split.workspace_bytes));
+    L.total = L.counters_at + (L.shares.any_shared() ? (size_t)L.shares.tiles * kConsumers * sizeof(uint32_t) : 0);
     return L;
 }
 
@@ -654,8 +644,8 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     p.counters = reinterpret_cast<uint32_t*>(ws + L.counters_at);
     p.slots = reinterpret_cast<float*>(ws + L.slots_at);
     p.xblocks = blocks;
-    p.M = d.M, p.N = d.N, p.KU = L.KU;
-    p.units_lo = L.tiles * L.KU / L.ctas, p.units_rem = L.tiles * L.KU % L.ctas;
+    p.M = d.M, p.N = d.N;
+    p.shares = L.shares;
     const int group = d.group_size > 0 ? d.group_size : d.K;
     p.G = d.K / group;
     p.zp_row_bytes = (p.G + 1) / 2;
@@ -669,13 +659,13 @@ int stream_launch(nnf_b200_ctx* ctx, cudaStream_t stream, const nnf_b200_linear_
     overlap_attribute(attr, &cfg.numAttrs);
     cfg.attrs = attr;
     cfg.stream = stream;
-    cfg.gridDim = dim3(kBatch, (L.KU + kPrepUnits - 1) / kPrepUnits);
+    cfg.gridDim = dim3(kBatch, (L.shares.KU + kPrepUnits - 1) / kPrepUnits);
     cfg.blockDim = dim3(kPrepThreads);
     e = cudaLaunchKernelEx(&cfg, stream_prep_kernel, static_cast<const __half*>(x), static_cast<const float*>(gain), blocks, (int)d.M, (int)d.K, d.rms_eps);
     if (e != cudaSuccess)
         return set_error(ctx, NNF_B200_ECUDA, std::string("stream_prep launch: ") + cudaGetErrorString(e));
     ctx->launches++;
-    cfg.gridDim = dim3(L.ctas);
+    cfg.gridDim = dim3(L.shares.ctas);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmem;
     e = cudaLaunchKernelEx(&cfg, dq_stream_kernel, p, tw[0], tw[1]);
