@@ -573,9 +573,17 @@ static StreamLayout stream_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear
 // cut K into a cluster that the device holds (halves of K, in practice), its sums meet in shared memory and it touches no workspace,
 // so that calls of one node on two streams may overlap.  Those stay there, also where this would be faster, as does a K of up to
 // 4096, which is not cut (gate/up pair 11008 x 4096 at 16 rows 25.5 / 23.7 us, small-M kernel / this).
-// Otherwise, measured at 16 rows (us; units per SM of 148): 4096 x 11008 (19) 19.6 / 18.7, the gate/up pair 28672 x 8192 (388)
-// 117 / 79, 8192 x 28672 (97) 68.8 / 44.6.  Up to 8 rows the small-M kernel keeps all activations in registers and is faster nearly
-// everywhere.
+// Otherwise by what the small-M kernel makes of the shape: `n` 16-row tiles and weight sets to walk for a warp, and warps of the CTA.
+// It is at its best with nearly all of its 16 warps at work and few tiles to walk, where this form pays for many CTAs to a tile.
+// Measured at 9, 12 and 16 rows, with and without the norm, 209 shapes of 16 to 194 units per SM of 148 (us at 16 rows without the
+// norm, small-M kernel / this; n, warps):
+//   4096 x 11008 (7, 11) 19.9 / 18.4, 8192 x 28672 (25, 16) 71.5 / 45.5, 28672 x 8192 pair (50, 16) 120 / 79.5,
+//   3936 x 12288 (7, 12) 20.0 / 18.8, 1680 x 11520 pair (6, 12) 17.5 / 16.9;
+//   left there: 3344 x 12288 (6, 12) 16.3 / 18.6, 4608 x 9728 (6, 13) 17.2 / 18.5, 672 x 28672 pair (4, 16) 16.6 / 19.2,
+//   3104 x 17920 (7, 14) 20.2 / 20.6, 2064 x 28672 with norm (7, 16) 26.9 / 29.0.
+// Of the 640 measured calls that this rule admits the slowest takes 0.98 times the small-M kernel's time, on average 0.71; of the
+// 183 that it leaves there the fastest would take 0.84.  Fewer than 16 units per SM were not measured.  Up to 8 rows the small-M
+// kernel keeps all activations in registers and is faster nearly everywhere.
 bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& plan)
 {
     const int group = d.group_size > 0 ? d.group_size : d.K;
@@ -596,7 +604,8 @@ bool stream_serves(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const
         if (plan.ctas_per_split <= held[plan.splits] * std::max(1, std::min(4, 16 / plan.warps)))
             return false;
     }
-    return d.K > 4096 && tiles * KU >= 16ll * sms;
+    const int sets = plan.dual ? 2 : 1, n = sets * ((plan.row_tiles + plan.ctas_per_split - 1) / plan.ctas_per_split);
+    return d.K > 4096 && tiles * KU >= 16ll * sms && (plan.warps <= 11 || n >= (d.K <= 15360 ? 8 - sets : 8));
 }
 
 size_t stream_workspace_bytes(const nnf_b200_ctx* ctx, const nnf_b200_linear_desc& d, const GemvPlan& plan)

@@ -37,3 +37,16 @@ def test_halves_that_meet_in_a_cluster_stay_there(lib, M, pair):
                 assert not out[7] & 16, (N, K)
                 assert need == _plan(lib, M, N, K, pair, split_k=2)[1], (N, K)
     assert found >= 100
+
+
+@pytest.mark.parametrize("M,norm", [(9, False), (16, True)])
+@pytest.mark.parametrize("N,K,pair,streams", [
+    (4096, 11008, False, True), (8192, 28672, False, True), (28672, 8192, True, True),   # the projections of 7B and 70B shapes
+    (3936, 12288, False, True), (1680, 11520, True, True),                               # (7 and 2 x 3 tiles to walk, 12 warps)
+    (3344, 12288, False, False), (4608, 9728, False, False), (672, 28672, True, False),  # measured slower there:
+    (3104, 17920, False, False), (2064, 28672, False, False),                            # few tiles to walk, many CTAs to a tile
+    (4096, 4096, False, False), (11008, 4096, True, False),                              # K is not cut
+])
+def test_sides_of_the_line(lib, N, K, pair, streams, M, norm):
+    assert bool(_plan(lib, M, N, K, pair, norm)[0][7] & 16) == streams
+    assert not _plan(lib, 8, N, K, pair, norm)[0][7] & 16
