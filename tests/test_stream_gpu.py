@@ -173,13 +173,9 @@ def test_both_forms_on_one_buffer(M, N, K, pair):
     """Calls of one descriptor follow one another on a buffer whichever form they take (the sum over ranks and smaller buffers take
     the split form): each finds its arrival counters zeroed.  296 tiles, one a CTA, among them: none is shared."""
     import torch
-    from nnfusion_b200.linear import DequantDot, DeviceWeight
+    from nnfusion_b200.linear import DequantDot
     gen = torch.Generator(device="cuda").manual_seed(N)
-
-    def weight():
-        wq, zp = (torch.randint(0, 256, (N, n), dtype=torch.uint8, device="cuda", generator=gen) for n in (K // 2, (K // 128 + 1) // 2))
-        return DeviceWeight(N, K, 4, 128, wq, (torch.rand(N, K // 128, device="cuda", generator=gen) * 0.018 + 0.002).half(), zp)
-    op = DequantDot(*[weight() for _ in range(1 + pair)])
+    op = DequantDot(*[_device_weight(gen, N, K) for _ in range(1 + pair)])
     x = torch.randn(M, K, device="cuda", generator=gen).half()
     d, plan = _plan_bits(op, M, x.dtype)
     assert plan[7] & 16
@@ -209,3 +205,82 @@ def test_both_forms_on_one_buffer(M, N, K, pair):
         assert torch.equal(run(ws, streaming), want[streaming])
         assert int(ws[:counters].count_nonzero()) == 0
     op.ctx.device_status()
+
+
+def _device_weight(gen, N, K, odd=False):
+    """Random weights on the device; odd: scales and zero-points that start 2 bytes and 1 byte past a 16-byte boundary."""
+    import torch
+    from nnfusion_b200.linear import DeviceWeight
+    wq, zp = (torch.randint(0, 256, (N, n), dtype=torch.uint8, device="cuda", generator=gen) for n in (K // 2, (K // 128 + 1) // 2))
+    scale = (torch.rand(N, K // 128, device="cuda", generator=gen) * 0.018 + 0.002).half()
+    if odd:
+        scale, zp = (torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape) for t in (scale, zp))
+        assert scale.data_ptr() % 16 == 2 and zp.data_ptr() % 16 == 1
+    return DeviceWeight(N, K, 4, 128, wq, scale, zp)
+
+
+@pytest.mark.parametrize("norm", [False, True])
+def test_not_finite_activations_stay_in_their_row(norm):
+    """A row with an infinity or a NaN gives what the small-M kernel gives (the offsets' sums make NaN of it), the others what they
+    give without it; the largest finite values stay finite where the result is."""
+    import torch
+    from nnfusion_b200.linear import DequantDot
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    N, K = 4096, 11008
+    op = DequantDot(_device_weight(gen, N, K), gain=torch.rand(K, device="cuda", generator=gen) + 0.5 if norm else None,
+                    y_dtype=torch.float32)
+    x = torch.randn(12, K, device="cuda", generator=gen).half()
+    x[9] = 0
+    x[9, 77] = 65504.0
+    clean, _ = _both_forms(op, x)
+    assert bool(torch.isfinite(clean).all())
+    x[2, 4000], x[5, 1], x[8, 11007] = float("inf"), float("nan"), -float("inf")
+    stream, split = _both_forms(op, x)
+    rows = [2, 5, 8]
+    assert torch.equal(torch.isnan(stream), torch.isnan(split)) and not bool(torch.isfinite(stream[rows]).any())
+    keep = [m for m in range(12) if m not in rows]
+    assert torch.equal(stream[keep], clean[keep])
+
+
+def test_scales_and_zero_points_off_their_boundaries():
+    import torch
+    from nnfusion_b200.linear import DequantDot
+    N, K = 4100, 11008
+    ops = [DequantDot(_device_weight(torch.Generator(device="cuda").manual_seed(3), N, K, odd)) for odd in (False, True)]
+    x = torch.randn(9, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(4)).half()
+    assert torch.equal(*[_both_forms(op, x)[0] for op in ops])
+
+
+@pytest.mark.parametrize("M", [16, 48])
+def test_two_host_threads_on_one_context(M):
+    """Nodes made and called for the first time by two threads at once: the tensor maps of their weights go into the context's
+    cache under its lock, and every call gets its own."""
+    import threading
+    import torch
+    from nnfusion_b200.linear import DequantDot
+    N, K, nodes = 4096, 11008, 12
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    weights = [[_device_weight(gen, N, K) for _ in range(nodes)] for _ in range(2)]
+    x = torch.randn(M, K, device="cuda", generator=gen).half()
+    want = [[DequantDot(w)(x) for w in ws] for ws in weights]
+    again = [[_device_weight(gen, 16, K) for _ in range(nodes)] for _ in range(2)]   # (new addresses: new entries)
+    torch.cuda.synchronize()
+    got, errors, start = [[], []], [], threading.Barrier(2)
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait(timeout=30)
+                for w, small in zip(weights[i], again[i]):
+                    DequantDot(small)(x)
+                    got[i].append(DequantDot(w)(x))
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # (shown by the assertion below)
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=120)
+    assert not errors and not any(t.is_alive() for t in threads)
+    assert all(torch.equal(a, b) for p, q in zip(want, got) for a, b in zip(p, q)) and [len(g) for g in got] == [nodes] * 2
