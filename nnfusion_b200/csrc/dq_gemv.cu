@@ -85,41 +85,6 @@ struct GemvParams
     int slot_floats;
 };
 
-__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// Same, starting a sum: the addend is zero.
-__device__ __forceinline__ void mma16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-
-// (w & MASK) | orv.  The OR-ed constant comes in a register that the caller fills once (see held_constant): with
-// two immediates the compiler re-creates one of them in front of every use.
-template <uint32_t MASK>
-__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t orv)
-{
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(orv)); // (a & b) | c
-    return r;
-}
-// A constant the compiler cannot see through, so that it stays in its register.
-__device__ __forceinline__ uint32_t held_constant(uint32_t v)
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
-
 __device__ __forceinline__ uint32_t hsub2_u32(uint32_t a, uint32_t b)
 {
     uint32_t r;

@@ -74,33 +74,6 @@ struct StreamParams
     int y_f32, scale_f32, has_addend;
 };
 
-__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// Same, starting a sum: the addend is zero.
-__device__ __forceinline__ void mma16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-// (w & MASK) | orv, the OR-ed constant in a register that the caller fills once
-template <uint32_t MASK>
-__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t orv)
-{
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(orv));
-    return r;
-}
-__device__ __forceinline__ uint32_t held(uint32_t v)
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
 // 16-byte aligned addresses, a size that is a multiple of 16
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
 {
@@ -213,7 +186,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         const uint32_t w_at[2] = {smem_s + (uint32_t)(r0 * 64 + ((t ^ ((r0 >> 1) & 3)) << 4)), smem_s + (uint32_t)(r1 * 64 + ((t ^ ((r1 >> 1) & 3)) << 4))};
         const uint32_t x_at = x_ring + (uint32_t)(g * 64 + t * 16);
         const uint32_t nc_at = x_ring + (uint32_t)(kBatch * 256 + t * 16);
-        const uint32_t k6400 = held(0x64006400u), k5400 = held(0x54005400u);
+        const uint32_t k6400 = held_constant(0x64006400u), k5400 = held_constant(0x54005400u);
 
         // Scales and zero-points: lane t of a row's four asks for those of unit 4 i + t, four units ahead; a unit's come round by
         // shuffles.  (A warp's rows lie in as many lines: asked for unit by unit they would take the load unit's turns from shared
