@@ -59,7 +59,7 @@ constexpr int kEpiBarrier = 1;                // named barrier of the epilogue w
 // BX: the most batch rows of a tile, 64, 128 or 256.
 // SMALL: tiles of up to 128 batch rows, whose multiplication takes no longer than the conversion of the weights: four
 // groups of conversion warps instead of two (about 220 clocks per k-block instead of 380; a k-block of 128 batch rows takes
-// the tensor core 256) and a raw ring of 128 KB (HBM's latency at full rate is about 100 KB per SM), paid for with half of
+// the tensor core 256) and a raw ring of 128 KB (160 KB up to 64 batch rows; HBM's latency at full rate is about 100 KB per SM), paid for with half of
 // the epilogue warps and a smaller x ring.
 // Up to 64 batch rows the two accumulators leave room for 12 converted k-blocks instead of 8, three stages instead of two: a
 // stage's conversion, its multiplies and the handing over between them follow one another, and what bounds these tiles is how
@@ -1267,8 +1267,8 @@ static GemmLayout gemm_layout(const nnf_b200_ctx* ctx, const nnf_b200_linear_des
     // Batch tiles of equal width and how K is shared, by an estimate that ranks the choices: its constants were fitted to 20
     // shapes of 32 to 4096 batch rows times every choice, without what all choices share (the launch, the first loads, the
     // last stores), so that the microseconds themselves come out 20 to 40 % low (4096 x 11008 x 4096: 227 for 320 measured;
-    // 48 x 4096 x 11008: 13.9 for 18.9).  What a k-block takes: up to 128 batch rows the conversion of the weights (and
-    // handing it over), 0.21 to 0.24; above, where two groups of warps convert, 0.31 to 0.345.  Whole tiles cost whole waves.
+    // 48 x 4096 x 11008: 13.9 for 18.4; fitted when tiles of up to 64 rows had two stages of converted weights, and not again since
+    // they have three).  What a k-block takes: up to 128 batch rows the conversion of the weights (and handing it over), 0.19 to 0.24; above, where two groups of warps convert, 0.31 to 0.345.  Whole tiles cost whole waves.
     // Partial sums through the workspace (store, ticket, read back) cost 9 to 26 us, inside a cluster 1 to 4 us.
     const double kb = (double)d.K / 64.0 * L.sets;
     auto pairs_of = [&](int tiles, bool whole) {

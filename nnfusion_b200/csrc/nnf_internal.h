@@ -76,7 +76,8 @@ int check_linear_call(const nnf_b200_linear_desc* d, const void* x, const nnf_b2
 void overlap_attribute(cudaLaunchAttribute* attr, unsigned* count);
 
 // Cached 2-D byte tensor map [rows][row_bytes] with a box of box_rows x box_bytes (swizzled over box_bytes, 64 or 128), copied
-// out under the cache's lock: threads may share a context; false if the driver refuses it.
+// out under the cache's lock (Python threads share a context, and prepared calls run without the interpreter lock; the launch count
+// and the last error's text are not guarded); false if the driver refuses it.
 bool weight_tensor_map(nnf_b200_ctx* ctx, const void* base, int rows, int row_bytes, int box_bytes, int box_rows, CUtensorMap* out);
 
 // allow_direct = false keeps the plan on the ring kernel (the one that takes the zero-points out before the multiply).
