@@ -343,7 +343,6 @@ __global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
 {
     using C = Cfg<BX>;
     constexpr int KBC = (WBITS == 4) ? 4 : 2;           // k-blocks per raw chunk
-    constexpr int RAW_BYTES = (WBITS == 4) ? 32 : 64;   // raw bytes per row and k-block
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* xs = base;                                        // [x stages][2][BX / 2 rows][128 B]
@@ -668,10 +667,12 @@ __global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
                 if (!ok)
                     break;
                 tcgen05_fence_after();
-                // A k-block at a time, in halves: raw bytes -> 32 fp16 (q - zp) * scale in k order (register i holds k = 2i in its low
-                // half and k = 2i + 1 in its high half).  (A loop: unrolled over the visit, a fifth of the issue slots went to
-                // instruction fetch; half a k-block per trip, and the quantisation parameters made anew in each, were a sixth of
-                // the conversion's instructions.)
+                // Half a k-block: raw bytes -> 32 fp16 (q - zp) * scale in k order (register i holds k = 2i in its low half and
+                // k = 2i + 1 in its high half).  (A loop: unrolled over the visit, a fifth of the issue slots went to instruction
+                // fetch.  uint4 takes a k-block per trip: half of one, and the quantisation parameters made anew in each, were a
+                // sixth of the conversion's instructions.  uint8 takes half of one: a whole one's
+                // bytes are eight registers too many, 172 instead of 128 bytes of spills a thread; 128 x 2048 x 8192 18.0 us for 17.7.)
+                constexpr int HALVES = WBITS == 4 ? 2 : 1; // of a k-block per trip
                 __half2 scale2, zc; // scale; uint4: (1024 + zp, 64 + zp), uint8: 1024 + zp in both halves
                 auto set_params = [&](int j) {
                     const uint32_t sraw = s_now[j], zraw = z_now[j];
@@ -684,17 +685,16 @@ __global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
                 };
                 set_params(0);
 #pragma unroll 1
-                for (int kbi = 0; kbi < nkb; kbi++)
+                for (int trip = 0; trip < nkb * (2 / HALVES); trip++)
                 {
-                    constexpr int NV = RAW_BYTES / 16;
-                    uint4 raw[NV];
+                    uint4 raw[2];
 #pragma unroll
-                    for (int v = 0; v < NV; v++)
-                        raw[v] = lds128(row + (uint32_t)((((in_chunk + kbi) * NV + v) ^ (r & 7)) * 16));
-                    if (!ONE_GROUP && kbi > 0)
+                    for (int v = 0; v < 2; v++)
+                        raw[v] = lds128(row + (uint32_t)((((in_chunk * (2 / HALVES) + trip) * 2 + v) ^ (r & 7)) * 16));
+                    if (!ONE_GROUP && trip == 2 / HALVES)
                         set_params(NP - 1);
 #pragma unroll
-                    for (int half = 0; half < 2; half++)
+                    for (int half = 0; half < HALVES; half++)
                     {
                         uint32_t a[16];
                         if (WBITS == 4)
@@ -717,8 +717,7 @@ __global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
 #pragma unroll
                             for (int v = 0; v < 2; v++)
                             {
-                                const uint4 q = raw[(2 * half + v) % NV];
-                                const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+                                const uint32_t w4[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
 #pragma unroll
                                 for (int wi = 0; wi < 4; wi++)
 #pragma unroll
@@ -730,7 +729,7 @@ __global__ void __launch_bounds__(Cfg<BX>::THREADS, 1)
                                     }
                             }
                         }
-                        tmem_st_32x16(col + (uint32_t)(kbi * kASlotCols + half * 16), a);
+                        tmem_st_32x16(col + (uint32_t)((trip * HALVES + half) * 16), a);
                     }
                 }
                 tcgen05_wait_st();
